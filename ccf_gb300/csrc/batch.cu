@@ -287,12 +287,16 @@ ccf_status Engine::prepare_batch(std::vector<Field*>& fields, int verbose)
 			CCF_TRY(f.leaf_mass_df.ensure((size_t)nl * MAX_NEAR), "cudaMalloc(leaves)");
 			CCF_TRY(f.leaf_loc_df.ensure((size_t)nl * 2 * (P + 1)), "cudaMalloc(leaves)");
 			CCF_TRY(f.leaf_ih_df.ensure(nl), "cudaMalloc(leaves)");
+			CCF_TRY(f.leaf_near_pk.ensure((size_t)nl * NEAR_PAIRS * NEAR_PAIR_F4), "cudaMalloc(leaves)");
+			CCF_TRY(f.leaf_loc_pk.ensure((size_t)nl * 2 * (P + 1)), "cudaMalloc(leaves)");
 			CCF_TRY(f.star_hilo.ensure(f.d.num_stars), "cudaMalloc(star hilo)");
 			CCF_TRY(f.star_mass_df.ensure(f.d.num_stars), "cudaMalloc(star hilo)");
 			g.leaf_near_df = f.leaf_near_df.ptr;
 			g.leaf_mass_df = f.leaf_mass_df.ptr;
 			g.leaf_loc_df = f.leaf_loc_df.ptr;
 			g.leaf_ih_df = f.leaf_ih_df.ptr;
+			g.leaf_near_pk = f.leaf_near_pk.ptr;
+			g.leaf_loc_pk = f.leaf_loc_pk.ptr;
 			g.star_hilo = f.star_hilo.ptr;
 			g.star_mass_df = f.star_mass_df.ptr;
 		}

@@ -198,4 +198,189 @@ CCF_D dfc dfc_fma(dfc a, dfc b, dfc c)
 }
 CCF_D float4 dfc_pack(dfc a) { return make_float4(a.re.hi, a.im.hi, a.re.lo, a.im.lo); }
 
+/* ---------------- two double-floats per instruction ----------------
+
+Two independent double-float chains side by side in the halves of 64-bit
+register pairs, on the packed FP32 instructions (add / mul / fma .f32x2).
+They run at the scalar ones' rate per operation, but one instruction carries
+two: the evaluators of the tracker are held by instruction issue and fetch
+(FMA pipe 41 %, issue 47 %, no_instruction the largest stall), not by the
+FMA pipe, and their chains of dependent operations halve.  Every half goes
+through the operations of the scalar primitive of the same name, rounded the
+same way; a - b is fma(b, -1, a), the same rounding as a subtraction. */
+typedef unsigned long long pk;   /* (low half, high half) */
+
+CCF_D pk pk_make(float a, float b)
+{
+	pk r;
+	asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+	return r;
+}
+CCF_D float pk_lo(pk v)
+{
+	float a, b;
+	asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+	return a;
+}
+CCF_D float pk_hi(pk v)
+{
+	float a, b;
+	asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+	return b;
+}
+CCF_D pk pk_add(pk a, pk b)
+{
+	pk r;
+	asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+	return r;
+}
+CCF_D pk pk_mul(pk a, pk b)
+{
+	pk r;
+	asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+	return r;
+}
+CCF_D pk pk_fma(pk a, pk b, pk c)
+{
+	pk r;
+	asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+	return r;
+}
+CCF_D pk pk_minus_one() { return 0xbf800000bf800000ull; }
+CCF_D pk pk_sub(pk a, pk b) { return pk_fma(b, pk_minus_one(), a); }
+CCF_D pk pk_neg(pk a) { return pk_mul(a, pk_minus_one()); }
+
+struct dfp   /* two double-floats */
+{
+	pk hi, lo;
+};
+
+CCF_D dfp dfp_make(dfl a, dfl b) { return {pk_make(a.hi, b.hi), pk_make(a.lo, b.lo)}; }
+CCF_D dfl dfp_first(dfp a) { return {pk_lo(a.hi), pk_lo(a.lo)}; }
+CCF_D dfl dfp_second(dfp a) { return {pk_hi(a.hi), pk_hi(a.lo)}; }
+CCF_D dfp dfp_neg(dfp a) { return {pk_neg(a.hi), pk_neg(a.lo)}; }
+
+CCF_D dfp two_sum(pk a, pk b)
+{
+	const pk s = pk_add(a, b);
+	const pk v = pk_sub(s, a);
+	return {s, pk_add(pk_sub(a, pk_sub(s, v)), pk_sub(b, v))};
+}
+/* a - b */
+CCF_D dfp two_diff(pk a, pk b)
+{
+	const pk s = pk_sub(a, b);
+	const pk v = pk_sub(s, a);
+	return {s, pk_sub(pk_sub(a, pk_sub(s, v)), pk_add(b, v))};
+}
+CCF_D dfp fast_two_sum(pk a, pk b)
+{
+	const pk s = pk_add(a, b);
+	return {s, pk_sub(b, pk_sub(s, a))};
+}
+/* na = -a */
+CCF_D dfp fast_two_sum_neg(pk a, pk na, pk b)
+{
+	const pk s = pk_add(a, b);
+	return {s, pk_sub(b, pk_add(s, na))};
+}
+CCF_D dfp dfp_sub(dfp a, dfp b)
+{
+	dfp s = two_diff(a.hi, b.hi);
+	const dfp t = two_diff(a.lo, b.lo);
+	s = fast_two_sum(s.hi, pk_add(s.lo, t.hi));
+	return fast_two_sum(s.hi, pk_add(s.lo, t.lo));
+}
+CCF_D dfp dfp_mul(dfp a, dfp b)
+{
+	const pk p = pk_mul(a.hi, b.hi), np = pk_neg(p);
+	pk lo = pk_fma(a.hi, b.hi, np);
+	lo = pk_fma(a.hi, b.lo, lo);
+	lo = pk_fma(a.lo, b.hi, lo);
+	return fast_two_sum_neg(p, np, lo);
+}
+CCF_D dfp dfp_sumsq(dfp x, dfp y)
+{
+	const pk p = pk_mul(x.hi, x.hi);
+	const pk pe = pk_fma(x.hi, x.hi, pk_neg(p));
+	const pk q = pk_mul(y.hi, y.hi);
+	const pk qe = pk_fma(y.hi, y.hi, pk_neg(q));
+	const dfp s = two_sum(p, q);
+	const pk lo = pk_add(pk_add(pe, qe), pk_fma(pk_add(x.hi, x.hi), x.lo, pk_fma(pk_add(y.hi, y.hi), y.lo, s.lo)));
+	return fast_two_sum(s.hi, lo);
+}
+CCF_D dfp dfp_rcp(dfp a)
+{
+	const pk q1 = pk_make(rcp32(pk_lo(a.hi)), rcp32(pk_hi(a.hi)));
+	const pk p = pk_mul(a.hi, q1), np = pk_neg(p);
+	const pk e = pk_fma(a.lo, q1, pk_fma(a.hi, q1, np));
+	const dfp t = fast_two_sum_neg(p, np, e);
+	const pk r = pk_sub(pk_sub(0x3f8000003f800000ull, t.hi), t.lo);
+	return fast_two_sum(q1, pk_mul(r, q1));
+}
+/* x^2 - y^2 (df_dot2) */
+CCF_D dfp dfp_diffsq(dfp x, dfp y)
+{
+	const pk p = pk_mul(x.hi, x.hi);
+	const pk pe = pk_fma(x.hi, x.hi, pk_neg(p));
+	const pk q = pk_mul(y.hi, y.hi);
+	const pk qe = pk_fma(y.hi, y.hi, pk_neg(q));
+	const dfp s = two_diff(p, q);
+	const pk e1 = pk_fma(x.lo, x.hi, pk_fma(x.hi, x.lo, pe));
+	const pk e2 = pk_fma(y.lo, y.hi, pk_fma(y.hi, y.lo, qe));
+	return fast_two_sum(s.hi, pk_add(pk_sub(e1, e2), s.lo));
+}
+/* a += x y: the running sums of dfacc_fma */
+CCF_D void dfp_acc_fma(dfp& a, dfp x, dfp y)
+{
+	const pk p = pk_mul(x.hi, y.hi);
+	const pk pe = pk_fma(x.hi, y.hi, pk_neg(p));
+	const dfp s = two_sum(a.hi, p);
+	a.hi = s.hi;
+	a.lo = pk_add(a.lo, pk_add(s.lo, pk_fma(x.hi, y.lo, pk_fma(x.lo, y.hi, pe))));
+}
+/* the sum of the two running sums of a dfp_acc_fma accumulator */
+CCF_D dfl dfp_acc_total(dfp a)
+{
+	const dfp t = fast_two_sum(a.hi, a.lo);
+	return df_add(dfp_first(t), dfp_second(t));
+}
+
+/* x y + u z + c with -y and -z at hand (df_dot2_add): the product errors
+   come out negated and save the negations of the products */
+CCF_D dfp dfp_dot2_add(dfp x, dfp y, dfp ny, dfp u, dfp z, dfp nz, dfp c)
+{
+	const pk p = pk_mul(x.hi, y.hi);
+	const pk q = pk_mul(u.hi, z.hi);
+	const dfp s = two_sum(p, q);
+	const dfp t = two_sum(s.hi, c.hi);
+	const pk e1 = pk_fma(x.lo, ny.hi, pk_fma(x.hi, ny.lo, pk_fma(x.hi, ny.hi, p)));
+	const pk e2 = pk_fma(u.lo, nz.hi, pk_fma(u.hi, nz.lo, pk_fma(u.hi, nz.hi, q)));
+	return fast_two_sum(t.hi, pk_sub(pk_add(pk_add(s.lo, t.lo), c.lo), pk_add(e1, e2)));
+}
+
+/* two complex double-floats */
+struct dfpc
+{
+	dfp re, im;
+};
+/* a multiplier of dfpc_fma with its negatives */
+struct dfpc_mult
+{
+	dfp re, im, nre, nim;
+};
+CCF_D dfpc_mult dfpc_mult_make(dfp re, dfp im) { return {re, im, dfp_neg(re), dfp_neg(im)}; }
+CCF_D dfpc dfpc_load(float4 hi, float4 lo)
+{
+	return {{pk_make(hi.x, hi.y), pk_make(lo.x, lo.y)}, {pk_make(hi.z, hi.w), pk_make(lo.z, lo.w)}};
+}
+CCF_D dfc dfpc_first(dfpc a) { return {dfp_first(a.re), dfp_first(a.im)}; }
+CCF_D dfc dfpc_second(dfpc a) { return {dfp_second(a.re), dfp_second(a.im)}; }
+/* a b + c (one Horner step of each half) */
+CCF_D dfpc dfpc_fma(dfpc a, const dfpc_mult& b, dfpc c)
+{
+	return {dfp_dot2_add(a.re, b.re, b.nre, a.im, b.nim, b.im, c.re),
+		dfp_dot2_add(a.re, b.im, b.nim, a.im, b.re, b.nre, c.im)};
+}
+
 } /* namespace ccf */

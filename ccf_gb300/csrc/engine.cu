@@ -578,8 +578,11 @@ ccf_status Engine::build_fmm(Field& f)
 		CCF_TRY(f.leaf_mass_df.ensure((size_t)nl * MAX_NEAR), "cudaMalloc(leaves)");
 		CCF_TRY(f.leaf_loc_df.ensure((size_t)nl * 2 * (P + 1)), "cudaMalloc(leaves)");
 		CCF_TRY(f.leaf_ih_df.ensure(nl), "cudaMalloc(leaves)");
+		CCF_TRY(f.leaf_near_pk.ensure((size_t)nl * NEAR_PAIRS * NEAR_PAIR_F4), "cudaMalloc(leaves)");
+		CCF_TRY(f.leaf_loc_pk.ensure((size_t)nl * 2 * (P + 1)), "cudaMalloc(leaves)");
 		launch_leaf_df(s, nl, P, f.leaf_center.ptr, f.leaf_inv_half.ptr, f.leaf_near_count.ptr, f.leaf_near.ptr,
-			f.leaf_loc.ptr, f.leaf_near_df.ptr, f.leaf_mass_df.ptr, f.leaf_loc_df.ptr, f.leaf_ih_df.ptr);
+			f.leaf_loc.ptr, f.leaf_near_df.ptr, f.leaf_mass_df.ptr, f.leaf_loc_df.ptr, f.leaf_ih_df.ptr,
+			f.leaf_near_pk.ptr, f.leaf_loc_pk.ptr);
 		CCF_TRY(cudaGetLastError(), "leaf_df_kernel");
 		/* split stars: poles of the Aberth sums and the off-field direct sums */
 		CCF_TRY(f.star_hilo.ensure(d.num_stars), "cudaMalloc(star hilo)");
@@ -660,6 +663,22 @@ ccf_status Engine::finish_view(Field& f, int P, double near_sum, int lerr, Uploa
 			}
 		}
 		inv_corner_df = split4(sp.inv_corner);
+		/* even and odd terms side by side (horner_halves_df) */
+		auto pairs = [](const std::vector<float4>& c) {
+			std::vector<float4> out;
+			for (size_t i = 0; i < c.size(); i += 2)
+			{
+				const float4 a = c[i], b = i + 1 < c.size() ? c[i + 1] : make_float4(0, 0, 0, 0);
+				out.push_back(make_float4(a.x, b.x, a.y, b.y));
+				out.push_back(make_float4(a.z, b.z, a.w, b.w));
+			}
+			return out;
+		};
+		const std::vector<float4> d1p = pairs(d1df), ap = pairs(adf);
+		CCF_TRY(f.sm_d1_pair.ensure(d1p.size()), "cudaMalloc(smooth)");
+		CCF_TRY(f.sm_a_pair.ensure(ap.size()), "cudaMalloc(smooth)");
+		CCF_TRY(put(f.sm_d1_pair.ptr, d1p.data(), d1p.size() * sizeof(float4)), "smooth");
+		CCF_TRY(put(f.sm_a_pair.ptr, ap.data(), ap.size() * sizeof(float4)), "smooth");
 		CCF_TRY(f.sm_d1_df.ensure(d1df.size()), "cudaMalloc(smooth)");
 		CCF_TRY(f.sm_a_df.ensure(adf.size()), "cudaMalloc(smooth)");
 		CCF_TRY(put(f.sm_d1_df.ptr, d1df.data(), d1df.size() * sizeof(float4)), "smooth");
@@ -709,7 +728,7 @@ ccf_status Engine::finish_view(Field& f, int P, double near_sum, int lerr, Uploa
 			CCF_TRY(f.leaf_loc_fold64.ensure((size_t)nl * 3 * (P + 1)), "cudaMalloc(fold)");
 			launch_fold_smooth(s, nl, P, f.leaf_center.ptr, f.leaf_inv_half.ptr, f.leaf_loc.ptr, f.fold_coef.ptr, 2 * M + 1,
 				f.fold_coef.ptr + 2 * M + 1, 2 * M, f.fold_coef.ptr + 4 * M + 1, na, 0.95 * std::hypot(d.corner_x1, d.corner_x2),
-				f.leaf_loc_df_fold.ptr, f.leaf_loc3f_fold.ptr, f.leaf_loc_fold64.ptr, f.leaf_fold.ptr);
+				f.leaf_loc_df_fold.ptr, f.leaf_loc_pk.ptr, f.leaf_loc3f_fold.ptr, f.leaf_loc_fold64.ptr, f.leaf_fold.ptr);
 			CCF_TRY(cudaGetLastError(), "fold_smooth_kernel");
 			fold_host.resize(nl);
 			CCF_TRY(cudaMemcpyAsync(fold_host.data(), f.leaf_fold.ptr, nl, cudaMemcpyDeviceToHost, s), "fold");
@@ -761,6 +780,8 @@ ccf_status Engine::finish_view(Field& f, int P, double near_sum, int lerr, Uploa
 	V.leaf_ih_df = f.leaf_ih_df.ptr;
 	V.smooth_d1_df = f.sm_d1_df.ptr;
 	V.smooth_a_df = f.sm_a_df.ptr;
+	V.smooth_d1_pair = f.sm_d1_pair.ptr;
+	V.smooth_a_pair = f.sm_a_pair.ptr;
 	V.inv_corner_df = inv_corner_df;
 	V.star_df = f.star_hilo.ptr;
 	V.star_mass_df = f.star_mass_df.ptr;
@@ -768,6 +789,8 @@ ccf_status Engine::finish_view(Field& f, int P, double near_sum, int lerr, Uploa
 	V.leaf_loc_df_fold = fold_ok ? f.leaf_loc_df_fold.ptr : nullptr;
 	V.leaf_loc3f_fold = fold_ok ? f.leaf_loc3f_fold.ptr : nullptr;
 	V.leaf_loc_fold64 = fold_ok ? f.leaf_loc_fold64.ptr : nullptr;
+	V.leaf_near_pk = f.leaf_near_pk.ptr;
+	V.leaf_loc_pk = f.leaf_loc_pk.ptr;
 	CCF_TRY(f.view_dev.ensure(1), "cudaMalloc(view)");
 	CCF_TRY(put(f.view_dev.ptr, &V, sizeof(V)), "view");
 	return CCF_OK;
@@ -1061,6 +1084,8 @@ ccf_status Engine::solve(std::vector<Field*>& fields, int verbose)
 		T.num_rows_dev = nullptr;
 		T.items_per_row = 0;
 		T.max_sub = TRACK_TSUB;
+		T.scales = 0;
+		for (Field* f : fields) T.scales |= f->params.write_mu_length_scales ? 1 : 0;
 		T.num_items = 0;
 		long long max_row_points = 0;   /* the column check's points of the longest row */
 		for (size_t r = 0; r < rc.size(); r++)

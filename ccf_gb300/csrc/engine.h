@@ -156,7 +156,7 @@ struct Field
 	DBuf<NearStar> leaf_near;
 	DBuf<double2> leaf_loc;
 	DBuf<float2> leaf_loc3f;
-	DBuf<float4> leaf_near_df, leaf_loc_df, leaf_loc_df_fold;
+	DBuf<float4> leaf_near_df, leaf_loc_df, leaf_loc_df_fold, leaf_near_pk, leaf_loc_pk;
 	DBuf<float2> leaf_mass_df, leaf_ih_df, leaf_loc3f_fold;
 	DBuf<double2> leaf_loc_fold64;
 	DBuf<unsigned char> leaf_fold;
@@ -166,7 +166,7 @@ struct Field
 	/* smooth-mass polynomials */
 	DBuf<double2> sm_d1, sm_d2, sm_a;
 	DBuf<float2> sm_d2f;
-	DBuf<float4> sm_d1_df, sm_a_df;
+	DBuf<float4> sm_d1_df, sm_a_df, sm_d1_pair, sm_a_pair;
 
 	/* device view */
 	FieldView view;

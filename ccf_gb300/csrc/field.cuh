@@ -30,6 +30,16 @@ struct NearStar
 	double x, y, m, pad;
 };
 
+/* Near stars of a leaf in pairs for the packed evaluators, NEAR_PAIR_F4
+   float4 per pair of stars (0, 1): (x0, x1, y0, y1) leading parts, the same
+   low parts, (m0, m1) leading and low; positions relative to the leaf centre.
+   An odd list ends with a star of mass 0 at NEAR_PAD (its terms vanish; the
+   distance keeps its 1/d, which the pole sum takes without the mass, below
+   1e-15). */
+constexpr int NEAR_PAIRS = MAX_NEAR / 2;
+constexpr int NEAR_PAIR_F4 = 3;
+constexpr float NEAR_PAD = 1e15f;
+
 struct FieldView
 {
 	/* lens parameters */
@@ -84,6 +94,8 @@ struct FieldView
 	const float2* leaf_ih_df;    /* [leaf] 1/h */
 	const float4* smooth_d1_df;  /* [smooth_m] */
 	const float4* smooth_a_df;   /* [taylor_smooth + 2] A_n c^n: the alpha polynomial in zbar / c */
+	const float4* smooth_d1_pair;   /* smooth_d1_df and smooth_a_df, the even and odd terms in pairs */
+	const float4* smooth_a_pair;    /* (horner_halves_df) */
 	float4 inv_corner_df;
 	const float4* star_df;       /* [num_stars] star positions, split (x_hi, y_hi, x_lo, y_lo) */
 	const float2* star_mass_df;  /* [num_stars] */
@@ -93,6 +105,11 @@ struct FieldView
 	const float4* leaf_loc_df_fold;   /* like leaf_loc_df */
 	const float2* leaf_loc3f_fold;    /* like leaf_loc3f */
 	const double2* leaf_loc_fold64;   /* like leaf_loc, in FP64 (the FP64 polish) */
+	/* the tracker's leaf records, two values side by side for the packed
+	   evaluator (eval_track_pk) */
+	const float4* leaf_near_pk;  /* [(leaf * NEAR_PAIRS + pair) * NEAR_PAIR_F4 + k], see near_pair */
+	const float4* leaf_loc_pk;   /* [(leaf * (P + 1) + i) * 2 + {0 leading, 1 low}]: alpha_i and
+	                                (d/dzbar)_(i+1), the folded blocks where the leaf is folded */
 };
 
 /* leaf containing z, or -1 when z lies outside the root box (the reference
@@ -102,6 +119,7 @@ struct FieldView
 CCF_D int find_leaf(const FieldView& F, double2 z)
 {
 	int n = 0;
+#pragma unroll 1
 	for (int depth = 0; depth < 64; depth++)
 	{
 		double2 c = F.node_center[n];
@@ -134,6 +152,58 @@ CCF_D double smooth_dz(const FieldView& F, double2 z)
 	return -F.kappa_star * heaviside(F.corner_abs - hypot(z.x, z.y));
 }
 
+/* The exact rectangular forms (approx = 0): four complex logarithms or
+   reciprocals.  Out of line, as all rarely taken FP64 code of the evaluators:
+   inlined at every call it made the tracker's loop 0.9 MB of instructions,
+   and instruction fetch its largest stall.  The polish, a small kernel whose
+   FP64 chains are its time, defines CCF_COLD to inline them (0.35 ms on the
+   bench field against 0.43 with the calls). */
+#ifndef CCF_COLD
+#define CCF_COLD static __device__ __noinline__
+#endif
+CCF_COLD double2 smooth_dzbar_exact_rect(const FieldView& F, double2 zb)
+{
+	const double k = F.kappa_star;
+	const double2 z = cconj(zb);
+	double2 c = F.corner;
+	double2 l1 = clog64(csub(cconj(c), zb));
+	double2 l2 = clog64(csub(c, zb));
+	double2 l3 = clog64(csub(make_double2(-c.x, -c.y), zb));
+	double2 l4 = clog64(csub(make_double2(-c.x, c.y), zb));
+	double2 s = cadd(csub(csub(l1, l2), l3), l4);
+	double2 d = cmul(s, make_double2(0, -k / PI));
+	d.x -= k * boxcar(z, c);
+	return d;
+}
+
+CCF_COLD double2 smooth_d2zbar_exact_rect(const FieldView& F, double2 zb)
+{
+	const double k = F.kappa_star;
+	double2 c = F.corner;
+	double2 i1 = cinv(csub(cconj(c), zb));
+	double2 i2 = cinv(csub(c, zb));
+	double2 i3 = cinv(csub(make_double2(-c.x, -c.y), zb));
+	double2 i4 = cinv(csub(make_double2(-c.x, c.y), zb));
+	double2 s = csub(cadd(cadd(make_double2(-i1.x, -i1.y), i2), i3), i4);
+	return cmul(s, make_double2(0, -k / PI));
+}
+
+CCF_COLD double2 smooth_alpha_exact_rect(const FieldView& F, double2 z)
+{
+	const double k = F.kappa_star;
+	const double2 zb = cconj(z);
+	double2 c = F.corner;
+	double2 c1 = csub(c, zb);
+	double2 c2 = csub(cconj(c), zb);
+	double2 c3 = csub(make_double2(-c.x, -c.y), zb);
+	double2 c4 = csub(make_double2(-c.x, c.y), zb);
+	double2 s = csub(cadd(csub(cmul(c1, clog64(c1)), cmul(c2, clog64(c2))), cmul(c3, clog64(c3))), cmul(c4, clog64(c4)));
+	double2 a = cmul(s, make_double2(0, -k / PI));
+	a.x -= k * 2 * (c.x + z.x) * boxcar(z, c);
+	a.x -= k * 4 * c.x * heaviside(c.y + z.y) * heaviside(c.y - z.y) * heaviside(z.x - c.x);
+	return a;
+}
+
 /* d alpha_smooth / d zbar (alpha_smooth.cuh:186-236) */
 CCF_D double2 smooth_dzbar(const FieldView& F, double2 z)
 {
@@ -152,15 +222,7 @@ CCF_D double2 smooth_dzbar(const FieldView& F, double2 z)
 			acc.x += F.smooth_k1;
 			return acc;
 		}
-		double2 c = F.corner;
-		double2 l1 = clog64(csub(cconj(c), zb));
-		double2 l2 = clog64(csub(c, zb));
-		double2 l3 = clog64(csub(make_double2(-c.x, -c.y), zb));
-		double2 l4 = clog64(csub(make_double2(-c.x, c.y), zb));
-		double2 s = cadd(csub(csub(l1, l2), l3), l4);
-		double2 d = cmul(s, make_double2(0, -k / PI));
-		d.x -= k * boxcar(z, c);
-		return d;
+		return smooth_dzbar_exact_rect(F, zb);
 	}
 	if (F.approx) return make_double2(0, 0);
 	/* the reference applies the exterior form everywhere for the exact disc */
@@ -184,13 +246,7 @@ CCF_D double2 smooth_d2zbar(const FieldView& F, double2 z)
 			for (int m = F.smooth_m - 2; m >= 0; m--) acc = cadd(cmul(acc, u), F.smooth_d2[m]);
 			return cmul(acc, cmul(zb, F.inv_corner2));
 		}
-		double2 c = F.corner;
-		double2 i1 = cinv(csub(cconj(c), zb));
-		double2 i2 = cinv(csub(c, zb));
-		double2 i3 = cinv(csub(make_double2(-c.x, -c.y), zb));
-		double2 i4 = cinv(csub(make_double2(-c.x, c.y), zb));
-		double2 s = csub(cadd(cadd(make_double2(-i1.x, -i1.y), i2), i3), i4);
-		return cmul(s, make_double2(0, -k / PI));
+		return smooth_d2zbar_exact_rect(F, zb);
 	}
 	if (F.approx) return make_double2(0, 0);
 	double2 z3 = cmul(cmul(zb, zb), zb);
@@ -213,16 +269,7 @@ CCF_D double2 smooth_alpha(const FieldView& F, double2 z)
 			a.x -= k * 2 * (F.corner.x + z.x);
 			return a;
 		}
-		double2 c = F.corner;
-		double2 c1 = csub(c, zb);
-		double2 c2 = csub(cconj(c), zb);
-		double2 c3 = csub(make_double2(-c.x, -c.y), zb);
-		double2 c4 = csub(make_double2(-c.x, c.y), zb);
-		double2 s = csub(cadd(csub(cmul(c1, clog64(c1)), cmul(c2, clog64(c2))), cmul(c3, clog64(c3))), cmul(c4, clog64(c4)));
-		double2 a = cmul(s, make_double2(0, -k / PI));
-		a.x -= k * 2 * (c.x + z.x) * boxcar(z, c);
-		a.x -= k * 4 * c.x * heaviside(c.y + z.y) * heaviside(c.y - z.y) * heaviside(z.x - c.x);
-		return a;
+		return smooth_alpha_exact_rect(F, z);
 	}
 	if (F.approx || hypot(z.x, z.y) <= F.corner_abs) return make_double2(-k * z.x, -k * z.y);
 	return cscale(cinv(zb), -k * F.corner_abs * F.corner_abs);

@@ -40,6 +40,7 @@ CCF_D SumsDF leaf_sums_df(const FieldView& F, int leaf, double2 z)
 	const int n = F.leaf_near_count[leaf];
 	const float4* P = F.leaf_near_df + (size_t)leaf * MAX_NEAR;
 	const float2* M = F.leaf_mass_df + (size_t)leaf * MAX_NEAR;
+#pragma unroll 1
 	for (int i = 0; i < n; i++)
 	{
 		const dfc s = dfc_load(P[i]);
@@ -114,6 +115,7 @@ CCF_D dfc horner_df(const float4* L, int P, int first, dfc dz)
 	   latency overlaps the previous step's arithmetic */
 	dfc acc = dfc_load(L[P]);
 	float4 nxt = L[P - 1];
+#pragma unroll 1
 	for (int i = P - 1; i >= first; i--)
 	{
 		const float4 cur = nxt;
@@ -140,6 +142,7 @@ CCF_D double2 smooth_dzbar_df(const FieldView& F, double2 z)
 	const dfc r = dfc_mul(zb, dfc_load(F.inv_corner_df));
 	const dfc u = dfc_mul(r, r);
 	dfc acc = dfc_load(F.smooth_d1_df[F.smooth_m - 1]);
+#pragma unroll 1
 	for (int m = F.smooth_m - 2; m >= 0; m--) acc = dfc_fma(acc, u, dfc_load(F.smooth_d1_df[m]));
 	acc = dfc_mul(acc, u);
 	double2 d = dfc_to(acc);
@@ -156,6 +159,7 @@ CCF_D double2 smooth_alpha_df(const FieldView& F, double2 z)
 	const dfc w = dfc_mul(dfc_from(make_double2(z.x, -z.y)), dfc_load(F.inv_corner_df));
 	const int n = F.taylor_smooth + 1;
 	dfc acc = dfc_load(F.smooth_a_df[n]);
+#pragma unroll 1
 	for (int i = n - 1; i >= 0; i--) acc = dfc_fma(acc, w, dfc_load(F.smooth_a_df[i]));
 	double2 a = cmul(dfc_to(acc), make_double2(0, -k / PI));
 	a.x -= k * 2 * (F.corner.x + z.x);
@@ -214,7 +218,8 @@ struct TrackConst
 	float r2;
 	float aabs;            /* |a|, rounded up */
 	double w1x, w1y, wc1;  /* the lens map's linear terms with the Taylor or folded smooth-mass
-	                          forms: w = (w1x x + wc1, w1y y) + the star and series terms */
+	                          forms, or the disc's approximate one: w = (w1x x + wc1, w1y y) +
+	                          the star and series terms */
 };
 
 CCF_D TrackConst track_const(const FieldView& F)
@@ -229,10 +234,171 @@ CCF_D TrackConst track_const(const FieldView& F)
 	k.ic2 = make_float2((float)F.inv_corner2.x, (float)F.inv_corner2.y);
 	k.r2 = (float)(SMOOTH_DF_RANGE * F.corner_abs * F.corner_abs);
 	k.aabs = __fadd_ru(fabsf(k.a.hi), fabsf(k.a.lo));
-	k.w1x = 1 - F.kappa_tot + F.shear + 2 * F.kappa_star;
-	k.w1y = 1 - F.kappa_tot - F.shear;
-	k.wc1 = 2 * F.kappa_star * F.corner.x;
+	const bool disc = !F.rectangular && F.approx;   /* alpha_s = -kappa_star z */
+	k.w1x = 1 - F.kappa_tot + F.shear + (disc ? 1 : 2) * F.kappa_star;
+	k.w1y = 1 - F.kappa_tot - F.shear + (disc ? F.kappa_star : 0);
+	k.wc1 = disc ? 0 : 2 * F.kappa_star * F.corner.x;
 	return k;
+}
+
+/* a pair of near stars (NEAR_PAIRS) */
+struct NearPair
+{
+	dfp x, y, m;
+};
+CCF_D NearPair near_pair(float4 hi, float4 lo, float4 m)
+{
+	return {{pk_make(hi.x, hi.y), pk_make(lo.x, lo.y)}, {pk_make(hi.z, hi.w), pk_make(lo.z, lo.w)},
+		{pk_make(m.x, m.y), pk_make(m.z, m.w)}};
+}
+
+/* A leaf's local expansion at dz: alpha, sum_{i >= 1} L0[i] dz^(i - 1), and
+   d alpha / d zbar, sum_{i >= 2} L1[i] dz^(i - 2), in double-float side by
+   side -- entry i of the block holds L0[i] and L1[i + 1] as (re0, re1, im0,
+   im1) leading and low parts (leaf_df_leaf, fold_smooth_kernel), so both end
+   after entry 1 -- and d2 alpha / d zbar2, sum_{i >= 3} L3[i] dz^(i - 3), in
+   FP32 in the same loop. */
+struct LeafPoly
+{
+	dfc al, dl;
+	float2 d2l;
+};
+
+CCF_D LeafPoly leaf_poly_pk(const float4* L, const float2* L3, int P, dfc dz)
+{
+	const dfpc_mult b = dfpc_mult_make(dfp_make(dz.re, dz.re), dfp_make(dz.im, dz.im));
+	const float2 dzf = make_float2(dz.re.hi, dz.im.hi);
+	/* each entry is loaded one step ahead of its use, so the load's latency
+	   overlaps the previous step's arithmetic */
+	dfpc acc = dfpc_load(L[2 * P], L[2 * P + 1]);
+	float2 a3 = make_float2(0.f, 0.f), n3 = a3;
+	float4 nh = L[2 * P - 2], nl = L[2 * P - 1];
+#pragma unroll 1
+	for (int i = P - 1; i >= 1; i--)
+	{
+		const dfpc c = dfpc_load(nh, nl);
+		const float2 c3 = n3;
+		nh = L[2 * i - 2];
+		nl = L[2 * i - 1];
+		n3 = L3[i + 1];
+		acc = dfpc_fma(acc, b, c);
+		a3 = fadd(fmulc(a3, dzf), c3);
+	}
+	return {dfpc_first(acc), dfpc_second(acc), a3};
+}
+
+/* sum_i c_i x^i, i < 2 n, from x and v = x^2: entry k of the pair array holds
+   c_2k and c_(2k + 1) as in leaf_poly_pk, and the two polynomials in v run
+   side by side */
+CCF_D dfc horner_halves_df(const float4* C, int n, dfc v, dfc x)
+{
+	const dfpc_mult b = dfpc_mult_make(dfp_make(v.re, v.re), dfp_make(v.im, v.im));
+	dfpc acc = dfpc_load(C[2 * n - 2], C[2 * n - 1]);
+#pragma unroll 1
+	for (int k = n - 2; k >= 0; k--) acc = dfpc_fma(acc, b, dfpc_load(C[2 * k], C[2 * k + 1]));
+	return dfc_fma(dfpc_second(acc), x, dfpc_first(acc));
+}
+
+/* the near stars' part of an evaluation: sums of m / d, m / d^2 (double-float),
+   m / d^3, 1 / d (FP32) and |m / d^2| */
+struct TrackSums
+{
+	dfc s1, s2;
+	float2 s3, pole;
+	float tabs;
+};
+
+CCF_D TrackSums track_sums(const FieldView& F, int leaf, const dfc& zr)
+{
+	dfacc s1r = {0.f, 0.f}, s1i = s1r, s2r = s1r, s2i = s1r;
+	float2 s3 = make_float2(0.f, 0.f), pole = make_float2(0.f, 0.f);
+	float tabs = 0.f;   /* sum of |m / d^2| */
+	const int n = F.leaf_near_count[leaf];
+	const float4* Pn = F.leaf_near_df + (size_t)leaf * MAX_NEAR;
+	const float2* Mn = F.leaf_mass_df + (size_t)leaf * MAX_NEAR;
+	/* the next star is loaded while this one's terms are formed */
+	float4 pn = Pn[0];
+	float2 mn = Mn[0];
+#pragma unroll 1
+	for (int i = 0; i < n; i++)
+	{
+		const dfc s = dfc_load(pn);
+		const float2 mm = mn;
+		pn = Pn[min(i + 1, MAX_NEAR - 1)];
+		mn = Mn[min(i + 1, MAX_NEAR - 1)];
+		const dfl m = {mm.x, mm.y};
+		const dfl dx = df_sub(zr.re, s.re);
+		const dfl dy = df_sub(zr.im, s.im);
+		const dfl r = df_rcp(df_sumsq(dx, dy));
+		const dfl ix = df_mul(dx, r);
+		const dfl iy = df_neg(df_mul(dy, r));                     /* 1/d */
+		/* ix^2 - iy^2 to 2^-47 of 1/|d|^2, the size of the term */
+		const dfl i2x = df_dot2(ix, ix, df_neg(iy), iy);
+		dfl i2y = df_mul(ix, iy);
+		i2y = {2.f * i2y.hi, 2.f * i2y.lo};                        /* 1/d^2 */
+		dfacc_fma(s2r, m, i2x);
+		dfacc_fma(s2i, m, i2y);
+		dfacc_fma(s1r, m, ix);
+		dfacc_fma(s1i, m, iy);
+		pole.x += ix.hi;
+		pole.y += iy.hi;
+		const float i3x = i2x.hi * ix.hi - i2y.hi * iy.hi;
+		const float i3y = i2x.hi * iy.hi + i2y.hi * ix.hi;        /* 1/d^3 */
+		s3.x = fmaf(m.hi, i3x, s3.x);
+		s3.y = fmaf(m.hi, i3y, s3.y);
+		tabs = fmaf(m.hi, fmaf(ix.hi, ix.hi, iy.hi * iy.hi), tabs);
+	}
+	const dfc s1 = {dfacc_get(s1r), dfacc_get(s1i)}, s2 = {dfacc_get(s2r), dfacc_get(s2i)};
+	return {s1, s2, s3, pole, tabs};
+}
+
+/* the same, two stars at a time (NEAR_PAIRS), with 1/d = (jx, -jy): the sums
+   run over m jx, m jy, m (jx^2 - jy^2) and m jx jy, their signs and the factor
+   2 of 2 jx jy put in at the end (exact) */
+CCF_D TrackSums track_sums_pk(const FieldView& F, int leaf, const dfc& zr)
+{
+	const dfp zxp = dfp_make(zr.re, zr.re), zyp = dfp_make(zr.im, zr.im);
+	dfp s1x = {0, 0}, s1y = s1x, s2x = s1x, s2y = s1x;
+	pk s3x = 0, s3y = 0, polex = 0, poley = 0;
+	pk tab = 0;   /* sum of |m / d^2| */
+	const int np = (F.leaf_near_count[leaf] + 1) >> 1;
+	const float4* Pn = F.leaf_near_pk + (size_t)leaf * NEAR_PAIRS * NEAR_PAIR_F4;
+	/* the next pair is loaded while this one's terms are formed */
+	float4 nh = Pn[0], nl = Pn[1], nm = Pn[2];
+#pragma unroll 1
+	for (int i = 0; i < np; i++)
+	{
+		const NearPair s = near_pair(nh, nl, nm);
+		const int k = 3 * min(i + 1, NEAR_PAIRS - 1);
+		nh = Pn[k];
+		nl = Pn[k + 1];
+		nm = Pn[k + 2];
+		const dfp dx = dfp_sub(zxp, s.x), dy = dfp_sub(zyp, s.y);
+		const dfp r = dfp_rcp(dfp_sumsq(dx, dy));
+		const dfp jx = dfp_mul(dx, r), jy = dfp_mul(dy, r);
+		/* 1/d^2 = (kx, -2 ky); kx to 2^-47 of 1/|d|^2, the size of the term */
+		const dfp kx = dfp_diffsq(jx, jy), ky = dfp_mul(jx, jy);
+		dfp_acc_fma(s2x, s.m, kx);
+		dfp_acc_fma(s2y, s.m, ky);
+		dfp_acc_fma(s1x, s.m, jx);
+		dfp_acc_fma(s1y, s.m, jy);
+		polex = pk_add(polex, jx.hi);
+		poley = pk_add(poley, jy.hi);
+		/* 1/d^3 = (kx jx - 2 ky jy, -(kx jy + 2 ky jx)) */
+		const pk t = pk_add(ky.hi, ky.hi);
+		const pk i3x = pk_fma(pk_neg(t), jy.hi, pk_mul(kx.hi, jx.hi));
+		const pk i3y = pk_fma(t, jx.hi, pk_mul(kx.hi, jy.hi));
+		s3x = pk_fma(s.m.hi, i3x, s3x);
+		s3y = pk_fma(s.m.hi, i3y, s3y);
+		tab = pk_fma(s.m.hi, pk_fma(jx.hi, jx.hi, pk_mul(jy.hi, jy.hi)), tab);
+	}
+	const dfl s2h = dfp_acc_total(s2y);
+	const dfc s1 = {dfp_acc_total(s1x), df_neg(dfp_acc_total(s1y))};
+	const dfc s2 = {dfp_acc_total(s2x), {-2.f * s2h.hi, -2.f * s2h.lo}};
+	const float2 s3 = make_float2(pk_lo(s3x) + pk_hi(s3x), -(pk_lo(s3y) + pk_hi(s3y)));
+	float2 pole = make_float2(pk_lo(polex) + pk_hi(polex), -(pk_lo(poley) + pk_hi(poley)));
+	const float tabs = pk_lo(tab) + pk_hi(tab);
+	return {s1, s2, s3, pole, tabs};
 }
 
 /* Everything one corrector iteration of the continuation tracker needs at a
@@ -247,7 +413,8 @@ CCF_D TrackConst track_const(const FieldView& F)
      wpart  the star, local and smooth-Taylor part of the lens map w
             (as eval_point_df): w = ((1 - kappa + gamma) x, (1 - kappa - gamma) y)
             + wpart, plus 2 kappa_star (corner.x + x) when wmode is 1 (the
-            Taylor form was evaluated here), minus smooth_alpha(z) when wmode
+            Taylor form was evaluated here, or its counterpart of the disc;
+            TrackConst::w1x, w1y, wc1), minus smooth_alpha(z) when wmode
             is 0; when wmode is 2, wpart is the whole of w.
 
    The FP32 terms are the high words of the double-float 1/d and 1/d^2 the
@@ -278,67 +445,59 @@ CCF_D float2 fdiv_scaled(float2 a, float2 b)
 	return make_float2((ax * bx + ay * by) * r, (ay * bx - ax * by) * r);
 }
 
+/* the smooth mass's part of an evaluation where its FP64 forms are taken: the
+   exact forms, and the Taylor form outside the corner circle (out of line) */
+struct SmoothFar
+{
+	dfc ds;
+	float2 d2s;
+};
+static __device__ __noinline__ SmoothFar smooth_far(const FieldView& F, double2 z)
+{
+	const double2 t = smooth_d2zbar(F, z);
+	return {dfc_from(smooth_dzbar(F, z)), make_float2((float)t.x, (float)t.y)};
+}
+
+template <bool PK>
 CCF_D TrackEval eval_track_df(const FieldView& F, const TrackConst& K, int leaf, double2 z, double2 rel, dfl cph, dfl sph,
 	bool disc_exact)
 {
 	const dfc zr = dfc_from(rel);
-	dfacc s1r = {0.f, 0.f}, s1i = s1r, s2r = s1r, s2i = s1r;
-	float2 s3 = make_float2(0.f, 0.f), pole = make_float2(0.f, 0.f);
-	float tabs = 0.f;   /* sum of |m / d^2| */
-	const int n = F.leaf_near_count[leaf];
-	const float4* Pn = F.leaf_near_df + (size_t)leaf * MAX_NEAR;
-	const float2* Mn = F.leaf_mass_df + (size_t)leaf * MAX_NEAR;
-	/* the next star is loaded while this one's terms are formed */
-	float4 pn = Pn[0];
-	float2 mn = Mn[0];
-	for (int i = 0; i < n; i++)
-	{
-		const dfc s = dfc_load(pn);
-		const float2 mm = mn;
-		pn = Pn[min(i + 1, MAX_NEAR - 1)];
-		mn = Mn[min(i + 1, MAX_NEAR - 1)];
-		const dfl m = {mm.x, mm.y};
-		const dfl dx = df_sub(zr.re, s.re);
-		const dfl dy = df_sub(zr.im, s.im);
-		const dfl r = df_rcp(df_sumsq(dx, dy));
-		const dfl ix = df_mul(dx, r);
-		const dfl iy = df_neg(df_mul(dy, r));                     /* 1/d */
-		/* ix^2 - iy^2 to 2^-47 of 1/|d|^2, the size of the term */
-		const dfl i2x = df_dot2(ix, ix, df_neg(iy), iy);
-		dfl i2y = df_mul(ix, iy);
-		i2y = {2.f * i2y.hi, 2.f * i2y.lo};                        /* 1/d^2 */
-		dfacc_fma(s2r, m, i2x);
-		dfacc_fma(s2i, m, i2y);
-		dfacc_fma(s1r, m, ix);
-		dfacc_fma(s1i, m, iy);
-		pole.x += ix.hi;
-		pole.y += iy.hi;
-		const float i3x = i2x.hi * ix.hi - i2y.hi * iy.hi;
-		const float i3y = i2x.hi * iy.hi + i2y.hi * ix.hi;        /* 1/d^3 */
-		s3.x = fmaf(m.hi, i3x, s3.x);
-		s3.y = fmaf(m.hi, i3y, s3.y);
-		tabs = fmaf(m.hi, fmaf(ix.hi, ix.hi, iy.hi * iy.hi), tabs);
-	}
-	const dfc s1 = {dfacc_get(s1r), dfacc_get(s1i)}, s2 = {dfacc_get(s2r), dfacc_get(s2i)};
+	const TrackSums S = PK ? track_sums_pk(F, leaf, zr) : track_sums(F, leaf, zr);
+	const dfc s1 = S.s1, s2 = S.s2;
+	const float2 s3 = S.s3;
+	float2 pole = S.pole;
+	const float tabs = S.tabs;
 	const int P = F.order;
 	const float2 ihf = F.leaf_ih_df[leaf];
 	const dfl ih = {ihf.x, ihf.y};
 	const dfc dz = {df_mul(zr.re, ih), df_mul(zr.im, ih)};
 	/* a leaf with the smooth-mass series folded into its expansion skips the series */
 	const bool folded = F.leaf_fold != nullptr && F.leaf_fold[leaf];
-	const float4* L = (folded ? F.leaf_loc_df_fold : F.leaf_loc_df) + (size_t)leaf * 2 * (P + 1);
-	const dfc al = horner_df(L, P, 1, dz);
-	const dfc dl = horner_df(L + (P + 1), P, 2, dz);
-	const float2 dzf = make_float2(dz.re.hi, dz.im.hi);
 	const float2* L3 = (folded ? F.leaf_loc3f_fold : F.leaf_loc3f) + (size_t)leaf * (P + 1);
-	float2 d2l = L3[P], l3n = L3[P - 1];
-	for (int i = P - 1; i >= 3; i--)
+	LeafPoly lp;
+	if constexpr (PK)
 	{
-		const float2 c = l3n;
-		l3n = L3[i - 1];
-		d2l = fadd(fmulc(d2l, dzf), c);
+		lp = leaf_poly_pk(F.leaf_loc_pk + (size_t)leaf * 2 * (P + 1), L3, P, dz);
 	}
-
+	else
+	{
+		const float4* L = (folded ? F.leaf_loc_df_fold : F.leaf_loc_df) + (size_t)leaf * 2 * (P + 1);
+		lp.al = horner_df(L, P, 1, dz);
+		lp.dl = horner_df(L + (P + 1), P, 2, dz);
+		const float2 dzf = make_float2(dz.re.hi, dz.im.hi);
+		float2 d2l = L3[P], l3n = L3[P - 1];
+#pragma unroll 1
+		for (int i = P - 1; i >= 3; i--)
+		{
+			const float2 c = l3n;
+			l3n = L3[i - 1];
+			d2l = fadd(fmulc(d2l, dzf), c);
+		}
+		lp.d2l = d2l;
+	}
+	const dfc al = lp.al, dl = lp.dl;
+	const float2 d2l = lp.d2l;
 	/* smooth mass: d alpha / d zbar (double-float), d2 alpha / d zbar2 (FP32)
 	   and the Taylor part of alpha (double-float) */
 	TrackEval e;
@@ -346,8 +505,15 @@ CCF_D TrackEval eval_track_df(const FieldView& F, const TrackConst& K, int leaf,
 	float2 d2s;
 	const float zx = (float)z.x, zy = (float)z.y;
 	const bool taylor = F.rectangular && F.approx && F.smooth_m > 0 && zx * zx + zy * zy < K.r2;
-	e.wmode = (taylor || folded) ? 1 : 0;
-	if (folded)
+	/* the disc's approximate form has no anti-analytic part */
+	const bool disc = !F.rectangular && F.approx;
+	e.wmode = (taylor || folded || disc) ? 1 : 0;
+	if (disc)
+	{
+		ds = {{0.f, 0.f}, {0.f, 0.f}};
+		d2s = make_float2(0.f, 0.f);
+	}
+	else if (folded)
 	{
 		/* the series are in the leaf's blocks: only d alpha_s / d zbar's constant */
 		ds = {K.k1, {0.f, 0.f}};
@@ -358,13 +524,26 @@ CCF_D TrackEval eval_track_df(const FieldView& F, const TrackConst& K, int leaf,
 		const dfc zb = dfc_from(make_double2(z.x, -z.y));
 		const dfc wc = dfc_mul(zb, dfc_load(F.inv_corner_df));   /* zbar / c */
 		const dfc u = dfc_mul(wc, wc);
-		dfc acc = dfc_load(F.smooth_d1_df[F.smooth_m - 1]);
-		for (int m = F.smooth_m - 2; m >= 0; m--) acc = dfc_fma(acc, u, dfc_load(F.smooth_d1_df[m]));
+		dfc acc, aa;
+		if constexpr (PK)
+		{
+			/* each series as its even and odd terms side by side: d1 in u^2,
+			   alpha in u = wc^2 */
+			acc = horner_halves_df(F.smooth_d1_pair, (F.smooth_m + 1) / 2, dfc_mul(u, u), u);
+			aa = horner_halves_df(F.smooth_a_pair, (F.taylor_smooth + 3) / 2, u, wc);
+		}
+		else
+		{
+			acc = dfc_load(F.smooth_d1_df[F.smooth_m - 1]);
+#pragma unroll 1
+			for (int m = F.smooth_m - 2; m >= 0; m--) acc = dfc_fma(acc, u, dfc_load(F.smooth_d1_df[m]));
+			const int na = F.taylor_smooth + 1;
+			aa = dfc_load(F.smooth_a_df[na]);
+#pragma unroll 1
+			for (int i = na - 1; i >= 0; i--) aa = dfc_fma(aa, wc, dfc_load(F.smooth_a_df[i]));
+		}
 		ds = dfc_mul(acc, u);
 		ds.re = df_add(ds.re, K.k1);
-		const int na = F.taylor_smooth + 1;
-		dfc aa = dfc_load(F.smooth_a_df[na]);
-		for (int i = na - 1; i >= 0; i--) aa = dfc_fma(aa, wc, dfc_load(F.smooth_a_df[i]));
 		/* (0, -k / pi) A: re = (k / pi) A.im, im = -(k / pi) A.re */
 		sa.re = df_mul(K.kpi, aa.im);
 		sa.im = df_neg(df_mul(K.kpi, aa.re));
@@ -372,14 +551,15 @@ CCF_D TrackEval eval_track_df(const FieldView& F, const TrackConst& K, int leaf,
 		const float2 r = fmulc(zbf, K.ic);
 		const float2 uf = fmulc(r, r);
 		float2 a2 = F.smooth_d2f[F.smooth_m - 1];
+#pragma unroll 1
 		for (int m = F.smooth_m - 2; m >= 0; m--) a2 = fadd(fmulc(a2, uf), F.smooth_d2f[m]);
 		d2s = fmulc(a2, fmulc(zbf, K.ic2));
 	}
 	else
 	{
-		ds = dfc_from(smooth_dzbar(F, z));
-		const double2 t = smooth_d2zbar(F, z);
-		d2s = make_float2((float)t.x, (float)t.y);
+		const SmoothFar t = smooth_far(F, z);
+		ds = t.ds;
+		d2s = t.d2s;
 	}
 	const dfl a = F.approx ? K.a : df_from_double(1 - F.kappa_tot - smooth_dz(F, z));
 

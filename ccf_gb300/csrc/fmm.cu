@@ -383,27 +383,54 @@ void launch_leaf_build(cudaStream_t s, const TreeDev& T, int num_nodes, const in
 namespace ccf
 {
 
+/* entry i, half k (0: alpha_i, 1: (d/dzbar)_(i+1)) of a leaf's paired
+   expansion block (FieldView::leaf_loc_pk); f: the block's floats */
+CCF_D void store_loc_pk(float* f, int i, int k, float2 re, float2 im)
+{
+	f += 8 * i + k;
+	f[0] = re.x;
+	f[2] = im.x;
+	f[4] = re.y;
+	f[6] = im.y;
+}
+
 /* double-float copies of the leaf records for the mixed-precision evaluators:
    near stars relative to the leaf centre (formed in FP64, then split),
-   masses, the alpha and d/dzbar coefficient blocks, and 1/h.  One warp per
-   leaf. */
+   masses, the alpha and d/dzbar coefficient blocks, and 1/h; and the packed
+   forms of the near stars (an odd list padded with a star of mass 0 at
+   NEAR_PAD) and of the blocks.  One warp per leaf. */
 CCF_D void leaf_df_leaf(int l, int i, int P, const double2* __restrict__ leaf_center,
 	const double* __restrict__ leaf_inv_half, const int* __restrict__ near_count, const NearStar* __restrict__ near,
 	const double2* __restrict__ loc, float4* __restrict__ near_df, float2* __restrict__ mass_df, float4* __restrict__ loc_df,
-	float2* __restrict__ ih_df)
+	float2* __restrict__ ih_df, float4* __restrict__ near_pk, float4* __restrict__ loc_pk)
 {
 	const double2 c = leaf_center[l];
 	auto split = [](double x) {
 		float h = __double2float_rn(x);
 		return make_float2(h, __double2float_rn(x - (double)h));
 	};
-	if (i < near_count[l])
+	const int n = near_count[l];
+	if (i < ((n + 1) & ~1))
 	{
-		NearStar s = near[(size_t)l * MAX_NEAR + i];
-		float2 x = split(s.x - c.x), y = split(s.y - c.y);
-		near_df[(size_t)l * MAX_NEAR + i] = make_float4(x.x, y.x, x.y, y.y);
-		mass_df[(size_t)l * MAX_NEAR + i] = split(s.m);
+		float2 x = make_float2(NEAR_PAD, 0.f), y = x, m = make_float2(0.f, 0.f);
+		if (i < n)
+		{
+			NearStar s = near[(size_t)l * MAX_NEAR + i];
+			x = split(s.x - c.x);
+			y = split(s.y - c.y);
+			m = split(s.m);
+			near_df[(size_t)l * MAX_NEAR + i] = make_float4(x.x, y.x, x.y, y.y);
+			mass_df[(size_t)l * MAX_NEAR + i] = m;
+		}
+		float* f = reinterpret_cast<float*>(near_pk + ((size_t)l * NEAR_PAIRS + (i >> 1)) * NEAR_PAIR_F4) + (i & 1);
+		f[0] = x.x;
+		f[2] = y.x;
+		f[4] = x.y;
+		f[6] = y.y;
+		f[8] = m.x;
+		f[10] = m.y;
 	}
+	float* pk = reinterpret_cast<float*>(loc_pk + (size_t)l * 2 * (P + 1));
 	if (i <= P)
 	{
 		for (int k = 0; k < 2; k++)
@@ -411,7 +438,10 @@ CCF_D void leaf_df_leaf(int l, int i, int P, const double2* __restrict__ leaf_ce
 			double2 v = loc[((size_t)l * 3 + k) * (P + 1) + i];
 			float2 re = split(v.x), im = split(v.y);
 			loc_df[((size_t)l * 2 + k) * (P + 1) + i] = make_float4(re.x, im.x, re.y, im.y);
+			if (k == 0) store_loc_pk(pk, i, 0, re, im);
+			else if (i > 0) store_loc_pk(pk, i - 1, 1, re, im);
 		}
+		if (i == 0) store_loc_pk(pk, P, 1, make_float2(0, 0), make_float2(0, 0));
 	}
 	if (i == 0) ih_df[l] = split(leaf_inv_half[l]);
 }
@@ -419,20 +449,22 @@ CCF_D void leaf_df_leaf(int l, int i, int P, const double2* __restrict__ leaf_ce
 __global__ void leaf_df_kernel(int num_leaves, int P, const double2* __restrict__ leaf_center,
 	const double* __restrict__ leaf_inv_half, const int* __restrict__ near_count, const NearStar* __restrict__ near,
 	const double2* __restrict__ loc, float4* __restrict__ near_df, float2* __restrict__ mass_df, float4* __restrict__ loc_df,
-	float2* __restrict__ ih_df)
+	float2* __restrict__ ih_df, float4* __restrict__ near_pk, float4* __restrict__ loc_pk)
 {
 	const int l = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
 	if (l >= num_leaves) return;
-	leaf_df_leaf(l, threadIdx.x & 31, P, leaf_center, leaf_inv_half, near_count, near, loc, near_df, mass_df, loc_df, ih_df);
+	leaf_df_leaf(l, threadIdx.x & 31, P, leaf_center, leaf_inv_half, near_count, near, loc, near_df, mass_df, loc_df, ih_df,
+		near_pk, loc_pk);
 }
 
 void launch_leaf_df(cudaStream_t s, int num_leaves, int P, const double2* leaf_center, const double* leaf_inv_half,
 	const int* near_count, const NearStar* near, const double2* loc, float4* near_df, float2* mass_df, float4* loc_df,
-	float2* ih_df)
+	float2* ih_df, float4* near_pk, float4* loc_pk)
 {
 	const int warps = 4;
 	leaf_df_kernel<<<(num_leaves + warps - 1) / warps, warps * 32, 0, s>>>(num_leaves, P, leaf_center, leaf_inv_half,
-		near_count, near, loc, near_df, mass_df, loc_df, ih_df);
+		near_count, near, loc, near_df, mass_df, loc_df, ih_df,
+		near_pk, loc_pk);
 }
 
 } /* namespace ccf */
@@ -501,7 +533,8 @@ CCF_D double fold_tail(const double2* __restrict__ e, int n, double2 z0, double 
 __global__ void __launch_bounds__(96) fold_smooth_kernel(int num_leaves, int P, const double2* __restrict__ leaf_center,
 	const double* __restrict__ leaf_inv_half, const double2* __restrict__ loc, const double2* __restrict__ ef, int nf,
 	const double2* __restrict__ er, int nr, const double2* __restrict__ eq, int nq, double radius,
-	float4* __restrict__ loc_df, float2* __restrict__ loc3f, double2* __restrict__ loc64, unsigned char* __restrict__ fold)
+	float4* __restrict__ loc_df, float4* __restrict__ loc_pk, float2* __restrict__ loc3f, double2* __restrict__ loc64,
+	unsigned char* __restrict__ fold)
 {
 	__shared__ double inv[FOLD_MAXD + 1];
 	__shared__ int s_ok[3];
@@ -541,6 +574,9 @@ __global__ void __launch_bounds__(96) fold_smooth_kernel(int num_leaves, int P, 
 	{
 		const float2 x = split(a.x), y = split(a.y);
 		loc_df[((size_t)l * 2 + part) * (P + 1) + i] = make_float4(x.x, y.x, x.y, y.y);
+		float* pk = reinterpret_cast<float*>(loc_pk + (size_t)l * 2 * (P + 1));
+		if (part == 0) store_loc_pk(pk, i, 0, x, y);
+		else if (i > 0) store_loc_pk(pk, i - 1, 1, x, y);
 	}
 	else
 	{
@@ -551,11 +587,11 @@ __global__ void __launch_bounds__(96) fold_smooth_kernel(int num_leaves, int P, 
 
 void launch_fold_smooth(cudaStream_t s, int num_leaves, int P, const double2* leaf_center, const double* leaf_inv_half,
 	const double2* loc, const double2* ef, int nf, const double2* er, int nr, const double2* eq, int nq, double radius,
-	float4* loc_df, float2* loc3f, double2* loc64, unsigned char* fold)
+	float4* loc_df, float4* loc_pk, float2* loc3f, double2* loc64, unsigned char* fold)
 {
 	if (num_leaves <= 0) return;
 	fold_smooth_kernel<<<num_leaves, 96, 0, s>>>(num_leaves, P, leaf_center, leaf_inv_half, loc, ef, nf, er, nr, eq, nq,
-		radius, loc_df, loc3f, loc64, fold);
+		radius, loc_df, loc_pk, loc3f, loc64, fold);
 }
 
 } /* namespace ccf */
@@ -638,7 +674,7 @@ __global__ void __launch_bounds__(512) leaf_batch_kernel(const BatchSeg* __restr
 	{
 		for (int l = warp; l < nl; l += nw)
 			leaf_df_leaf(l, lane, S.P, S.leaf_center, S.leaf_inv_half, S.leaf_near_count, S.leaf_near, S.leaf_loc,
-				S.leaf_near_df, S.leaf_mass_df, S.leaf_loc_df, S.leaf_ih_df);
+				S.leaf_near_df, S.leaf_mass_df, S.leaf_loc_df, S.leaf_ih_df, S.leaf_near_pk, S.leaf_loc_pk);
 		for (int i = tid; i < S.n; i += blockDim.x)
 		{
 			S.star_hilo[i] = split_hilo(S.pos[i]);

@@ -252,6 +252,7 @@ struct TrackArgs
 	const int* num_rows_dev;    /* when set: the number of rows, on the device */
 	int items_per_row;          /* when > 0: item = row * items_per_row + chunk */
 	int max_sub;                /* longest sub-step (TSUB = a whole phi step) */
+	int scales;                 /* a field of the launch writes length scales */
 };
 
 /* stars.cu */
@@ -316,6 +317,8 @@ struct BatchSeg
 	float2* leaf_mass_df;
 	float4* leaf_loc_df;
 	float2* leaf_ih_df;
+	float4* leaf_near_pk;
+	float4* leaf_loc_pk;
 	float4* star_hilo;
 	float2* star_mass_df;
 };
@@ -405,10 +408,10 @@ void launch_leaf_build(cudaStream_t s, const TreeDev& T, int num_nodes, const in
 
 void launch_leaf_df(cudaStream_t s, int num_leaves, int P, const double2* leaf_center, const double* leaf_inv_half,
 	const int* near_count, const NearStar* near, const double2* loc, float4* near_df, float2* mass_df, float4* loc_df,
-	float2* ih_df);
+	float2* ih_df, float4* near_pk, float4* loc_pk);
 void launch_fold_smooth(cudaStream_t s, int num_leaves, int P, const double2* leaf_center, const double* leaf_inv_half,
 	const double2* loc, const double2* ef, int nf, const double2* er, int nr, const double2* eq, int nq, double radius,
-	float4* loc_df, float2* loc3f, double2* loc64, unsigned char* fold);
+	float4* loc_df, float4* loc_pk, float2* loc3f, double2* loc64, unsigned char* fold);
 
 /* solver.cu */
 int solver_blocks_per_sm(bool mixed);

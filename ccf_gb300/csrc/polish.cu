@@ -38,6 +38,7 @@ run over every star, is taken by the whole warp, the lanes splitting the
 stars.  A point beyond the list's capacity is polished by the scan itself,
 one warp per point.
 ******************************************************************************/
+#define CCF_COLD static __device__ __forceinline__
 #include "kernels.h"
 
 namespace ccf

@@ -752,47 +752,24 @@ constexpr int TABLE_PROBES = 1024;       /* linear-probe bound of the column tab
                                             longest cluster of a table of 1e5 slots is ~60) */
 constexpr double CELL_PER_THETA = 1048576.0;   /* 2^20 cells per theta_star */
 
-/* 2 sum_i 1/(z - z_i) over the near stars of the leaf; zero off the root box.
-   FP32 on the leaf-relative split positions in mixed precision (it only
-   scales the step), FP64 otherwise. */
-template <bool MIXED>
+/* 2 sum_i 1/(z - z_i) over the near stars of the leaf; zero off the root box
+   (the FP64 tracker; eval_track_df forms its own) */
 CCF_D double2 near_pole_sum(const FieldView& F, int leaf, double2 z)
 {
 	if (leaf < 0) return make_double2(0, 0);
 	const int n = F.leaf_near_count[leaf];
-	const double2 c = F.leaf_center[leaf];
-	const double rx = z.x - c.x, ry = z.y - c.y;
-	if constexpr (MIXED)
+	const NearStar* P = F.leaf_near + (size_t)leaf * MAX_NEAR;
+	double ax = 0, ay = 0;
+#pragma unroll 1
+	for (int i = 0; i < n; i++)
 	{
-		const float hx = (float)rx, hy = (float)ry;
-		const float lx = (float)(rx - (double)hx), ly = (float)(ry - (double)hy);
-		const float4* P = F.leaf_near_df + (size_t)leaf * MAX_NEAR;
-		float ax = 0.f, ay = 0.f;
-		for (int i = 0; i < n; i++)
-		{
-			const float4 s = P[i];
-			const float dx = (hx - s.x) + (lx - s.z);
-			const float dy = (hy - s.y) + (ly - s.w);
-			const float r = rcp32(fmaf(dx, dx, fmaf(dy, dy, 1e-30f)));
-			ax = fmaf(dx, r, ax);
-			ay = fmaf(dy, r, ay);
-		}
-		return make_double2(2.0 * ax, -2.0 * ay);
+		const NearStar s = P[i];
+		const double dx = z.x - s.x, dy = z.y - s.y;
+		const double r = rcp64(fma(dx, dx, fma(dy, dy, 1e-300)));
+		ax = fma(dx, r, ax);
+		ay = fma(dy, r, ay);
 	}
-	else
-	{
-		const NearStar* P = F.leaf_near + (size_t)leaf * MAX_NEAR;
-		double ax = 0, ay = 0;
-		for (int i = 0; i < n; i++)
-		{
-			const NearStar s = P[i];
-			const double dx = z.x - s.x, dy = z.y - s.y;
-			const double r = rcp64(fma(dx, dx, fma(dy, dy, 1e-300)));
-			ax = fma(dx, r, ax);
-			ay = fma(dy, r, ay);
-		}
-		return make_double2(2 * ax, -2 * ay);
-	}
+	return make_double2(2 * ax, -2 * ay);
 }
 
 /* 64-bit key of the cell of z (never 0, the empty slot); the mixing is the
@@ -825,37 +802,42 @@ CCF_D unsigned long long table_insert(unsigned long long* tab, unsigned long lon
 }
 
 /* Predictor of the continuation: the polynomial through the last accepted
-   positions of the root (newest first, hz[k * TNT], k < hn <= TRACK_HIST),
-   extrapolated to sub-step position t.  When the history is a run of whole
-   phi steps and t is the next one, the extrapolation of order hn has the
-   binomial weights (5, -10, 10, -5, 1 for five points): along the smooth
+   positions of the root, extrapolated to sub-step position t.  hz is the
+   lane's ring of TRACK_HIST positions, slot head the newest (the next slots
+   the older ones), hn of them valid.  When the history is a run of whole phi
+   steps and t is the next one (uniform), the extrapolation of order hn has
+   the binomial weights (5, -10, 10, -5, 1 for five points): along the smooth
    paths of the critical curves its error is below 1e-9 theta_star for most
    roots, so they converge at the first evaluation.  After sub-steps (uneven
-   history) it falls back to the secant through the two newest points. */
+   history) it falls back to the secant through the two newest points, t0 and
+   t1 the older and the newer one's positions. */
 constexpr int TRACK_HIST = 5;
 __constant__ double c_extrap_w[TRACK_HIST][TRACK_HIST] = {
 	{1, 0, 0, 0, 0}, {2, -1, 0, 0, 0}, {3, -3, 1, 0, 0}, {4, -6, 4, -1, 0}, {5, -10, 10, -5, 1}};
 
-CCF_D double2 track_predict(const double2* hz, const int* ht, int hn, int t)
+CCF_D int ring_next(int slot) { return slot + 1 == TRACK_HIST ? 0 : slot + 1; }
+
+CCF_D double2 track_predict(const double2* hz, int head, int hn, bool uniform, int t0, int t1, int t)
 {
-	bool uniform = t - ht[0] == TSUB;
-	for (int k = 0; k + 1 < hn; k++) uniform = uniform && ht[k * TNT] - ht[(k + 1) * TNT] == TSUB;
-	const double2 z1 = hz[0];
+	const double2 z1 = hz[head * TNT];
 	if (uniform && hn > 1)
 	{
 		double x = 0, y = 0;
+		int slot = head;
+#pragma unroll 1
 		for (int k = 0; k < hn; k++)
 		{
-			const double2 q = hz[k * TNT];
+			const double2 q = hz[slot * TNT];
 			const double wk = c_extrap_w[hn - 1][k];
 			x = fma(wk, q.x, x);
 			y = fma(wk, q.y, y);
+			slot = ring_next(slot);
 		}
 		return make_double2(x, y);
 	}
 	if (hn < 2) return z1;
-	const double2 z0 = hz[TNT];
-	const double w = (double)(t - ht[0]) / (double)(ht[0] - ht[TNT]);
+	const double2 z0 = hz[ring_next(head) * TNT];
+	const double w = (double)(t - t1) / (double)(t1 - t0);
 	return make_double2(z1.x + w * (z1.x - z0.x), z1.y + w * (z1.y - z0.y));
 }
 
@@ -889,6 +871,7 @@ CCF_D void offfield_sums_warp_df(const FieldView& F, bool need, double2 z, NearS
 		a.s2 = a.s1;
 		dfc s3 = a.s1;
 		float2 s3f = make_float2(0.f, 0.f);
+#pragma unroll 1
 		for (int i = lane; i < F.num_stars; i += 32)
 			star_term_df<NEED1, false>(a, s3, s3f, zd, F.star_df[i], F.star_mass_df[i]);
 		dfl w[4] = {a.s1.re, a.s1.im, a.s2.re, a.s2.im};
@@ -1048,6 +1031,20 @@ __device__ __noinline__ TrackEval track_offfield(const FieldView& F, bool off, d
 	return r;
 }
 
+/* find_leaf out of line, for the lanes that left their leaf */
+__device__ __noinline__ int find_leaf_far(const FieldView& F, double2 z) { return find_leaf(F, z); }
+
+/* slot of branch b, column k in the output rows of a root (out_slot), row =
+   root * w_nb */
+CCF_D size_t out_slot_row(const FieldOut& O, size_t row, int b, int k)
+{
+	int bi = b - O.w_b0;
+	if (bi < 0) bi += O.nb;
+	const int ki = k - O.w_k0;
+	if (bi >= O.w_nb || ki < 0 || ki >= O.w_cols) return NO_OUT;
+	return (row + bi) * O.w_cols + ki;
+}
+
 /* Is z inside the box of `leaf`?  rel = z - leaf centre. */
 CCF_D bool in_leaf_box(const FieldView& F, int leaf, double2 z, double2& rel)
 {
@@ -1104,20 +1101,30 @@ __global__ void track_mark_kernel(const TrackArgs T)
 	}
 }
 
+/* cos, sin of a sub-step position t that is no whole step (out of line) */
+__device__ __noinline__ double2 track_phase_sub(const FieldOut& O, int c, int side, int t)
+{
+	double2 cs;
+	sincos(track_phi(c, O.nb, O.nphi, side, t), &cs.y, &cs.x);
+	return cs;
+}
+
 /* cos, sin of sub-step position t of row (c, side): the field's phase table
-   for whole steps, else computed */
-CCF_D void track_phase(const FieldOut& O, int c, int side, int t, double& cp, double& sp, dfl& cpd, dfl& spd)
+   for the whole step whose global step is gp, else computed */
+CCF_D void track_phase(const FieldOut& O, int c, int side, int t, int gp, double& cp, double& sp, dfl& cpd, dfl& spd)
 {
 	if (t % TSUB == 0)
 	{
-		const PhaseEntry e = O.phase[row_global_step(O.nb, O.half, c, side, t / TSUB)];
+		const PhaseEntry e = O.phase[gp];
 		cp = e.cs.x;
 		sp = e.cs.y;
 		cpd = {e.cs_df.x, e.cs_df.z};
 		spd = {e.cs_df.y, e.cs_df.w};
 		return;
 	}
-	sincos(track_phi(c, O.nb, O.nphi, side, t), &sp, &cp);
+	const double2 cs = track_phase_sub(O, c, side, t);
+	cp = cs.x;
+	sp = cs.y;
 	cpd = df_from_double(cp);
 	spd = df_from_double(sp);
 }
@@ -1166,7 +1173,7 @@ cudaError_t launch_phase_table(cudaStream_t s, int nb, int nphi, PhaseEntry* out
    the direct evaluation of the outputs (a warp-wide call).  Every lane of the
    warp stays in the loop to the end: the evaluation off the root box and
    the direct epilogue are warp-wide calls. */
-template <bool MIXED>
+template <bool MIXED, bool PK>
 __global__ void __launch_bounds__(TNT, 3) track_kernel(const TrackArgs T)
 {
 	__shared__ FieldView sF[TNT / 32];
@@ -1174,12 +1181,10 @@ __global__ void __launch_bounds__(TNT, 3) track_kernel(const TrackArgs T)
 	__shared__ RowDesc sR[TNT / 32];
 	__shared__ TrackConst sK[TNT / 32];
 	__shared__ double s_maxerr[TNT / 32];
-	__shared__ double2 s_hz[TRACK_HIST * TNT];   /* accepted positions of each lane's root, newest first */
-	__shared__ int s_ht[TRACK_HIST * TNT];
+	__shared__ double2 s_hz[TRACK_HIST * TNT];   /* accepted positions of each lane's root (a ring per lane) */
 	const unsigned full = 0xffffffffu;
 	const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
 	double2* const hz = s_hz + threadIdx.x;
-	int* const ht = s_ht + threadIdx.x;
 
 	while (true)
 	{
@@ -1233,7 +1238,7 @@ __global__ void __launch_bounds__(TNT, 3) track_kernel(const TrackArgs T)
 		const int a = solo_root >= 0 ? solo_root : chunk * 32 + lane;
 		const bool valid = solo_root >= 0 ? lane == 0 : (a < R && (T.items_per_row > 0 || !T.is_solo[RD.base + a]));
 		const int max_sub = T.max_sub;
-		const int c = RD.branch, side = RD.side, nb = O.nb, nphi = O.nphi;
+		const int c = RD.branch, side = RD.side, nb = O.nb, nphi = O.nphi, period = 2 * O.half;
 		const int j0 = O.step_first, j1 = RD.steps;
 		const int cap = O.max_iters_step;
 		const double tol = STEP_TOL * F.theta;
@@ -1248,23 +1253,32 @@ __global__ void __launch_bounds__(TNT, 3) track_kernel(const TrackArgs T)
 		const bool direct_out = !MIXED || O.mu != nullptr;
 		unsigned long long lane_maxerr = 0;   /* bits of the lane's largest 1/mu bound (non-negative) */
 
-		double2 z1 = valid ? T.master[RD.base + a] : make_double2(0, 0);
+		const double2 z1 = valid ? T.master[RD.base + a] : make_double2(0, 0);
 		int t1 = (j0 - 1) * TSUB;
+		int head = 0, hn = 1;   /* the ring's newest slot and its length */
 		hz[0] = z1;
-		ht[0] = t1;
-		int hn = 1;
+		int t0 = t1;            /* the position before t1, once hn > 1 */
+		int run = 0;            /* whole-step gaps in a row up to t1 */
 		int leaf = -1;
 		unsigned flags = 0;
 		unsigned long long nev = 0, nhalf = 0;
 		int maxev = 0;
 
 		int j = j0;
+		/* global step of step j and its output column (row_slots), kept as j
+		   advances: gp = the step's phase, column kk of branch bb */
+		int gp = row_global_step(nb, O.half, c, side, j);
+		int bb = (gp + O.half) / period;
+		int kk = gp + O.half - bb * period;
+		if (bb == nb) bb = 0;
+		const int nbr = side ? (c + O.seg) % nb : (c - O.seg + nb) % nb;   /* the next solved centre that way */
+		const size_t out_row = (size_t)a * O.w_nb;
 		bool act = valid;
 		int tt = min(t1 + max_sub, j * TSUB);
 		double2 z = z1;
 		double cp = 0, sp = 0;
 		dfl cpd = {0.f, 0.f}, spd = {0.f, 0.f};
-		track_phase(O, c, side, tt, cp, sp, cpd, spd);
+		track_phase(O, c, side, tt, gp, cp, sp, cpd, spd);
 		int it = 0, evs = 0;
 		real prev2 = 0;
 		bool lost = !valid;
@@ -1280,7 +1294,7 @@ __global__ void __launch_bounds__(TNT, 3) track_kernel(const TrackArgs T)
 			double2 rel = make_double2(0, 0);
 			if (act && !(leaf >= 0 && in_leaf_box(F, leaf, z, rel)))
 			{
-				leaf = find_leaf(F, z);
+				leaf = find_leaf_far(F, z);
 				if (leaf >= 0) in_leaf_box(F, leaf, z, rel);
 			}
 			const bool off = act && leaf < 0;
@@ -1295,7 +1309,7 @@ __global__ void __launch_bounds__(TNT, 3) track_kernel(const TrackArgs T)
 			e.wmode = 2;
 			if constexpr (MIXED)
 			{
-				if (act && leaf >= 0) e = eval_track_df(F, K, leaf, z, rel, cpd, spd, disc_exact);
+				if (act && leaf >= 0) e = eval_track_df<PK>(F, K, leaf, z, rel, cpd, spd, disc_exact);
 				if (__any_sync(full, off))
 				{
 					const TrackEval o = track_offfield(F, off, z, cp, sp, disc_exact, (float)stuck2);
@@ -1309,7 +1323,7 @@ __global__ void __launch_bounds__(TNT, 3) track_kernel(const TrackArgs T)
 				const FdF g = eval_fdf_warp<false>(F, act, z, leaf, false, zero_sums(), cp, sp);
 				if (act)
 				{
-					double2 S = near_pole_sum<false>(F, leaf, z);
+					double2 S = near_pole_sum(F, leaf, z);
 					if (disc_exact)
 					{
 						const double2 iz = cinv(z);
@@ -1375,16 +1389,12 @@ __global__ void __launch_bounds__(TNT, 3) track_kernel(const TrackArgs T)
 				if (conv)
 				{
 					const int dist = tt - t1;
-					for (int k = min(hn, TRACK_HIST - 1); k > 0; k--)
-					{
-						hz[k * TNT] = hz[(k - 1) * TNT];
-						ht[k * TNT] = ht[(k - 1) * TNT];
-					}
+					head = head == 0 ? TRACK_HIST - 1 : head - 1;
 					hn = min(hn + 1, TRACK_HIST);
-					z1 = z;
+					run = dist == TSUB ? min(run + 1, TRACK_HIST - 1) : 0;
+					t0 = t1;
 					t1 = tt;
-					hz[0] = z1;
-					ht[0] = t1;
+					hz[head * TNT] = z;
 					refine = false;
 					if (tt == j * TSUB)
 					{
@@ -1392,10 +1402,19 @@ __global__ void __launch_bounds__(TNT, 3) track_kernel(const TrackArgs T)
 						zf = z;
 						ecp = cp;
 						esp = sp;
-						int ob[2], ok[2];
-						const int nslot = row_slots(nb, O.half, O.seg, c, side, j, ob, ok);
-						out = out_slot(O, a, ob[0], ok[0]);
-						if (nslot > 1) out2 = out_slot(O, a, ob[1], ok[1]);
+						/* the slots of row_slots for step j */
+						const bool first = !(kk == 0 && side == 1 && O.seg == 1 && bb == nbr);
+						out = first ? out_slot_row(O, out_row, bb, kk) : NO_OUT;
+						if (kk == 0)
+						{
+							const int bp = bb == 0 ? nb - 1 : bb - 1;
+							if (!(side == 0 && O.seg == 1 && bp == nbr))
+							{
+								const size_t o2 = out_slot_row(O, out_row, bp, period);
+								if (first) out2 = o2;
+								else out = o2;
+							}
+						}
 						if constexpr (MIXED)
 						{
 							if (!direct_out)
@@ -1470,6 +1489,24 @@ __global__ void __launch_bounds__(TNT, 3) track_kernel(const TrackArgs T)
 						evs = 0;
 						j++;
 						if (j > j1) act = false;
+						if (side)
+						{
+							gp = gp + 1 == nphi ? 0 : gp + 1;
+							if (++kk == period)
+							{
+								kk = 0;
+								bb = bb + 1 == nb ? 0 : bb + 1;
+							}
+						}
+						else
+						{
+							gp = gp == 0 ? nphi - 1 : gp - 1;
+							if (--kk < 0)
+							{
+								kk = period - 1;
+								bb = bb == 0 ? nb - 1 : bb - 1;
+							}
+						}
 						tn = min(t1 + max_sub, j * TSUB);
 					}
 					else
@@ -1502,10 +1539,10 @@ __global__ void __launch_bounds__(TNT, 3) track_kernel(const TrackArgs T)
 				{
 					/* next target: predict, restart the corrector */
 					tt = tn;
-					z = track_predict(hz, ht, hn, tt);
+					z = track_predict(hz, head, hn, tt - t1 == TSUB && run >= hn - 1, t0, t1, tt);
 					it = 0;
 					prev2 = 0;
-					track_phase(O, c, side, tt, cp, sp, cpd, spd);
+					track_phase(O, c, side, tt, gp, cp, sp, cpd, spd);
 				}
 			}
 
@@ -1656,16 +1693,17 @@ cudaError_t launch_track(cudaStream_t s, const TrackArgs& a, bool mixed)
 	int& n = per_sm[mixed ? 1 : 0];
 	if (n == 0)
 	{
-		if (mixed) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, track_kernel<true>, TNT, 0);
-		else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, track_kernel<false>, TNT, 0);
+		if (mixed) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, track_kernel<true, true>, TNT, 0);
+		else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, track_kernel<false, false>, TNT, 0);
 		if (n < 1) n = 1;
 	}
 	int dev = 0, sms = 0;
 	cudaGetDevice(&dev);
 	cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
 	const int blocks = std::max(1, std::min(sms * n, (a.num_items + TNT / 32 - 1) / (TNT / 32)));
-	if (mixed) track_kernel<true><<<blocks, TNT, 0, s>>>(a);
-	else track_kernel<false><<<blocks, TNT, 0, s>>>(a);
+	if (!mixed) track_kernel<false, false><<<blocks, TNT, 0, s>>>(a);
+	else if (a.scales) track_kernel<true, false><<<blocks, TNT, 0, s>>>(a);
+	else track_kernel<true, true><<<blocks, TNT, 0, s>>>(a);
 	return cudaGetLastError();
 }
 

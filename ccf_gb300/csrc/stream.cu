@@ -429,6 +429,7 @@ ccf_status Engine::solve_chunked(Field& f, int verbose)
 			T.num_rows_dev = nullptr;
 			T.items_per_row = 0;
 			T.max_sub = TRACK_TSUB;
+			T.scales = f.params.write_mu_length_scales ? 1 : 0;
 			T.num_items = grows * ((R + 31) / 32);
 			T.solo = P.solo.ptr;
 			T.num_solo = reinterpret_cast<int*>(P.solo.ptr + ncont);
