@@ -122,11 +122,49 @@ Engine::~Engine()
 		cudaStreamDestroy(chunk.copy);
 		for (cudaEvent_t e : {chunk.ready, chunk.copied[0], chunk.copied[1], chunk.done}) cudaEventDestroy(e);
 	}
+	if (side.side)
+	{
+		cudaStreamSynchronize(side.side);
+		cudaStreamDestroy(side.side);
+		cudaEventDestroy(side.fork);
+		cudaEventDestroy(side.join);
+	}
 	if (stream)
 	{
 		cudaStreamSynchronize(stream);   /* its pool buffers go back to the cache after this */
 		cudaStreamDestroy(stream);
 	}
+}
+
+/* room for the roots that leave the box: a few per row do (20 of 160 000 on
+   the 20 000-star field); those beyond it stay in their items */
+constexpr int FAR_EVICT_CAP = 8192;
+
+cudaError_t Engine::far_setup(TrackArgs& T, long long roots, long long smooth, int max_stars)
+{
+	cudaError_t e;
+	if (!side.side)
+	{
+		if ((e = cudaEventCreateWithFlags(&side.fork, cudaEventDisableTiming)) != cudaSuccess) return e;
+		if ((e = cudaEventCreateWithFlags(&side.join, cudaEventDisableTiming)) != cudaSuccess) return e;
+		if ((e = cudaStreamCreateWithFlags(&side.side, cudaStreamNonBlocking)) != cudaSuccess) return e;
+	}
+	T.evict_cap = (int)std::min<long long>(roots, FAR_EVICT_CAP);
+	if ((e = pools.evict.ensure(T.evict_cap)) != cudaSuccess) return e;
+	T.evict = pools.evict.ptr;
+	T.num_evict = pools.rerun_count.ptr + 6;
+	T.evict_counter = pools.rerun_count.ptr + 7;
+	T.far_evicted = T.solo_far = 0;
+	T.num_roots = roots;
+	T.solo_guess = T.num_rows + smooth / 3;
+	T.max_stars = max_stars;
+	return cudaSuccess;
+}
+
+void Engine::far_counts(TrackArgs& T2)
+{
+	T2.num_evict = pools.rerun_count.ptr + 8;
+	T2.evict_counter = pools.rerun_count.ptr + 9;
 }
 
 ccf_status Engine::cuda_fail(cudaError_t e, const char* what)
@@ -1020,7 +1058,7 @@ ccf_status Engine::solve(std::vector<Field*>& fields, int verbose)
 		CCF_TRY(P.track_table.ensure(table_slots), "cudaMalloc(tables)");
 		CCF_TRY(P.row_stats.ensure(TRACK_ROW_STATS * rc.size()), "cudaMalloc(rows)");
 		CCF_TRY(P.rows_rerun.ensure(rc.size()), "cudaMalloc(rows)");
-		CCF_TRY(P.rerun_count.ensure(6), "cudaMalloc(rows)");
+		CCF_TRY(P.rerun_count.ensure(10), "cudaMalloc(rows)");
 		CCF_TRY(P.rows_rerun2.ensure(rc.size()), "cudaMalloc(rows)");
 		CCF_TRY(P.row_stats2.ensure(TRACK_ROW_STATS * rc.size()), "cudaMalloc(rows)");
 		CCF_TRY(P.item_start.ensure(rc.size()), "cudaMalloc(rows)");
@@ -1101,10 +1139,15 @@ ccf_status Engine::solve(std::vector<Field*>& fields, int verbose)
 		T.solo = P.solo.ptr;
 		T.num_solo = reinterpret_cast<int*>(P.solo.ptr + ncont);
 		T.is_solo = P.is_solo.ptr;
+		int max_stars = 0;
+		for (Field* f : fields) max_stars = std::max(max_stars, f->d.num_stars);
+		long long smooth_roots = 0;
+		for (const RowDesc& r : rc) smooth_roots += fields[r.field]->d.num_roots - 2 * fields[r.field]->d.num_stars;
+		CCF_TRY(far_setup(T, ncont, smooth_roots, max_stars), "cudaMalloc(far roots)");
 		CCF_TRY(cudaMemsetAsync(T.num_solo, 0, sizeof(int), s), "memset");
 		CCF_TRY(cudaMemsetAsync(P.track_table.ptr, 0, table_slots * sizeof(unsigned long long), s), "memset");
 		CCF_TRY(cudaMemsetAsync(P.row_stats.ptr, 0, TRACK_ROW_STATS * rc.size() * sizeof(unsigned long long), s), "memset");
-		CCF_TRY(cudaMemsetAsync(P.rerun_count.ptr, 0, 6 * sizeof(int), s), "memset");
+		CCF_TRY(cudaMemsetAsync(P.rerun_count.ptr, 0, 10 * sizeof(int), s), "memset");
 		CCF_TRY(cudaMemsetAsync(P.row_stats2.ptr, 0, TRACK_ROW_STATS * rc.size() * sizeof(unsigned long long), s), "memset");
 		CCF_TRY(P.item_order.ensure((size_t)T.num_items + 1), "cudaMalloc(items)");
 		CCF_TRY(P.item_work.ensure(3 * (size_t)T.num_items + 3), "cudaMalloc(items)");
@@ -1112,9 +1155,9 @@ ccf_status Engine::solve(std::vector<Field*>& fields, int verbose)
 		   last wave's length is a sizeable share of it (track_item_order_kernel) */
 		reorder = (long long)T.num_items < 32LL * num_sms * TRACK_WARPS_PER_SM;
 		T.item_order = reorder ? P.item_order.ptr : nullptr;
-		CCF_TRY(launch_track_mark(s, T), "track_mark");
+		CCF_TRY(launch_track_mark(s, T, P.item_work.ptr), "track_mark");
 		if (reorder) CCF_TRY(launch_track_item_order(s, T, P.item_work.ptr, P.item_order.ptr), "track_item_order");
-		CCF_TRY(launch_track(s, T, mixed), "track_ccs");
+		CCF_TRY(launch_track(s, T, mixed, side), "track_ccs");
 		CCF_TRY(launch_track_check(s, T, max_row_points), "track_check");
 		CCF_TRY(launch_collect_rerun(s, T, P.rows_rerun.ptr, P.rerun_count.ptr), "collect_rerun");
 		/* rows that failed: tracked again from their centre with sub-steps of at
@@ -1130,8 +1173,9 @@ ccf_status Engine::solve(std::vector<Field*>& fields, int verbose)
 		T2.max_sub = TRACK_TSUB / TRACK_FINE_SUB;
 		T2.row_stats = P.row_stats2.ptr;
 		T2.counter = P.rerun_count.ptr + 4;
+		far_counts(T2);
 		CCF_TRY(launch_clear_tables(s, T2), "clear_tables");
-		CCF_TRY(launch_track(s, T2, mixed), "track_ccs_fine");
+		CCF_TRY(launch_track(s, T2, mixed, side), "track_ccs_fine");
 		CCF_TRY(launch_track_check(s, T2, max_row_points), "track_check");
 		CCF_TRY(launch_collect_rerun(s, T2, P.rows_rerun2.ptr, P.rerun_count.ptr + 3), "collect_rerun");
 		A.rows = P.rows_rerun2.ptr;
@@ -1170,13 +1214,14 @@ ccf_status Engine::solve(std::vector<Field*>& fields, int verbose)
 
 	ccf_status status = CCF_OK;
 	/* root seeds, initial solve, continuation (tracker: phase table, item
-	   marking, item order (2), tracking, column check, row collection, table clearing,
-	   re-tracking, column check, row collection and the full-sum launch for
+	   marking, item order, tracking (the items and two far launches), column check, row
+	   collection, table clearing, re-tracking (items, far), column check, row collection and the
+	   full-sum launch for
 	   the rows to re-run), FP64 polish; the launches are shared by the
 	   batch's fields and counted with the first */
 	for (int fi = 0; fi < nf; fi++)
 	{
-		ccf_status rc = finish_stats(*fields[fi], seg[fi], track, verbose, fi > 0 ? 0 : track ? (reorder ? 16 : 14) : 5);
+		ccf_status rc = finish_stats(*fields[fi], seg[fi], track, verbose, fi > 0 ? 0 : track ? (reorder ? 18 : 17) : 5);
 		if (rc != CCF_OK) status = rc;
 	}
 	return status;

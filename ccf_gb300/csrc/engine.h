@@ -206,9 +206,12 @@ struct SolverPools
 	DBuf<unsigned long long> track_table;   /* column tables of the tracker */
 	DBuf<unsigned long long> row_stats, row_stats2;   /* TRACK_ROW_STATS per row: tracking, re-tracking */
 	DBuf<int> rerun_count;                  /* [0] rows to re-track, [1] [2] tracker work counters,
-	                                           [3] rows to re-run, [4] [5] re-tracking work counters */
+	                                           [3] rows to re-run, [4] [5] re-tracking work counters,
+	                                           [6] [7] roots that left the box and the next of them,
+	                                           [8] [9] the same of the re-tracking */
 	DBuf<int> item_start;                   /* first tracker work item of each continuation row */
 	DBuf<int2> solo;                        /* tracker roots run alone, and their count after them */
+	DBuf<FarState> evict;                   /* tracker roots that left the root box */
 	DBuf<unsigned char> is_solo;            /* per continuation root */
 	DBuf<unsigned long long> polish_list;   /* [0] count, then the points the FP64 polish works on */
 	DBuf<FieldView> views;
@@ -306,7 +309,14 @@ public:
 	bool ensure_device(int dev);
 
 private:
+	/* the device buffers and counts of the tracker's far launches into T (the
+	   first tracking; T2 takes its counts from far_counts); roots = all rows',
+	   smooth = those of them beyond two per star (the Taylor form's), of which
+	   about a third start off the root box or leave it */
+	cudaError_t far_setup(TrackArgs& T, long long roots, long long smooth, int max_stars);
+	void far_counts(TrackArgs& T2);
 
+	TrackSide side;   /* the stream the far launch runs on, beside the items */
 	SolverPools pools;
 	/* solve_chunked: the centre columns of the initial solve, two chunk
 	   buffers of output windows, their FieldOut records, a copy stream and

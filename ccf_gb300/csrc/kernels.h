@@ -230,6 +230,17 @@ constexpr unsigned long long TRACK_LOST = 2;         /* a root that did not conv
 constexpr unsigned long long TRACK_NONFINITE = 4;    /* a non-finite 1/mu bound */
 constexpr unsigned long long TRACK_TABLE_FULL = 8;   /* the column table probe limit was reached */
 
+/* a root handed from the item launch to the far launch: the tracker's state
+   at the top of an iteration (track_kernel) */
+constexpr int TRACK_HIST = 5;   /* accepted positions a root's predictor uses */
+struct FarState
+{
+	double2 hz[TRACK_HIST];
+	double2 z;
+	double prev2;
+	int row, root, head, hn, run, t0, t1, j, tt, it, evs, refine;
+};
+
 struct TrackArgs
 {
 	const FieldView* fields;
@@ -241,10 +252,22 @@ struct TrackArgs
 	unsigned long long* row_stats;   /* TRACK_ROW_STATS per row, zeroed before the launch */
 	const int* item_start;      /* [num_rows]: first work item (32 roots) of each row */
 	int num_items;
-	int* counter;               /* [0] next solo root, [1] next item in order; zeroed before the launch */
-	int2* solo;                 /* (row, root) of the roots that start off the root box: one warp each, first ... */
+	int* counter;               /* [0] next solo root, [1] next item; zeroed before the launch */
+	int2* solo;                 /* (row, root) of the roots that start off the root box or are about to
+	                               leave it: tracked alone ... */
 	int* num_solo;              /* ... their number (zeroed before the marking launch) */
-	unsigned char* is_solo;     /* [master index]: the root runs solo, not in its item */
+	unsigned char* is_solo;     /* [master index]: the root is in that list, not in its item */
+	/* roots of the items that leave the root box: handed over to a second far
+	   launch (beyond evict_cap of them they stay in their item) */
+	FarState* evict;
+	int* num_evict;             /* their number (zeroed before the launch) */
+	int* evict_counter;         /* next one (zeroed before the launch) */
+	int evict_cap;
+	int solo_far;               /* the solo roots go to a far launch (set by launch_track) */
+	int far_evicted;            /* a far launch: 0 takes the solo list, 1 the handed-over roots */
+	long long num_roots;        /* the launch's roots (all rows), at most: bounds the far launches */
+	long long solo_guess;       /* about how many of them run alone */
+	int max_stars;              /* the largest field's stars */
 	const int* item_order;      /* [num_items]: the queue's order of the items; null: in order */
 	/* re-tracking of rows that failed the check: the rows are a device-side
 	   list of *num_rows_dev rows, items_per_row fixed-size items each (no
@@ -416,11 +439,18 @@ void launch_fold_smooth(cudaStream_t s, int num_leaves, int P, const double2* le
 /* solver.cu */
 int solver_blocks_per_sm(bool mixed);
 cudaError_t launch_solve(cudaStream_t s, const SolveArgs& a, bool mixed, bool initial);
-cudaError_t launch_track_mark(cudaStream_t s, const TrackArgs& a);
+cudaError_t launch_track_mark(cudaStream_t s, const TrackArgs& a, int* cls);
 cudaError_t launch_track_item_order(cudaStream_t s, const TrackArgs& a, int* work, int* order);
 constexpr int TRACK_WARPS_PER_SM = 12;   /* resident tracker warps per SM (3 CTAs of 4 warps) */
 cudaError_t launch_phase_table(cudaStream_t s, int nb, int nphi, PhaseEntry* out);
-cudaError_t launch_track(cudaStream_t s, const TrackArgs& a, bool mixed);
+/* a second stream for the far launch, and the events that fork and join it
+   (side null: everything on s) */
+struct TrackSide
+{
+	cudaStream_t side = nullptr;
+	cudaEvent_t fork = nullptr, join = nullptr;
+};
+cudaError_t launch_track(cudaStream_t s, const TrackArgs& a, bool mixed, const TrackSide& side);
 cudaError_t launch_track_check(cudaStream_t s, const TrackArgs& a, long long max_row_points);
 cudaError_t launch_collect_rerun(cudaStream_t s, const TrackArgs& a, RowDesc* rerun, int* count);
 cudaError_t launch_clear_tables(cudaStream_t s, const TrackArgs& a);

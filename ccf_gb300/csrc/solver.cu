@@ -37,6 +37,7 @@ GB300 design:
 #include "field_df.cuh"
 #include "kernels.h"
 
+#include <atomic>
 #include <cooperative_groups.h>
 #include <type_traits>
 
@@ -803,7 +804,7 @@ CCF_D unsigned long long table_insert(unsigned long long* tab, unsigned long lon
 
 /* Predictor of the continuation: the polynomial through the last accepted
    positions of the root, extrapolated to sub-step position t.  hz is the
-   lane's ring of TRACK_HIST positions, slot head the newest (the next slots
+   lane's ring of TRACK_HIST positions (NL lanes side by side), slot head the newest (the next slots
    the older ones), hn of them valid.  When the history is a run of whole phi
    steps and t is the next one (uniform), the extrapolation of order hn has
    the binomial weights (5, -10, 10, -5, 1 for five points): along the smooth
@@ -811,15 +812,15 @@ CCF_D unsigned long long table_insert(unsigned long long* tab, unsigned long lon
    roots, so they converge at the first evaluation.  After sub-steps (uneven
    history) it falls back to the secant through the two newest points, t0 and
    t1 the older and the newer one's positions. */
-constexpr int TRACK_HIST = 5;
 __constant__ double c_extrap_w[TRACK_HIST][TRACK_HIST] = {
 	{1, 0, 0, 0, 0}, {2, -1, 0, 0, 0}, {3, -3, 1, 0, 0}, {4, -6, 4, -1, 0}, {5, -10, 10, -5, 1}};
 
 CCF_D int ring_next(int slot) { return slot + 1 == TRACK_HIST ? 0 : slot + 1; }
 
+template <int NL>
 CCF_D double2 track_predict(const double2* hz, int head, int hn, bool uniform, int t0, int t1, int t)
 {
-	const double2 z1 = hz[head * TNT];
+	const double2 z1 = hz[head * NL];
 	if (uniform && hn > 1)
 	{
 		double x = 0, y = 0;
@@ -827,7 +828,7 @@ CCF_D double2 track_predict(const double2* hz, int head, int hn, bool uniform, i
 #pragma unroll 1
 		for (int k = 0; k < hn; k++)
 		{
-			const double2 q = hz[slot * TNT];
+			const double2 q = hz[slot * NL];
 			const double wk = c_extrap_w[hn - 1][k];
 			x = fma(wk, q.x, x);
 			y = fma(wk, q.y, y);
@@ -836,7 +837,7 @@ CCF_D double2 track_predict(const double2* hz, int head, int hn, bool uniform, i
 		return make_double2(x, y);
 	}
 	if (hn < 2) return z1;
-	const double2 z0 = hz[ring_next(head) * TNT];
+	const double2 z0 = hz[ring_next(head) * NL];
 	const double w = (double)(t - t1) / (double)(t1 - t0);
 	return make_double2(z1.x + w * (z1.x - z0.x), z1.y + w * (z1.y - z0.y));
 }
@@ -899,6 +900,168 @@ CCF_D void offfield_sums_warp_df(const FieldView& F, bool need, double2 z, NearS
 			out.s3 = NEED3 ? make_double2(s3f.x, s3f.y) : make_double2(0, 0);
 		}
 	}
+}
+
+/* The far launch (track_kernel, FAR): one CTA per root off the root box, so
+   that its direct sums over every star take N / (32 FAR_MAX_WARPS) terms per
+   lane instead of N / 32.  On a 20 000-star field such an evaluation took one warp
+   0.29 ms, and the two items whose roots left the box one after another ran
+   334 and 404 ms, ten times the rest of the launch.  Warp 0 runs the tracker
+   on its lane 0; the other warps wait for points to sum (FarShared, the
+   barriers of far_sums_begin / far_sums_end), while warp 0 forms the
+   smooth-mass series. */
+constexpr int FAR_MAX_WARPS = 8;
+/* From this many stars on a root that leaves the box within an item goes to
+   the far launch that follows the items; below, one off-box evaluation by its
+   item's warp is short enough (64 star pairs a lane) to be done there, and the
+   launch that would only begin after the items costs more.  When rows are
+   tracked again, their off-box roots sit in the items from the start, and all
+   of them go to that launch. */
+constexpr int FAR_EVICT_STARS = 4096;
+
+struct FarShared
+{
+	double2 z;                       /* the point whose stars are summed */
+	int go;                          /* 0: the helpers leave */
+	double red[FAR_MAX_WARPS][6];    /* each warp's share: s1, s2, s3 */
+};
+
+/* a warp's share of the direct star sums at z: star pairs first, first + stride, ...
+   (a pair: stars p and p + pairs); the sums go to out[6] */
+template <bool MIXED>
+__device__ __noinline__ void far_share(const FieldView& F, double2 z, int first, int stride, double* out)
+{
+	const unsigned full = 0xffffffffu;
+	const int lane = threadIdx.x & 31;
+	const int N = F.num_stars, pairs = (N + 1) >> 1;
+	if constexpr (MIXED)
+	{
+		const dfc zd = dfc_from(z);
+		const dfp zx = dfp_make(zd.re, zd.re), zy = dfp_make(zd.im, zd.im);
+		dfp s1x = {0, 0}, s1y = s1x, s2x = s1x, s2y = s1x;
+		pk s3x = 0, s3y = 0;
+		/* the next pair is loaded while this one's terms are formed; without a
+		   second star: the last one again, with mass 0 */
+		float4 na = F.star_df[min(first, N - 1)], nb = F.star_df[min(first + pairs, N - 1)];
+		float2 nma = F.star_mass_df[min(first, N - 1)], nmb = F.star_mass_df[min(first + pairs, N - 1)];
+#pragma unroll 1
+		for (int p = first; p < pairs; p += stride)
+		{
+			const float4 a = na, b = nb;
+			const float2 ma = nma, mb = p + pairs < N ? nmb : make_float2(0.f, 0.f);
+			const int pn = min(p + stride, N - 1), qn = min(p + stride + pairs, N - 1);
+			na = F.star_df[pn];
+			nb = F.star_df[qn];
+			nma = F.star_mass_df[pn];
+			nmb = F.star_mass_df[qn];
+			const dfp m = {pk_make(ma.x, mb.x), pk_make(ma.y, mb.y)};
+			const dfp dx = dfp_sub(zx, {pk_make(a.x, b.x), pk_make(a.z, b.z)});
+			const dfp dy = dfp_sub(zy, {pk_make(a.y, b.y), pk_make(a.w, b.w)});
+			const dfp r = dfp_rcp(dfp_sumsq(dx, dy));
+			const dfp jx = dfp_mul(dx, r), jy = dfp_mul(dy, r);
+			const dfp kx = dfp_diffsq(jx, jy), ky = dfp_mul(jx, jy);
+			dfp_acc_fma(s2x, m, kx);
+			dfp_acc_fma(s2y, m, ky);
+			dfp_acc_fma(s1x, m, jx);
+			dfp_acc_fma(s1y, m, jy);
+			const pk t = pk_add(ky.hi, ky.hi);
+			s3x = pk_fma(m.hi, pk_fma(pk_neg(t), jy.hi, pk_mul(kx.hi, jx.hi)), s3x);
+			s3y = pk_fma(m.hi, pk_fma(t, jx.hi, pk_mul(kx.hi, jy.hi)), s3y);
+		}
+		/* signs and the factor 2 as in track_sums_pk */
+		dfl w[4] = {dfp_acc_total(s1x), df_neg(dfp_acc_total(s1y)), dfp_acc_total(s2x), dfp_acc_total(s2y)};
+		w[3] = {-2.f * w[3].hi, -2.f * w[3].lo};
+		float2 s3 = make_float2(pk_lo(s3x) + pk_hi(s3x), -(pk_lo(s3y) + pk_hi(s3y)));
+#pragma unroll 1
+		for (int o = 16; o > 0; o >>= 1)
+		{
+#pragma unroll
+			for (int c = 0; c < 4; c++)
+			{
+				const dfl u = {__shfl_xor_sync(full, w[c].hi, o), __shfl_xor_sync(full, w[c].lo, o)};
+				w[c] = df_add(w[c], u);
+			}
+			s3.x += __shfl_xor_sync(full, s3.x, o);
+			s3.y += __shfl_xor_sync(full, s3.y, o);
+		}
+		if (lane == 0)
+		{
+#pragma unroll
+			for (int c = 0; c < 4; c++) out[c] = df_to_double(w[c]);
+			out[4] = s3.x;
+			out[5] = s3.y;
+		}
+	}
+	else
+	{
+		NearSums a = zero_sums();
+		for (int p = first; p < pairs; p += stride)
+		{
+			const double2 u = F.star_pos[p];
+			star_term<true, true>(a, z, u.x, u.y, F.star_mass[p]);
+			if (p + pairs < N)
+			{
+				const double2 v = F.star_pos[p + pairs];
+				star_term<true, true>(a, z, v.x, v.y, F.star_mass[p + pairs]);
+			}
+		}
+		double v[6] = {a.s1.x, a.s1.y, a.s2.x, a.s2.y, a.s3.x, a.s3.y};
+#pragma unroll
+		for (int c = 0; c < 6; c++)
+		{
+			for (int o = 16; o > 0; o >>= 1) v[c] += __shfl_xor_sync(full, v[c], o);
+			if (lane == 0) out[c] = v[c];
+		}
+	}
+}
+
+/* warps 1 .. of a far CTA: sum the stars at each point warp 0 posts */
+template <bool MIXED>
+__device__ void far_helper(const FieldView& F, FarShared& S)
+{
+	const int helpers = (blockDim.x >> 5) - 1, w = (threadIdx.x >> 5) - 1;
+	while (true)
+	{
+		__syncthreads();
+		if (!S.go) return;
+		far_share<MIXED>(F, S.z, w * 32 + (threadIdx.x & 31), helpers * 32, S.red[w]);
+		__syncthreads();
+	}
+}
+
+/* warp 0 posts the point z of its lane 0 (begin), and takes the sums (end);
+   between the two it is free while the helpers sum.  A CTA of one warp sums in
+   end.  All 32 lanes call both. */
+CCF_D void far_sums_begin(FarShared& S, double2 z)
+{
+	if (threadIdx.x == 0)
+	{
+		S.z = z;
+		S.go = 1;
+	}
+	__syncthreads();
+}
+template <bool MIXED>
+CCF_D NearSums far_sums_end(const FieldView& F, FarShared& S)
+{
+	const int warps = blockDim.x >> 5;
+	int shares = warps - 1;
+	if (warps == 1)
+	{
+		far_share<MIXED>(F, S.z, threadIdx.x & 31, 32, S.red[0]);
+		shares = 1;
+	}
+	__syncthreads();
+	/* lane c adds the shares' component c */
+	const unsigned full = 0xffffffffu;
+	const int c = min((int)(threadIdx.x & 31), 5);
+	double v = 0;
+	for (int w = 0; w < shares; w++) v += S.red[w][c];
+	NearSums n;
+	n.s1 = make_double2(__shfl_sync(full, v, 0), __shfl_sync(full, v, 1));
+	n.s2 = make_double2(__shfl_sync(full, v, 2), __shfl_sync(full, v, 3));
+	n.s3 = make_double2(__shfl_sync(full, v, 4), __shfl_sync(full, v, 5));
+	return n;
 }
 
 /* The FP64 smooth-mass series of the rectangular Taylor form at a point
@@ -964,19 +1127,31 @@ __device__ __noinline__ SmoothSeries smooth_series_warp(const FieldView& F, doub
 	return out;
 }
 
+/* |a| for the error bound, never below it: in FP32 (2^-20 above) where a's
+   square stays in the FP32 range, else in FP64 (an FP64 hypot is a chain of
+   ~30 instructions of 64 cycles) */
+CCF_D double bound_abs(double2 a)
+{
+	const double m = fmax(fabs(a.x), fabs(a.y));
+	if (m < 1e18 && m > 1e-18) return (double)(hypotf((float)a.x, (float)a.y) * (1.f + 0x1p-20f));
+	return hypot(a.x, a.y);
+}
+
 /* The iteration quantities of the tracker (TrackEval) for the warp's lanes
    with off set, which lie outside the root box: direct double-float sums over
-   every star, then f, f', the step and the whole lens map (wmode 2) in FP64
-   (far from the field the smooth-mass Taylor terms leave the FP32 range).
-   Kept out of line, as the rare path of the iteration.  All 32 lanes must
-   call it. */
+   every star (by the warp, one lane at a time; CTA: lane 0's by the CTA),
+   then f, f', the step and the whole lens map (wmode 2) in FP64 (far from the
+   field the smooth-mass Taylor terms leave the FP32 range).  Kept out of line,
+   as the rare path of the iteration.  All 32 lanes must call it. */
+template <bool CTA>
 __device__ __noinline__ TrackEval track_offfield(const FieldView& F, bool off, double2 z, double cphi, double sphi,
-	bool disc_exact, float wtol2)
+	bool disc_exact, float wtol2, FarShared* far)
 {
 	const unsigned full = 0xffffffffu;
 	const int lane = threadIdx.x & 31;
 	NearSums ns = zero_sums();
-	offfield_sums_warp_df<true, true>(F, off, z, ns);
+	if constexpr (CTA) far_sums_begin(*far, z);
+	else offfield_sums_warp_df<true, true>(F, off, z, ns);
 	/* the Taylor form's series outside the corner circle, warp-wide per point */
 	const bool series = F.rectangular && F.approx && F.smooth_m > 0 && !smooth_df_ok(F, z);
 	SmoothSeries sm;
@@ -989,6 +1164,7 @@ __device__ __noinline__ TrackEval track_offfield(const FieldView& F, bool off, d
 		const SmoothSeries t = smooth_series_warp(F, make_double2(__shfl_sync(full, z.x, src), __shfl_sync(full, z.y, src)));
 		if (lane == src) sm = t;
 	}
+	if constexpr (CTA) ns = far_sums_end<true>(F, *far);
 	TrackEval r;
 	r.step = make_float2(0.f, 0.f);
 	r.as2 = 0;
@@ -1016,9 +1192,9 @@ __device__ __noinline__ TrackEval track_offfield(const FieldView& F, bool off, d
 	r.as2 = as2 < 3e38 ? (float)as2 : INFINITY;   /* a step beyond the FP32 range fails */
 	r.fz = make_float2((float)f.x, (float)f.y);
 	const double2 fs = cmul(df, make_double2(r.step.x, r.step.y));
-	r.af = __double2float_ru(hypot(f.x - fs.x, f.y - fs.y) +
-		7.2e-15 * (F.theta2 * hypot(ns.s2.x, ns.s2.y) + hypot(ds.x, ds.y) + 1 + F.shear) +
-		1.2e-16 * hypot(z.x, z.y) * hypot(df.x, df.y));
+	r.af = __double2float_ru(bound_abs(make_double2(f.x - fs.x, f.y - fs.y)) +
+		7.2e-15 * (F.theta2 * bound_abs(ns.s2) + bound_abs(ds) + 1 + F.shear) +
+		1.2e-16 * bound_abs(z) * bound_abs(df));
 	/* the lens map only where the point can be final: a step below the
 	   tolerance, or a stalled root kept as it is */
 	if (r.as2 < wtol2)
@@ -1071,34 +1247,6 @@ CCF_D int item_row(const TrackArgs& T, int item)
 		else hi = mid - 1;
 	}
 	return lo;
-}
-
-/* Roots that start outside the root box evaluate f by direct sums over
-   every star, which the warp computes together, one such point at a time.  In
-   a warp of 32 tracked roots a few of them would multiply the cost of every
-   iteration of the other 31 and make their item the longest of the launch,
-   so each of these roots is tracked alone by a warp of its own (its lane 0;
-   the other lanes only help with the sums) and is left out of its item.
-   This kernel lists them (in no particular order: a root's results do not
-   depend on when or where it runs). */
-__global__ void track_mark_kernel(const TrackArgs T)
-{
-	const int item = blockIdx.x * blockDim.x + threadIdx.x;
-	if (item >= T.num_items) return;
-	const int row = item_row(T, item);
-	const RowDesc rd = T.rows[row];
-	const FieldView* F = T.fields + rd.field;
-	const int R = F->num_roots;
-	const double2 c = F->node_center[0];
-	const double h = F->node_half[0];
-	const int a0 = (item - T.item_start[row]) * 32;
-	for (int a = a0; a < min(a0 + 32, R); a++)
-	{
-		const double2 z = T.master[rd.base + a];
-		const bool off = fabs(z.x - c.x) > h || fabs(z.y - c.y) > h;
-		T.is_solo[rd.base + a] = off ? 1 : 0;
-		if (off) T.solo[atomicAdd(T.num_solo, 1)] = make_int2(row, a);
-	}
 }
 
 /* cos, sin of a sub-step position t that is no whole step (out of line) */
@@ -1173,50 +1321,86 @@ cudaError_t launch_phase_table(cudaStream_t s, int nb, int nphi, PhaseEntry* out
    the direct evaluation of the outputs (a warp-wide call).  Every lane of the
    warp stays in the loop to the end: the evaluation off the root box and
    the direct epilogue are warp-wide calls. */
-template <bool MIXED, bool PK>
-__global__ void __launch_bounds__(TNT, 3) track_kernel(const TrackArgs T)
+template <bool MIXED, bool PK, bool FAR>
+__global__ void __launch_bounds__(FAR ? 32 * FAR_MAX_WARPS : TNT, FAR ? 2 : 3) track_kernel(const TrackArgs T)
 {
-	__shared__ FieldView sF[TNT / 32];
-	__shared__ FieldOut sO[TNT / 32];
-	__shared__ RowDesc sR[TNT / 32];
-	__shared__ TrackConst sK[TNT / 32];
-	__shared__ double s_maxerr[TNT / 32];
-	__shared__ double2 s_hz[TRACK_HIST * TNT];   /* accepted positions of each lane's root (a ring per lane) */
+	constexpr int NL = FAR ? 32 : TNT;   /* tracking lanes of the CTA */
+	__shared__ FieldView sF[NL / 32];
+	__shared__ FieldOut sO[NL / 32];
+	__shared__ RowDesc sR[NL / 32];
+	__shared__ TrackConst sK[NL / 32];
+	__shared__ double s_maxerr[NL / 32];
+	__shared__ double2 s_hz[TRACK_HIST * NL];   /* accepted positions of each lane's root (a ring per lane) */
+	__shared__ FarShared s_far;                 /* (the far launch) */
 	const unsigned full = 0xffffffffu;
 	const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
 	double2* const hz = s_hz + threadIdx.x;
 
+	if constexpr (FAR)
+	{
+		if (w > 0)
+		{
+			far_helper<MIXED>(sF[0], s_far);
+			return;
+		}
+	}
+
 	while (true)
 	{
-		/* the solo roots first, then the items in order */
+		/* the far launch: the next listed root; else the next item in the queue's order */
 		int item = 0, solo_root = -1, row = 0;
-		if (lane == 0)
+		const FarState* resume = nullptr;
+		if constexpr (FAR)
 		{
-			const int q = T.items_per_row > 0 ? 0 : atomicAdd(&T.counter[0], 1);
-			if (T.items_per_row == 0 && q < *T.num_solo)
+			int q = 0;
+			if (lane == 0) q = atomicAdd(T.far_evicted ? T.evict_counter : &T.counter[0], 1);
+			q = __shfl_sync(full, q, 0);
+			if (q >= (T.far_evicted ? min(*T.num_evict, T.evict_cap) : *T.num_solo)) break;
+			if (T.far_evicted)
+			{
+				resume = T.evict + q;
+				row = resume->row;
+				solo_root = resume->root;
+			}
+			else
 			{
 				const int2 sr = T.solo[q];
 				row = sr.x;
 				solo_root = sr.y;
 			}
-			else
+		}
+		else
+		{
+			/* the solo roots first, when no far launch takes them */
+			if (T.items_per_row == 0 && !T.solo_far)
 			{
-				item = atomicAdd(&T.counter[1], 1);
+				int q = 0;
+				if (lane == 0) q = atomicAdd(&T.counter[0], 1);
+				q = __shfl_sync(full, q, 0);
+				if (q < *T.num_solo)
+				{
+					const int2 sr = T.solo[q];
+					row = sr.x;
+					solo_root = sr.y;
+				}
 			}
-		}
-		item = __shfl_sync(full, item, 0);
-		solo_root = __shfl_sync(full, solo_root, 0);
-		if (T.items_per_row > 0)
-		{
-			if (item >= *T.num_rows_dev * T.items_per_row) break;
-			row = item / T.items_per_row;
-		}
-		else if (solo_root < 0)
-		{
-			if (item >= T.num_items) break;
-			/* the queue's order of the items (track_item_order_kernel) */
-			if (T.item_order) item = T.item_order[item];
-			row = item_row(T, item);
+			if (solo_root < 0)
+			{
+				if (lane == 0) item = atomicAdd(&T.counter[1], 1);
+				item = __shfl_sync(full, item, 0);
+				if (T.items_per_row > 0)
+				{
+					if (item >= *T.num_rows_dev * T.items_per_row) break;
+					row = item / T.items_per_row;
+				}
+				else
+				{
+					if (item >= T.num_items) break;
+					/* the queue's order of the items (track_item_order_kernel) */
+					if (T.item_order) item = T.item_order[item];
+					row = item_row(T, item);
+				}
+			}
 		}
 		row = __shfl_sync(full, row, 0);
 		__syncwarp();
@@ -1265,6 +1449,7 @@ __global__ void __launch_bounds__(TNT, 3) track_kernel(const TrackArgs T)
 		int maxev = 0;
 
 		int j = j0;
+		if (FAR && resume) j = resume->j;
 		/* global step of step j and its output column (row_slots), kept as j
 		   advances: gp = the step's phase, column kk of branch bb */
 		int gp = row_global_step(nb, O.half, c, side, j);
@@ -1278,11 +1463,28 @@ __global__ void __launch_bounds__(TNT, 3) track_kernel(const TrackArgs T)
 		double2 z = z1;
 		double cp = 0, sp = 0;
 		dfl cpd = {0.f, 0.f}, spd = {0.f, 0.f};
-		track_phase(O, c, side, tt, gp, cp, sp, cpd, spd);
 		int it = 0, evs = 0;
 		real prev2 = 0;
 		bool lost = !valid;
 		bool refine = false;
+		if (FAR && resume)
+		{
+			/* a root handed over by its item: go on where it stopped */
+			const FarState& fs = *resume;
+			for (int k = 0; k < TRACK_HIST; k++) hz[k * NL] = fs.hz[k];
+			z = fs.z;
+			head = fs.head;
+			hn = fs.hn;
+			run = fs.run;
+			t0 = fs.t0;
+			t1 = fs.t1;
+			tt = fs.tt;
+			it = fs.it;
+			evs = fs.evs;
+			prev2 = (real)fs.prev2;
+			refine = fs.refine != 0;
+		}
+		track_phase(O, c, side, tt, gp, cp, sp, cpd, spd);
 		unsigned unconv = 0;
 		/* corrector iterations per (sub-)step target: the sweep cap of the
 		   step, at most TRACK_ITERS (4 TRACK_ITERS at the finest sub-step) */
@@ -1296,6 +1498,31 @@ __global__ void __launch_bounds__(TNT, 3) track_kernel(const TrackArgs T)
 			{
 				leaf = find_leaf_far(F, z);
 				if (leaf >= 0) in_leaf_box(F, leaf, z, rel);
+			}
+			if (!FAR && act && leaf < 0 && solo_root < 0 && !T.scales && (F.num_stars >= FAR_EVICT_STARS || T.items_per_row > 0))
+			{
+				/* the root left the root box: to the second far launch */
+				const int q = atomicAdd(T.num_evict, 1);
+				if (q < T.evict_cap)
+				{
+					FarState& fs = T.evict[q];
+					for (int k = 0; k < TRACK_HIST; k++) fs.hz[k] = hz[k * NL];
+					fs.z = z;
+					fs.prev2 = (double)prev2;
+					fs.row = row;
+					fs.root = a;
+					fs.head = head;
+					fs.hn = hn;
+					fs.run = run;
+					fs.t0 = t0;
+					fs.t1 = t1;
+					fs.j = j;
+					fs.tt = tt;
+					fs.it = it;
+					fs.evs = evs;
+					fs.refine = refine ? 1 : 0;
+					act = false;
+				}
 			}
 			const bool off = act && leaf < 0;
 			double2 step = make_double2(0, 0);
@@ -1312,7 +1539,7 @@ __global__ void __launch_bounds__(TNT, 3) track_kernel(const TrackArgs T)
 				if (act && leaf >= 0) e = eval_track_df<PK>(F, K, leaf, z, rel, cpd, spd, disc_exact);
 				if (__any_sync(full, off))
 				{
-					const TrackEval o = track_offfield(F, off, z, cp, sp, disc_exact, (float)stuck2);
+					const TrackEval o = track_offfield<FAR && PK>(F, off, z, cp, sp, disc_exact, (float)stuck2, &s_far);
 					if (off) e = o;
 				}
 				step = make_double2((double)e.step.x, (double)e.step.y);
@@ -1320,7 +1547,14 @@ __global__ void __launch_bounds__(TNT, 3) track_kernel(const TrackArgs T)
 			}
 			else
 			{
-				const FdF g = eval_fdf_warp<false>(F, act, z, leaf, false, zero_sums(), cp, sp);
+				NearSums fsum = zero_sums();
+				const bool far_pt = FAR && !T.scales && __any_sync(full, off);
+				if (far_pt)
+				{
+					far_sums_begin(s_far, z);
+					fsum = far_sums_end<false>(F, s_far);
+				}
+				const FdF g = eval_fdf_warp<false>(F, act, z, leaf, far_pt && off, fsum, cp, sp);
 				if (act)
 				{
 					double2 S = near_pole_sum(F, leaf, z);
@@ -1394,7 +1628,7 @@ __global__ void __launch_bounds__(TNT, 3) track_kernel(const TrackArgs T)
 					run = dist == TSUB ? min(run + 1, TRACK_HIST - 1) : 0;
 					t0 = t1;
 					t1 = tt;
-					hz[head * TNT] = z;
+					hz[head * NL] = z;
 					refine = false;
 					if (tt == j * TSUB)
 					{
@@ -1539,7 +1773,7 @@ __global__ void __launch_bounds__(TNT, 3) track_kernel(const TrackArgs T)
 				{
 					/* next target: predict, restart the corrector */
 					tt = tn;
-					z = track_predict(hz, head, hn, tt - t1 == TSUB && run >= hn - 1, t0, t1, tt);
+					z = track_predict<NL>(hz, head, hn, tt - t1 == TSUB && run >= hn - 1, t0, t1, tt);
 					it = 0;
 					prev2 = 0;
 					track_phase(O, c, side, tt, gp, cp, sp, cpd, spd);
@@ -1556,8 +1790,15 @@ __global__ void __launch_bounds__(TNT, 3) track_kernel(const TrackArgs T)
 					double2 r2;
 					leafo = (leaf >= 0 && in_leaf_box(F, leaf, zf, r2)) ? leaf : find_leaf(F, zf);
 				}
-				if (!point_epilogue_warp<MIXED>(F, O, emit_direct, zf, leafo, false, zero_sums(), out, out2, ecp, esp, &s_maxerr[w],
-						stuck))
+				NearSums fsum = zero_sums();
+				const bool far_pt = FAR && !MIXED && !T.scales && __any_sync(full, emit_direct && leafo < 0);
+				if (far_pt)
+				{
+					far_sums_begin(s_far, zf);
+					fsum = far_sums_end<false>(F, s_far);
+				}
+				if (!point_epilogue_warp<MIXED>(F, O, emit_direct, zf, leafo, far_pt && leafo < 0, fsum, out, out2, ecp, esp,
+						&s_maxerr[w], stuck))
 					flags |= (unsigned)TRACK_NONFINITE;
 			}
 		}
@@ -1579,6 +1820,12 @@ __global__ void __launch_bounds__(TNT, 3) track_kernel(const TrackArgs T)
 			atomicAdd(&O.stats[2], nev);
 			if (nhalf) atomicAdd(&O.stats[10], nhalf);
 		}
+		__syncwarp();
+	}
+	if constexpr (FAR)
+	{
+		if (lane == 0) s_far.go = 0;
+		__syncthreads();   /* the helpers leave */
 	}
 }
 
@@ -1616,21 +1863,58 @@ __global__ void collect_rerun_kernel(const TrackArgs T, RowDesc* rerun, int* cou
 	}
 }
 
-/* The queue order of the tracker's work items: by the smallest |f'| of
-   their roots at the branch centre, smallest first, in TRACK_ORDER_CLASSES
-   classes of |f'| theta_star (below 0.03, 0.1, 0.3, 1, 3, and the rest).
-   Roots with a small |f'| move fast along the curve (dz/dphi = i a e^{-i phi}
-   / f'), where the predictor misses the 1e-9 theta_star tolerance and the
-   corrector takes a second evaluation at most steps; their items run
-   longer.  A launch of persistent warps ends one item after its queue
-   empties (on the bench field the SMs idled 20 % of the launch), so the long
-   items go first and the launch ends on short ones.  The items keep their
-   roots; only the order changes, and with it nothing in the results.
-   Class: one warp per item, a lane per root (solo roots do not run in their
-   item); order: one CTA, a stable counting sort by block scans. */
-constexpr int TRACK_ORDER_CLASSES = 6;
+/* Before the tracking, one lane per root at its branch centre:
 
-__global__ void track_item_flag_kernel(const TrackArgs T, int* cls)
+   Solo roots.  A root off the root box evaluates f by direct sums over every
+   star; in a warp of 32 tracked roots it would multiply the cost of every
+   iteration of the other 31, so the roots that start off the box are left out
+   of their items and tracked alone; with them, where a root that leaves the box
+   goes to the far launch (FAR_EVICT_STARS), the roots near the box's side that
+   leave it on the way, as far as TRACK_EXIT_STEPS Euler steps along
+   dz/dphi = -i a e^{-i phi} / f' tell, so that they run beside the items
+   instead of after them.  They are listed in no particular order: a root's
+   results do not depend on when or where it runs.
+
+   Classes.  The queue takes the work items by the smallest |f'| of their
+   roots, smallest first, in TRACK_ORDER_CLASSES classes of |f'| theta_star
+   (below 0.03, 0.1, 0.3, 1, 3, and the rest).  Roots with a small |f'| move
+   fast along the curve, where the predictor misses the 1e-9 theta_star
+   tolerance and the corrector takes a second evaluation at most steps; their
+   items run longer.  A launch of persistent warps ends one item after its
+   queue empties (on the bench field the SMs idled 20 % of the launch), so the
+   long items go first and the launch ends on short ones.  The items keep
+   their roots; only the order changes, and with it nothing in the results.
+   (The order itself: one CTA, a stable counting sort by block scans.) */
+constexpr int TRACK_ORDER_CLASSES = 6;
+constexpr double TRACK_EXIT_RIM = 0.2;   /* half-lengths: only a root this near the box's side is asked ... */
+constexpr float TRACK_EXIT_SLOW = 3;     /* ... and whose slope at the centre times this would carry it out */
+constexpr int TRACK_EXIT_STEPS = 4;
+
+/* does the root z (at the centre of row rd, f' = d there) leave the root box on its row? */
+__device__ __noinline__ bool track_leaves_box(const FieldView& F, const FieldOut& O, const RowDesc& rd, double2 z, float2 d)
+{
+	const double2 bc = F.node_center[0];
+	const double h = F.node_half[0];
+	const float dphi = (float)(2 * PI / O.nphi) * (rd.side ? rd.steps : -rd.steps);
+	const float a = (float)(1 - F.kappa_tot + F.kappa_star) * dphi;
+	const float phi = (float)(PI / O.nb + rd.branch * 2 * PI / O.nb);
+	for (int m = 0; m < TRACK_EXIT_STEPS; m++)
+	{
+		float sp, cp;
+		sincosf(phi + dphi * m / TRACK_EXIT_STEPS, &sp, &cp);
+		/* -i a e^{-i phi} = a (-sin phi, -cos phi) */
+		const float2 v = fdivc(make_float2(-a * sp, -a * cp), d);
+		if (m == 0 && fabs(z.x - bc.x) + TRACK_EXIT_SLOW * fabsf(v.x) <= h && fabs(z.y - bc.y) + TRACK_EXIT_SLOW * fabsf(v.y) <= h)
+			return false;
+		z.x += v.x / TRACK_EXIT_STEPS;
+		z.y += v.y / TRACK_EXIT_STEPS;
+		if (!(fabs(z.x - bc.x) <= h && fabs(z.y - bc.y) <= h)) return true;
+		if (m + 1 < TRACK_EXIT_STEPS) d = eval_df32(F, find_leaf(F, z), z, make_double2(0, 0));
+	}
+	return false;
+}
+
+__global__ void track_mark_kernel(const TrackArgs T, int* cls)
 {
 	const int item = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
 	const int lane = threadIdx.x & 31;
@@ -1640,15 +1924,26 @@ __global__ void track_item_flag_kernel(const TrackArgs T, int* cls)
 	const FieldView& F = T.fields[rd.field];
 	const int a = (item - T.item_start[row]) * 32 + lane;
 	int c = TRACK_ORDER_CLASSES - 1;
-	if (a < F.num_roots && !T.is_solo[rd.base + a])
+	if (a < F.num_roots)
 	{
 		const double2 z = T.master[rd.base + a];
-		const int leaf = find_leaf(F, z);
+		const double2 bc = F.node_center[0];
+		const double h = F.node_half[0];
+		bool solo = fabs(z.x - bc.x) > h || fabs(z.y - bc.y) > h;
+		const int leaf = solo ? -1 : find_leaf(F, z);
 		if (leaf >= 0)
 		{
 			const float2 d = eval_df32(F, leaf, z, make_double2(0, 0));
 			const float x = hypotf(d.x, d.y) * (float)F.theta;
+			if (F.num_stars >= FAR_EVICT_STARS && fmax(fabs(z.x - bc.x), fabs(z.y - bc.y)) > (1 - TRACK_EXIT_RIM) * h)
+				solo = track_leaves_box(F, T.outs[rd.field], rd, z, d);
 			c = x < 0.03f ? 0 : x < 0.1f ? 1 : x < 0.3f ? 2 : x < 1.f ? 3 : x < 3.f ? 4 : 5;
+		}
+		T.is_solo[rd.base + a] = solo ? 1 : 0;
+		if (solo)
+		{
+			T.solo[atomicAdd(T.num_solo, 1)] = make_int2(row, a);
+			c = TRACK_ORDER_CLASSES - 1;   /* it does not run in its item */
 		}
 	}
 	c = (int)__reduce_min_sync(0xffffffffu, (unsigned)c);
@@ -1673,38 +1968,130 @@ __global__ void __launch_bounds__(1024) track_item_order_kernel(int n, const int
 cudaError_t launch_track_item_order(cudaStream_t s, const TrackArgs& a, int* work, int* order)
 {
 	if (a.num_items == 0) return cudaSuccess;
-	track_item_flag_kernel<<<(a.num_items + 3) / 4, 128, 0, s>>>(a, work);
 	track_item_order_kernel<<<1, 1024, 0, s>>>(a.num_items, work, work + a.num_items, work + 2 * (size_t)a.num_items, order);
 	return cudaGetLastError();
 }
 
-cudaError_t launch_track_mark(cudaStream_t s, const TrackArgs& a)
+cudaError_t launch_track_mark(cudaStream_t s, const TrackArgs& a, int* cls)
 {
 	if (a.num_items == 0) return cudaSuccess;
-	track_mark_kernel<<<(a.num_items + 127) / 128, 128, 0, s>>>(a);
+	track_mark_kernel<<<(a.num_items + 3) / 4, 128, 0, s>>>(a, cls);
 	return cudaGetLastError();
 }
 
-cudaError_t launch_track(cudaStream_t s, const TrackArgs& a, bool mixed)
+namespace
 {
-	if (a.num_items == 0) return cudaSuccess;
-	/* persistent warps: as many CTAs as are resident at once */
-	static int per_sm[2] = {0, 0};
-	int& n = per_sm[mixed ? 1 : 0];
+/* percent of the SM's shared memory and L1 that the tracker's launches set
+   aside as shared memory: 64 KiB hold the items' three CTAs and a far one; the
+   leaf records are read through the rest */
+constexpr int TRACK_CARVEOUT = 28;
+
+/* CTAs of the tracker that are resident on one SM at once (asked once per
+   form and CTA size) */
+template <bool MIXED, bool PK, bool FAR>
+int resident(int threads)
+{
+	static std::atomic<int> known[FAR_MAX_WARPS + 1];
+	int n = known[threads / 32].load(std::memory_order_relaxed);
 	if (n == 0)
 	{
-		if (mixed) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, track_kernel<true, true>, TNT, 0);
-		else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, track_kernel<false, false>, TNT, 0);
-		if (n < 1) n = 1;
+		/* one shared-memory split for both kinds of launch: an SM must be empty
+		   to change it, so with splits of their own the far launch and the items
+		   never shared one */
+		cudaFuncSetAttribute(track_kernel<MIXED, PK, FAR>, cudaFuncAttributePreferredSharedMemoryCarveout, TRACK_CARVEOUT);
+		cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, track_kernel<MIXED, PK, FAR>, threads, 0);
+		n = std::max(n, 1);
+		known[threads / 32].store(n, std::memory_order_relaxed);
 	}
+	return n;
+}
+
+/* Warps of a far CTA: all but one (or the only one) sum stars.  A star pair
+   takes a lane ~0.2 us and warp 0's own work on an evaluation (FP64) ~10 us,
+   so the stars are split until a lane has about 16 pairs. */
+int far_warps(int stars)
+{
+	return stars <= 1024 ? 1 : stars <= 2048 ? 3 : stars <= 4096 ? 5 : FAR_MAX_WARPS;
+}
+
+/* Whether the roots that start off the box go to a far launch, or to warps of
+   the item launch, one root each, before the items.  An evaluation of such a
+   root takes a warp 25 000 cycles and 7.5 per star, one of an item's 50 000
+   while the GPU is full; both walk the same steps.  Beside the items a far
+   launch takes a third of their registers (8.8 ms against 7.1 on the 2000-star
+   field, 744 such roots); it pays where one root by one warp would outlast the
+   items (the 20 000-star field: 92 ms against 35).  With length scales the
+   roots stay with the items, whose order of summation their far FP64 sums
+   show (1e-6 of a length scale). */
+bool solos_far(const TrackArgs& a, int sms)
+{
+	const double root = 1.15 * (25000 + 7.5 * a.max_stars);
+	const double items = 1.6 * 50000 * a.num_items / (double)(sms * TRACK_WARPS_PER_SM);
+	return !a.scales && a.max_stars >= FAR_EVICT_STARS && 2 * root > 0.5 * items;
+}
+
+template <bool MIXED, bool PK>
+cudaError_t launch_far(cudaStream_t s, const TrackArgs& a, int sms, int evicted)
+{
+	TrackArgs f = a;
+	f.far_evicted = evicted;
+	const int threads = 32 * far_warps(a.max_stars);
+	const long long most = evicted ? std::min<long long>(a.num_roots, a.evict_cap) : a.num_roots;
+	/* beside items that fill the GPU one CTA per SM, so that the items keep two
+	   thirds of the registers; else as many as are resident */
+	const bool beside = !evicted && a.num_items >= sms * TRACK_WARPS_PER_SM / 2;
+	const int blocks = (int)std::min<long long>((long long)sms * (beside ? 1 : resident<MIXED, PK, true>(threads)), most);
+	if (blocks > 0) track_kernel<MIXED, PK, true><<<blocks, threads, 0, s>>>(f);
+	return cudaGetLastError();
+}
+
+/* The far launch of the roots that start off the root box (solos_far; first
+   tracking only), on the side stream when there is one; the items; then the
+   far launch of the roots that left the box. */
+template <bool MIXED, bool PK>
+cudaError_t launch_track_form(cudaStream_t s, const TrackArgs& a, int sms, const TrackSide& side)
+{
+	cudaError_t e = cudaSuccess;
+	TrackArgs t = a;
+	const bool first = a.items_per_row == 0;
+	t.solo_far = first && solos_far(a, sms);
+	if (t.solo_far && side.side)
+	{
+		if ((e = cudaEventRecord(side.fork, s)) != cudaSuccess) return e;
+		if ((e = cudaStreamWaitEvent(side.side, side.fork, 0)) != cudaSuccess) return e;
+		if ((e = launch_far<MIXED, PK>(side.side, t, sms, 0)) != cudaSuccess) return e;
+		if ((e = cudaEventRecord(side.join, side.side)) != cudaSuccess) return e;
+	}
+	else if (t.solo_far && (e = launch_far<MIXED, PK>(s, t, sms, 0)) != cudaSuccess) return e;
+	/* persistent warps: as many CTAs as are resident at once, and no more than
+	   there is work for: the warps of a small launch otherwise race for it, and
+	   SMs whose warps all won share one FP64 pipe.  The solo roots are counted
+	   in (a 17-star rectangle has 36 of them and 6 items: 7.5 ms against 30 with
+	   the items' two CTAs), but not where the outputs are FP64 epilogues, which
+	   a CTA more per SM does not speed up (11.3 ms against 12.8 in FP64 on a
+	   600-star rectangle) */
+	const long long work = t.num_items + (first && !t.solo_far && PK ? t.solo_guess : 0);
+	const int blocks = (int)std::max<long long>(1, std::min<long long>(sms * resident<MIXED, PK, false>(TNT),
+		(work + TNT / 32 - 1) / (TNT / 32)));
+	track_kernel<MIXED, PK, false><<<blocks, TNT, 0, s>>>(t);
+	if ((e = cudaGetLastError()) != cudaSuccess) return e;
+	if (t.solo_far && side.side && (e = cudaStreamWaitEvent(s, side.join, 0)) != cudaSuccess) return e;
+	if (!a.scales && (!first || a.max_stars >= FAR_EVICT_STARS)) e = launch_far<MIXED, PK>(s, t, sms, 1);
+	return e;
+}
+}
+
+cudaError_t launch_track(cudaStream_t s, const TrackArgs& a, bool mixed, const TrackSide& side)
+{
+	if (a.num_items == 0) return cudaSuccess;
 	int dev = 0, sms = 0;
 	cudaGetDevice(&dev);
 	cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-	const int blocks = std::max(1, std::min(sms * n, (a.num_items + TNT / 32 - 1) / (TNT / 32)));
-	if (!mixed) track_kernel<false, false><<<blocks, TNT, 0, s>>>(a);
-	else if (a.scales) track_kernel<true, false><<<blocks, TNT, 0, s>>>(a);
-	else track_kernel<true, true><<<blocks, TNT, 0, s>>>(a);
-	return cudaGetLastError();
+	if (!mixed) return launch_track_form<false, false>(s, a, sms, side);
+	/* length scales: the scalar evaluator (the packed one's other rounding, 1e-14
+	   in a root, becomes 4e-8 in a length scale next to a cusp) */
+	if (a.scales) return launch_track_form<true, false>(s, a, sms, side);
+	return launch_track_form<true, true>(s, a, sms, side);
 }
 
 /* zeroes the column tables of the rows to re-track (a device-side list) */

@@ -312,7 +312,7 @@ ccf_status Engine::solve_chunked(Field& f, int verbose)
 		CCF_TRY_S(P.row_stats2.ensure(TRACK_ROW_STATS * grows), "cudaMalloc(rows)");
 		CCF_TRY_S(P.rows_rerun.ensure(grows), "cudaMalloc(rows)");
 		CCF_TRY_S(P.rows_rerun2.ensure(grows), "cudaMalloc(rows)");
-		CCF_TRY_S(P.rerun_count.ensure(6), "cudaMalloc(rows)");
+		CCF_TRY_S(P.rerun_count.ensure(10), "cudaMalloc(rows)");
 		CCF_TRY_S(P.item_start.ensure(rc.size()), "cudaMalloc(rows)");
 		CCF_TRY_S(P.solo.ensure((size_t)ncont + 1), "cudaMalloc(rows)");
 		CCF_TRY_S(P.is_solo.ensure((size_t)ncont), "cudaMalloc(rows)");
@@ -434,10 +434,11 @@ ccf_status Engine::solve_chunked(Field& f, int verbose)
 			T.solo = P.solo.ptr;
 			T.num_solo = reinterpret_cast<int*>(P.solo.ptr + ncont);
 			T.is_solo = P.is_solo.ptr;
+			CCF_TRY_S(far_setup(T, (long long)grows * R, (long long)grows * (R - 2 * f.d.num_stars), f.d.num_stars), "cudaMalloc(far roots)");
 			CCF_TRY_S(cudaMemsetAsync(T.num_solo, 0, sizeof(int), s), "memset");
 			CCF_TRY_S(cudaMemsetAsync(P.track_table.ptr, 0, gr.table_slots * sizeof(unsigned long long), s), "memset");
 			CCF_TRY_S(cudaMemsetAsync(P.row_stats.ptr, 0, TRACK_ROW_STATS * grows * sizeof(unsigned long long), s), "memset");
-			CCF_TRY_S(cudaMemsetAsync(P.rerun_count.ptr, 0, 6 * sizeof(int), s), "memset");
+			CCF_TRY_S(cudaMemsetAsync(P.rerun_count.ptr, 0, 10 * sizeof(int), s), "memset");
 			CCF_TRY_S(cudaMemsetAsync(P.row_stats2.ptr, 0, TRACK_ROW_STATS * grows * sizeof(unsigned long long), s), "memset");
 			CCF_TRY_S(P.item_order.ensure((size_t)T.num_items + 1), "cudaMalloc(items)");
 			CCF_TRY_S(P.item_work.ensure(3 * (size_t)T.num_items + 3), "cudaMalloc(items)");
@@ -446,9 +447,9 @@ ccf_status Engine::solve_chunked(Field& f, int verbose)
 			const bool reorder = (long long)T.num_items < 32LL * num_sms * TRACK_WARPS_PER_SM;
 			if (reorder) reordered_groups++;
 			T.item_order = reorder ? P.item_order.ptr : nullptr;
-			CCF_TRY_S(launch_track_mark(s, T), "track_mark");
+			CCF_TRY_S(launch_track_mark(s, T, P.item_work.ptr), "track_mark");
 			if (reorder) CCF_TRY_S(launch_track_item_order(s, T, P.item_work.ptr, P.item_order.ptr), "track_item_order");
-			CCF_TRY_S(launch_track(s, T, mixed), "track_ccs");
+			CCF_TRY_S(launch_track(s, T, mixed, side), "track_ccs");
 			CCF_TRY_S(launch_track_check(s, T, (long long)R * seg * half), "track_check");
 			CCF_TRY_S(launch_collect_rerun(s, T, P.rows_rerun.ptr, P.rerun_count.ptr), "collect_rerun");
 			TrackArgs T2 = T;
@@ -460,8 +461,9 @@ ccf_status Engine::solve_chunked(Field& f, int verbose)
 			T2.max_sub = TRACK_TSUB / TRACK_FINE_SUB;
 			T2.row_stats = P.row_stats2.ptr;
 			T2.counter = P.rerun_count.ptr + 4;
+			far_counts(T2);
 			CCF_TRY_S(launch_clear_tables(s, T2), "clear_tables");
-			CCF_TRY_S(launch_track(s, T2, mixed), "track_ccs_fine");
+			CCF_TRY_S(launch_track(s, T2, mixed, side), "track_ccs_fine");
 			CCF_TRY_S(launch_track_check(s, T2, (long long)R * seg * half), "track_check");
 			CCF_TRY_S(launch_collect_rerun(s, T2, P.rows_rerun2.ptr, P.rerun_count.ptr + 3), "collect_rerun");
 			A.rows = P.rows_rerun2.ptr;
@@ -500,11 +502,11 @@ ccf_status Engine::solve_chunked(Field& f, int verbose)
 	CCF_TRY_S(cudaEventRecord(f.ev[5], s), "event");
 	CCF_TRY_S(cudaStreamSynchronize(s), "solver");
 	/* seeds, (phase table), initial solve, its polish (2); per group the
-	   tracker's 8 launches (marking, tracking, column check, collection,
-	   table clearing, re-tracking, column check, collection) and the full-sum
+	   tracker's 11 launches (marking, tracking in three, column check, collection,
+	   table clearing, re-tracking in two, column check, collection) and the full-sum
 	   launch, or the full-sum launch alone, then the polish (2); and the item
-	   order's 2 where a group reorders its items */
-	return finish_stats(f, seg, track, verbose, (track ? 5 : 4) + (track ? 11 : 3) * ngroups + 2 * reordered_groups);
+	   order where a group reorders its items */
+	return finish_stats(f, seg, track, verbose, (track ? 5 : 4) + (track ? 14 : 3) * ngroups + reordered_groups);
 }
 
 } /* namespace ccf */

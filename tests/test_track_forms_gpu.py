@@ -39,3 +39,20 @@ def test_packed_evaluator_finds_the_full_sum_zeros(n, rectangular):
         assert d["non_finite"] == 0 and d["non_bijective_cols"] == 0
         assert d["max_dist"] <= 1e-11
     assert np.max(t["errs"]) <= 1e-9
+
+
+@pytest.mark.parametrize("n, rectangular, num_phi, nb", [
+    (4096, 1, 32, 2),     # the far launch from its smallest field on, roots that leave the box among the items
+    (4501, 1, 24, 1),     # an odd number of stars, long rows
+    (4501, 0, 24, 1),     # a disc: few roots off the box
+    (150, 1, 24, 2),      # coarse steps: rows tracked again, their off-box roots handed over
+    (17, 1, 40, 1),       # more solo roots than items
+])
+def test_roots_off_the_box_find_the_full_sum_zeros(n, rectangular, num_phi, nb):
+    cfg = dict(kappa_tot=0.45, kappa_star=0.4, shear=0.3, mass_function="equal", rectangular=rectangular, num_stars=n,
+               num_phi=num_phi, num_branches=nb, random_seed=7 + n)
+    t = run(cfg)
+    a = run(cfg, continuation="aberth")
+    d = O.match_sets(t["ccs"], a["ccs"], nb)
+    assert d["non_finite"] == 0 and d["non_bijective_cols"] == 0
+    assert d["max_dist"] <= 1e-11
