@@ -136,6 +136,54 @@ Engine::~Engine()
 	}
 }
 
+/* device memory for the partial sums of the rows a launch_rows works on at
+   once: a 40 060-root row takes 41 MB, one of the 2000-star field 1.6 MB */
+constexpr long long PARTIAL_BYTES = 256LL << 20;
+
+ccf_status Engine::rows_setup(SolveArgs& A, int which, const std::vector<Field*>& fields, bool mixed, const int rows[2],
+	const int cluster[2])
+{
+	SolverPools& P = pools;
+	cudaStream_t s = stream;
+	/* sized for both launches at once: a buffer that grew between them would go
+	   back to the cache under the first */
+	long long stride[2] = {0, 0}, slots[2], part_bytes = 0, most_slots = 0;
+	int bytes = 0, maxR = 0;
+	for (const Field* f : fields) maxR = std::max(maxR, f->d.num_roots);
+	for (int k = 0; k < 2; k++)
+	{
+		for (const Field* f : fields)
+		{
+			long long n = 0;
+			bytes = rows_partials(f->d.num_roots, f->d.num_stars, cluster[k], mixed, &n);
+			stride[k] = std::max(stride[k], n);
+		}
+		slots[k] = std::max<long long>(1, std::min<long long>(rows[k], PARTIAL_BYTES / (stride[k] * bytes)));
+		part_bytes = std::max(part_bytes, slots[k] * stride[k] * bytes);
+		most_slots = std::max(most_slots, slots[k]);
+	}
+	CCF_TRY(P.row_state.ensure((size_t)rows[0] + rows[1]), "cudaMalloc(rows)");
+	CCF_TRY(P.row_control.ensure(4), "cudaMalloc(rows)");
+	CCF_TRY(P.row_part.ensure((size_t)part_bytes), "cudaMalloc(rows)");
+	/* a unit's share is 256 roots; the blocks of a row's segments may end short */
+	const long long units = maxR / 256 + 17;
+	CCF_TRY(P.row_share.ensure((size_t)(most_slots * units * 256)), "cudaMalloc(rows)");
+	CCF_TRY(P.row_counts.ensure((size_t)(most_slots * units)), "cudaMalloc(rows)");
+	A.share = P.row_share.ptr;
+	A.counts = P.row_counts.ptr;
+	A.share_stride = units * 256;
+	A.counts_stride = units;
+	A.cluster = cluster[which];
+	A.state = P.row_state.ptr + (which ? rows[0] : 0);
+	A.control = P.row_control.ptr + 2 * which;
+	A.part = P.row_part.ptr;
+	A.part_slots = (int)slots[which];
+	A.part_stride = stride[which];
+	CCF_TRY(cudaMemsetAsync(A.state, 0, (size_t)rows[which] * sizeof(RowState), s), "memset");
+	CCF_TRY(cudaMemsetAsync(A.control, 0, 2 * sizeof(int), s), "memset");
+	return CCF_OK;
+}
+
 /* room for the roots that leave the box: a few per row do (20 of 160 000 on
    the 20 000-star field); those beyond it stay in their items */
 constexpr int FAR_EVICT_CAP = 8192;
@@ -1084,20 +1132,25 @@ ccf_status Engine::solve(std::vector<Field*>& fields, int verbose)
 	if (verbose >= 1) std::cout << "Finding initial roots...\n";
 	A.rows = P.rows_init.ptr;
 	A.num_rows = (int)ri.size();
-	A.cluster = init_cluster > 0 ? init_cluster : pick_cluster(A.num_rows);
-	for (Field* f : fields) f->info.init_cluster = A.cluster;
+	/* the initial solve's and the continuation's rows, and the CTAs per row whose
+	   order of summation they keep */
+	const int solver_rows[2] = {(int)ri.size(), (int)rc.size()};
+	const int solver_cluster[2] = {init_cluster > 0 ? init_cluster : pick_cluster(solver_rows[0]), pick_cluster(solver_rows[1])};
+	for (Field* f : fields) f->info.init_cluster = solver_cluster[0];
 	A.master = P.master_init.ptr;
 	A.snap32 = mixed ? P.snap32_init.ptr : nullptr;
 	A.snap64 = mixed ? nullptr : P.snap64_init.ptr;
 	A.fin = P.fin_init.ptr;
 	A.list = P.list_init.ptr;
 	A.fval = P.fval_init.ptr;
-	CCF_TRY(launch_solve(s, A, mixed, true), "find_initial_roots");
+	int max_stars = 0;
+	for (Field* f : fields) max_stars = std::max(max_stars, f->d.num_stars);
+	if (ccf_status rs = rows_setup(A, 0, fields, mixed, solver_rows, solver_cluster); rs != CCF_OK) return rs;
+	CCF_TRY(launch_rows(s, A, mixed, true, num_sms, maxR, max_stars), "find_initial_roots");
 	for (Field* f : fields) CCF_TRY(cudaEventRecord(f->ev[4], s), "event");
 	if (verbose >= 1) std::cout << "Finding critical curve positions...\n";
 	A.rows = P.rows_cont.ptr;
 	A.num_rows = (int)rc.size();
-	A.cluster = pick_cluster(A.num_rows);
 	A.master = P.master_cont.ptr;
 	A.snap32 = mixed ? P.snap32_cont.ptr : nullptr;
 	A.snap64 = mixed ? nullptr : P.snap64_cont.ptr;
@@ -1139,8 +1192,6 @@ ccf_status Engine::solve(std::vector<Field*>& fields, int verbose)
 		T.solo = P.solo.ptr;
 		T.num_solo = reinterpret_cast<int*>(P.solo.ptr + ncont);
 		T.is_solo = P.is_solo.ptr;
-		int max_stars = 0;
-		for (Field* f : fields) max_stars = std::max(max_stars, f->d.num_stars);
 		long long smooth_roots = 0;
 		for (const RowDesc& r : rc) smooth_roots += fields[r.field]->d.num_roots - 2 * fields[r.field]->d.num_stars;
 		CCF_TRY(far_setup(T, ncont, smooth_roots, max_stars), "cudaMalloc(far roots)");
@@ -1181,7 +1232,8 @@ ccf_status Engine::solve(std::vector<Field*>& fields, int verbose)
 		A.rows = P.rows_rerun2.ptr;
 		A.num_rows_dev = P.rerun_count.ptr + 3;
 	}
-	CCF_TRY(launch_solve(s, A, mixed, false), "find_ccs");
+	if (ccf_status rs = rows_setup(A, 1, fields, mixed, solver_rows, solver_cluster); rs != CCF_OK) return rs;
+	CCF_TRY(launch_rows(s, A, mixed, false, num_sms, maxR, max_stars), "find_ccs");
 	/* FP64 polish of the points above the 1/mu target or left unconverged;
 	   it also forms the largest 1/mu error and the non-finite flag */
 	{

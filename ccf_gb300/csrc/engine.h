@@ -201,6 +201,10 @@ struct SolverPools
 	DBuf<float4> snap32_init, snap32_cont;
 	DBuf<unsigned char> fin_init, fin_cont;
 	DBuf<int> list_init, list_cont;
+	DBuf<RowState> row_state;               /* rows.cu: the rows' states, then of the continuation's */
+	DBuf<int> row_control;                  /* and their counters, two per launch */
+	DBuf<unsigned char> row_part;           /* the partial sums of the rows at work, */
+	DBuf<int> row_share, row_counts;        /* and the shares of their next lists */
 	DBuf<double2> fval_init, fval_cont;   /* f, f' per root */
 	DBuf<RowDesc> rows_init, rows_cont, rows_rerun, rows_rerun2;
 	DBuf<unsigned long long> track_table;   /* column tables of the tracker */
@@ -309,6 +313,10 @@ public:
 	bool ensure_device(int dev);
 
 private:
+	/* the cluster, row states and partial sums of a launch_rows into A (which: 0
+	   the initial solve, 1 the continuation; rows, cluster: both launches') */
+	ccf_status rows_setup(SolveArgs& A, int which, const std::vector<Field*>& fields, bool mixed, const int rows[2],
+		const int cluster[2]);
 	/* the device buffers and counts of the tracker's far launches into T (the
 	   first tracking; T2 takes its counts from far_counts); roots = all rows',
 	   smooth = those of them beyond two per star (the Taylor form's), of which

@@ -200,6 +200,18 @@ CCF_HD int row_global_step(int nb, int half, int c, int side, int j)
 	return ((P % nphi) + nphi) % nphi;
 }
 
+/* rows.cu: where a row of the full-sum solver stands */
+struct RowState
+{
+	unsigned long long ticket;   /* units of the open phase, next unit */
+	int done;                    /* units of the phase that are finished */
+	int phase, it, j;
+	int total, late;             /* roots of the sweep's list: active; made final by its check */
+	int split, tpt, chunks, tiles;   /* the shape of its sums */
+	int complete;
+	int pad[3];
+};
+
 struct SolveArgs
 {
 	const FieldView* fields;
@@ -216,6 +228,15 @@ struct SolveArgs
 	const float4* const* star_hilo;   /* per field, FP32 hi/lo stars (mixed) */
 	int* error;
 	const int* num_rows_dev;   /* when set, the rows to run are rows[0 .. *num_rows_dev), at most num_rows */
+	/* rows.cu */
+	RowState* state;       /* [num_rows], zeroed before the launch */
+	int* control;          /* next row to start, rows complete; zeroed before the launch */
+	void* part;            /* partial sums: part_slots rows of part_stride elements */
+	int part_slots;
+	long long part_stride;
+	int* share;            /* the units' shares of the next list, share_stride a slot */
+	int* counts;           /* and their lengths, counts_stride a slot */
+	long long share_stride, counts_stride;
 };
 
 /* Per-root tracking of the continuation rows (solver.cu, track_kernel).
@@ -439,6 +460,11 @@ void launch_fold_smooth(cudaStream_t s, int num_leaves, int P, const double2* le
 /* solver.cu */
 int solver_blocks_per_sm(bool mixed);
 cudaError_t launch_solve(cudaStream_t s, const SolveArgs& a, bool mixed, bool initial);
+/* rows.cu: launch_solve with every row spread over the GPU; cluster then only
+   sets the order of summation.  rows_partials: the elements of one row's
+   partial sums, and the bytes of one */
+int rows_partials(int R, int N, int cluster, bool mixed, long long* elements);
+cudaError_t launch_rows(cudaStream_t s, const SolveArgs& a, bool mixed, bool initial, int num_sms, int max_roots, int max_stars);
 cudaError_t launch_track_mark(cudaStream_t s, const TrackArgs& a, int* cls);
 cudaError_t launch_track_item_order(cudaStream_t s, const TrackArgs& a, int* work, int* order);
 constexpr int TRACK_WARPS_PER_SM = 12;   /* resident tracker warps per SM (3 CTAs of 4 warps) */

@@ -367,20 +367,24 @@ ccf_status Engine::solve_chunked(Field& f, int verbose)
 	A.error = P.error.ptr;
 	A.rows = P.rows_init.ptr;
 	A.num_rows = K;
-	{
+	auto pick_cluster = [&](int rows) {
 		const int slots = num_sms * slots_per_sm;
 		int cl = 1;
-		while (cl < 16 && (long long)K * cl * 2 <= slots && R / (cl * 2) >= 256) cl *= 2;
-		A.cluster = p.init_cluster > 0 ? p.init_cluster : cl;
-		f.info.init_cluster = A.cluster;
-	}
+		while (cl < 16 && (long long)rows * cl * 2 <= slots && R / (cl * 2) >= 256) cl *= 2;
+		return cl;
+	};
+	const int solver_rows[2] = {K, grows};
+	const int solver_cluster[2] = {p.init_cluster > 0 ? p.init_cluster : pick_cluster(K), pick_cluster(grows)};
+	f.info.init_cluster = solver_cluster[0];
 	A.master = P.master_init.ptr;
 	A.snap32 = mixed ? P.snap32_init.ptr : nullptr;
 	A.snap64 = mixed ? nullptr : P.snap64_init.ptr;
 	A.fin = P.fin_init.ptr;
 	A.list = P.list_init.ptr;
 	A.fval = P.fval_init.ptr;
-	CCF_TRY_S(launch_solve(s, A, mixed, true), "find_initial_roots");
+	const std::vector<Field*> one(1, &f);
+	if (ccf_status rs = rows_setup(A, 0, one, mixed, solver_rows, solver_cluster); rs != CCF_OK) return rs;
+	CCF_TRY_S(launch_rows(s, A, mixed, true, num_sms, R, f.d.num_stars), "find_initial_roots");
 	CCF_TRY_S(cudaEventRecord(f.ev[4], s), "event");
 	CCF_TRY_S(polish(C.outs.ptr, (long long)R * nb), "polish");
 	/* the solved centres' columns go out at once */
@@ -476,13 +480,8 @@ ccf_status Engine::solve_chunked(Field& f, int verbose)
 			A.num_rows = grows;
 			A.num_rows_dev = nullptr;
 		}
-		{
-			const int slots = num_sms * slots_per_sm;
-			int cl = 1;
-			while (cl < 16 && (long long)grows * cl * 2 <= slots && R / (cl * 2) >= 256) cl *= 2;
-			A.cluster = cl;
-		}
-		CCF_TRY_S(launch_solve(s, A, mixed, false), "find_ccs");
+		if (ccf_status rs = rows_setup(A, 1, one, mixed, solver_rows, solver_cluster); rs != CCF_OK) return rs;
+		CCF_TRY_S(launch_rows(s, A, mixed, false, num_sms, R, f.d.num_stars), "find_ccs");
 		CCF_TRY_S(polish(og, (long long)R * gr.w_nb * cols), "polish");
 		/* the chunk goes out while the next group computes */
 		CCF_TRY_S(cudaEventRecord(C.ready, s), "event");

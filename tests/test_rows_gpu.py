@@ -1,0 +1,82 @@
+"""The full-sum rows cut into units over the whole GPU (rows.cu) against the
+cluster-per-row kernel that ccf_continue_branch_noalloc keeps: the same order of
+summation, so the same roots to the bit, whatever number of CTAs takes the
+units.  Sizes at the edges of the units: rows of one block and one unit, blocks
+and chunks that end short, several tiles, more rows than fit the partial sums'
+slots, steps with no root left after the first check.
+"""
+import ctypes
+
+import numpy as np
+import pytest
+
+from ccf_gb300 import CCF, run_batch
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+def field(n, rectangular, nb=1, num_phi=16, **kw):
+    return CCF(kappa_tot=0.4, kappa_star=0.35, shear=0.2, mass_function="uniform", m_lower=0.5, m_upper=1.5,
+               rectangular=rectangular, num_stars=n, num_branches=nb, num_phi=num_phi, random_seed=31 + n, **kw)
+
+
+@pytest.mark.parametrize("precision", ["mixed", "fp64"])
+@pytest.mark.parametrize("n", [1, 16, 127, 128, 129, 255, 512, 513, 700])
+def test_rows_do_not_depend_on_the_number_of_ctas(n, precision):
+    """One field alone (every CTA on its rows) and in a batch of eight (a CTA
+    has about one row): the launches differ, the roots are the same bits.  Both
+    have rows enough for clusters of one CTA, so the order of summation is one."""
+    a = field(n, 0, nb=8, num_phi=64, continuation="aberth", precision=precision, init_cluster=1)
+    assert a.run(-1), a.last_error()
+    r = a.results()
+    fs = [field(n, 0, nb=8, num_phi=64, continuation="aberth", precision=precision, init_cluster=1) for _ in range(8)]
+    for i, f in enumerate(fs[1:]):
+        f.random_seed = 500 + i
+    assert run_batch(fs, -1), fs[0].last_error()
+    b = fs[0].results()
+    centre = 64 // 8 // 2
+    assert np.array_equal(r["ccs"][:, centre], b["ccs"][:, centre])
+    d = O.match_sets(r["ccs"], b["ccs"], 8)
+    assert d["non_finite"] == 0 and d["non_bijective_cols"] == 0
+    assert d["max_dist"] <= 1e-11
+    assert r["info"]["unconverged"] == 0
+
+
+@pytest.mark.parametrize("n, rectangular", [(1, 0), (100, 1), (300, 0), (520, 1)])
+def test_rows_are_repeatable(n, rectangular):
+    outs = []
+    for _ in range(2):
+        c = field(n, rectangular, nb=2, num_phi=32, continuation="aberth")
+        assert c.run(-1), c.last_error()
+        outs.append(c.results())
+    assert np.array_equal(outs[0]["ccs"], outs[1]["ccs"])
+    assert np.array_equal(outs[0]["caustics"], outs[1]["caustics"])
+    assert np.array_equal(outs[0]["errs"], outs[1]["errs"])
+
+
+@pytest.mark.parametrize("n, rectangular", [(1, 0), (20, 0), (129, 0), (300, 0), (520, 0)])
+def test_rows_are_the_cluster_kernels(n, rectangular):
+    """Branch 0, side 0 of a full-sum run, and the same steps from the same
+    centre by ccf_continue_branch_noalloc."""
+    import torch
+    nb, num_phi = 2, 32
+    half = num_phi // nb // 2
+    c = field(n, rectangular, nb=nb, num_phi=num_phi, continuation="aberth")
+    assert c.run(-1), c.last_error()
+    r = c.results()
+    R = r["info"]["num_roots"]
+    start = torch.from_numpy(np.ascontiguousarray(r["ccs"].reshape(R, nb, -1)[:, 0, half]).view(np.float64).copy()).cuda()
+    shape = r["ccs"].shape
+    ccs = torch.zeros(shape[0] * shape[1] * 2, dtype=torch.float64, device="cuda")
+    errs = torch.zeros(shape[0] * shape[1], dtype=torch.float64, device="cuda")
+    f = c._L.ccf_continue_branch_noalloc
+    f.argtypes = [ctypes.c_void_p, ctypes.c_int, ctypes.c_int, ctypes.c_int] + [ctypes.c_void_p] * 5
+    f.restype = ctypes.c_int
+    assert f(c._h, 0, 0, half, start.data_ptr(), ccs.data_ptr(), errs.data_ptr(), None, None) == 0, c.last_error()
+    torch.cuda.synchronize()
+    z = ccs.cpu().numpy().view(np.complex128).reshape(R, nb, -1)[:, 0, :half]
+    want = r["ccs"].reshape(R, nb, -1)[:, 0, :half]
+    # the centre's snapshot is refreshed one sweep apart in the two, by less than the 1e-9 theta_star tolerance:
+    # the sums' 1e-9 changes a converging step's end quadratically less
+    assert np.max(np.abs(z - want)) <= 1e-11
