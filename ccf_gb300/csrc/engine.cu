@@ -1158,6 +1158,7 @@ ccf_status Engine::solve(std::vector<Field*>& fields, int verbose)
 	A.list = P.list_cont.ptr;
 	A.fval = P.fval_cont.ptr;
 	bool reorder = false;
+	int output_launches = 0;
 	if (track)
 	{
 		/* every root on its own path; rows that fail the column check run
@@ -1177,6 +1178,7 @@ ccf_status Engine::solve(std::vector<Field*>& fields, int verbose)
 		T.max_sub = TRACK_TSUB;
 		T.scales = 0;
 		for (Field* f : fields) T.scales |= f->params.write_mu_length_scales ? 1 : 0;
+		output_launches = !mixed || T.scales ? 2 : 0;
 		T.num_items = 0;
 		long long max_row_points = 0;   /* the column check's points of the longest row */
 		for (size_t r = 0; r < rc.size(); r++)
@@ -1209,6 +1211,7 @@ ccf_status Engine::solve(std::vector<Field*>& fields, int verbose)
 		CCF_TRY(launch_track_mark(s, T, P.item_work.ptr), "track_mark");
 		if (reorder) CCF_TRY(launch_track_item_order(s, T, P.item_work.ptr, P.item_order.ptr), "track_item_order");
 		CCF_TRY(launch_track(s, T, mixed, side), "track_ccs");
+		CCF_TRY(launch_track_outputs(s, T, mixed, max_row_points), "track_outputs");
 		CCF_TRY(launch_track_check(s, T, max_row_points), "track_check");
 		CCF_TRY(launch_collect_rerun(s, T, P.rows_rerun.ptr, P.rerun_count.ptr), "collect_rerun");
 		/* rows that failed: tracked again from their centre with sub-steps of at
@@ -1227,6 +1230,7 @@ ccf_status Engine::solve(std::vector<Field*>& fields, int verbose)
 		far_counts(T2);
 		CCF_TRY(launch_clear_tables(s, T2), "clear_tables");
 		CCF_TRY(launch_track(s, T2, mixed, side), "track_ccs_fine");
+		CCF_TRY(launch_track_outputs(s, T2, mixed, max_row_points), "track_outputs");
 		CCF_TRY(launch_track_check(s, T2, max_row_points), "track_check");
 		CCF_TRY(launch_collect_rerun(s, T2, P.rows_rerun2.ptr, P.rerun_count.ptr + 3), "collect_rerun");
 		A.rows = P.rows_rerun2.ptr;
@@ -1266,14 +1270,13 @@ ccf_status Engine::solve(std::vector<Field*>& fields, int verbose)
 
 	ccf_status status = CCF_OK;
 	/* root seeds, initial solve, continuation (tracker: phase table, item
-	   marking, item order, tracking (the items and two far launches), column check, row
-	   collection, table clearing, re-tracking (items, far), column check, row collection and the
-	   full-sum launch for
-	   the rows to re-run), FP64 polish; the launches are shared by the
+	   marking, item order, tracking (the items and two far launches), FP64 outputs, column
+	   check, row collection, table clearing, re-tracking (items, far), FP64 outputs, column
+	   check, row collection and the full-sum launch for the rows to re-run), FP64 polish; the launches are shared by the
 	   batch's fields and counted with the first */
 	for (int fi = 0; fi < nf; fi++)
 	{
-		ccf_status rc = finish_stats(*fields[fi], seg[fi], track, verbose, fi > 0 ? 0 : track ? (reorder ? 18 : 17) : 5);
+		ccf_status rc = finish_stats(*fields[fi], seg[fi], track, verbose, fi > 0 ? 0 : track ? (reorder ? 18 : 17) + output_launches : 5);
 		if (rc != CCF_OK) status = rc;
 	}
 	return status;

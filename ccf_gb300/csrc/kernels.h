@@ -477,6 +477,8 @@ struct TrackSide
 	cudaEvent_t fork = nullptr, join = nullptr;
 };
 cudaError_t launch_track(cudaStream_t s, const TrackArgs& a, bool mixed, const TrackSide& side);
+/* the FP64 outputs of a tracking launch (none where the tracker wrote them itself) */
+cudaError_t launch_track_outputs(cudaStream_t s, const TrackArgs& a, bool mixed, long long max_row_points);
 cudaError_t launch_track_check(cudaStream_t s, const TrackArgs& a, long long max_row_points);
 cudaError_t launch_collect_rerun(cudaStream_t s, const TrackArgs& a, RowDesc* rerun, int* count);
 cudaError_t launch_clear_tables(cudaStream_t s, const TrackArgs& a);

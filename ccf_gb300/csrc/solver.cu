@@ -552,6 +552,8 @@ constexpr double TRACK_STUCK = 1e-2;            /* theta_star: a root whose corr
                                                    (the full Aberth step leaves such roots unconverged
                                                    too: pairs of nearly coincident zeros); larger steps
                                                    are a lost root and send the row to the re-run */
+/* a slot's 1/mu error until track_outputs_kernel has formed it: neither a bound (>= 0) nor an unconverged mark (<= -1) */
+constexpr double OUTPUT_DUE = -0.25, OUTPUT_DUE_STALLED = -0.5;
 constexpr double TRACK_FS_REFINE = 1e-9;        /* bound on |f| above which a converged root takes one more step */
 constexpr int TABLE_PROBES = 1024;       /* linear-probe bound of the column tables (load <= 1/2: the
                                             longest cluster of a table of 1e5 slots is ~60) */
@@ -1243,6 +1245,10 @@ __global__ void __launch_bounds__(FAR ? 32 * FAR_MAX_WARPS : TNT, FAR ? 2 : 3) t
 		const double inv_cell = CELL_PER_THETA / F.theta;
 		const unsigned long long slots = 2ull * (unsigned long long)R;
 		const bool direct_out = !MIXED || O.mu != nullptr;
+		/* ... whose FP64 outputs track_outputs_kernel forms after the launch,
+		   unless they lie in host memory, from where it would read the roots,
+		   or the CTA sums the root's stars (FP64 far launch) */
+		const bool deferred = direct_out && !O.check_inline && !(FAR && !MIXED);
 		unsigned long long lane_maxerr = 0;   /* bits of the lane's largest 1/mu bound (non-negative) */
 
 		const double2 z1 = valid ? T.master[RD.base + a] : make_double2(0, 0);
@@ -1522,6 +1528,20 @@ __global__ void __launch_bounds__(FAR ? 32 * FAR_MAX_WARPS : TNT, FAR ? 2 : 3) t
 								else flags |= (unsigned)TRACK_NONFINITE;
 							}
 						}
+						if (deferred)
+						{
+							const double mark = stuck ? OUTPUT_DUE_STALLED : OUTPUT_DUE;
+							if (out != NO_OUT)
+							{
+								O.ccs[out] = zf;
+								O.errs[out] = mark;
+							}
+							if (out2 != NO_SLOT)
+							{
+								O.ccs[out2] = zf;
+								O.errs[out2] = mark;
+							}
+						}
 						/* the column check: by track_check_kernel after the launch, from
 						   the stored root, unless the outputs lie in host memory or the
 						   window does not hold this column */
@@ -1590,7 +1610,7 @@ __global__ void __launch_bounds__(FAR ? 32 * FAR_MAX_WARPS : TNT, FAR ? 2 : 3) t
 			}
 
 			/* direct outputs (FP64 solver, length scales): warp-wide */
-			const bool emit_direct = direct_out && emit;
+			const bool emit_direct = direct_out && !deferred && emit;
 			if (__any_sync(full, emit_direct))
 			{
 				int leafo = 0;
@@ -1957,6 +1977,82 @@ __global__ void track_check_kernel(const TrackArgs T)
 		}
 		if (flags) atomicOr(&T.row_stats[TRACK_ROW_STATS * (size_t)q + 1], (unsigned long long)flags);
 	}
+}
+
+/* The FP64 outputs of a tracking launch (the FP64 solver, and fields that
+   write length scales), after it: one lane per stored point, the 1/mu error,
+   the caustic and the length scale from the stored root, by the same function
+   and so with the same bits as in the tracking loop.  There a warp formed them
+   for the few lanes that had just converged, at a full warp's cost on the
+   1/64-rate FP64 pipe (half the continuation of a 419-star rectangle with
+   length scales, 420 phi steps: 9.1 ms, 4.7 with this launch; 600 stars in
+   FP64, 256 steps: 11.0 ms, 8.2).  Bound by that pipe at full lanes.  Consecutive lanes are consecutive phi steps of one root,
+   mostly in one leaf.  The roots are read back from the output arrays, their
+   slot's 1/mu error saying that the outputs are due.  A row that lost a root
+   has slots without one and is tracked again or re-run: it is skipped. */
+template <bool MIXED>
+__global__ void __launch_bounds__(128) track_outputs_kernel(const TrackArgs T)
+{
+	__shared__ FieldView sF;
+	__shared__ FieldOut sO;
+	__shared__ double s_max;
+	const unsigned full = 0xffffffffu;
+	const int nrows = T.num_rows_dev ? *T.num_rows_dev : T.num_rows;
+	for (int q = blockIdx.y; q < nrows; q += gridDim.y)
+	{
+		const RowDesc RD = T.rows[q];
+		if (T.outs[RD.field].check_inline || (T.row_stats[TRACK_ROW_STATS * (size_t)q + 1] & TRACK_LOST) ||
+			(MIXED && !T.outs[RD.field].mu))
+			continue;
+		__syncthreads();
+		if (threadIdx.x == 0)
+		{
+			sF = T.fields[RD.field];
+			sO = T.outs[RD.field];
+			s_max = 0;
+		}
+		__syncthreads();
+		const FieldView& F = sF;
+		const FieldOut& O = sO;
+		const int R = F.num_roots;
+		const int j0 = O.step_first, nsteps = RD.steps - j0 + 1;
+		const long long n = (long long)R * max(nsteps, 0);
+		unsigned flags = 0;
+		for (long long i0 = (long long)blockIdx.x * blockDim.x; i0 < n; i0 += (long long)gridDim.x * blockDim.x)
+		{
+			const long long i = i0 + threadIdx.x;
+			bool v = i < n;
+			const int a = v ? (int)(i / nsteps) : 0, j = v ? j0 + (int)(i - (long long)a * nsteps) : j0;
+			int ob[2], ok[2];
+			const int nslot = row_slots(O.nb, O.half, O.seg, RD.branch, RD.side, j, ob, ok);
+			const size_t out = out_slot(O, a, ob[0], ok[0]);
+			const size_t out2 = nslot > 1 ? out_slot(O, a, ob[1], ok[1]) : NO_SLOT;
+			const size_t from = out != NO_OUT ? out : out2;
+			const double due = v && from != NO_SLOT ? O.errs[from] : 0;
+			const bool stuck = due == OUTPUT_DUE_STALLED;
+			v = stuck || due == OUTPUT_DUE;
+			const double2 z = v ? O.ccs[from] : make_double2(0, 0);
+			const double2 cs = O.phase[row_global_step(O.nb, O.half, RD.branch, RD.side, j)].cs;
+			const int leaf = v ? find_leaf(F, z) : 0;
+			if (!point_epilogue_warp<MIXED>(F, O, v, z, leaf, false, zero_sums(), out, out2, cs.x, cs.y, &s_max, stuck))
+				flags |= (unsigned)TRACK_NONFINITE;
+		}
+		flags = __reduce_or_sync(full, flags);
+		unsigned long long* rs = T.row_stats + TRACK_ROW_STATS * (size_t)q;
+		if ((threadIdx.x & 31) == 0 && flags) atomicOr(&rs[1], (unsigned long long)flags);
+		__syncthreads();
+		if (threadIdx.x == 0 && s_max > 0) atomicMax(&rs[0], (unsigned long long)__double_as_longlong(s_max));
+	}
+}
+
+cudaError_t launch_track_outputs(cudaStream_t s, const TrackArgs& a, bool mixed, long long max_row_points)
+{
+	if (a.num_rows == 0 || max_row_points <= 0 || (mixed && !a.scales)) return cudaSuccess;
+	/* a bounded number of CTAs per row: the re-tracking's launch finds few rows */
+	const dim3 grid((unsigned)std::min<long long>((max_row_points + 127) / 128, 4096), (unsigned)std::min(a.num_rows, 65535));
+	if (mixed) track_outputs_kernel<true><<<grid, 128, 0, s>>>(a);
+	else track_outputs_kernel<false><<<grid, 128, 0, s>>>(a);
+	return cudaGetLastError();
 }
 
 cudaError_t launch_track_check(cudaStream_t s, const TrackArgs& a, long long max_row_points)

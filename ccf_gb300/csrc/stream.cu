@@ -454,6 +454,7 @@ ccf_status Engine::solve_chunked(Field& f, int verbose)
 			CCF_TRY_S(launch_track_mark(s, T, P.item_work.ptr), "track_mark");
 			if (reorder) CCF_TRY_S(launch_track_item_order(s, T, P.item_work.ptr, P.item_order.ptr), "track_item_order");
 			CCF_TRY_S(launch_track(s, T, mixed, side), "track_ccs");
+			CCF_TRY_S(launch_track_outputs(s, T, mixed, (long long)R * seg * half), "track_outputs");
 			CCF_TRY_S(launch_track_check(s, T, (long long)R * seg * half), "track_check");
 			CCF_TRY_S(launch_collect_rerun(s, T, P.rows_rerun.ptr, P.rerun_count.ptr), "collect_rerun");
 			TrackArgs T2 = T;
@@ -468,6 +469,7 @@ ccf_status Engine::solve_chunked(Field& f, int verbose)
 			far_counts(T2);
 			CCF_TRY_S(launch_clear_tables(s, T2), "clear_tables");
 			CCF_TRY_S(launch_track(s, T2, mixed, side), "track_ccs_fine");
+			CCF_TRY_S(launch_track_outputs(s, T2, mixed, (long long)R * seg * half), "track_outputs");
 			CCF_TRY_S(launch_track_check(s, T2, (long long)R * seg * half), "track_check");
 			CCF_TRY_S(launch_collect_rerun(s, T2, P.rows_rerun2.ptr, P.rerun_count.ptr + 3), "collect_rerun");
 			A.rows = P.rows_rerun2.ptr;
@@ -503,9 +505,9 @@ ccf_status Engine::solve_chunked(Field& f, int verbose)
 	/* seeds, (phase table), initial solve, its polish (2); per group the
 	   tracker's 11 launches (marking, tracking in three, column check, collection,
 	   table clearing, re-tracking in two, column check, collection) and the full-sum
-	   launch, or the full-sum launch alone, then the polish (2); and the item
+	   launch, the FP64 outputs of both trackings where they are formed after them, or the full-sum launch alone, then the polish (2); and the item
 	   order where a group reorders its items */
-	return finish_stats(f, seg, track, verbose, (track ? 5 : 4) + (track ? 14 : 3) * ngroups + reordered_groups);
+	return finish_stats(f, seg, track, verbose, (track ? 5 : 4) + (track ? 14 + (!mixed || f.params.write_mu_length_scales ? 2 : 0) : 3) * ngroups + reordered_groups);
 }
 
 } /* namespace ccf */

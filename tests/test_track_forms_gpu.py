@@ -56,3 +56,32 @@ def test_roots_off_the_box_find_the_full_sum_zeros(n, rectangular, num_phi, nb):
     d = O.match_sets(t["ccs"], a["ccs"], nb)
     assert d["non_finite"] == 0 and d["non_bijective_cols"] == 0
     assert d["max_dist"] <= 1e-11
+
+
+@pytest.mark.parametrize("precision, mu", [("fp64", 0), ("fp64", 1), ("mixed", 1)])
+@pytest.mark.parametrize("n, rectangular, num_phi, nb", [
+    (1, 0, 6, 1),         # fewer points than one warp
+    (9, 0, 64, 2),        # rows of less than a CTA
+    (33, 1, 94, 1),       # roots off the box, a ragged last warp
+    (150, 1, 24, 2),      # coarse steps: rows tracked again and re-run
+])
+def test_outputs_formed_after_the_tracking(monkeypatch, n, rectangular, num_phi, nb, precision, mu):
+    """The launch that forms FP64 outputs and length scales reaches every
+    point: the caustics are the oracle's lens map of the stored roots (FP64 on
+    both sides, the same tree and expansions: 1e-11 of the map's size, the
+    multipole evaluation's rounding), and the same bits come out with the
+    outputs in host memory and one group of centres at a time."""
+    monkeypatch.setenv("CCF_GB300_CHUNK_BYTES", "1")
+    field = dict(kappa_tot=0.45, kappa_star=0.4, shear=0.3, mass_function="equal", rectangular=rectangular,
+                 num_stars=n, random_seed=40 + n)
+    cfg = dict(field, num_phi=num_phi, num_branches=nb, precision=precision, write_mu_length_scales=mu)
+    a = run(cfg)
+    z = a["ccs"].ravel()
+    w = O.eval_field(z, **field)["w"]
+    assert np.all(np.abs(a["caustics"].ravel() - w) <= 1e-11 * (1 + np.abs(w) + np.abs(z)))
+    if mu:
+        assert np.all(a["mu_length_scales"] > 0)
+    for host in (1, 2):
+        b = run(cfg, host_outputs=host)
+        for k in ("ccs", "caustics", "errs") + (("mu_length_scales",) if mu else ()):
+            assert np.array_equal(a[k], b[k]), k
