@@ -1202,6 +1202,7 @@ ccf_status Engine::solve(std::vector<Field*>& fields, int verbose)
 		CCF_TRY(cudaMemsetAsync(P.row_stats.ptr, 0, TRACK_ROW_STATS * rc.size() * sizeof(unsigned long long), s), "memset");
 		CCF_TRY(cudaMemsetAsync(P.rerun_count.ptr, 0, 10 * sizeof(int), s), "memset");
 		CCF_TRY(cudaMemsetAsync(P.row_stats2.ptr, 0, TRACK_ROW_STATS * rc.size() * sizeof(unsigned long long), s), "memset");
+		T.run_items = T.num_items;
 		CCF_TRY(P.item_order.ensure((size_t)T.num_items + 1), "cudaMalloc(items)");
 		CCF_TRY(P.item_work.ensure(3 * (size_t)T.num_items + 3), "cudaMalloc(items)");
 		/* long items first where the launch is a few waves of items, and its

@@ -299,6 +299,86 @@ CCF_D dfc horner_halves_df(const float4* C, int n, dfc v, dfc x)
 	return dfc_fma(dfpc_second(acc), x, dfpc_first(acc));
 }
 
+/* Evaluation of one root by a group of G lanes (a power of two, G > 1, lane sub
+   of the group, mask gm): the lanes hold the same root, take every G-th near
+   pair and every G-th coefficient, and add up by shuffles, so that a warp
+   runs 32 / G roots in chains about G times shorter.  The exchange is
+   symmetric (a + b and b + a round alike), so all lanes end with the same
+   bits and take the same decisions.  All G lanes must call these. */
+template <int G>
+CCF_D float group_sum(float v, unsigned gm)
+{
+#pragma unroll
+	for (int o = 1; o < G; o <<= 1) v = __fadd_rn(v, __shfl_xor_sync(gm, v, o));
+	return v;
+}
+template <int G>
+CCF_D dfl group_sum(dfl v, unsigned gm)
+{
+#pragma unroll
+	for (int o = 1; o < G; o <<= 1)
+	{
+		const dfl u = {__shfl_xor_sync(gm, v.hi, o), __shfl_xor_sync(gm, v.lo, o)};
+		v = df_add(v, u);
+	}
+	return v;
+}
+template <int G>
+CCF_D dfc group_sum(dfc v, unsigned gm) { return {group_sum<G>(v.re, gm), group_sum<G>(v.im, gm)}; }
+template <int G>
+CCF_D float2 group_sum(float2 v, unsigned gm) { return make_float2(group_sum<G>(v.x, gm), group_sum<G>(v.y, gm)); }
+
+/* a lane's share of a split polynomial in x: its powers x^sub and x^G */
+template <int G>
+struct SplitPowers
+{
+	dfc first, stride;
+};
+template <int G>
+CCF_D SplitPowers<G> split_powers(dfc x, int sub)
+{
+	SplitPowers<G> w = {{{1.f, 0.f}, {0.f, 0.f}}, x};
+#pragma unroll
+	for (int b = 1; b < G; b <<= 1)
+	{
+		const dfc t = dfc_mul(w.first, w.stride);
+		if (sub & b) w.first = t;
+		w.stride = dfc_mul(w.stride, w.stride);
+	}
+	return w;
+}
+
+/* this lane's part of the two polynomials sum_k C_k x^k, k < n, of a pair array */
+template <int G>
+CCF_D dfpc poly_split(const float4* C, int n, const SplitPowers<G>& w, int sub)
+{
+	const dfpc_mult b = dfpc_mult_make(dfp_make(w.stride.re, w.stride.re), dfp_make(w.stride.im, w.stride.im));
+	const dfpc zero = {{0, 0}, {0, 0}};
+	dfpc acc = zero;
+#pragma unroll 1
+	for (int k = sub < n ? sub + (n - 1 - sub) / G * G : -1; k >= sub; k -= G) acc = dfpc_fma(acc, b, dfpc_load(C[2 * k], C[2 * k + 1]));
+	return dfpc_fma(acc, dfpc_mult_make(dfp_make(w.first.re, w.first.re), dfp_make(w.first.im, w.first.im)), zero);
+}
+
+/* sum_k c_k x^k, k < n, in FP32, over the group */
+template <int G>
+CCF_D float2 poly_split_f(const float2* c, int n, const SplitPowers<G>& w, int sub, unsigned gm)
+{
+	const float2 x = make_float2(w.stride.re.hi, w.stride.im.hi);
+	float2 acc = make_float2(0.f, 0.f);
+#pragma unroll 1
+	for (int k = sub < n ? sub + (n - 1 - sub) / G * G : -1; k >= sub; k -= G) acc = fadd(fmulc(acc, x), c[k]);
+	return group_sum<G>(fmulc(acc, make_float2(w.first.re.hi, w.first.im.hi)), gm);
+}
+
+/* horner_halves_df over the group: c_2k + c_(2k+1) x in v = x^2 */
+template <int G>
+CCF_D dfc halves_split(const float4* C, int n, const SplitPowers<G>& wv, dfc x, int sub, unsigned gm)
+{
+	const dfpc a = poly_split<G>(C, n, wv, sub);
+	return group_sum<G>(dfc_fma(dfpc_second(a), x, dfpc_first(a)), gm);
+}
+
 /* the near stars' part of an evaluation: sums of m / d, m / d^2 (double-float),
    m / d^3, 1 / d (FP32) and |m / d^2| */
 struct TrackSums
@@ -355,7 +435,8 @@ CCF_D TrackSums track_sums(const FieldView& F, int leaf, const dfc& zr)
 /* the same, two stars at a time (NEAR_PAIRS), with 1/d = (jx, -jy): the sums
    run over m jx, m jy, m (jx^2 - jy^2) and m jx jy, their signs and the factor
    2 of 2 jx jy put in at the end (exact) */
-CCF_D TrackSums track_sums_pk(const FieldView& F, int leaf, const dfc& zr)
+template <int G>
+CCF_D TrackSums track_sums_pk(const FieldView& F, int leaf, const dfc& zr, int sub, unsigned gm)
 {
 	const dfp zxp = dfp_make(zr.re, zr.re), zyp = dfp_make(zr.im, zr.im);
 	dfp s1x = {0, 0}, s1y = s1x, s2x = s1x, s2y = s1x;
@@ -364,12 +445,12 @@ CCF_D TrackSums track_sums_pk(const FieldView& F, int leaf, const dfc& zr)
 	const int np = (F.leaf_near_count[leaf] + 1) >> 1;
 	const float4* Pn = F.leaf_near_pk + (size_t)leaf * NEAR_PAIRS * NEAR_PAIR_F4;
 	/* the next pair is loaded while this one's terms are formed */
-	float4 nh = Pn[0], nl = Pn[1], nm = Pn[2];
+	float4 nh = Pn[3 * sub], nl = Pn[3 * sub + 1], nm = Pn[3 * sub + 2];
 #pragma unroll 1
-	for (int i = 0; i < np; i++)
+	for (int i = sub; i < np; i += G)
 	{
 		const NearPair s = near_pair(nh, nl, nm);
-		const int k = 3 * min(i + 1, NEAR_PAIRS - 1);
+		const int k = 3 * min(i + G, NEAR_PAIRS - 1);
 		nh = Pn[k];
 		nl = Pn[k + 1];
 		nm = Pn[k + 2];
@@ -398,6 +479,8 @@ CCF_D TrackSums track_sums_pk(const FieldView& F, int leaf, const dfc& zr)
 	const float2 s3 = make_float2(pk_lo(s3x) + pk_hi(s3x), -(pk_lo(s3y) + pk_hi(s3y)));
 	float2 pole = make_float2(pk_lo(polex) + pk_hi(polex), -(pk_lo(poley) + pk_hi(poley)));
 	const float tabs = pk_lo(tab) + pk_hi(tab);
+	if constexpr (G > 1)
+		return {group_sum<G>(s1, gm), group_sum<G>(s2, gm), group_sum<G>(s3, gm), group_sum<G>(pole, gm), group_sum<G>(tabs, gm)};
 	return {s1, s2, s3, pole, tabs};
 }
 
@@ -458,12 +541,13 @@ static __device__ __noinline__ SmoothFar smooth_far(const FieldView& F, double2 
 	return {dfc_from(smooth_dzbar(F, z)), make_float2((float)t.x, (float)t.y)};
 }
 
-template <bool PK>
+template <bool PK, int G>
 CCF_D TrackEval eval_track_df(const FieldView& F, const TrackConst& K, int leaf, double2 z, double2 rel, dfl cph, dfl sph,
-	bool disc_exact)
+	bool disc_exact, int sub, unsigned gm)
 {
+	static_assert(PK || G == 1, "only the packed evaluator is split over lanes");
 	const dfc zr = dfc_from(rel);
-	const TrackSums S = PK ? track_sums_pk(F, leaf, zr) : track_sums(F, leaf, zr);
+	const TrackSums S = PK ? track_sums_pk<G>(F, leaf, zr, sub, gm) : track_sums(F, leaf, zr);
 	const dfc s1 = S.s1, s2 = S.s2;
 	const float2 s3 = S.s3;
 	float2 pole = S.pole;
@@ -476,7 +560,16 @@ CCF_D TrackEval eval_track_df(const FieldView& F, const TrackConst& K, int leaf,
 	const bool folded = F.leaf_fold != nullptr && F.leaf_fold[leaf];
 	const float2* L3 = (folded ? F.leaf_loc3f_fold : F.leaf_loc3f) + (size_t)leaf * (P + 1);
 	LeafPoly lp;
-	if constexpr (PK)
+	if constexpr (G > 1)
+	{
+		/* entries 1 .. P of the pair block (leaf_poly_pk) */
+		const SplitPowers<G> w = split_powers<G>(dz, sub);
+		const dfpc a = poly_split<G>(F.leaf_loc_pk + (size_t)leaf * 2 * (P + 1) + 2, P, w, sub);
+		lp.al = group_sum<G>(dfpc_first(a), gm);
+		lp.dl = group_sum<G>(dfpc_second(a), gm);
+		lp.d2l = poly_split_f<G>(L3 + 3, P - 2, w, sub, gm);
+	}
+	else if constexpr (PK)
 	{
 		lp = leaf_poly_pk(F.leaf_loc_pk + (size_t)leaf * 2 * (P + 1), L3, P, dz);
 	}
@@ -525,7 +618,16 @@ CCF_D TrackEval eval_track_df(const FieldView& F, const TrackConst& K, int leaf,
 		const dfc wc = dfc_mul(zb, dfc_load(F.inv_corner_df));   /* zbar / c */
 		const dfc u = dfc_mul(wc, wc);
 		dfc acc, aa;
-		if constexpr (PK)
+		float2 a2;
+		if constexpr (G > 1)
+		{
+			const SplitPowers<G> wu = split_powers<G>(u, sub);
+			const dfc u2 = dfc_mul(u, u);
+			acc = halves_split<G>(F.smooth_d1_pair, (F.smooth_m + 1) / 2, split_powers<G>(u2, sub), u, sub, gm);
+			aa = halves_split<G>(F.smooth_a_pair, (F.taylor_smooth + 3) / 2, wu, wc, sub, gm);
+			a2 = poly_split_f<G>(F.smooth_d2f, F.smooth_m, wu, sub, gm);
+		}
+		else if constexpr (PK)
 		{
 			/* each series as its even and odd terms side by side: d1 in u^2,
 			   alpha in u = wc^2 */
@@ -548,11 +650,14 @@ CCF_D TrackEval eval_track_df(const FieldView& F, const TrackConst& K, int leaf,
 		sa.re = df_mul(K.kpi, aa.im);
 		sa.im = df_neg(df_mul(K.kpi, aa.re));
 		const float2 zbf = make_float2(zx, -zy);
-		const float2 r = fmulc(zbf, K.ic);
-		const float2 uf = fmulc(r, r);
-		float2 a2 = F.smooth_d2f[F.smooth_m - 1];
+		if constexpr (G == 1)
+		{
+			const float2 r = fmulc(zbf, K.ic);
+			const float2 uf = fmulc(r, r);
+			a2 = F.smooth_d2f[F.smooth_m - 1];
 #pragma unroll 1
-		for (int m = F.smooth_m - 2; m >= 0; m--) a2 = fadd(fmulc(a2, uf), F.smooth_d2f[m]);
+			for (int m = F.smooth_m - 2; m >= 0; m--) a2 = fadd(fmulc(a2, uf), F.smooth_d2f[m]);
+		}
 		d2s = fmulc(a2, fmulc(zbf, K.ic2));
 	}
 	else

@@ -273,6 +273,8 @@ struct TrackArgs
 	unsigned long long* row_stats;   /* TRACK_ROW_STATS per row, zeroed before the launch */
 	const int* item_start;      /* [num_rows]: first work item (32 roots) of each row */
 	int num_items;
+	long long run_items;        /* the items of the whole run, of which this launch may hold one group
+	                               (stream.cu): what decides the forms with other roundings */
 	int* counter;               /* [0] next solo root, [1] next item; zeroed before the launch */
 	int2* solo;                 /* (row, root) of the roots that start off the root box or are about to
 	                               leave it: tracked alone ... */

@@ -1017,6 +1017,17 @@ __device__ __noinline__ TrackEval track_offfield(const FieldView& F, bool off, d
 	return r;
 }
 
+/* the evaluation that lane src holds, in every lane (all 32 call it) */
+CCF_D TrackEval group_first(TrackEval e, int src)
+{
+	const unsigned full = 0xffffffffu;
+	float* const v[10] = {&e.step.x, &e.step.y, &e.as2, &e.fz.x, &e.fz.y, &e.af, &e.wpart.re.hi, &e.wpart.re.lo, &e.wpart.im.hi, &e.wpart.im.lo};
+#pragma unroll
+	for (int k = 0; k < 10; k++) *v[k] = __shfl_sync(full, *v[k], src);
+	e.wmode = __shfl_sync(full, e.wmode, src);
+	return e;
+}
+
 /* find_leaf out of line, for the lanes that left their leaf */
 __device__ __noinline__ int find_leaf_far(const FieldView& F, double2 z) { return find_leaf(F, z); }
 
@@ -1119,6 +1130,11 @@ cudaError_t launch_phase_table(cudaStream_t s, int nb, int nphi, PhaseEntry* out
    global counter until none are left, so a slow item delays only its own
    warp and no CTA waits at a barrier for its slowest warp.
 
+   A small launch holds each root in a group of G lanes, which split its near
+   stars and its polynomials and do the rest alike (an item is then G units of
+   work): what bounds such a launch is the chain of one root's evaluations
+   (launch_track has the rule and both sides' times).
+
    Each lane walks its own root through the phi steps of the row: one
    evaluation per iteration of the warp's loop, whatever step and sub-step
    the lane is at, so a lane that converges in one evaluation does not wait
@@ -1131,8 +1147,8 @@ cudaError_t launch_phase_table(cudaStream_t s, int nb, int nphi, PhaseEntry* out
    the direct evaluation of the outputs (a warp-wide call).  Every lane of the
    warp stays in the loop to the end: the evaluation off the root box and
    the direct epilogue are warp-wide calls. */
-template <bool MIXED, bool PK, bool FAR>
-__global__ void __launch_bounds__(FAR ? 32 * FAR_MAX_WARPS : TNT, FAR ? 2 : 3) track_kernel(const TrackArgs T)
+template <bool MIXED, bool PK, bool FAR, int G>
+__global__ void __launch_bounds__(FAR ? 32 * FAR_MAX_WARPS : TNT, FAR || G > 1 ? 2 : 3) track_kernel(const TrackArgs T)
 {
 	constexpr int NL = FAR ? 32 : TNT;   /* tracking lanes of the CTA */
 	__shared__ FieldView sF[NL / 32];
@@ -1145,6 +1161,9 @@ __global__ void __launch_bounds__(FAR ? 32 * FAR_MAX_WARPS : TNT, FAR ? 2 : 3) t
 	const unsigned full = 0xffffffffu;
 	const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
 	double2* const hz = s_hz + threadIdx.x;
+	/* the G lanes that hold one root (all of them its whole state) */
+	const int sub = lane & (G - 1);
+	const unsigned gm = ((1u << G) - 1u) << (lane - sub);
 
 	if constexpr (FAR)
 	{
@@ -1158,7 +1177,7 @@ __global__ void __launch_bounds__(FAR ? 32 * FAR_MAX_WARPS : TNT, FAR ? 2 : 3) t
 	while (true)
 	{
 		/* the far launch: the next listed root; else the next item in the queue's order */
-		int item = 0, solo_root = -1, row = 0;
+		int item = 0, part = 0, solo_root = -1, row = 0;
 		const FarState* resume = nullptr;
 		if constexpr (FAR)
 		{
@@ -1198,6 +1217,8 @@ __global__ void __launch_bounds__(FAR ? 32 * FAR_MAX_WARPS : TNT, FAR ? 2 : 3) t
 			{
 				if (lane == 0) item = atomicAdd(&T.counter[1], 1);
 				item = __shfl_sync(full, item, 0);
+				part = item % G;   /* an item is G work units of 32 / G roots */
+				item /= G;
 				if (T.items_per_row > 0)
 				{
 					if (item >= *T.num_rows_dev * T.items_per_row) break;
@@ -1229,8 +1250,8 @@ __global__ void __launch_bounds__(FAR ? 32 * FAR_MAX_WARPS : TNT, FAR ? 2 : 3) t
 		const TrackConst& K = sK[w];
 		const int R = F.num_roots;
 		const int chunk = T.items_per_row > 0 ? item - row * T.items_per_row : item - T.item_start[row];
-		const int a = solo_root >= 0 ? solo_root : chunk * 32 + lane;
-		const bool valid = solo_root >= 0 ? lane == 0 : (a < R && (T.items_per_row > 0 || !T.is_solo[RD.base + a]));
+		const int a = solo_root >= 0 ? solo_root : chunk * 32 + part * (32 / G) + lane / G;
+		const bool valid = solo_root >= 0 ? lane < G : (a < R && (T.items_per_row > 0 || !T.is_solo[RD.base + a]));
 		const int max_sub = T.max_sub;
 		const int c = RD.branch, side = RD.side, nb = O.nb, nphi = O.nphi, period = 2 * O.half;
 		const int j0 = O.step_first, j1 = RD.steps;
@@ -1316,8 +1337,11 @@ __global__ void __launch_bounds__(FAR ? 32 * FAR_MAX_WARPS : TNT, FAR ? 2 : 3) t
 			if (!FAR && act && leaf < 0 && solo_root < 0 && !T.scales && (F.num_stars >= FAR_EVICT_STARS || T.items_per_row > 0))
 			{
 				/* the root left the root box: to the second far launch */
-				const int q = atomicAdd(T.num_evict, 1);
-				if (q < T.evict_cap)
+				int q = 0;
+				if (sub == 0) q = atomicAdd(T.num_evict, 1);
+				if constexpr (G > 1) q = __shfl_sync(gm, q, lane - sub);
+				if (q < T.evict_cap && sub > 0) act = false;
+				else if (q < T.evict_cap)
 				{
 					FarState& fs = T.evict[q];
 					for (int k = 0; k < TRACK_HIST; k++) fs.hz[k] = hz[k * NL];
@@ -1350,10 +1374,11 @@ __global__ void __launch_bounds__(FAR ? 32 * FAR_MAX_WARPS : TNT, FAR ? 2 : 3) t
 			e.wmode = 2;
 			if constexpr (MIXED)
 			{
-				if (act && leaf >= 0) e = eval_track_df<PK>(F, K, leaf, z, rel, cpd, spd, disc_exact);
+				if (act && leaf >= 0) e = eval_track_df<PK, G>(F, K, leaf, z, rel, cpd, spd, disc_exact, sub, gm);
 				if (__any_sync(full, off))
 				{
-					const TrackEval o = track_offfield<FAR && PK>(F, off, z, cp, sp, disc_exact, (float)stuck2, &s_far);
+					TrackEval o = track_offfield<FAR && PK>(F, off && sub == 0, z, cp, sp, disc_exact, (float)stuck2, &s_far);
+					if constexpr (G > 1) o = group_first(o, lane - sub);
 					if (off) e = o;
 				}
 				step = make_double2((double)e.step.x, (double)e.step.y);
@@ -1466,7 +1491,7 @@ __global__ void __launch_bounds__(FAR ? 32 * FAR_MAX_WARPS : TNT, FAR ? 2 : 3) t
 						}
 						if constexpr (MIXED)
 						{
-							if (!direct_out)
+							if (!direct_out && sub == 0)
 							{
 								/* the lens map at the evaluated point ze, corrected to zf = ze - s:
 								   w(zf) = w(ze) - a s - (conj(f) + a e^{i phi}) conj(s).  With
@@ -1545,7 +1570,7 @@ __global__ void __launch_bounds__(FAR ? 32 * FAR_MAX_WARPS : TNT, FAR ? 2 : 3) t
 						/* the column check: by track_check_kernel after the launch, from
 						   the stored root, unless the outputs lie in host memory or the
 						   window does not hold this column */
-						if (O.check_inline || out == NO_OUT)
+						if ((O.check_inline || out == NO_OUT) && sub == 0)
 							flags |= (unsigned)table_insert(T.table + RD.cont_base + (size_t)(j - j0) * slots, slots,
 								cell_key(zf, inv_cell));
 						maxev = max(maxev, evs);
@@ -1633,11 +1658,11 @@ __global__ void __launch_bounds__(FAR ? 32 * FAR_MAX_WARPS : TNT, FAR ? 2 : 3) t
 		}
 		if (valid && lost) flags |= (unsigned)TRACK_LOST;
 		for (int o = 16; o > 0; o >>= 1) lane_maxerr = max(lane_maxerr, __shfl_xor_sync(full, lane_maxerr, o));
-		unconv = __reduce_add_sync(full, unconv);
+		unconv = __reduce_add_sync(full, unconv) / G;   /* counted by each lane of a root */
 		flags = __reduce_or_sync(full, flags);
 		maxev = (int)__reduce_max_sync(full, (unsigned)maxev);
-		nev = warp_sum_u64(nev);
-		nhalf = warp_sum_u64(nhalf);
+		nev = warp_sum_u64(nev) / G;
+		nhalf = warp_sum_u64(nhalf) / G;
 		__syncwarp();
 		if (lane == 0)
 		{
@@ -1817,7 +1842,7 @@ constexpr int TRACK_CARVEOUT = 28;
 
 /* CTAs of the tracker that are resident on one SM at once (asked once per
    form and CTA size) */
-template <bool MIXED, bool PK, bool FAR>
+template <bool MIXED, bool PK, bool FAR, int G>
 int resident(int threads)
 {
 	static std::atomic<int> known[FAR_MAX_WARPS + 1];
@@ -1827,8 +1852,8 @@ int resident(int threads)
 		/* one shared-memory split for both kinds of launch: an SM must be empty
 		   to change it, so with splits of their own the far launch and the items
 		   never shared one */
-		cudaFuncSetAttribute(track_kernel<MIXED, PK, FAR>, cudaFuncAttributePreferredSharedMemoryCarveout, TRACK_CARVEOUT);
-		cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, track_kernel<MIXED, PK, FAR>, threads, 0);
+		cudaFuncSetAttribute(track_kernel<MIXED, PK, FAR, G>, cudaFuncAttributePreferredSharedMemoryCarveout, TRACK_CARVEOUT);
+		cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, track_kernel<MIXED, PK, FAR, G>, threads, 0);
 		n = std::max(n, 1);
 		known[threads / 32].store(n, std::memory_order_relaxed);
 	}
@@ -1855,7 +1880,7 @@ int far_warps(int stars)
 bool solos_far(const TrackArgs& a, int sms)
 {
 	const double root = 1.15 * (25000 + 7.5 * a.max_stars);
-	const double items = 1.6 * 50000 * a.num_items / (double)(sms * TRACK_WARPS_PER_SM);
+	const double items = 1.6 * 50000 * a.run_items / (double)(sms * TRACK_WARPS_PER_SM);
 	return !a.scales && a.max_stars >= FAR_EVICT_STARS && 2 * root > 0.5 * items;
 }
 
@@ -1869,15 +1894,15 @@ cudaError_t launch_far(cudaStream_t s, const TrackArgs& a, int sms, int evicted)
 	/* beside items that fill the GPU one CTA per SM, so that the items keep two
 	   thirds of the registers; else as many as are resident */
 	const bool beside = !evicted && a.num_items >= sms * TRACK_WARPS_PER_SM / 2;
-	const int blocks = (int)std::min<long long>((long long)sms * (beside ? 1 : resident<MIXED, PK, true>(threads)), most);
-	if (blocks > 0) track_kernel<MIXED, PK, true><<<blocks, threads, 0, s>>>(f);
+	const int blocks = (int)std::min<long long>((long long)sms * (beside ? 1 : resident<MIXED, PK, true, 1>(threads)), most);
+	if (blocks > 0) track_kernel<MIXED, PK, true, 1><<<blocks, threads, 0, s>>>(f);
 	return cudaGetLastError();
 }
 
 /* The far launch of the roots that start off the root box (solos_far; first
    tracking only), on the side stream when there is one; the items; then the
    far launch of the roots that left the box. */
-template <bool MIXED, bool PK>
+template <bool MIXED, bool PK, int G = 1>
 cudaError_t launch_track_form(cudaStream_t s, const TrackArgs& a, int sms, const TrackSide& side)
 {
 	cudaError_t e = cudaSuccess;
@@ -1899,10 +1924,10 @@ cudaError_t launch_track_form(cudaStream_t s, const TrackArgs& a, int sms, const
 	   the items' two CTAs), but not where the outputs are FP64 epilogues, which
 	   a CTA more per SM does not speed up (11.3 ms against 12.8 in FP64 on a
 	   600-star rectangle) */
-	const long long work = t.num_items + (first && !t.solo_far && PK ? t.solo_guess : 0);
-	const int blocks = (int)std::max<long long>(1, std::min<long long>(sms * resident<MIXED, PK, false>(TNT),
+	const long long work = (long long)t.num_items * G + (first && !t.solo_far && PK ? t.solo_guess : 0);
+	const int blocks = (int)std::max<long long>(1, std::min<long long>(sms * resident<MIXED, PK, false, G>(TNT),
 		(work + TNT / 32 - 1) / (TNT / 32)));
-	track_kernel<MIXED, PK, false><<<blocks, TNT, 0, s>>>(t);
+	track_kernel<MIXED, PK, false, G><<<blocks, TNT, 0, s>>>(t);
 	if ((e = cudaGetLastError()) != cudaSuccess) return e;
 	if (t.solo_far && side.side && (e = cudaStreamWaitEvent(s, side.join, 0)) != cudaSuccess) return e;
 	if (!a.scales && (!first || a.max_stars >= FAR_EVICT_STARS)) e = launch_far<MIXED, PK>(s, t, sms, 1);
@@ -1920,6 +1945,19 @@ cudaError_t launch_track(cudaStream_t s, const TrackArgs& a, bool mixed, const T
 	/* length scales: the scalar evaluator (the packed one's other rounding, 1e-14
 	   in a root, becomes 4e-8 in a length scale next to a cusp) */
 	if (a.scales) return launch_track_form<true, false>(s, a, sms, side);
+	/* Lanes per root: as many as leave at most eight warps per SM.  An iteration
+	   of a warp alone takes ~10 us with one lane per root, ~7.3 with four and
+	   ~6.5 with eight, but the root's own FP64 work then runs in four or eight
+	   times as many warps.  Continuation of equal-mass discs, 64 phi steps per
+	   branch, with 1 / 2 / 4 / 8 lanes: 18 items 1.50 / 1.20 / 0.99 / 0.91 ms,
+	   152 items 1.30 / 1.03 / 0.94 / 0.96, 304 items 1.17 / 0.97 / 0.93 / 1.33,
+	   512 items 1.21 / 1.06 / 1.32 / 1.97, 800 items 1.62 / 1.64 / 1.88 / 3.0.  When rows are
+	   tracked again two of them are counted, their number being on the device. */
+	const long long units = a.items_per_row > 0 ? 2LL * a.items_per_row : a.run_items;
+	const int lanes = (int)(8LL * sms / units);
+	if (lanes >= 8) return launch_track_form<true, true, 8>(s, a, sms, side);
+	if (lanes >= 4) return launch_track_form<true, true, 4>(s, a, sms, side);
+	if (lanes >= 2) return launch_track_form<true, true, 2>(s, a, sms, side);
 	return launch_track_form<true, true>(s, a, sms, side);
 }
 

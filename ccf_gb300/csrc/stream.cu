@@ -435,6 +435,7 @@ ccf_status Engine::solve_chunked(Field& f, int verbose)
 			T.max_sub = TRACK_TSUB;
 			T.scales = f.params.write_mu_length_scales ? 1 : 0;
 			T.num_items = grows * ((R + 31) / 32);
+			T.run_items = (long long)ngroups * T.num_items;
 			T.solo = P.solo.ptr;
 			T.num_solo = reinterpret_cast<int*>(P.solo.ptr + ncont);
 			T.is_solo = P.is_solo.ptr;

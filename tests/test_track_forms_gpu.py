@@ -13,7 +13,7 @@ one's to the same tolerance.
 import numpy as np
 import pytest
 
-from ccf_gb300 import CCF
+from ccf_gb300 import CCF, run_batch
 from oracle import oracle as O
 
 pytestmark = pytest.mark.gpu
@@ -85,3 +85,29 @@ def test_outputs_formed_after_the_tracking(monkeypatch, n, rectangular, num_phi,
         b = run(cfg, host_outputs=host)
         for k in ("ccs", "caustics", "errs") + (("mu_length_scales",) if mu else ()):
             assert np.array_equal(a[k], b[k]), k
+
+
+@pytest.mark.parametrize("n, rectangular, num_phi, nb", [
+    (1, 0, 16, 1),        # one star, fewer roots than lanes
+    (3, 1, 40, 1),        # an odd near list, roots off the box
+    (33, 0, 24, 3),       # groups past the last root
+    (150, 1, 24, 2),      # rows tracked again and re-run
+    (300, 1, 64, 8),      # a middling launch, smooth-mass series not folded into every leaf
+])
+def test_roots_split_over_lanes_find_the_same_zeros(n, rectangular, num_phi, nb):
+    """A small launch evaluates each root with 2, 4 or 8 lanes, a launch that
+    fills the GPU with one: the same field alone and in a batch of enough
+    copies.  Both converge to a step below 1e-9 theta_star quadratically and
+    so agree within the tracker tests' 1e-11."""
+    cfg = dict(kappa_tot=0.45, kappa_star=0.4, shear=0.3, mass_function="equal", rectangular=rectangular, num_stars=n,
+               num_phi=num_phi, num_branches=nb, random_seed=60 + n)
+    a = run(cfg)
+    items = 2 * a["info"]["centres_solved"] * ((a["info"]["num_roots"] + 31) // 32)
+    for per_sm in (1, 2, 4):    # more items than that per SM: 4, 2 and 1 lanes per root
+        copies = [CCF(**cfg) for _ in range(per_sm * 152 // items + 1)]
+        if len(copies) == 1:
+            continue
+        run_batch(copies)
+        d = O.match_sets(a["ccs"], copies[-1].results()["ccs"], nb)
+        assert d["non_finite"] == 0 and d["non_bijective_cols"] == 0
+        assert d["max_dist"] <= 1e-11
