@@ -337,18 +337,22 @@ struct SplitPowers
 template <int G>
 CCF_D SplitPowers<G> split_powers(dfc x, int sub)
 {
+	const dfc zero = {{0.f, 0.f}, {0.f, 0.f}};
 	SplitPowers<G> w = {{{1.f, 0.f}, {0.f, 0.f}}, x};
 #pragma unroll
 	for (int b = 1; b < G; b <<= 1)
 	{
-		const dfc t = dfc_mul(w.first, w.stride);
+		const dfc t = b == 1 ? w.stride : dfc_fma(w.first, w.stride, zero);
 		if (sub & b) w.first = t;
-		w.stride = dfc_mul(w.stride, w.stride);
+		w.stride = dfc_fma(w.stride, w.stride, zero);
 	}
 	return w;
 }
 
-/* this lane's part of the two polynomials sum_k C_k x^k, k < n, of a pair array */
+/* this lane's part of the two polynomials sum_k C_k x^k, 1 <= k < n, of a pair
+   array.  The constant terms, the largest, are left to the caller, who adds
+   them after the exchange: with them in it each exchange would round at their
+   size (a caustic's rms error against FP64 8 % above the serial Horner's). */
 template <int G>
 CCF_D dfpc poly_split(const float4* C, int n, const SplitPowers<G>& w, int sub)
 {
@@ -356,7 +360,7 @@ CCF_D dfpc poly_split(const float4* C, int n, const SplitPowers<G>& w, int sub)
 	const dfpc zero = {{0, 0}, {0, 0}};
 	dfpc acc = zero;
 #pragma unroll 1
-	for (int k = sub < n ? sub + (n - 1 - sub) / G * G : -1; k >= sub; k -= G) acc = dfpc_fma(acc, b, dfpc_load(C[2 * k], C[2 * k + 1]));
+	for (int k = sub < n ? sub + (n - 1 - sub) / G * G : -1; k >= sub; k -= G) acc = dfpc_fma(acc, b, k > 0 ? dfpc_load(C[2 * k], C[2 * k + 1]) : zero);
 	return dfpc_fma(acc, dfpc_mult_make(dfp_make(w.first.re, w.first.re), dfp_make(w.first.im, w.first.im)), zero);
 }
 
@@ -375,8 +379,10 @@ CCF_D float2 poly_split_f(const float2* c, int n, const SplitPowers<G>& w, int s
 template <int G>
 CCF_D dfc halves_split(const float4* C, int n, const SplitPowers<G>& wv, dfc x, int sub, unsigned gm)
 {
-	const dfpc a = poly_split<G>(C, n, wv, sub);
-	return group_sum<G>(dfc_fma(dfpc_second(a), x, dfpc_first(a)), gm);
+	const dfpc a = poly_split<G>(C, n, wv, sub), c0 = dfpc_load(C[0], C[1]);
+	const dfc r = dfc_fma(dfpc_second(c0), x, group_sum<G>(dfc_fma(dfpc_second(a), x, dfpc_first(a)), gm));
+	const dfc c = dfpc_first(c0);
+	return {df_add(r.re, c.re), df_add(r.im, c.im)};
 }
 
 /* the near stars' part of an evaluation: sums of m / d, m / d^2 (double-float),
@@ -564,9 +570,12 @@ CCF_D TrackEval eval_track_df(const FieldView& F, const TrackConst& K, int leaf,
 	{
 		/* entries 1 .. P of the pair block (leaf_poly_pk) */
 		const SplitPowers<G> w = split_powers<G>(dz, sub);
-		const dfpc a = poly_split<G>(F.leaf_loc_pk + (size_t)leaf * 2 * (P + 1) + 2, P, w, sub);
-		lp.al = group_sum<G>(dfpc_first(a), gm);
-		lp.dl = group_sum<G>(dfpc_second(a), gm);
+		const float4* C = F.leaf_loc_pk + (size_t)leaf * 2 * (P + 1) + 2;
+		const dfpc a = poly_split<G>(C, P, w, sub), c0 = dfpc_load(C[0], C[1]);
+		const dfc ra = group_sum<G>(dfpc_first(a), gm), rd = group_sum<G>(dfpc_second(a), gm);
+		const dfc ca = dfpc_first(c0), cd = dfpc_second(c0);
+		lp.al = {df_add(ra.re, ca.re), df_add(ra.im, ca.im)};
+		lp.dl = {df_add(rd.re, cd.re), df_add(rd.im, cd.im)};
 		lp.d2l = poly_split_f<G>(L3 + 3, P - 2, w, sub, gm);
 	}
 	else if constexpr (PK)
