@@ -1334,7 +1334,7 @@ __global__ void __launch_bounds__(FAR ? 32 * FAR_MAX_WARPS : TNT, FAR || G > 1 ?
 				leaf = find_leaf_far(F, z);
 				if (leaf >= 0) in_leaf_box(F, leaf, z, rel);
 			}
-			if (!FAR && act && leaf < 0 && solo_root < 0 && !T.scales && (F.num_stars >= FAR_EVICT_STARS || T.items_per_row > 0))
+			if (!FAR && act && leaf < 0 && solo_root < 0 && ((!T.scales && F.num_stars >= FAR_EVICT_STARS) || T.items_per_row > 0))
 			{
 				/* the root left the root box: to the second far launch */
 				int q = 0;
@@ -1930,7 +1930,7 @@ cudaError_t launch_track_form(cudaStream_t s, const TrackArgs& a, int sms, const
 	track_kernel<MIXED, PK, false, G><<<blocks, TNT, 0, s>>>(t);
 	if ((e = cudaGetLastError()) != cudaSuccess) return e;
 	if (t.solo_far && side.side && (e = cudaStreamWaitEvent(s, side.join, 0)) != cudaSuccess) return e;
-	if (!a.scales && (!first || a.max_stars >= FAR_EVICT_STARS)) e = launch_far<MIXED, PK>(s, t, sms, 1);
+	if (!first || (!a.scales && a.max_stars >= FAR_EVICT_STARS)) e = launch_far<MIXED, PK>(s, t, sms, 1);
 	return e;
 }
 }
