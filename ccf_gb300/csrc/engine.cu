@@ -30,6 +30,9 @@ The engine never resets the device and reuses its buffers across runs.
 #include <numeric>
 #include <thread>
 
+#include <sys/mman.h>
+#include <unistd.h>
+
 namespace ccf
 {
 
@@ -1499,6 +1502,74 @@ cudaError_t Engine::copy_out(void* dst, const void* src, size_t bytes)
 	return e;
 }
 
+#ifndef MADV_POPULATE_WRITE
+#define MADV_POPULATE_WRITE 23   /* Linux 5.14 */
+#endif
+
+/* Maps the pages of new pageable destinations from several threads before the
+   copies, without changing what they hold.  An array fresh from the allocator
+   has no pages, and the copy faulted them in and cleared them one after
+   another (new arrays of 24 fields, 524 MB: 29 ms, 16 with this, 4.5 into
+   arrays that have their pages).  Destinations the driver knows (page-locked,
+   managed, device memory) are left alone, and where the kernel has no such
+   call or no thread can be started the copy maps them as before. */
+static void populate(std::vector<std::pair<void*, size_t>> dst)
+{
+	constexpr size_t PER_THREAD = 2 << 20;
+	constexpr size_t MAX_THREADS = 4;   /* eight wait for one another in the kernel */
+	const size_t page = (size_t)sysconf(_SC_PAGESIZE);
+	struct Span
+	{
+		char* p;
+		size_t n;
+	};
+	std::vector<Span> spans;
+	size_t total = 0;
+	for (auto& d : dst)
+	{
+		cudaPointerAttributes a;
+		const bool pageable = d.second >= PER_THREAD && cudaPointerGetAttributes(&a, d.first) == cudaSuccess &&
+			a.type == cudaMemoryTypeUnregistered;
+		cudaGetLastError();
+		if (!pageable) continue;
+		/* whole pages inside the destination */
+		const uintptr_t b = ((uintptr_t)d.first + page - 1) / page * page, e = ((uintptr_t)d.first + d.second) / page * page;
+		/* an array used before has its pages */
+		bool mapped = e > b;
+		for (const uintptr_t q : {b, b + (e - b) / page / 2 * page, e - page})
+		{
+			unsigned char in = 0;
+			mapped = mapped && mincore((void*)q, page, &in) == 0 && (in & 1);
+		}
+		if (e <= b || mapped) continue;
+		spans.push_back({(char*)b, e - b});
+		total += e - b;
+	}
+	const size_t hw = std::max(1u, std::thread::hardware_concurrency());
+	const size_t threads = std::min({total / PER_THREAD, MAX_THREADS, std::max<size_t>(1, hw / 2)});
+	if (threads < 2) return;
+	/* thread t takes the t-th share of every span */
+	auto work = [&](size_t t) {
+		for (const Span& v : spans)
+		{
+			const size_t pages = v.n / page, b = pages * t / threads, e = pages * (t + 1) / threads;
+			if (e > b) madvise(v.p + b * page, (e - b) * page, MADV_POPULATE_WRITE);
+		}
+	};
+	std::vector<std::thread> team;
+	size_t started = 1;
+	try
+	{
+		team.reserve(threads);
+		for (; started < threads; started++) team.emplace_back(work, started);
+	}
+	catch (const std::exception&)
+	{
+	}
+	work(0);
+	for (auto& th : team) th.join();
+}
+
 ccf_status Engine::copy_results(Field& f, double* ccs, double* caustics, double* errs, double* mu, double* stars)
 {
 	if (!f.ran) { error = "Error. No results: run() has not completed."; return CCF_ERR_NOT_RUN; }
@@ -1518,6 +1589,12 @@ ccf_status Engine::copy_results(Field& f, double* ccs, double* caustics, double*
 		error = "Error. Length scales were not requested (write_mu_length_scales = 0).";
 		return CCF_ERR_INVALID_ARGUMENT;
 	}
+	std::vector<std::pair<void*, size_t>> dst;
+	for (double* p : {ccs, caustics})
+		if (p) dst.push_back({p, npts * sizeof(double2)});
+	for (double* p : {errs, mu})
+		if (p) dst.push_back({p, npts * sizeof(double)});
+	populate(std::move(dst));
 	if (ccs) CCF_TRY(copy(ccs, f.out_ccs, npts * sizeof(double2)), "copy ccs");
 	if (errs) CCF_TRY(copy(errs, f.out_errs, npts * sizeof(double)), "copy errs");
 	if (caustics) CCF_TRY(copy(caustics, f.out_caustics, npts * sizeof(double2)), "copy caustics");
