@@ -168,13 +168,13 @@ ccf_status Engine::rows_setup(SolveArgs& A, int which, const std::vector<Field*>
 	CCF_TRY(P.row_state.ensure((size_t)rows[0] + rows[1]), "cudaMalloc(rows)");
 	CCF_TRY(P.row_control.ensure(4), "cudaMalloc(rows)");
 	CCF_TRY(P.row_part.ensure((size_t)part_bytes), "cudaMalloc(rows)");
-	/* a unit's share is 256 roots; the blocks of a row's segments may end short */
-	const long long units = maxR / 256 + 17;
-	CCF_TRY(P.row_share.ensure((size_t)(most_slots * units * 256)), "cudaMalloc(rows)");
+	/* a unit's share is 64 to 256 roots; the blocks of a row's segments may end short */
+	const long long units = maxR / ROWS_MIN_BLOCK + 17, shares = maxR + 17 * 256;
+	CCF_TRY(P.row_share.ensure((size_t)(most_slots * shares)), "cudaMalloc(rows)");
 	CCF_TRY(P.row_counts.ensure((size_t)(most_slots * units)), "cudaMalloc(rows)");
 	A.share = P.row_share.ptr;
 	A.counts = P.row_counts.ptr;
-	A.share_stride = units * 256;
+	A.share_stride = shares;
 	A.counts_stride = units;
 	A.cluster = cluster[which];
 	A.state = P.row_state.ptr + (which ? rows[0] : 0);

@@ -464,27 +464,26 @@ CCF_D float2 smooth_d2zbar_f32(const FieldView& F, double2 z)
 /* f'(z) in FP32 for the mixed-precision solver: only the step size depends
    on it, never the converged root.  Off-field points take s3_off, the direct
    sum over every star. */
-CCF_D float2 eval_df32(const FieldView& F, int leaf, double2 z, double2 s3_off)
+CCF_D void star_term_df32(float2& s3, double2 z, const NearStar& s)
 {
-	float2 s3 = make_float2(0, 0);
+	float dx = (float)(z.x - s.x), dy = (float)(z.y - s.y), m = (float)s.m;
+	float r = rcp32(dx * dx + dy * dy);
+	float ix = dx * r, iy = -dy * r;
+	float i2x = ix * ix - iy * iy, i2y = 2 * ix * iy;
+	float i3x = i2x * ix - i2y * iy, i3y = i2x * iy + i2y * ix;
+	s3.x = fmaf(m, i3x, s3.x);
+	s3.y = fmaf(m, i3y, s3.y);
+}
+
+/* the same from the near stars' sum of m / d^3 (near_s3, a root in a leaf) */
+CCF_D float2 eval_df32_from(const FieldView& F, int leaf, double2 z, double2 s3_off, float2 near_s3)
+{
+	float2 s3 = near_s3;
 	float2 d2l = make_float2(0, 0);
 	bool folded = false;
 	if (leaf >= 0)
 	{
 		folded = F.leaf_fold != nullptr && F.leaf_fold[leaf];
-		int n = F.leaf_near_count[leaf];
-		const NearStar* ns = F.leaf_near + (size_t)leaf * MAX_NEAR;
-		for (int i = 0; i < n; i++)
-		{
-			NearStar s = ns[i];
-			float dx = (float)(z.x - s.x), dy = (float)(z.y - s.y), m = (float)s.m;
-			float r = rcp32(dx * dx + dy * dy);
-			float ix = dx * r, iy = -dy * r;
-			float i2x = ix * ix - iy * iy, i2y = 2 * ix * iy;
-			float i3x = i2x * ix - i2y * iy, i3y = i2x * iy + i2y * ix;
-			s3.x = fmaf(m, i3x, s3.x);
-			s3.y = fmaf(m, i3y, s3.y);
-		}
 		const int P = F.order;
 		double2 dzd = leaf_dz(F, leaf, z);
 		float2 dz = make_float2((float)dzd.x, (float)dzd.y);
@@ -503,13 +502,24 @@ CCF_D float2 eval_df32(const FieldView& F, int leaf, double2 z, double2 s3_off)
 	return make_float2(-2 * t2 * s3.x - d2l.x - d2s.x, -2 * t2 * s3.y - d2l.y + d2s.y);
 }
 
+CCF_D float2 eval_df32(const FieldView& F, int leaf, double2 z, double2 s3_off)
+{
+	float2 s3 = make_float2(0, 0);
+	if (leaf >= 0)
+	{
+		int n = F.leaf_near_count[leaf];
+		const NearStar* ns = F.leaf_near + (size_t)leaf * MAX_NEAR;
+		for (int i = 0; i < n; i++) star_term_df32(s3, z, ns[i]);
+	}
+	return eval_df32_from(F, leaf, z, s3_off, s3);
+}
+
 /* f'(z) for the mixed-precision solver: the FP32 evaluation, or FP64 where
    that is not finite (far outside the field the smooth-mass Taylor terms
    leave the FP32 range, and an infinite f' would make a zero step).
    Off-field points take s3_off, the direct sum over every star. */
-CCF_D double2 eval_df_mixed(const FieldView& F, int leaf, double2 z, double2 s3_off)
+CCF_D double2 eval_df_widen(const FieldView& F, int leaf, double2 z, double2 s3_off, float2 d)
 {
-	const float2 d = eval_df32(F, leaf, z, s3_off);
 	if (isfinite(d.x) && isfinite(d.y)) return make_double2(d.x, d.y);
 	double2 s3 = s3_off, d2l = make_double2(0, 0);
 	if (leaf >= 0)
@@ -520,6 +530,10 @@ CCF_D double2 eval_df_mixed(const FieldView& F, int leaf, double2 z, double2 s3_
 	}
 	const double2 d2s = smooth_d2zbar(F, z);
 	return make_double2(-2 * F.theta2 * s3.x - d2l.x - d2s.x, -2 * F.theta2 * s3.y - d2l.y + d2s.y);
+}
+CCF_D double2 eval_df_mixed(const FieldView& F, int leaf, double2 z, double2 s3_off)
+{
+	return eval_df_widen(F, leaf, z, s3_off, eval_df32(F, leaf, z, s3_off));
 }
 
 /* everything the epilogue needs at a final root: the 1/mu error bound

@@ -209,8 +209,11 @@ struct RowState
 	int total, late;             /* roots of the sweep's list: active; made final by its check */
 	int split, tpt, chunks, tiles;   /* the shape of its sums */
 	int complete;
-	int pad[3];
+	int blk;                     /* roots per unit of the phases that evaluate roots */
+	int pad[2];
 };
+
+constexpr int ROWS_MIN_BLOCK = 64;   /* fewest roots of a unit of rows_kernel */
 
 struct SolveArgs
 {

@@ -17,7 +17,7 @@ Here a row's sweep is two phases of independent units,
          stars): FP32 (FP64) partial sums per target, chunk and source share;
 
 with a first check before them and the outputs (epilogue, and the next phi
-step's first check) after them, both over blocks of 256 consecutive roots.  The
+step's first check) after them, both over blocks of 64 to 256 consecutive roots.  The
 steps go over the list, not the row: after a few sweeps a block of the row
 holds a handful of active roots and costs as much as a full one.  The list
 keeps the row's order (each unit writes its survivors in order, and the CTA
@@ -45,6 +45,7 @@ per target, chunk and share, so large launches run PARTIAL_BYTES of rows at a
 time; ccf_continue_branch_noalloc, which has no memory for them, keeps
 solve_kernel.
 ******************************************************************************/
+#define CCF_EVAL_UNROLL 4
 #include "solver_dev.cuh"
 
 #include <algorithm>
@@ -77,13 +78,28 @@ CCF_D unsigned long long load_cg(const unsigned long long* p) { return __ldcg(p)
 CCF_D int load_volatile(const int* p) { return *(const volatile int*)p; }
 
 /* start of segment r of a row of R roots: the roots that CTA r of a cluster of
-   csize owns in solve_kernel.  Blocks of 256 roots start at these. */
+   csize owns in solve_kernel.  A row's blocks of roots start at these. */
 CCF_D int segment_start(int R, int csize, int r) { return (int)((long long)R * r / csize); }
-CCF_D int row_blocks(int R, int csize)
+constexpr int MIN_BLOCK = ROWS_MIN_BLOCK;
+constexpr int NO_ROOT = 1 << 20;   /* a thread past its unit's block */
+CCF_D int row_blocks(int R, int csize, int blk)
 {
 	int n = 0;
-	for (int r = 0; r < csize; r++) n += (segment_start(R, csize, r + 1) - segment_start(R, csize, r) + NT - 1) / NT;
+	for (int r = 0; r < csize; r++) n += (segment_start(R, csize, r + 1) - segment_start(R, csize, r) + blk - 1) / blk;
 	return n;
+}
+
+/* Roots per unit of a phase that evaluates n roots of each row (a step, a
+   first check, an epilogue): 64, 128 or 256, the fewest that leave no more
+   units than CTAs.  A unit's time is its roots' FP64 work and the chain of one
+   evaluation: with two warps in a CTA instead of eight each scheduler's FP64
+   pipe serves one of them (a step of 64 roots 33 us, of 256 51; the full-sum
+   continuation of 400 stars, 4 branches of 32 steps, 4.8 ms against 5.5). */
+CCF_D int block_roots(int n, int rows, int ctas)
+{
+	int blk = MIN_BLOCK;
+	while (blk < NT && (long long)rows * ((n + blk - 1) / blk) > ctas) blk *= 2;
+	return blk;
 }
 
 /* The source split of a sweep with `total` active roots, for the shortest
@@ -137,9 +153,11 @@ struct RowShared
 	int row;                /* the row F, O, R belong to; -1: none */
 	int cur;                /* the row this CTA started; -1: none */
 	int unit, units, phase, it, j, total, late, split;
+	int blk;                /* roots per unit of the phase (not of the sums) */
 	SumsShape shape;
 	int last;               /* this CTA finished the phase's last unit */
-	int seg_start[MAX_CLUSTER + 1];   /* of the row's segments, and their blocks of 256 before each */
+	int seg_blk;
+	int seg_start[MAX_CLUSTER + 1];   /* of the row's segments, and their blocks of seg_blk before each */
 	int seg_block[MAX_CLUSTER + 1];
 	int phase_j;            /* the step that sphi, cphi belong to; -1: none */
 	double sphi, cphi;
@@ -161,7 +179,7 @@ static_assert(OFF_CAP * (NT / 32) * 6 * sizeof(double) <= 2 * CHUNK * 16, "off-f
    ones go to the share's end: their snapshot is due with the next step's (after
    the sums, as the others').  Every thread of the CTA calls it. */
 template <bool MIXED>
-__device__ void check_roots(const SolveArgs& A, RowShared<MIXED>& S, int* share, int* counts, int a, bool act, double2 z,
+__device__ void check_roots(const SolveArgs& A, RowShared<MIXED>& S, int* share, int* counts, int blk, int a, bool act, double2 z,
 	double cphi, double sphi, bool initial)
 {
 	const FieldView& F = S.F;
@@ -222,7 +240,7 @@ __device__ void check_roots(const SolveArgs& A, RowShared<MIXED>& S, int* share,
 		nl += S.warp_late[w];
 	}
 	if (still) share[g] = a;
-	if (late) share[NT - 1 - gl] = a;
+	if (late) share[blk - 1 - gl] = a;
 	if (threadIdx.x == 0)
 	{
 		*counts = n | nl << 16;
@@ -238,7 +256,7 @@ __device__ void check_roots(const SolveArgs& A, RowShared<MIXED>& S, int* share,
    its start, the late ones from its end.  The whole CTA; the totals come back
    in Sh.total and Sh.late. */
 template <bool MIXED>
-__device__ void join_list(RowShared<MIXED>& S, const int* share, const int* counts, int units, int* list, int R)
+__device__ void join_list(RowShared<MIXED>& S, const int* share, const int* counts, int units, int blk, int* list, int R)
 {
 	const unsigned full = 0xffffffffu;
 	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -283,9 +301,9 @@ __device__ void join_list(RowShared<MIXED>& S, const int* share, const int* coun
 		{
 			const int kn = __shfl_sync(full, n, k), kl = __shfl_sync(full, nl, k);
 			const int kx = __shfl_sync(full, x, k), ky = __shfl_sync(full, y, k);
-			const int* from = share + (size_t)(u0 + warp * 32 + k) * NT;
+			const int* from = share + (size_t)(u0 + warp * 32 + k) * blk;
 			for (int i = lane; i < kn; i += 32) list[kx + i] = __ldcg(from + i);
-			for (int i = lane; i < kl; i += 32) list[R - 1 - (ky + i)] = __ldcg(from + NT - 1 - i);
+			for (int i = lane; i < kl; i += 32) list[R - 1 - (ky + i)] = __ldcg(from + blk - 1 - i);
 		}
 		carry += tx;
 		carry_late += ty;
@@ -532,6 +550,7 @@ __global__ void __launch_bounds__(NT, 2) rows_kernel(const SolveArgs A, const in
 			Sh.total = load_volatile(&st->total);
 			Sh.late = load_volatile(&st->late);
 			Sh.split = load_volatile(&st->split);
+			Sh.blk = load_volatile(&st->blk);
 			Sh.shape.tpt = load_volatile(&st->tpt);
 			Sh.shape.chunks = load_volatile(&st->chunks);
 			Sh.shape.tiles = load_volatile(&st->tiles);
@@ -568,7 +587,8 @@ __global__ void __launch_bounds__(NT, 2) rows_kernel(const SolveArgs A, const in
 						}
 						else
 						{
-							const int units = row_blocks(A.fields[rd.field].num_roots, csize);
+							const int nr0 = A.fields[rd.field].num_roots, blk = block_roots(nr0, rows_at_work, (int)gridDim.x);
+							const int units = row_blocks(nr0, csize, blk);
 							Sh.cur = nr;
 							Sh.claimed = nr;
 							Sh.unit = 0;
@@ -578,9 +598,11 @@ __global__ void __launch_bounds__(NT, 2) rows_kernel(const SolveArgs A, const in
 							Sh.j = first;
 							Sh.total = Sh.late = 0;
 							Sh.split = 1;
+							Sh.blk = blk;
 							got = true;
 							/* the state is zero: phase, it, counts */
 							st->j = first;
+							st->blk = blk;
 							if (units > 1)
 							{
 								__threadfence();
@@ -643,13 +665,15 @@ __global__ void __launch_bounds__(NT, 2) rows_kernel(const SolveArgs A, const in
 			__syncthreads();
 			if (threadIdx.x == 0)
 			{
+				const int blk = block_roots(A.fields[field].num_roots, rows_at_work, (int)gridDim.x);
 				int n = 0;
 				for (int r = 0; r < csize; r++)
 				{
 					Sh.seg_block[r] = n;
-					n += (Sh.seg_start[r + 1] - Sh.seg_start[r] + NT - 1) / NT;
+					n += (Sh.seg_start[r + 1] - Sh.seg_start[r] + blk - 1) / blk;
 				}
 				Sh.seg_block[csize] = n;
+				Sh.seg_blk = blk;
 			}
 		}
 		const FieldView& F = Sh.F;
@@ -678,7 +702,8 @@ __global__ void __launch_bounds__(NT, 2) rows_kernel(const SolveArgs A, const in
 		int* const list = A.list + base;
 		int* const shares = A.share + (size_t)(row % A.part_slots) * A.share_stride;
 		int* const counts = A.counts + (size_t)(row % A.part_slots) * A.counts_stride;
-		int* const share = shares + (size_t)Sh.unit * NT;
+		const int blk = Sh.blk, tid = threadIdx.x < blk ? (int)threadIdx.x : NO_ROOT;
+		int* const share = shares + (size_t)Sh.unit * blk;
 		typename PartT<MIXED>::T* part = reinterpret_cast<typename PartT<MIXED>::T*>(A.part) +
 			(size_t)(row % A.part_slots) * A.part_stride;
 
@@ -694,9 +719,9 @@ __global__ void __launch_bounds__(NT, 2) rows_kernel(const SolveArgs A, const in
 			if (Sh.phase == PHASE_STEP)
 			{
 				/* the roots of the list, then those made final by the last check */
-				const int g = Sh.unit * NT + threadIdx.x, total = Sh.total;
-				bool act = g < total;
-				const bool own = g < total + Sh.late;
+				const int g = Sh.unit * blk + threadIdx.x, total = Sh.total;
+				const bool own = tid < NO_ROOT && g < total + Sh.late;
+				bool act = own && g < total;
 				const int a = own ? __ldcg(list + (act ? g : R - 1 - (g - total))) : 0;
 				double2 z = own ? __ldcg(A.master + base + a) : make_double2(0, 0);
 				double2 totR, totS;
@@ -734,16 +759,16 @@ __global__ void __launch_bounds__(NT, 2) rows_kernel(const SolveArgs A, const in
 					if constexpr (MIXED) A.snap32[base + a] = split_hilo(z);
 					else A.snap64[base + a] = z;
 				}
-				if (Sh.it < max_it) check_roots<MIXED>(A, Sh, share, counts + Sh.unit, a, act, z, cphi, sphi, initial);
+				if (Sh.it < max_it) check_roots<MIXED>(A, Sh, share, counts + Sh.unit, blk, a, act, z, cphi, sphi, initial);
 			}
 			else
 			{
 				/* the block's roots */
 				int r = 0;
 				while (r + 1 < csize && Sh.unit >= Sh.seg_block[r + 1]) r++;
-				const int a = Sh.seg_start[r] + (Sh.unit - Sh.seg_block[r]) * NT + threadIdx.x;
+				const int a = Sh.seg_start[r] + (Sh.unit - Sh.seg_block[r]) * blk + threadIdx.x;
 				const int o1 = Sh.seg_start[r + 1];
-				const bool own = a < o1;
+				const bool own = tid < NO_ROOT && a < o1;
 				const double2 z = own ? __ldcg(A.master + base + a) : make_double2(0, 0);
 				bool check = true;
 				if (Sh.phase == PHASE_EPILOGUE)
@@ -814,7 +839,7 @@ __global__ void __launch_bounds__(NT, 2) rows_kernel(const SolveArgs A, const in
 				if (check)
 				{
 					if (own) A.fin[base + a] = 0;
-					check_roots<MIXED>(A, Sh, share, counts + Sh.unit, a, own, z, cphi, sphi, initial);
+					check_roots<MIXED>(A, Sh, share, counts + Sh.unit, blk, a, own, z, cphi, sphi, initial);
 				}
 			}
 		}
@@ -848,7 +873,7 @@ __global__ void __launch_bounds__(NT, 2) rows_kernel(const SolveArgs A, const in
 		__syncthreads();
 		if (!Sh.last) continue;
 		/* the next phase */
-		if (checked) join_list<MIXED>(Sh, shares, counts, Sh.units, list, R);
+		if (checked) join_list<MIXED>(Sh, shares, counts, Sh.units, blk, list, R);
 		if (threadIdx.x == 0)
 		{
 			unsigned long long* stats = O.stats;
@@ -857,7 +882,8 @@ __global__ void __launch_bounds__(NT, 2) rows_kernel(const SolveArgs A, const in
 			{
 				phase = PHASE_STEP;
 				Sh.it++;
-				units = (Sh.total + Sh.late + NT - 1) / NT;
+				Sh.blk = block_roots(Sh.total + Sh.late, rows_at_work, (int)gridDim.x);
+				units = (Sh.total + Sh.late + Sh.blk - 1) / Sh.blk;
 			}
 			else
 			{
@@ -887,6 +913,7 @@ __global__ void __launch_bounds__(NT, 2) rows_kernel(const SolveArgs A, const in
 				else
 				{
 					phase = PHASE_EPILOGUE;
+					Sh.blk = Sh.seg_blk;
 					units = Sh.seg_block[csize];
 				}
 			}
@@ -904,6 +931,7 @@ __global__ void __launch_bounds__(NT, 2) rows_kernel(const SolveArgs A, const in
 					st->total = Sh.total;
 					st->late = Sh.late;
 					st->split = Sh.split;
+					st->blk = Sh.blk;
 					st->tpt = Sh.shape.tpt;
 					st->chunks = Sh.shape.chunks;
 					st->tiles = Sh.shape.tiles;
@@ -942,7 +970,7 @@ cudaError_t launch_rows(cudaStream_t s, const SolveArgs& a, bool mixed, bool ini
 	}
 	/* as many CTAs as the rows can ever have units for */
 	const long long chunks = (max_roots + CHUNK - 1) / CHUNK + (max_stars + CHUNK - 1) / CHUNK;
-	const long long units = std::max<long long>(max_roots / NT + a.cluster, chunks * ((max_roots + 31) / 32));
+	const long long units = std::max<long long>(max_roots / MIN_BLOCK + a.cluster, chunks * ((max_roots + 31) / 32));
 	const int blocks = (int)std::min<long long>((long long)num_sms * per_sm, units * a.num_rows);
 	if (mixed) rows_kernel<true><<<blocks, NT, 0, s>>>(a, initial ? 1 : 0);
 	else rows_kernel<false><<<blocks, NT, 0, s>>>(a, initial ? 1 : 0);

@@ -150,8 +150,7 @@ static __device__ __noinline__ FdF eval_fdf_warp(const FieldView& F, bool valid,
 	{
 		/* f in double-float on the FP32 pipe, off-field points included;
 		   f' in FP32, or FP64 where FP32 overflows */
-		r.f = eval_f_df(F, leaf, z, cphi, sphi, ns);
-		r.df = eval_df_mixed(F, leaf, z, ns.s3);
+		eval_fdf_df(F, leaf, z, cphi, sphi, ns, r.f, r.df);
 	}
 	else
 	{

@@ -80,3 +80,19 @@ def test_rows_are_the_cluster_kernels(n, rectangular):
     # the centre's snapshot is refreshed one sweep apart in the two, by less than the 1e-9 theta_star tolerance:
     # the sums' 1e-9 changes a converging step's end quadratically less
     assert np.max(np.abs(z - want)) <= 1e-11
+
+
+@pytest.mark.parametrize("precision", ["mixed", "fp64"])
+@pytest.mark.parametrize("n", [31, 32, 33, 64, 65, 321])
+def test_rows_do_not_depend_on_the_blocks(n, precision):
+    """Alone a field's steps and checks go over blocks of 64 roots, in a batch
+    of 40 over 128 or 256: the same bits in the solved column."""
+    a = field(n, 0, nb=8, num_phi=64, continuation="aberth", precision=precision, init_cluster=1)
+    assert a.run(-1), a.last_error()
+    r = a.results()
+    fs = [field(n, 0, nb=8, num_phi=64, continuation="aberth", precision=precision, init_cluster=1) for _ in range(40)]
+    assert run_batch(fs, -1), fs[0].last_error()
+    for f in (fs[0], fs[-1]):
+        b = f.results()
+        assert np.array_equal(r["ccs"][:, 4], b["ccs"][:, 4])
+        assert O.match_sets(r["ccs"], b["ccs"], 8)["max_dist"] <= 1e-11
