@@ -190,8 +190,9 @@ ccf_status Engine::rows_setup(SolveArgs& A, int which, const std::vector<Field*>
 /* room for the roots that leave the box: a few per row do (20 of 160 000 on
    the 20 000-star field); those beyond it stay in their items */
 constexpr int FAR_EVICT_CAP = 8192;
+constexpr int OUT_LIST_CAP = 1 << 18;   /* 2 MB */
 
-cudaError_t Engine::far_setup(TrackArgs& T, long long roots, long long smooth, int max_stars)
+cudaError_t Engine::far_setup(TrackArgs& T, long long roots, long long smooth, int max_stars, long long out_points)
 {
 	cudaError_t e;
 	if (!side.side)
@@ -206,6 +207,10 @@ cudaError_t Engine::far_setup(TrackArgs& T, long long roots, long long smooth, i
 	T.num_evict = pools.rerun_count.ptr + 6;
 	T.evict_counter = pools.rerun_count.ptr + 7;
 	T.far_evicted = T.solo_far = 0;
+	T.out_cap = (int)std::min<long long>(out_points, OUT_LIST_CAP);
+	if (T.out_cap > 0 && (e = pools.out_list.ensure(T.out_cap)) != cudaSuccess) return e;
+	T.out_list = pools.out_list.ptr;
+	T.num_out = pools.rerun_count.ptr + 10;
 	T.num_roots = roots;
 	T.solo_guess = T.num_rows + smooth / 3;
 	T.max_stars = max_stars;
@@ -216,6 +221,7 @@ void Engine::far_counts(TrackArgs& T2)
 {
 	T2.num_evict = pools.rerun_count.ptr + 8;
 	T2.evict_counter = pools.rerun_count.ptr + 9;
+	T2.num_out = pools.rerun_count.ptr + 11;
 }
 
 ccf_status Engine::cuda_fail(cudaError_t e, const char* what)
@@ -1109,7 +1115,7 @@ ccf_status Engine::solve(std::vector<Field*>& fields, int verbose)
 		CCF_TRY(P.track_table.ensure(table_slots), "cudaMalloc(tables)");
 		CCF_TRY(P.row_stats.ensure(TRACK_ROW_STATS * rc.size()), "cudaMalloc(rows)");
 		CCF_TRY(P.rows_rerun.ensure(rc.size()), "cudaMalloc(rows)");
-		CCF_TRY(P.rerun_count.ensure(10), "cudaMalloc(rows)");
+		CCF_TRY(P.rerun_count.ensure(12), "cudaMalloc(rows)");
 		CCF_TRY(P.rows_rerun2.ensure(rc.size()), "cudaMalloc(rows)");
 		CCF_TRY(P.row_stats2.ensure(TRACK_ROW_STATS * rc.size()), "cudaMalloc(rows)");
 		CCF_TRY(P.item_start.ensure(rc.size()), "cudaMalloc(rows)");
@@ -1181,7 +1187,7 @@ ccf_status Engine::solve(std::vector<Field*>& fields, int verbose)
 		T.max_sub = TRACK_TSUB;
 		T.scales = 0;
 		for (Field* f : fields) T.scales |= f->params.write_mu_length_scales ? 1 : 0;
-		output_launches = !mixed || T.scales ? 2 : 0;
+		output_launches = !mixed || T.scales ? 4 : 0;
 		T.num_items = 0;
 		long long max_row_points = 0;   /* the column check's points of the longest row */
 		for (size_t r = 0; r < rc.size(); r++)
@@ -1199,11 +1205,11 @@ ccf_status Engine::solve(std::vector<Field*>& fields, int verbose)
 		T.is_solo = P.is_solo.ptr;
 		long long smooth_roots = 0;
 		for (const RowDesc& r : rc) smooth_roots += fields[r.field]->d.num_roots - 2 * fields[r.field]->d.num_stars;
-		CCF_TRY(far_setup(T, ncont, smooth_roots, max_stars), "cudaMalloc(far roots)");
+		CCF_TRY(far_setup(T, ncont, smooth_roots, max_stars, output_launches ? (long long)rc.size() * max_row_points : 0), "cudaMalloc(far roots)");
 		CCF_TRY(cudaMemsetAsync(T.num_solo, 0, sizeof(int), s), "memset");
 		CCF_TRY(cudaMemsetAsync(P.track_table.ptr, 0, table_slots * sizeof(unsigned long long), s), "memset");
 		CCF_TRY(cudaMemsetAsync(P.row_stats.ptr, 0, TRACK_ROW_STATS * rc.size() * sizeof(unsigned long long), s), "memset");
-		CCF_TRY(cudaMemsetAsync(P.rerun_count.ptr, 0, 10 * sizeof(int), s), "memset");
+		CCF_TRY(cudaMemsetAsync(P.rerun_count.ptr, 0, 12 * sizeof(int), s), "memset");
 		CCF_TRY(cudaMemsetAsync(P.row_stats2.ptr, 0, TRACK_ROW_STATS * rc.size() * sizeof(unsigned long long), s), "memset");
 		T.run_items = T.num_items;
 		CCF_TRY(P.item_order.ensure((size_t)T.num_items + 1), "cudaMalloc(items)");

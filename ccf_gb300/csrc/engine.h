@@ -212,9 +212,11 @@ struct SolverPools
 	DBuf<int> rerun_count;                  /* [0] rows to re-track, [1] [2] tracker work counters,
 	                                           [3] rows to re-run, [4] [5] re-tracking work counters,
 	                                           [6] [7] roots that left the box and the next of them,
-	                                           [8] [9] the same of the re-tracking */
+	                                           [8] [9] the same of the re-tracking, [10] [11] listed
+	                                           points of either */
 	DBuf<int> item_start;                   /* first tracker work item of each continuation row */
 	DBuf<int2> solo;                        /* tracker roots run alone, and their count after them */
+	DBuf<unsigned long long> out_list;      /* tracked points off the root box, for their FP64 outputs */
 	DBuf<FarState> evict;                   /* tracker roots that left the root box */
 	DBuf<unsigned char> is_solo;            /* per continuation root */
 	DBuf<unsigned long long> polish_list;   /* [0] count, then the points the FP64 polish works on */
@@ -321,7 +323,7 @@ private:
 	   first tracking; T2 takes its counts from far_counts); roots = all rows',
 	   smooth = those of them beyond two per star (the Taylor form's), of which
 	   about a third start off the root box or leave it */
-	cudaError_t far_setup(TrackArgs& T, long long roots, long long smooth, int max_stars);
+	cudaError_t far_setup(TrackArgs& T, long long roots, long long smooth, int max_stars, long long out_points);
 	void far_counts(TrackArgs& T2);
 
 	TrackSide side;   /* the stream the far launch runs on, beside the items */

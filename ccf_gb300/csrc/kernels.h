@@ -301,6 +301,11 @@ struct TrackArgs
 	const int* num_rows_dev;    /* when set: the number of rows, on the device */
 	int items_per_row;          /* when > 0: item = row * items_per_row + chunk */
 	int max_sub;                /* longest sub-step (TSUB = a whole phi step) */
+	/* the points off the root box whose FP64 outputs are due (launch_track_outputs):
+	   row << 32 | point of the row */
+	unsigned long long* out_list;
+	int* num_out;               /* their number (zeroed before the tracking launch) */
+	int out_cap;                /* beyond it they are formed with the others */
 	int scales;                 /* a field of the launch writes length scales */
 };
 

@@ -2023,11 +2023,59 @@ __global__ void track_check_kernel(const TrackArgs T)
    and so with the same bits as in the tracking loop.  There a warp formed them
    for the few lanes that had just converged, at a full warp's cost on the
    1/64-rate FP64 pipe (half the continuation of a 419-star rectangle with
-   length scales, 420 phi steps: 9.1 ms, 4.7 with this launch; 600 stars in
-   FP64, 256 steps: 11.0 ms, 8.2).  Bound by that pipe at full lanes.  Consecutive lanes are consecutive phi steps of one root,
+   length scales, 420 phi steps: 9.1 ms, 4.4 with these launches; 600 stars in
+   FP64, 256 steps: 11.0 ms, 7.9).  Bound by that pipe at full lanes.  Consecutive lanes are consecutive phi steps of one root,
    mostly in one leaf.  The roots are read back from the output arrays, their
    slot's 1/mu error saying that the outputs are due.  A row that lost a root
-   has slots without one and is tracked again or re-run: it is skipped. */
+   has slots without one and is tracked again or re-run: it is skipped.
+
+   A point off the root box is summed over every star by its whole warp, and
+   such roots stand together at the end of a rectangle's, so a few warps had 32
+   of those sums one after another and outlasted the launch by half.  They are
+   listed, and a second launch forms them eight to a warp (the rest of a point's
+   work costs a warp the same for one lane as for eight): on the 419-star
+   rectangle 1.15 + 0.30 ms, 1.7 before. */
+constexpr int OUT_GROUP = 8;
+
+/* the outputs of the lanes with v set: point i of row q's, at leaf */
+template <bool MIXED>
+__device__ bool track_point_outputs(const TrackArgs& T, const FieldView& F, const FieldOut& O, const RowDesc& RD, long long i,
+	bool listing, unsigned long long q, bool v, double* maxerr)
+{
+	const unsigned full = 0xffffffffu;
+	const int lane = threadIdx.x & 31;
+	const int j0 = O.step_first, nsteps = RD.steps - j0 + 1;
+	const int a = v ? (int)(i / nsteps) : 0, j = v ? j0 + (int)(i - (long long)a * nsteps) : j0;
+	int ob[2], ok[2];
+	const int nslot = row_slots(O.nb, O.half, O.seg, RD.branch, RD.side, j, ob, ok);
+	const size_t out = out_slot(O, a, ob[0], ok[0]);
+	const size_t out2 = nslot > 1 ? out_slot(O, a, ob[1], ok[1]) : NO_SLOT;
+	const size_t from = out != NO_OUT ? out : out2;
+	const double due = v && from != NO_SLOT ? O.errs[from] : 0;
+	const bool stuck = due == OUTPUT_DUE_STALLED;
+	v = stuck || due == OUTPUT_DUE;
+	const double2 z = v ? O.ccs[from] : make_double2(0, 0);
+	const double2 cs = O.phase[row_global_step(O.nb, O.half, RD.branch, RD.side, j)].cs;
+	const int leaf = v ? find_leaf(F, z) : 0;
+	if (listing)
+	{
+		const bool off = v && leaf < 0;
+		const unsigned m = __ballot_sync(full, off);
+		if (m)
+		{
+			int at = T.out_cap;
+			if (lane == 0 && *(const volatile int*)T.num_out < T.out_cap) at = atomicAdd(T.num_out, __popc(m));
+			at = __shfl_sync(full, at, 0) + __popc(m & ((1u << lane) - 1u));
+			if (off && at < T.out_cap)
+			{
+				T.out_list[at] = q << 32 | (unsigned long long)i;
+				v = false;
+			}
+		}
+	}
+	return point_epilogue_warp<MIXED>(F, O, v, z, leaf, false, zero_sums(), out, out2, cs.x, cs.y, maxerr, stuck);
+}
+
 template <bool MIXED>
 __global__ void __launch_bounds__(128) track_outputs_kernel(const TrackArgs T)
 {
@@ -2050,29 +2098,14 @@ __global__ void __launch_bounds__(128) track_outputs_kernel(const TrackArgs T)
 			s_max = 0;
 		}
 		__syncthreads();
-		const FieldView& F = sF;
-		const FieldOut& O = sO;
-		const int R = F.num_roots;
-		const int j0 = O.step_first, nsteps = RD.steps - j0 + 1;
+		const int R = sF.num_roots, nsteps = RD.steps - sO.step_first + 1;
 		const long long n = (long long)R * max(nsteps, 0);
+		const bool listing = n < 1LL << 32;
 		unsigned flags = 0;
 		for (long long i0 = (long long)blockIdx.x * blockDim.x; i0 < n; i0 += (long long)gridDim.x * blockDim.x)
 		{
 			const long long i = i0 + threadIdx.x;
-			bool v = i < n;
-			const int a = v ? (int)(i / nsteps) : 0, j = v ? j0 + (int)(i - (long long)a * nsteps) : j0;
-			int ob[2], ok[2];
-			const int nslot = row_slots(O.nb, O.half, O.seg, RD.branch, RD.side, j, ob, ok);
-			const size_t out = out_slot(O, a, ob[0], ok[0]);
-			const size_t out2 = nslot > 1 ? out_slot(O, a, ob[1], ok[1]) : NO_SLOT;
-			const size_t from = out != NO_OUT ? out : out2;
-			const double due = v && from != NO_SLOT ? O.errs[from] : 0;
-			const bool stuck = due == OUTPUT_DUE_STALLED;
-			v = stuck || due == OUTPUT_DUE;
-			const double2 z = v ? O.ccs[from] : make_double2(0, 0);
-			const double2 cs = O.phase[row_global_step(O.nb, O.half, RD.branch, RD.side, j)].cs;
-			const int leaf = v ? find_leaf(F, z) : 0;
-			if (!point_epilogue_warp<MIXED>(F, O, v, z, leaf, false, zero_sums(), out, out2, cs.x, cs.y, &s_max, stuck))
+			if (!track_point_outputs<MIXED>(T, sF, sO, RD, i, listing, (unsigned long long)q, i < n, &s_max))
 				flags |= (unsigned)TRACK_NONFINITE;
 		}
 		flags = __reduce_or_sync(full, flags);
@@ -2083,14 +2116,51 @@ __global__ void __launch_bounds__(128) track_outputs_kernel(const TrackArgs T)
 	}
 }
 
-cudaError_t launch_track_outputs(cudaStream_t s, const TrackArgs& a, bool mixed, long long max_row_points)
+/* the listed points, OUT_GROUP to a warp; the group's rows one after another
+   (mostly one) */
+template <bool MIXED>
+__global__ void __launch_bounds__(128) track_outputs_off_kernel(const TrackArgs T)
 {
-	if (a.num_rows == 0 || max_row_points <= 0 || (mixed && !a.scales)) return cudaSuccess;
+	const unsigned full = 0xffffffffu;
+	const int lane = threadIdx.x & 31;
+	const int n = min(*T.num_out, T.out_cap);
+	for (int g = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); g * OUT_GROUP < n; g += gridDim.x * (blockDim.x >> 5))
+	{
+		const int e = g * OUT_GROUP + lane;
+		const bool mine = lane < OUT_GROUP && e < n;
+		const unsigned long long at = mine ? T.out_list[e] : 0;
+		unsigned pend = __ballot_sync(full, mine);
+		while (pend)
+		{
+			const int q = (int)(__shfl_sync(full, at, __ffs(pend) - 1) >> 32);
+			const bool now = mine && (int)(at >> 32) == q;
+			pend &= ~__ballot_sync(full, now);
+			const RowDesc RD = T.rows[q];
+			unsigned long long* rs = T.row_stats + TRACK_ROW_STATS * (size_t)q;
+			if (!track_point_outputs<MIXED>(T, T.fields[RD.field], T.outs[RD.field], RD, (long long)(at & 0xffffffffu), false, 0, now,
+					reinterpret_cast<double*>(&rs[0])))
+				atomicOr(&rs[1], TRACK_NONFINITE);
+		}
+	}
+}
+
+template <bool MIXED>
+cudaError_t launch_track_outputs_form(cudaStream_t s, const TrackArgs& a, long long max_row_points)
+{
 	/* a bounded number of CTAs per row: the re-tracking's launch finds few rows */
 	const dim3 grid((unsigned)std::min<long long>((max_row_points + 127) / 128, 4096), (unsigned)std::min(a.num_rows, 65535));
-	if (mixed) track_outputs_kernel<true><<<grid, 128, 0, s>>>(a);
-	else track_outputs_kernel<false><<<grid, 128, 0, s>>>(a);
+	track_outputs_kernel<MIXED><<<grid, 128, 0, s>>>(a);
+	cudaError_t e = cudaGetLastError();
+	if (e != cudaSuccess) return e;
+	const int groups = (a.out_cap + OUT_GROUP - 1) / OUT_GROUP;
+	track_outputs_off_kernel<MIXED><<<std::min((groups + 3) / 4, 1024), 128, 0, s>>>(a);
 	return cudaGetLastError();
+}
+
+cudaError_t launch_track_outputs(cudaStream_t s, const TrackArgs& a, bool mixed, long long max_row_points)
+{
+	if (a.num_rows == 0 || max_row_points <= 0 || a.out_cap <= 0 || (mixed && !a.scales)) return cudaSuccess;
+	return mixed ? launch_track_outputs_form<true>(s, a, max_row_points) : launch_track_outputs_form<false>(s, a, max_row_points);
 }
 
 cudaError_t launch_track_check(cudaStream_t s, const TrackArgs& a, long long max_row_points)

@@ -312,7 +312,7 @@ ccf_status Engine::solve_chunked(Field& f, int verbose)
 		CCF_TRY_S(P.row_stats2.ensure(TRACK_ROW_STATS * grows), "cudaMalloc(rows)");
 		CCF_TRY_S(P.rows_rerun.ensure(grows), "cudaMalloc(rows)");
 		CCF_TRY_S(P.rows_rerun2.ensure(grows), "cudaMalloc(rows)");
-		CCF_TRY_S(P.rerun_count.ensure(10), "cudaMalloc(rows)");
+		CCF_TRY_S(P.rerun_count.ensure(12), "cudaMalloc(rows)");
 		CCF_TRY_S(P.item_start.ensure(rc.size()), "cudaMalloc(rows)");
 		CCF_TRY_S(P.solo.ensure((size_t)ncont + 1), "cudaMalloc(rows)");
 		CCF_TRY_S(P.is_solo.ensure((size_t)ncont), "cudaMalloc(rows)");
@@ -439,11 +439,12 @@ ccf_status Engine::solve_chunked(Field& f, int verbose)
 			T.solo = P.solo.ptr;
 			T.num_solo = reinterpret_cast<int*>(P.solo.ptr + ncont);
 			T.is_solo = P.is_solo.ptr;
-			CCF_TRY_S(far_setup(T, (long long)grows * R, (long long)grows * (R - 2 * f.d.num_stars), f.d.num_stars), "cudaMalloc(far roots)");
+			CCF_TRY_S(far_setup(T, (long long)grows * R, (long long)grows * (R - 2 * f.d.num_stars), f.d.num_stars,
+				!mixed || T.scales ? (long long)grows * R * seg * half : 0), "cudaMalloc(far roots)");
 			CCF_TRY_S(cudaMemsetAsync(T.num_solo, 0, sizeof(int), s), "memset");
 			CCF_TRY_S(cudaMemsetAsync(P.track_table.ptr, 0, gr.table_slots * sizeof(unsigned long long), s), "memset");
 			CCF_TRY_S(cudaMemsetAsync(P.row_stats.ptr, 0, TRACK_ROW_STATS * grows * sizeof(unsigned long long), s), "memset");
-			CCF_TRY_S(cudaMemsetAsync(P.rerun_count.ptr, 0, 10 * sizeof(int), s), "memset");
+			CCF_TRY_S(cudaMemsetAsync(P.rerun_count.ptr, 0, 12 * sizeof(int), s), "memset");
 			CCF_TRY_S(cudaMemsetAsync(P.row_stats2.ptr, 0, TRACK_ROW_STATS * grows * sizeof(unsigned long long), s), "memset");
 			CCF_TRY_S(P.item_order.ensure((size_t)T.num_items + 1), "cudaMalloc(items)");
 			CCF_TRY_S(P.item_work.ensure(3 * (size_t)T.num_items + 3), "cudaMalloc(items)");
@@ -508,7 +509,7 @@ ccf_status Engine::solve_chunked(Field& f, int verbose)
 	   table clearing, re-tracking in two, column check, collection) and the full-sum
 	   launch, the FP64 outputs of both trackings where they are formed after them, or the full-sum launch alone, then the polish (2); and the item
 	   order where a group reorders its items */
-	return finish_stats(f, seg, track, verbose, (track ? 5 : 4) + (track ? 14 + (!mixed || f.params.write_mu_length_scales ? 2 : 0) : 3) * ngroups + reordered_groups);
+	return finish_stats(f, seg, track, verbose, (track ? 5 : 4) + (track ? 14 + (!mixed || f.params.write_mu_length_scales ? 4 : 0) : 3) * ngroups + reordered_groups);
 }
 
 } /* namespace ccf */
