@@ -814,7 +814,8 @@ ccf_status Engine::finish_view(Field& f, int P, double near_sum, int lerr, Uploa
 				const cl v = cl(0.0L, kpi) * std::conj(cl(sp.a[n].real(), sp.a[n].imag()));
 				eq[n] = make_double2((double)v.real(), (double)v.imag());
 			}
-			CCF_TRY(f.fold_coef.ensure(coef.size()), "cudaMalloc(fold)");
+			/* the series, then the binomials of their shifts */
+			CCF_TRY(f.fold_coef.ensure(coef.size() + (fold_binom_size(2 * M + 1, 2 * M, na) + 1) / 2), "cudaMalloc(fold)");
 			CCF_TRY(cudaMemcpyAsync(f.fold_coef.ptr, coef.data(), coef.size() * sizeof(double2), cudaMemcpyHostToDevice, s),
 				"fold");
 			CCF_TRY(f.leaf_fold.ensure(nl), "cudaMalloc(fold)");
@@ -823,7 +824,8 @@ ccf_status Engine::finish_view(Field& f, int P, double near_sum, int lerr, Uploa
 			CCF_TRY(f.leaf_loc_fold64.ensure((size_t)nl * 3 * (P + 1)), "cudaMalloc(fold)");
 			launch_fold_smooth(s, nl, P, f.leaf_center.ptr, f.leaf_inv_half.ptr, f.leaf_loc.ptr, f.fold_coef.ptr, 2 * M + 1,
 				f.fold_coef.ptr + 2 * M + 1, 2 * M, f.fold_coef.ptr + 4 * M + 1, na, 0.95 * std::hypot(d.corner_x1, d.corner_x2),
-				f.leaf_loc_df_fold.ptr, f.leaf_loc_pk.ptr, f.leaf_loc3f_fold.ptr, f.leaf_loc_fold64.ptr, f.leaf_fold.ptr);
+				f.leaf_loc_df_fold.ptr, f.leaf_loc_pk.ptr, f.leaf_loc3f_fold.ptr, f.leaf_loc_fold64.ptr, f.leaf_fold.ptr,
+				reinterpret_cast<double*>(f.fold_coef.ptr + coef.size()));
 			CCF_TRY(cudaGetLastError(), "fold_smooth_kernel");
 			fold_host.resize(nl);
 			CCF_TRY(cudaMemcpyAsync(fold_host.data(), f.leaf_fold.ptr, nl, cudaMemcpyDeviceToHost, s), "fold");

@@ -45,18 +45,26 @@ CCF_D double2 shfl_c(double2 v, int src)
 }
 
 /* upward pass at one level: P2M for leaves holding stars, M2M for split
-   nodes.  The stars of a leaf are taken 32 at a time, one per lane, and
-   handed round the warp by shuffles; the powers come from warp_powers. */
-CCF_D void fmm_upward_node(const TreeDev& T, int n, int P, int p, const double2* __restrict__ pos,
+   nodes, by the block's UP_WARPS warps (every thread calls it).  The FP64 pipe
+   takes 64 cycles for each of a warp's instructions, and each of an SM's four
+   schedulers has one: the four children's translations run side by side, and
+   so do the powers of four stars at a time, which warp 0 adds up in order.
+   One warp per node: 36 us a level of a few nodes, 11 with four.  The stars of
+   a leaf are taken 32 at a time, one per lane, and handed round the warp by
+   shuffles; the powers come from warp_powers. */
+constexpr int UP_WARPS = 4;
+CCF_D void fmm_upward_node(const TreeDev& T, int n, int P, const double2* __restrict__ pos,
 	const double* __restrict__ mass, double2* __restrict__ multi, const double* __restrict__ B)
 {
+	__shared__ double2 terms[32][32];   /* [star][power], or [child][coefficient] */
+	const int p = threadIdx.x & 31, w = threadIdx.x >> 5;
 	const bool act = p <= P;
 	double2 r = make_double2(0, 0);
 	int ch = T.child[n];
 	if (ch < 0)
 	{
 		int s = T.star_start[n], ns = T.star_count[n];
-		if (ns == 0) return;   /* warp-uniform */
+		if (ns == 0) return;   /* block-uniform */
 		double2 c = T.center[n];
 		double ih = 1.0 / T.half[n];
 		for (int i0 = 0; i0 < ns; i0 += 32)
@@ -70,20 +78,26 @@ CCF_D void fmm_upward_node(const TreeDev& T, int n, int P, int p, const double2*
 				mq = mass[s + i0 + p];
 				wq = make_double2((q.x - c.x) * ih, (q.y - c.y) * ih);
 			}
-			for (int i = 0; i < nq; i++)
+			for (int i = w; i < nq; i += UP_WARPS) terms[i][p] = warp_powers(shfl_c(wq, i), p);
+			__syncthreads();
+			if (w == 0)
 			{
-				const double m = __shfl_sync(0xffffffffu, mq, i);
-				const double2 t = warp_powers(shfl_c(wq, i), p);
-				if (p == 0)
+				for (int i = 0; i < nq; i++)
 				{
-					r.x += m;
-				}
-				else
-				{
-					r.x -= t.x * m;
-					r.y -= t.y * m;
+					const double m = __shfl_sync(0xffffffffu, mq, i);
+					const double2 t = terms[i][p];
+					if (p == 0)
+					{
+						r.x += m;
+					}
+					else
+					{
+						r.x -= t.x * m;
+						r.y -= t.y * m;
+					}
 				}
 			}
+			__syncthreads();
 		}
 		if (p > 0)
 		{
@@ -93,40 +107,41 @@ CCF_D void fmm_upward_node(const TreeDev& T, int n, int P, int p, const double2*
 	}
 	else
 	{
+		static_assert(UP_WARPS == 4, "a warp per child");
 		double2 pc = T.center[n];
-		for (int q = 0; q < 4; q++)
+		int k = ch + w;
+		const double2* a = multi + (size_t)k * (P + 1);
+		double2 cc = T.center[k];
+		double ih = 1.0 / T.half[k];
+		double2 dz = make_double2((cc.x - pc.x) * ih, (cc.y - pc.y) * ih);
+		const double2 dzp = warp_powers(dz, p);
+		double2 v = make_double2(0, 0);
+		if (p == 0)
 		{
-			int k = ch + q;
-			const double2* a = multi + (size_t)k * (P + 1);
-			double2 cc = T.center[k];
-			double ih = 1.0 / T.half[k];
-			double2 dz = make_double2((cc.x - pc.x) * ih, (cc.y - pc.y) * ih);
-			const double2 dzp = warp_powers(dz, p);
-			double2 v = make_double2(0, 0);
-			if (p == 0)
-			{
-				v = a[0];
-			}
-			else if (act)
-			{
-				/* b_p = (sum_{i=1..p} a_i C(p-1, i-1) dz^(p-i) - a_0 dz^p / p) / 2^p */
-				double2 acc = cscale(a[1], binom_at(B, p - 1, 0));
-				for (int i = 2; i <= p; i++) acc = cadd(cmul(acc, dz), cscale(a[i], binom_at(B, p - 1, i - 1)));
-				double2 t = cscale(cmul(a[0], dzp), 1.0 / p);
-				v = cscale(csub(acc, t), ldexp(1.0, -p));
-			}
-			r = cadd(r, v);
+			v = a[0];
 		}
+		else if (act)
+		{
+			/* b_p = (sum_{i=1..p} a_i C(p-1, i-1) dz^(p-i) - a_0 dz^p / p) / 2^p */
+			double2 acc = cscale(a[1], binom_at(B, p - 1, 0));
+			for (int i = 2; i <= p; i++) acc = cadd(cmul(acc, dz), cscale(a[i], binom_at(B, p - 1, i - 1)));
+			double2 t = cscale(cmul(a[0], dzp), 1.0 / p);
+			v = cscale(csub(acc, t), ldexp(1.0, -p));
+		}
+		terms[w][p] = v;
+		__syncthreads();
+		if (w == 0)
+			for (int q = 0; q < 4; q++) r = cadd(r, terms[q][p]);
 	}
-	if (act) multi[(size_t)n * (P + 1) + p] = r;
+	if (w == 0 && act) multi[(size_t)n * (P + 1) + p] = r;
 }
 
-__global__ void fmm_upward_kernel(TreeDev T, int start, int count, int P, const double2* __restrict__ pos,
-	const double* __restrict__ mass, double2* __restrict__ multi, const double* __restrict__ B)
+/* one node per block of UP_WARPS warps */
+__global__ void __launch_bounds__(UP_WARPS * 32) fmm_upward_kernel(TreeDev T, int start, int count, int P,
+	const double2* __restrict__ pos, const double* __restrict__ mass, double2* __restrict__ multi, const double* __restrict__ B)
 {
-	int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-	if (w >= count) return;   /* warp-uniform */
-	fmm_upward_node(T, start + w, P, threadIdx.x & 31, pos, mass, multi, B);
+	if ((int)blockIdx.x >= count) return;   /* block-uniform */
+	fmm_upward_node(T, start + blockIdx.x, P, pos, mass, multi, B);
 }
 
 /* downward pass at one level >= 2: L2L from the parent, then M2L from the
@@ -361,8 +376,7 @@ __global__ void leaf_build_kernel(TreeDev T, int num_nodes, const int* __restric
 void launch_fmm_upward(cudaStream_t s, const TreeDev& T, int start, int count, int P, const double2* pos, const double* mass,
 	double2* multi, const double* B)
 {
-	long long threads = (long long)count * 32;
-	fmm_upward_kernel<<<(int)((threads + 127) / 128), 128, 0, s>>>(T, start, count, P, pos, mass, multi, B);
+	if (count > 0) fmm_upward_kernel<<<count, UP_WARPS * 32, 0, s>>>(T, start, count, P, pos, mass, multi, B);
 }
 void launch_fmm_downward(cudaStream_t s, const TreeDev& T, int start, int count, int P, const double2* pos, const double* mass,
 	const double2* multi, double2* local, const double* B)
@@ -489,57 +503,62 @@ namespace ccf
 constexpr int FOLD_MAXD = 256;
 static_assert(MAX_ORDER < 32, "one coefficient of a leaf block per lane");
 
-/* h^j times the j-th Taylor coefficient at z0 of sum_k e_k z^k, i.e.
-   h^j sum_{k >= j} C(k, j) e_k z0^(k - j): Horner from the top degree with
-   the binomial carried down the column, C(k, j) = C(k + 1, j) (k + 1 - j) / (k + 1)
-   (inv[k] = 1 / k).  Zero for j outside [0, n). */
-CCF_D double2 fold_coef(const double2* __restrict__ e, int n, double2 z0, double h, int j, const double* inv)
+/* The binomials of the three series' shifts, the same for every leaf: C(k, j)
+   of part's n coefficients at b[k * n + j], column j carried down from the top
+   degree, C(k, j) = C(k + 1, j) (k + 1 - j) / (k + 1).  One block per series,
+   one thread per column. */
+__global__ void __launch_bounds__(FOLD_MAXD) fold_binom_kernel(int nq, int nf, int nr, double* __restrict__ b)
 {
-	if (j < 0 || j >= n) return make_double2(0, 0);
-	double b = 1;   /* C(n - 1, j) */
-	for (int i = 0; i < j; i++) b *= (double)(n - 1 - i) * inv[i + 1];
-	double2 acc = make_double2(b * e[n - 1].x, b * e[n - 1].y);
+	__shared__ double inv[FOLD_MAXD + 1];
+	for (int k = threadIdx.x; k <= FOLD_MAXD; k += blockDim.x) inv[k] = k ? 1.0 / k : 0.0;
+	__syncthreads();
+	const int n = blockIdx.x == 0 ? nq : blockIdx.x == 1 ? nf : nr, j = threadIdx.x;
+	double* out = b + (blockIdx.x == 0 ? 0 : blockIdx.x == 1 ? nq * nq : nq * nq + nf * nf);
+	if (j >= n) return;
+	double v = 1;   /* C(n - 1, j) */
+	for (int i = 0; i < j; i++) v *= (double)(n - 1 - i) * inv[i + 1];
+	out[(n - 1) * n + j] = v;
 	for (int k = n - 2; k >= j; k--)
 	{
-		b *= (double)(k + 1 - j) * inv[k + 1];
-		const double2 ek = e[k];
-		acc = cmul(acc, z0);
-		acc.x += b * ek.x;
-		acc.y += b * ek.y;
+		v *= (double)(k + 1 - j) * inv[k + 1];
+		out[k * n + j] = v;
 	}
-	double hj = 1;
-	for (int i = 0; i < j; i++) hj *= h;
-	return make_double2(acc.x * hj, acc.y * hj);
 }
 
-/* sum over j = start, start + 32, ... < n of |coefficient j| sqrt(2)^j: one
-   lane's share of the terms beyond a block's order at the leaf corner */
-CCF_D double fold_tail(const double2* __restrict__ e, int n, double2 z0, double h, int start, const double* inv)
+/* hj = h^j times the j-th Taylor coefficient at z0 of sum_k e_k z^k, i.e.
+   h^j sum_{k >= j} C(k, j) e_k z0^(k - j): Horner from the top degree (b:
+   the series' binomials).  Zero for j outside [0, n). */
+CCF_D double2 fold_coef(const double2* __restrict__ e, int n, double2 z0, double hj, int j, const double* __restrict__ b)
 {
-	double t = 0;
-	for (int j = start; j < n; j += 32)
+	if (j < 0 || j >= n) return make_double2(0, 0);
+	const double top = b[(n - 1) * n + j];
+	double2 acc = make_double2(top * e[n - 1].x, top * e[n - 1].y);
+	for (int k = n - 2; k >= j; k--)
 	{
-		const double2 v = fold_coef(e, n, z0, h, j, inv);
-		t += hypot(v.x, v.y) * ldexp((j & 1) ? 1.4142135623730951 : 1.0, j >> 1);
+		const double bk = b[k * n + j];
+		const double2 ek = e[k];
+		acc = cmul(acc, z0);
+		acc.x += bk * ek.x;
+		acc.y += bk * ek.y;
 	}
-	return t;
+	return make_double2(acc.x * hj, acc.y * hj);
 }
 
 /* one leaf per CTA of three warps: warp 0 folds the alpha series (eq) into
    block 0, warp 1 the d alpha / d zbar series (ef) into block 1, warp 2 the
    d2 alpha / d zbar2 series (er) into block 2; each lane forms one shifted
-   coefficient and a share of its series' tail beyond the block's order, and
-   the leaf folds when all three tails are negligible */
+   coefficient and a share of its series' tail beyond the block's order (the
+   sum of |coefficient j| sqrt(2)^j at the leaf corner), and
+   the leaf folds when all three tails are negligible.  Bound by the FP64
+   pipe; with the binomials from a table and the powers of h from one product
+   12052 leaves take 1.66 ms, 3.45 with each leaf's own. */
 __global__ void __launch_bounds__(96) fold_smooth_kernel(int num_leaves, int P, const double2* __restrict__ leaf_center,
 	const double* __restrict__ leaf_inv_half, const double2* __restrict__ loc, const double2* __restrict__ ef, int nf,
 	const double2* __restrict__ er, int nr, const double2* __restrict__ eq, int nq, double radius,
 	float4* __restrict__ loc_df, float4* __restrict__ loc_pk, float2* __restrict__ loc3f, double2* __restrict__ loc64,
-	unsigned char* __restrict__ fold)
+	unsigned char* __restrict__ fold, const double* __restrict__ binom)
 {
-	__shared__ double inv[FOLD_MAXD + 1];
 	__shared__ int s_ok[3];
-	for (int k = threadIdx.x; k <= FOLD_MAXD; k += blockDim.x) inv[k] = k ? 1.0 / k : 0.0;
-	__syncthreads();
 	const int lane = threadIdx.x & 31, part = threadIdx.x >> 5;
 	const int l = blockIdx.x;
 	if (l >= num_leaves) return;   /* block-uniform */
@@ -556,8 +575,30 @@ __global__ void __launch_bounds__(96) fold_smooth_kernel(int num_leaves, int P, 
 	const double2* e = part == 0 ? eq : part == 1 ? ef : er;
 	const int n = part == 0 ? nq : part == 1 ? nf : nr;
 	const int i = lane;
-	const double2 v = i >= part + 1 && i <= P ? fold_coef(e, n, c, h, i - part - 1, inv) : make_double2(0, 0);
-	double t = fold_tail(e, n, c, h, P - part + lane, inv);
+	const double* b = binom + (part == 0 ? 0 : part == 1 ? nq * nq : nq * nq + nf * nf);
+	/* the powers of h for the lane's coefficient and the first two of its tail */
+	const int j0 = i >= part + 1 && i <= P ? i - part - 1 : -1, j1 = P - part + lane, j2 = j1 + 32;
+	double hp = 1, h0 = 1, h1 = 1, h2 = 1;
+	for (int k = 0; k < n; k++)
+	{
+		if (k == j0) h0 = hp;
+		if (k == j1) h1 = hp;
+		if (k == j2) h2 = hp;
+		hp *= h;
+	}
+	const double2 v = fold_coef(e, n, c, h0, j0, b);
+	double t = 0;
+	for (int j = j1; j < n; j += 32)
+	{
+		double hj = j == j1 ? h1 : h2;
+		if (j > j2)
+		{
+			hj = 1;
+			for (int k = 0; k < j; k++) hj *= h;
+		}
+		const double2 u = fold_coef(e, n, c, hj, j, b);
+		t += hypot(u.x, u.y) * ldexp((j & 1) ? 1.4142135623730951 : 1.0, j >> 1);
+	}
 	for (int o = 16; o; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
 	const double tol = 1e-15;
 	if (lane == 0) s_ok[part] = t <= tol ? 1 : 0;
@@ -585,13 +626,21 @@ __global__ void __launch_bounds__(96) fold_smooth_kernel(int num_leaves, int P, 
 	if (loc64) loc64[((size_t)l * 3 + part) * (P + 1) + i] = a;
 }
 
+size_t fold_binom_size(int nf, int nr, int nq)
+{
+	if (std::max({nf, nr, nq}) > FOLD_MAXD) return 0;
+	return (size_t)nf * nf + (size_t)nr * nr + (size_t)nq * nq;
+}
+
 void launch_fold_smooth(cudaStream_t s, int num_leaves, int P, const double2* leaf_center, const double* leaf_inv_half,
 	const double2* loc, const double2* ef, int nf, const double2* er, int nr, const double2* eq, int nq, double radius,
-	float4* loc_df, float4* loc_pk, float2* loc3f, double2* loc64, unsigned char* fold)
+	float4* loc_df, float4* loc_pk, float2* loc3f, double2* loc64, unsigned char* fold, double* binom)
 {
 	if (num_leaves <= 0) return;
+	/* (a series beyond FOLD_MAXD is not folded, and its binomials not read) */
+	if (fold_binom_size(nf, nr, nq) > 0) fold_binom_kernel<<<3, FOLD_MAXD, 0, s>>>(nq, nf, nr, binom);
 	fold_smooth_kernel<<<num_leaves, 96, 0, s>>>(num_leaves, P, leaf_center, leaf_inv_half, loc, ef, nf, er, nr, eq, nq,
-		radius, loc_df, loc_pk, loc3f, loc64, fold);
+		radius, loc_df, loc_pk, loc3f, loc64, fold, binom);
 }
 
 } /* namespace ccf */
@@ -622,10 +671,9 @@ __global__ void fmm_level_batch_kernel(const BatchSeg* __restrict__ segs, int L,
 	if (L > S.info[0]) return;   /* block-uniform */
 	if (upward)
 	{
-		/* four nodes per block, one warp each */
-		const int w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-		if (w >= S.info[3 + TREE_MAX_LEVELS + 1 + L]) return;   /* warp-uniform */
-		fmm_upward_node(S.T, S.info[3 + L] + w, S.P, threadIdx.x & 31, S.pos, S.mass, S.multi, S.B);
+		/* one node per block, UP_WARPS warps */
+		if ((int)blockIdx.x >= S.info[3 + TREE_MAX_LEVELS + 1 + L]) return;   /* block-uniform */
+		fmm_upward_node(S.T, S.info[3 + L] + blockIdx.x, S.P, S.pos, S.mass, S.multi, S.B);
 	}
 	else
 	{
@@ -697,9 +745,9 @@ void launch_fmm_batch(cudaStream_t s, const BatchSeg* segs, int nseg, int max_le
 	if (nseg <= 0) return;
 	const int gz = (int)std::min<long long>((max_coefficients + 255) / 256, 64);
 	fmm_zero_batch_kernel<<<dim3(std::max(gz, 1), nseg), 256, 0, s>>>(segs);
-	const int gx = std::max(1, (max_level_nodes + 3) / 4);
-	for (int L = max_levels; L >= 0; L--) fmm_level_batch_kernel<<<dim3(gx, nseg), 128, 0, s>>>(segs, L, 1);
-	static_assert(DOWN_PARTS * 32 == 128, "the level kernel's blocks");
+	for (int L = max_levels; L >= 0; L--)
+		fmm_level_batch_kernel<<<dim3(std::max(1, max_level_nodes), nseg), 128, 0, s>>>(segs, L, 1);
+	static_assert(DOWN_PARTS * 32 == 128 && UP_WARPS * 32 == 128, "the level kernel's blocks");
 	for (int L = 2; L <= max_levels; L++)
 		fmm_level_batch_kernel<<<dim3(std::max(1, max_level_nodes), nseg), 128, 0, s>>>(segs, L, 0);
 	leaf_number_batch_kernel<<<nseg, 1024, 0, s>>>(segs);

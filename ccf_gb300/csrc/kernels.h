@@ -465,7 +465,9 @@ void launch_leaf_df(cudaStream_t s, int num_leaves, int P, const double2* leaf_c
 	float2* ih_df, float4* near_pk, float4* loc_pk);
 void launch_fold_smooth(cudaStream_t s, int num_leaves, int P, const double2* leaf_center, const double* leaf_inv_half,
 	const double2* loc, const double2* ef, int nf, const double2* er, int nr, const double2* eq, int nq, double radius,
-	float4* loc_df, float4* loc_pk, float2* loc3f, double2* loc64, unsigned char* fold);
+	float4* loc_df, float4* loc_pk, float2* loc3f, double2* loc64, unsigned char* fold, double* binom);
+/* binom's doubles (0: the series are too long to be folded) */
+size_t fold_binom_size(int nf, int nr, int nq);
 
 /* solver.cu */
 int solver_blocks_per_sm(bool mixed);
