@@ -256,7 +256,8 @@ constexpr unsigned long long TRACK_TABLE_FULL = 8;   /* the column table probe l
 
 /* a root handed from the item launch to the far launch: the tracker's state
    at the top of an iteration (track_kernel) */
-constexpr int TRACK_HIST = 5;   /* accepted positions a root's predictor uses */
+constexpr int TRACK_HIST = 9;       /* accepted positions a root keeps for its predictor, */
+constexpr int TRACK_HIST_ROUGH = 5; /* and those it uses where the path is not smooth (track_predict) */
 struct FarState
 {
 	double2 hz[TRACK_HIST];

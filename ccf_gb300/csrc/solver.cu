@@ -554,6 +554,7 @@ constexpr double TRACK_STUCK = 1e-2;            /* theta_star: a root whose corr
                                                    are a lost root and send the row to the re-run */
 /* a slot's 1/mu error until track_outputs_kernel has formed it: neither a bound (>= 0) nor an unconverged mark (<= -1) */
 constexpr double OUTPUT_DUE = -0.25, OUTPUT_DUE_STALLED = -0.5;
+constexpr double TRACK_SMOOTH = 1e-7;           /* theta_star: a first step below it lets the predictor use all its points */
 constexpr double TRACK_FS_REFINE = 1e-9;        /* bound on |f| above which a converged root takes one more step */
 constexpr int TABLE_PROBES = 1024;       /* linear-probe bound of the column tables (load <= 1/2: the
                                             longest cluster of a table of 1e5 slots is ~60) */
@@ -618,12 +619,28 @@ CCF_D unsigned long long table_insert(unsigned long long* tab, unsigned long lon
    roots, so they converge at the first evaluation.  The steps may be
    sub-steps: a row tracked again in eighths of a step took 2.3 evaluations
    for each with the secant (one row of a 137-star field 14 ms), 1.0 with the
-   polynomial.  After an uneven history it falls back to the secant
+   polynomial.  Nine points are used while the path is smooth -- the last
+   target's first step was below TRACK_SMOOTH theta_star -- and five elsewhere:
+   six everywhere led some roots next to a star onto another's path (rows of the
+   20 000-star field failed their column check), while under this rule the same
+   rows as with five are tracked again on 435 fields of 11 kinds.  Against five
+   throughout: the continuation of 2000 stars 7.0 to 6.4 ms, 7001 stars 10.4 to
+   8.3, 20 000 stars 43.9 to 37.4, a 17-star rectangle (2.0 to 1.4 evaluations a
+   step) 5.9 to 4.1.  After an uneven history it falls back to the secant
    through the two newest points, t0 and t1 the older and the newer one's
-   positions; so it does after sub-steps where length scales are written,
-   which would show the other starting point's 1e-14 in the root. */
+   positions.  Where length scales are written it does so after sub-steps too
+   and stays with five points: they would show another starting point's 1e-14
+   in the root. */
 __constant__ double c_extrap_w[TRACK_HIST][TRACK_HIST] = {
-	{1, 0, 0, 0, 0}, {2, -1, 0, 0, 0}, {3, -3, 1, 0, 0}, {4, -6, 4, -1, 0}, {5, -10, 10, -5, 1}};
+	{1, 0, 0, 0, 0, 0, 0, 0, 0},
+	{2, -1, 0, 0, 0, 0, 0, 0, 0},
+	{3, -3, 1, 0, 0, 0, 0, 0, 0},
+	{4, -6, 4, -1, 0, 0, 0, 0, 0},
+	{5, -10, 10, -5, 1, 0, 0, 0, 0},
+	{6, -15, 20, -15, 6, -1, 0, 0, 0},
+	{7, -21, 35, -35, 21, -7, 1, 0, 0},
+	{8, -28, 56, -70, 56, -28, 8, -1, 0},
+	{9, -36, 84, -126, 126, -84, 36, -9, 1}};
 
 CCF_D int ring_next(int slot) { return slot + 1 == TRACK_HIST ? 0 : slot + 1; }
 
@@ -1262,6 +1279,7 @@ __global__ void __launch_bounds__(FAR ? 32 * FAR_MAX_WARPS : TNT, FAR || G > 1 ?
 		typedef typename std::conditional<MIXED, float, double>::type real;
 		const real tol2 = (real)(tol * tol);
 		const real stuck2 = (real)(TRACK_STUCK * TRACK_STUCK * F.theta * F.theta);
+		const real smooth2 = (real)(TRACK_SMOOTH * TRACK_SMOOTH * F.theta * F.theta);
 		const bool disc_exact = !F.rectangular && !F.approx;
 		const double inv_cell = CELL_PER_THETA / F.theta;
 		const unsigned long long slots = 2ull * (unsigned long long)R;
@@ -1300,6 +1318,7 @@ __global__ void __launch_bounds__(FAR ? 32 * FAR_MAX_WARPS : TNT, FAR || G > 1 ?
 		dfl cpd = {0.f, 0.f}, spd = {0.f, 0.f};
 		int it = 0, evs = 0;
 		real prev2 = 0;
+		bool smooth = false;    /* the target's first step was short (track_predict) */
 		bool lost = !valid;
 		bool refine = false;
 		if (FAR && resume)
@@ -1424,6 +1443,7 @@ __global__ void __launch_bounds__(FAR ? 32 * FAR_MAX_WARPS : TNT, FAR || G > 1 ?
 				const real contract = (real)(finest ? TRACK_CONTRACT_FINEST : TRACK_CONTRACT);
 				bool conv = false, fail = !isfinite(as2);
 				if (!fail && it > 0 && as2 >= tol2 && as2 > contract * contract * prev2) fail = true;
+				if (it == 0) smooth = as2 < smooth2;
 				if (!fail)
 				{
 					it++;
@@ -1627,7 +1647,8 @@ __global__ void __launch_bounds__(FAR ? 32 * FAR_MAX_WARPS : TNT, FAR || G > 1 ?
 				{
 					/* next target: predict, restart the corrector */
 					tt = tn;
-					z = track_predict<NL>(hz, head, hn, tt - t1 == t1 - t0 && run >= hn - 1, t0, t1, tt);
+					const int hp = min(hn, smooth && !T.scales ? TRACK_HIST : TRACK_HIST_ROUGH);
+				z = track_predict<NL>(hz, head, hp, tt - t1 == t1 - t0 && run >= hp - 1, t0, t1, tt);
 					it = 0;
 					prev2 = 0;
 					track_phase(O, c, side, tt, gp, cp, sp, cpd, spd);
@@ -1836,9 +1857,9 @@ cudaError_t launch_track_mark(cudaStream_t s, const TrackArgs& a, int* cls)
 namespace
 {
 /* percent of the SM's shared memory and L1 that the tracker's launches set
-   aside as shared memory: 64 KiB hold the items' three CTAs and a far one; the
+   aside as shared memory: 82 KiB hold the items' three CTAs and a far one; the
    leaf records are read through the rest */
-constexpr int TRACK_CARVEOUT = 28;
+constexpr int TRACK_CARVEOUT = 36;
 
 /* CTAs of the tracker that are resident on one SM at once (asked once per
    form and CTA size) */
