@@ -121,13 +121,20 @@ CCF_D int source_split(int total, int csize)
 }
 
 /* How a sweep's sums are cut into units: tpt targets per thread, 1 where two
-   would leave SMs without a unit; and chunks per unit, all of them where the
-   whole sweep is less work than handing units around (~5 us). */
+   would leave SMs without a unit, and 0 (one target per thread of the first
+   HALF_WARPS warps only) where such units would still be no more than the SMs:
+   a unit of eight warps runs two on each of the SM's four schedulers (with the
+   warps that have no target kept out of the loop, the initial solve of 600
+   stars in FP64 6.3 ms against 8.6, the full-sum continuation of 400 stars 4.1
+   against 4.3); and
+   chunks per unit, all of them where the whole sweep is less work than handing
+   units around (~5 us). */
 struct SumsShape
 {
 	int tpt, chunks, tiles, groups;
 };
 constexpr long long SUMS_ONE_UNIT = 1 << 16;   /* terms */
+constexpr int HALF_WARPS = NT / 64;
 CCF_D SumsShape sums_shape(int total, int S, int R, int N, int nch, int rows, int sms)
 {
 	SumsShape p;
@@ -139,6 +146,11 @@ CCF_D SumsShape sums_shape(int total, int S, int R, int N, int nch, int rows, in
 	{
 		p.tpt = 1;
 		p.tiles = (total + NT / S - 1) / (NT / S);
+		if (S <= HALF_WARPS && (long long)p.tiles * p.groups * rows <= sms)
+		{
+			p.tpt = 0;
+			p.tiles = (total + NT / 2 / S - 1) / (NT / 2 / S);
+		}
 	}
 	return p;
 }
@@ -370,12 +382,15 @@ __device__ void sums_unit(const SolveArgs& A, RowShared<MIXED>& Sh, const int* l
 	issue(ch0, 0);
 	const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 	const int part = warp % S, group = warp / S;
+	const int groups = (Sh.shape.tpt == 0 ? HALF_WARPS : NT / 32) / S;   /* of 32 TP targets */
+	/* a warp without a target only loads: it would take the others' issue slots */
+	const bool work = group < groups && (tile * groups + group) * 32 * TP < total;
 	int g[TP];
 	SrcT zs[TP];
 #pragma unroll
 	for (int t = 0; t < TP; t++)
 	{
-		g[t] = (tile * (NT / 32 / S) + group) * 32 * TP + t * 32 + lane;
+		g[t] = work ? (tile * groups + group) * 32 * TP + t * 32 + lane : total;
 		if constexpr (MIXED) zs[t] = g[t] < total ? __ldcg(rsrc + __ldcg(list + g[t])) : make_float4(0, 0, 0, 0);
 		else zs[t] = g[t] < total ? __ldcg(rsrc + __ldcg(list + g[t])) : make_double2(0, 0);
 	}
@@ -387,7 +402,7 @@ __device__ void sums_unit(const SolveArgs& A, RowShared<MIXED>& Sh, const int* l
 		cp_async_wait<1>();
 		__syncthreads();
 		const int n = count(ch);
-		const int j0 = (n * part) / S, j1 = (n * (part + 1)) / S;
+		const int j0 = (n * part) / S, j1 = work ? (n * (part + 1)) / S : j0;
 		const SrcT* sb = Sh.buf + buf * CHUNK;
 		typename PartT<MIXED>::T* out = part_out + ((size_t)ch * S + part) * total;
 		if constexpr (MIXED)
@@ -709,7 +724,7 @@ __global__ void __launch_bounds__(NT, 2) rows_kernel(const SolveArgs A, const in
 
 		if (Sh.phase == PHASE_SUMS)
 		{
-			if (Sh.shape.tpt == 1) sums_unit<MIXED, 1>(A, Sh, list, part);
+			if (Sh.shape.tpt <= 1) sums_unit<MIXED, 1>(A, Sh, list, part);
 			else sums_unit<MIXED, TPT>(A, Sh, list, part);
 		}
 		else

@@ -96,3 +96,20 @@ def test_rows_do_not_depend_on_the_blocks(n, precision):
         b = f.results()
         assert np.array_equal(r["ccs"][:, 4], b["ccs"][:, 4])
         assert O.match_sets(r["ccs"], b["ccs"], 8)["max_dist"] <= 1e-11
+
+
+@pytest.mark.parametrize("precision", ["mixed", "fp64"])
+@pytest.mark.parametrize("n, nb", [(63, 1), (65, 4), (260, 2), (600, 1)])
+def test_rows_do_not_depend_on_the_sums_tiles(n, nb, precision):
+    """A row alone has sums units of half the warps, forty copies of it full
+    ones: the same bits in the solved column."""
+    def make():
+        return field(n, 1, nb=nb, num_phi=8 * nb, continuation="aberth", precision=precision, init_cluster=1)
+    a = make()
+    assert a.run(-1), a.last_error()
+    r = a.results()
+    fs = [make() for _ in range(40)]
+    assert run_batch(fs, -1), fs[0].last_error()
+    b = fs[-1].results()
+    assert np.array_equal(r["ccs"][:, 4], b["ccs"][:, 4])
+    assert O.match_sets(r["ccs"], b["ccs"], nb)["max_dist"] <= 1e-11
