@@ -427,6 +427,59 @@ CCF_D dfc halves_split(const float4* C, int n, const SplitPowers<G>& wv, dfc x, 
 	return {df_add(r.re, c.re), df_add(r.im, c.im)};
 }
 
+/* The Taylor forms of the smooth mass outside the corner circle, FP64, over the
+   group: a lane's Horner passes over the three series are ~460 instructions
+   of 64 cycles each, a lane's share of eight ~130.  The constant terms are
+   added after the exchange, as above. */
+struct SplitPowers64
+{
+	double2 first, stride;
+};
+template <int G>
+CCF_D SplitPowers64 split_powers64(double2 x, int sub)
+{
+	SplitPowers64 w = {make_double2(1, 0), x};
+#pragma unroll
+	for (int b = 1; b < G; b <<= 1)
+	{
+		const double2 t = b == 1 ? w.stride : cmul(w.first, w.stride);
+		if (sub & b) w.first = t;
+		w.stride = cmul(w.stride, w.stride);
+	}
+	return w;
+}
+/* sum_k c_k x^k, k < n */
+template <int G>
+CCF_D double2 poly_split64(const double2* c, int n, const SplitPowers64& w, int sub, unsigned gm)
+{
+	double2 acc = make_double2(0, 0);
+#pragma unroll 1
+	for (int k = sub < n ? sub + (n - 1 - sub) / G * G : -1; k >= sub; k -= G)
+	{
+		acc = cmul(acc, w.stride);
+		if (k > 0) acc = cadd(acc, c[k]);
+	}
+	acc = cmul(acc, w.first);
+#pragma unroll
+	for (int o = 1; o < G; o <<= 1)
+	{
+		acc.x += __shfl_xor_sync(gm, acc.x, o);
+		acc.y += __shfl_xor_sync(gm, acc.y, o);
+	}
+	return cadd(acc, c[0]);
+}
+/* whether the field's smooth mass takes the Taylor form */
+CCF_D bool smooth_taylor(const FieldView& F) { return F.rectangular && F.approx && F.smooth_m > 0; }
+/* smooth_alpha of a field of that form */
+template <int G>
+CCF_D double2 smooth_alpha_split(const FieldView& F, double2 z, int sub, unsigned gm)
+{
+	const double2 acc = poly_split64<G>(F.smooth_a, F.taylor_smooth + 2, split_powers64<G>(cconj(z), sub), sub, gm);
+	double2 a = cmul(acc, make_double2(0, -F.kappa_star / PI));
+	a.x -= F.kappa_star * 2 * (F.corner.x + z.x);
+	return a;
+}
+
 /* the near stars' part of an evaluation: sums of m / d, m / d^2 (double-float),
    m / d^3, 1 / d (FP32) and |m / d^2| */
 struct TrackSums
@@ -589,6 +642,24 @@ static __device__ __noinline__ SmoothFar smooth_far(const FieldView& F, double2 
 	return {dfc_from(smooth_dzbar(F, z)), make_float2((float)t.x, (float)t.y)};
 }
 
+template <int G>
+CCF_D SmoothFar smooth_far_split(const FieldView& F, double2 z, int sub, unsigned gm)
+{
+	if constexpr (G > 1)
+	{
+		if (smooth_taylor(F))
+		{
+			const double2 zb = cconj(z), r = cmul(zb, F.inv_corner), u = cmul(r, r);
+			const SplitPowers64 w = split_powers64<G>(u, sub);
+			double2 ds = cmul(poly_split64<G>(F.smooth_d1, F.smooth_m, w, sub, gm), u);
+			ds.x += F.smooth_k1;
+			const double2 d2s = cmul(poly_split64<G>(F.smooth_d2, F.smooth_m, w, sub, gm), cmul(zb, F.inv_corner2));
+			return {dfc_from(ds), make_float2((float)d2s.x, (float)d2s.y)};
+		}
+	}
+	return smooth_far(F, z);
+}
+
 template <bool PK, int G>
 CCF_D TrackEval eval_track_df(const FieldView& F, const TrackConst& K, int leaf, double2 z, double2 rel, dfl cph, dfl sph,
 	bool disc_exact, int sub, unsigned gm)
@@ -713,7 +784,7 @@ CCF_D TrackEval eval_track_df(const FieldView& F, const TrackConst& K, int leaf,
 	}
 	else
 	{
-		const SmoothFar t = smooth_far(F, z);
+		const SmoothFar t = smooth_far_split<G>(F, z, sub, gm);
 		ds = t.ds;
 		d2s = t.d2s;
 	}

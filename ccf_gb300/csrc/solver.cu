@@ -1511,6 +1511,12 @@ __global__ void __launch_bounds__(FAR ? 32 * FAR_MAX_WARPS : TNT, FAR || G > 1 ?
 						}
 						if constexpr (MIXED)
 						{
+							double2 sa_group;   /* the smooth mass's deflection, by the group */
+							if constexpr (G > 1)
+							{
+								if (!direct_out && e.wmode == 0 && smooth_taylor(F))
+									sa_group = smooth_alpha_split<G>(F, make_double2(zf.x + step.x, zf.y + step.y), sub, gm);
+							}
 							if (!direct_out && sub == 0)
 							{
 								/* the lens map at the evaluated point ze, corrected to zf = ze - s:
@@ -1543,7 +1549,7 @@ __global__ void __launch_bounds__(FAR ? 32 * FAR_MAX_WARPS : TNT, FAR || G > 1 ?
 								{
 									const double2 ze = make_double2(zf.x + step.x, zf.y + step.y);
 									const double2 wp = dfc_to(e.wpart);
-									const double2 sa = smooth_alpha(F, ze);
+									const double2 sa = G > 1 && smooth_taylor(F) ? sa_group : smooth_alpha(F, ze);
 									wx = (1 - F.kappa_tot + F.shear) * ze.x + wp.x - sa.x;
 									wy = (1 - F.kappa_tot - F.shear) * ze.y + wp.y - sa.y;
 								}
