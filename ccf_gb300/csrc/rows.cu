@@ -93,10 +93,15 @@ CCF_D int row_blocks(int R, int csize, int blk)
    first check, an epilogue): 64, 128 or 256, the fewest that leave no more
    units than CTAs.  A unit's time is its roots' FP64 work and the chain of one
    evaluation: with two warps in a CTA instead of eight each scheduler's FP64
-   pipe serves one of them (a step of 64 roots 33 us, of 256 51; the full-sum
+   pipe serves one of them, and a rectangle's off-box roots, whose star sums
+   take a CTA one after another, are spread.  A row of one such unit of 256 stays
+   in its CTA, which saves handing units around: up to 256 roots (full-sum
+   continuation of a 60-star disc 8.0 ms, 8.6 in blocks of 64; a 60-star
+   rectangle 22 in blocks of 64, 25.7 in one), 128 of a rectangle (a step of 64 roots 33 us, of 256 51; the full-sum
    continuation of 400 stars, 4 branches of 32 steps, 4.8 ms against 5.5). */
-CCF_D int block_roots(int n, int rows, int ctas)
+CCF_D int block_roots(int n, int rows, int ctas, bool rectangular)
 {
+	if (n <= (rectangular ? NT / 2 : NT)) return NT;
 	int blk = MIN_BLOCK;
 	while (blk < NT && (long long)rows * ((n + blk - 1) / blk) > ctas) blk *= 2;
 	return blk;
@@ -191,7 +196,7 @@ static_assert(OFF_CAP * (NT / 32) * 6 * sizeof(double) <= 2 * CHUNK * 16, "off-f
    ones go to the share's end: their snapshot is due with the next step's (after
    the sums, as the others').  Every thread of the CTA calls it. */
 template <bool MIXED>
-__device__ void check_roots(const SolveArgs& A, RowShared<MIXED>& S, int* share, int* counts, int blk, int a, bool act, double2 z,
+__device__ void check_roots(const SolveArgs& A, RowShared<MIXED>& S, int* share, int* share_end, int* counts, int a, bool act, double2 z,
 	double cphi, double sphi, bool initial)
 {
 	const FieldView& F = S.F;
@@ -252,10 +257,18 @@ __device__ void check_roots(const SolveArgs& A, RowShared<MIXED>& S, int* share,
 		nl += S.warp_late[w];
 	}
 	if (still) share[g] = a;
-	if (late) share[blk - 1 - gl] = a;
+	if (late) share_end[-1 - gl] = a;
 	if (threadIdx.x == 0)
 	{
-		*counts = n | nl << 16;
+		if (counts)
+		{
+			*counts = n | nl << 16;
+		}
+		else
+		{
+			S.total = n;
+			S.late = nl;
+		}
 		if (evals)
 		{
 			atomicAdd(&S.O.stats[2], (unsigned long long)evals);
@@ -602,7 +615,7 @@ __global__ void __launch_bounds__(NT, 2) rows_kernel(const SolveArgs A, const in
 						}
 						else
 						{
-							const int nr0 = A.fields[rd.field].num_roots, blk = block_roots(nr0, rows_at_work, (int)gridDim.x);
+							const int nr0 = A.fields[rd.field].num_roots, blk = block_roots(nr0, rows_at_work, (int)gridDim.x, A.fields[rd.field].rectangular != 0);
 							const int units = row_blocks(nr0, csize, blk);
 							Sh.cur = nr;
 							Sh.claimed = nr;
@@ -680,7 +693,7 @@ __global__ void __launch_bounds__(NT, 2) rows_kernel(const SolveArgs A, const in
 			__syncthreads();
 			if (threadIdx.x == 0)
 			{
-				const int blk = block_roots(A.fields[field].num_roots, rows_at_work, (int)gridDim.x);
+				const int blk = block_roots(A.fields[field].num_roots, rows_at_work, (int)gridDim.x, A.fields[field].rectangular != 0);
 				int n = 0;
 				for (int r = 0; r < csize; r++)
 				{
@@ -718,7 +731,11 @@ __global__ void __launch_bounds__(NT, 2) rows_kernel(const SolveArgs A, const in
 		int* const shares = A.share + (size_t)(row % A.part_slots) * A.share_stride;
 		int* const counts = A.counts + (size_t)(row % A.part_slots) * A.counts_stride;
 		const int blk = Sh.blk, tid = threadIdx.x < blk ? (int)threadIdx.x : NO_ROOT;
-		int* const share = shares + (size_t)Sh.unit * blk;
+		/* the unit's share of the next list; the list itself when it is the only unit */
+		const bool only = Sh.units == 1;
+		int* const share = only ? list : shares + (size_t)Sh.unit * blk;
+		int* const share_end = only ? list + R : share + blk;
+		int* const share_count = only ? nullptr : counts + Sh.unit;
 		typename PartT<MIXED>::T* part = reinterpret_cast<typename PartT<MIXED>::T*>(A.part) +
 			(size_t)(row % A.part_slots) * A.part_stride;
 
@@ -774,7 +791,7 @@ __global__ void __launch_bounds__(NT, 2) rows_kernel(const SolveArgs A, const in
 					if constexpr (MIXED) A.snap32[base + a] = split_hilo(z);
 					else A.snap64[base + a] = z;
 				}
-				if (Sh.it < max_it) check_roots<MIXED>(A, Sh, share, counts + Sh.unit, blk, a, act, z, cphi, sphi, initial);
+				if (Sh.it < max_it) check_roots<MIXED>(A, Sh, share, share_end, share_count, a, act, z, cphi, sphi, initial);
 			}
 			else
 			{
@@ -854,7 +871,7 @@ __global__ void __launch_bounds__(NT, 2) rows_kernel(const SolveArgs A, const in
 				if (check)
 				{
 					if (own) A.fin[base + a] = 0;
-					check_roots<MIXED>(A, Sh, share, counts + Sh.unit, blk, a, own, z, cphi, sphi, initial);
+					check_roots<MIXED>(A, Sh, share, share_end, share_count, a, own, z, cphi, sphi, initial);
 				}
 			}
 		}
@@ -888,7 +905,7 @@ __global__ void __launch_bounds__(NT, 2) rows_kernel(const SolveArgs A, const in
 		__syncthreads();
 		if (!Sh.last) continue;
 		/* the next phase */
-		if (checked) join_list<MIXED>(Sh, shares, counts, Sh.units, blk, list, R);
+		if (checked && Sh.units > 1) join_list<MIXED>(Sh, shares, counts, Sh.units, blk, list, R);
 		if (threadIdx.x == 0)
 		{
 			unsigned long long* stats = O.stats;
@@ -897,7 +914,7 @@ __global__ void __launch_bounds__(NT, 2) rows_kernel(const SolveArgs A, const in
 			{
 				phase = PHASE_STEP;
 				Sh.it++;
-				Sh.blk = block_roots(Sh.total + Sh.late, rows_at_work, (int)gridDim.x);
+				Sh.blk = block_roots(Sh.total + Sh.late, rows_at_work, (int)gridDim.x, F.rectangular != 0);
 				units = (Sh.total + Sh.late + Sh.blk - 1) / Sh.blk;
 			}
 			else
