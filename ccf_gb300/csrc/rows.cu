@@ -904,8 +904,9 @@ __global__ void __launch_bounds__(NT, 2) rows_kernel(const SolveArgs A, const in
 		}
 		__syncthreads();
 		if (!Sh.last) continue;
-		/* the next phase */
-		if (checked && Sh.units > 1) join_list<MIXED>(Sh, shares, counts, Sh.units, blk, list, R);
+		/* the next phase (only, like checked, was read before: without a list to
+		   join thread 0 moves on at once) */
+		if (checked && !only) join_list<MIXED>(Sh, shares, counts, Sh.units, blk, list, R);
 		if (threadIdx.x == 0)
 		{
 			unsigned long long* stats = O.stats;
