@@ -1518,7 +1518,7 @@ cudaError_t Engine::copy_out(void* dst, const void* src, size_t bytes)
    copies, without changing what they hold.  An array fresh from the allocator
    has no pages, and the copy faulted them in and cleared them one after
    another (new arrays of 24 fields, 524 MB: 29 ms, 16 with this, 4.5 into
-   arrays that have their pages).  Destinations the driver knows (page-locked,
+   arrays that have their pages).  Destinations CUDA knows (page-locked,
    managed, device memory) are left alone, and where the kernel has no such
    call or no thread can be started the copy maps them as before. */
 static void populate(std::vector<std::pair<void*, size_t>> dst)

@@ -1948,10 +1948,10 @@ cudaError_t launch_track_form(cudaStream_t s, const TrackArgs& a, int sms, const
 	   there is work for: the warps of a small launch otherwise race for it, and
 	   SMs whose warps all won share one FP64 pipe.  The solo roots are counted
 	   in (a 17-star rectangle has 36 of them and 6 items: 7.5 ms against 30 with
-	   the items' two CTAs), but not where the outputs are FP64 epilogues, which
-	   a CTA more per SM does not speed up (11.3 ms against 12.8 in FP64 on a
-	   600-star rectangle) */
-	const long long work = (long long)t.num_items * G + (first && !t.solo_far && PK ? t.solo_guess : 0);
+	   the items' two CTAs; a 419-star rectangle with length scales 4.0 ms against
+	   4.4), but not in FP64, where a CTA more per SM only shares its FP64 pipes
+	   (8.0 ms against 9.5 on a 600-star rectangle) */
+	const long long work = (long long)t.num_items * G + (first && !t.solo_far && MIXED ? t.solo_guess : 0);
 	const int blocks = (int)std::max<long long>(1, std::min<long long>(sms * resident<MIXED, PK, false, G>(TNT),
 		(work + TNT / 32 - 1) / (TNT / 32)));
 	track_kernel<MIXED, PK, false, G><<<blocks, TNT, 0, s>>>(t);

@@ -57,9 +57,9 @@ typedef enum ccf_precision
 typedef enum ccf_continuation
 {
 	CCF_CONTINUATION_TRACK = 0,  /* default: every root follows its own path in
-	                                phi with a quartic predictor (the polynomial
-	                                through its last five positions; the secant
-	                                after sub-steps) and a corrector whose Aberth
+	                                phi with a polynomial predictor (through its
+	                                last five positions, nine on a smooth path;
+	                                the secant after sub-steps) and a corrector whose Aberth
 	                                correction keeps the poles of the leaf's near
 	                                stars only; every column is checked for two
 	                                roots on one zero.  A row that fails the check
