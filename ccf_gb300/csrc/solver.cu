@@ -1949,11 +1949,13 @@ cudaError_t launch_track_form(cudaStream_t s, const TrackArgs& a, int sms, const
 	   SMs whose warps all won share one FP64 pipe.  The solo roots are counted
 	   in (a 17-star rectangle has 36 of them and 6 items: 7.5 ms against 30 with
 	   the items' two CTAs; a 419-star rectangle with length scales 4.0 ms against
-	   4.4), but not in FP64, where a CTA more per SM only shares its FP64 pipes
+	   4.4), in FP64 up to a CTA per SM, where one more only shares its FP64 pipes
 	   (8.0 ms against 9.5 on a 600-star rectangle) */
-	const long long work = (long long)t.num_items * G + (first && !t.solo_far && MIXED ? t.solo_guess : 0);
-	const int blocks = (int)std::max<long long>(1, std::min<long long>(sms * resident<MIXED, PK, false, G>(TNT),
-		(work + TNT / 32 - 1) / (TNT / 32)));
+	const auto ctas = [](long long warps) { return (warps + TNT / 32 - 1) / (TNT / 32); };
+	const long long items = ctas((long long)t.num_items * G);
+	const long long both = ctas((long long)t.num_items * G + (first && !t.solo_far ? t.solo_guess : 0));
+	const long long most = MIXED ? both : std::max(items, std::min<long long>(both, sms));
+	const int blocks = (int)std::max<long long>(1, std::min<long long>(sms * resident<MIXED, PK, false, G>(TNT), most));
 	track_kernel<MIXED, PK, false, G><<<blocks, TNT, 0, s>>>(t);
 	if ((e = cudaGetLastError()) != cudaSuccess) return e;
 	if (t.solo_far && side.side && (e = cudaStreamWaitEvent(s, side.join, 0)) != cudaSuccess) return e;
