@@ -1597,12 +1597,19 @@ ccf_status Engine::copy_results(Field& f, double* ccs, double* caustics, double*
 		error = "Error. Length scales were not requested (write_mu_length_scales = 0).";
 		return CCF_ERR_INVALID_ARGUMENT;
 	}
-	std::vector<std::pair<void*, size_t>> dst;
-	for (double* p : {ccs, caustics})
-		if (p) dst.push_back({p, npts * sizeof(double2)});
-	for (double* p : {errs, mu})
-		if (p) dst.push_back({p, npts * sizeof(double)});
-	populate(std::move(dst));
+	try
+	{
+		std::vector<std::pair<void*, size_t>> dst;
+		for (double* p : {ccs, caustics})
+			if (p) dst.push_back({p, npts * sizeof(double2)});
+		for (double* p : {errs, mu})
+			if (p) dst.push_back({p, npts * sizeof(double)});
+		populate(std::move(dst));
+	}
+	catch (const std::bad_alloc&)
+	{
+		/* the copies map the pages */
+	}
 	if (ccs) CCF_TRY(copy(ccs, f.out_ccs, npts * sizeof(double2)), "copy ccs");
 	if (errs) CCF_TRY(copy(errs, f.out_errs, npts * sizeof(double)), "copy errs");
 	if (caustics) CCF_TRY(copy(caustics, f.out_caustics, npts * sizeof(double2)), "copy caustics");

@@ -9,7 +9,7 @@ a launch of few rows left most of the GPU idle (2 rows of 40 060 roots ran on
 waits at the cluster's barrier for its slowest CTA (barrier the largest stall).
 Here a row's sweep is two phases of independent units,
 
-  step   256 roots of the row's list: the Aberth step from the sweep's
+  step   64 to 256 roots of the row's list: the Aberth step from the sweep's
          correction sums, their snapshot, then the Newton check of the next
          sweep (f, f', and the roots whose Newton step is below the tolerance
          made final) and the unit's share of the next list;
@@ -38,7 +38,8 @@ The results are those of solve_kernel to the bit, for any number of CTAs: a
 unit's partial sums run over the same sources in the same order, the chunks'
 FP32 sums are added in FP64 in chunk order, the source shares S of a tile are
 those solve_kernel's cluster of `cluster` CTAs would choose, and off-box points
-are summed by a 256-thread CTA in blocks of the same roots.  (With another
+are summed by a 256-thread CTA (solve_kernel has a warp sum those beyond
+OFF_CAP of a block, which a block of 64 never has).  (With another
 order of summation a few rows in 1e5 trade roots: the iteration is chaotic
 before it converges.)  The price is the partial sums in memory, 8 or 16 bytes
 per target, chunk and share, so large launches run PARTIAL_BYTES of rows at a
