@@ -16,6 +16,7 @@ Per batch of fields:
 The engine never resets the device and reuses its buffers across runs.
 ******************************************************************************/
 #include "engine.h"
+#include "rows_plan.h"
 
 #include <algorithm>
 #include <atomic>
@@ -169,7 +170,7 @@ ccf_status Engine::rows_setup(SolveArgs& A, int which, const std::vector<Field*>
 	CCF_TRY(P.row_control.ensure(4), "cudaMalloc(rows)");
 	CCF_TRY(P.row_part.ensure((size_t)part_bytes), "cudaMalloc(rows)");
 	/* a unit's share is 64 to 256 roots; the blocks of a row's segments may end short */
-	const long long units = maxR / ROWS_MIN_BLOCK + 17, shares = maxR + 17 * 256;
+	const long long units = maxR / MIN_BLOCK + 17, shares = maxR + 17 * 256;
 	CCF_TRY(P.row_share.ensure((size_t)(most_slots * shares)), "cudaMalloc(rows)");
 	CCF_TRY(P.row_counts.ensure((size_t)(most_slots * units)), "cudaMalloc(rows)");
 	A.share = P.row_share.ptr;
@@ -1298,7 +1299,6 @@ ccf_status Engine::solve(std::vector<Field*>& fields, int verbose)
    unless a 1/mu error is not finite */
 ccf_status Engine::finish_stats(Field& f, int seg, bool track, int verbose, int launches)
 {
-	(void)track;
 	unsigned long long st[STATS_WORDS];
 	CCF_TRY(cudaMemcpy(st, f.stats.ptr, STATS_WORDS * sizeof(unsigned long long), cudaMemcpyDeviceToHost), "stats");
 	ccf_info& info = f.info;
@@ -1332,7 +1332,15 @@ ccf_status Engine::finish_stats(Field& f, int seg, bool track, int verbose, int 
 	info.kernel_launches += launches;
 	info.centres_solved = f.params.num_branches / seg;
 	ccf_status status = CCF_OK;
-	if (info.has_nan)
+	/* the full-sum solver's rows: a centre each, and both sides of it or the rows handed to it by the tracker */
+	const unsigned long long rows = (unsigned long long)info.centres_solved;
+	if (st[STAT_ROWS_DONE] != rows + (track ? st[9] : 2 * rows))
+	{
+		f.error = "Error. The full-sum solver left rows unfinished.";
+		error = f.error;
+		status = CCF_ERR_NUMERIC;
+	}
+	else if (info.has_nan)
 	{
 		f.error = "Error. Errors in 1/mu contain values which are not positive real numbers.";
 		error = f.error;

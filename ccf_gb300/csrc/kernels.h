@@ -94,7 +94,8 @@ struct FieldOut
 	                                step, [7] updates in the initial solve, [8] terms in the initial
 	                                solve, [9] continuation rows re-run by the full-sum solver, [10]
 	                                tracker sub-step halvings, [11] TRACK_* flags of the re-run rows,
-	                                [12] rows tracked again with fine sub-steps; [16] .. [20] the
+	                                [12] rows tracked again with fine sub-steps, [13] rows the
+	                                full-sum solver finished (STAT_ROWS_DONE); [16] .. [20] the
 	                                FP64 polish (STAT_POLISHED_*) */
 };
 
@@ -119,6 +120,7 @@ CCF_HD void full_window(FieldOut& O)
 
 /* statistics words of a field (FieldOut::stats) */
 constexpr int STATS_WORDS = 24;
+constexpr int STAT_ROWS_DONE = 13;          /* rows of the field that rows_kernel ran to their end */
 constexpr int STAT_POLISHED_MAX_ERR = 16;   /* largest 1/mu error after the polish (double bits) */
 constexpr int STAT_POLISHED_NAN = 17;       /* a non-finite 1/mu error after the polish */
 constexpr int STAT_POLISHED = 18;           /* points the polish worked on */
@@ -212,8 +214,6 @@ struct RowState
 	int blk;                     /* roots per unit of the phases that evaluate roots */
 	int pad[2];
 };
-
-constexpr int ROWS_MIN_BLOCK = 64;   /* fewest roots of a unit of rows_kernel */
 
 struct SolveArgs
 {

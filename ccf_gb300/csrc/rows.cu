@@ -66,100 +66,11 @@ enum RowPhase
 	PHASE_EPILOGUE = 3
 };
 
-/* ticket of a row: units << 22 | next unit (0: none) */
-constexpr int TICKET_BITS = 22;
-constexpr unsigned long long TICKET_MASK = (1ull << TICKET_BITS) - 1;
 constexpr int POLL_LIMIT = 1 << 21;   /* polls in a row without work (~1 us each) after which a CTA leaves */
-
-CCF_D int ticket_next(unsigned long long t) { return (int)(t & TICKET_MASK); }
-CCF_D int ticket_units(unsigned long long t) { return (int)((t >> TICKET_BITS) & TICKET_MASK); }
 
 /* loads of what other CTAs wrote: past L1 */
 CCF_D unsigned long long load_cg(const unsigned long long* p) { return __ldcg(p); }
 CCF_D int load_volatile(const int* p) { return *(const volatile int*)p; }
-
-/* start of segment r of a row of R roots: the roots that CTA r of a cluster of
-   csize owns in solve_kernel.  A row's blocks of roots start at these. */
-CCF_D int segment_start(int R, int csize, int r) { return (int)((long long)R * r / csize); }
-constexpr int MIN_BLOCK = ROWS_MIN_BLOCK;
-constexpr int NO_ROOT = 1 << 20;   /* a thread past its unit's block */
-CCF_D int row_blocks(int R, int csize, int blk)
-{
-	int n = 0;
-	for (int r = 0; r < csize; r++) n += (segment_start(R, csize, r + 1) - segment_start(R, csize, r) + blk - 1) / blk;
-	return n;
-}
-
-/* Roots per unit of a phase that evaluates n roots of each row (a step, a
-   first check, an epilogue): 64, 128 or 256, the fewest that leave no more
-   units than CTAs.  A unit's time is its roots' FP64 work and the chain of one
-   evaluation: with two warps in a CTA instead of eight each scheduler's FP64
-   pipe serves one of them, and a rectangle's off-box roots, whose star sums
-   take a CTA one after another, are spread.  A row of one such unit of 256 stays
-   in its CTA, which saves handing units around: up to 256 roots (full-sum
-   continuation of a 60-star disc 8.0 ms, 8.6 in blocks of 64; a 60-star
-   rectangle 22 in blocks of 64, 25.7 in one), 128 of a rectangle (a step of 64 roots 33 us, of 256 51; the full-sum
-   continuation of 400 stars, 4 branches of 32 steps, 4.8 ms against 5.5). */
-CCF_D int block_roots(int n, int rows, int ctas, bool rectangular)
-{
-	if (n <= (rectangular ? NT / 2 : NT)) return NT;
-	int blk = MIN_BLOCK;
-	while (blk < NT && (long long)rows * ((n + blk - 1) / blk) > ctas) blk *= 2;
-	return blk;
-}
-
-/* The source split of a sweep with `total` active roots, for the shortest
-   sweep of a cluster of csize CTAs (solve_kernel). */
-CCF_D int source_split(int total, int csize)
-{
-	int S = 1, best = 1 << 30;
-	for (int s2 = 1; s2 <= NT / 32; s2 *= 2)
-	{
-		const int nt = (total + TILE / s2 - 1) / (TILE / s2);
-		const int cost = ((nt + csize - 1) / csize) * (NT / 32 + 7 * (NT / 32) / s2);
-		if (cost < best)
-		{
-			best = cost;
-			S = s2;
-		}
-	}
-	return S;
-}
-
-/* How a sweep's sums are cut into units: tpt targets per thread, 1 where two
-   would leave SMs without a unit, and 0 (one target per thread of the first
-   HALF_WARPS warps only) where such units would still be no more than the SMs:
-   a unit of eight warps runs two on each of the SM's four schedulers (with the
-   warps that have no target kept out of the loop, the initial solve of 600
-   stars in FP64 6.3 ms against 8.6, the full-sum continuation of 400 stars 4.1
-   against 4.3); and
-   chunks per unit, all of them where the whole sweep is less work than handing
-   units around (~5 us). */
-struct SumsShape
-{
-	int tpt, chunks, tiles, groups;
-};
-constexpr long long SUMS_ONE_UNIT = 1 << 16;   /* terms */
-constexpr int HALF_WARPS = NT / 64;
-CCF_D SumsShape sums_shape(int total, int S, int R, int N, int nch, int rows, int sms)
-{
-	SumsShape p;
-	p.chunks = (long long)total * (R + N) <= SUMS_ONE_UNIT ? nch : 1;
-	p.groups = (nch + p.chunks - 1) / p.chunks;
-	p.tpt = TPT;
-	p.tiles = (total + TILE / S - 1) / (TILE / S);
-	if ((long long)p.tiles * p.groups * rows < sms)
-	{
-		p.tpt = 1;
-		p.tiles = (total + NT / S - 1) / (NT / S);
-		if (S <= HALF_WARPS && (long long)p.tiles * p.groups * rows <= sms)
-		{
-			p.tpt = 0;
-			p.tiles = (total + NT / 2 / S - 1) / (NT / 2 / S);
-		}
-	}
-	return p;
-}
 
 /* shared memory of a CTA */
 template <bool MIXED>
@@ -610,6 +521,7 @@ __global__ void __launch_bounds__(NT, 2) rows_kernel(const SolveArgs A, const in
 						if (first > last)
 						{
 							/* no steps to run */
+							atomicAdd(&A.outs[rd.field].stats[STAT_ROWS_DONE], 1ull);
 							st->complete = 1;
 							__threadfence();
 							atomicAdd(&A.control[1], 1);
@@ -635,7 +547,7 @@ __global__ void __launch_bounds__(NT, 2) rows_kernel(const SolveArgs A, const in
 							if (units > 1)
 							{
 								__threadfence();
-								atomicExch(&st->ticket, (unsigned long long)units << TICKET_BITS | 1ull);
+								atomicExch(&st->ticket, ticket_open(units) | 1ull);
 							}
 						}
 					}
@@ -929,6 +841,7 @@ __global__ void __launch_bounds__(NT, 2) rows_kernel(const SolveArgs A, const in
 				}
 				if (Sh.j > j1)
 				{
+					atomicAdd(&stats[STAT_ROWS_DONE], 1ull);
 					__threadfence();
 					st->complete = 1;
 					__threadfence();
@@ -970,7 +883,7 @@ __global__ void __launch_bounds__(NT, 2) rows_kernel(const SolveArgs A, const in
 					st->chunks = Sh.shape.chunks;
 					st->tiles = Sh.shape.tiles;
 					__threadfence();
-					atomicExch(&st->ticket, (unsigned long long)units << TICKET_BITS | 1ull);
+					atomicExch(&st->ticket, ticket_open(units) | 1ull);
 				}
 			}
 		}

@@ -1,0 +1,110 @@
+/******************************************************************************
+rows_plan.h -- how the full-sum solver's work is cut: the CTA's shape, the
+blocks and units of a row (rows.cu), and the ticket its units are drawn from.
+Host and device code, so that the plan can be checked on the host.
+******************************************************************************/
+#pragma once
+
+#include "common.cuh"
+
+namespace ccf
+{
+
+constexpr int NT = 256;          /* threads per CTA */
+constexpr int MAX_CLUSTER = 16;  /* CTAs per row (above 8: the non-portable cluster sizes) */
+constexpr int TPT = 2;           /* targets per thread */
+constexpr int TILE = NT * TPT;   /* targets per tile */
+constexpr int CHUNK = 1024;      /* sources per shared-memory stage */
+
+/* ticket of a row: the units of the open phase and the next unit (0: none) in
+   one word, each as wide as the int it is read into (of 22 bits a first sweep
+   of 610 000 stars, 4.3e6 units, left 66 000) */
+constexpr int TICKET_BITS = 32;
+CCF_HD unsigned long long ticket_open(int units) { return (unsigned long long)(unsigned)units << TICKET_BITS; }
+CCF_HD int ticket_next(unsigned long long t) { return (int)(unsigned)t; }
+CCF_HD int ticket_units(unsigned long long t) { return (int)(t >> TICKET_BITS); }
+
+/* start of segment r of a row of R roots: the roots that CTA r of a cluster of
+   csize owns in solve_kernel.  A row's blocks of roots start at these. */
+CCF_HD int segment_start(int R, int csize, int r) { return (int)((long long)R * r / csize); }
+constexpr int MIN_BLOCK = 64;      /* fewest roots of a unit of rows_kernel */
+constexpr int NO_ROOT = 1 << 20;   /* a thread past its unit's block */
+CCF_HD int row_blocks(int R, int csize, int blk)
+{
+	int n = 0;
+	for (int r = 0; r < csize; r++) n += (segment_start(R, csize, r + 1) - segment_start(R, csize, r) + blk - 1) / blk;
+	return n;
+}
+
+/* Roots per unit of a phase that evaluates n roots of each row (a step, a
+   first check, an epilogue): 64, 128 or 256, the fewest that leave no more
+   units than CTAs.  A unit's time is its roots' FP64 work and the chain of one
+   evaluation: with two warps in a CTA instead of eight each scheduler's FP64
+   pipe serves one of them, and a rectangle's off-box roots, whose star sums
+   take a CTA one after another, are spread.  A row of one such unit of 256 stays
+   in its CTA, which saves handing units around: up to 256 roots (full-sum
+   continuation of a 60-star disc 8.0 ms, 8.6 in blocks of 64; a 60-star
+   rectangle 22 in blocks of 64, 25.7 in one), 128 of a rectangle (a step of 64 roots 33 us, of 256 51; the full-sum
+   continuation of 400 stars, 4 branches of 32 steps, 4.8 ms against 5.5). */
+CCF_HD int block_roots(int n, int rows, int ctas, bool rectangular)
+{
+	if (n <= (rectangular ? NT / 2 : NT)) return NT;
+	int blk = MIN_BLOCK;
+	while (blk < NT && (long long)rows * ((n + blk - 1) / blk) > ctas) blk *= 2;
+	return blk;
+}
+
+/* The source split of a sweep with `total` active roots, for the shortest
+   sweep of a cluster of csize CTAs (solve_kernel). */
+CCF_HD int source_split(int total, int csize)
+{
+	int S = 1, best = 1 << 30;
+	for (int s2 = 1; s2 <= NT / 32; s2 *= 2)
+	{
+		const int nt = (total + TILE / s2 - 1) / (TILE / s2);
+		const int cost = ((nt + csize - 1) / csize) * (NT / 32 + 7 * (NT / 32) / s2);
+		if (cost < best)
+		{
+			best = cost;
+			S = s2;
+		}
+	}
+	return S;
+}
+
+/* How a sweep's sums are cut into units: tpt targets per thread, 1 where two
+   would leave SMs without a unit, and 0 (one target per thread of the first
+   HALF_WARPS warps only) where such units would still be no more than the SMs:
+   a unit of eight warps runs two on each of the SM's four schedulers (with the
+   warps that have no target kept out of the loop, the initial solve of 600
+   stars in FP64 6.3 ms against 8.6, the full-sum continuation of 400 stars 4.1
+   against 4.3); and
+   chunks per unit, all of them where the whole sweep is less work than handing
+   units around (~5 us). */
+struct SumsShape
+{
+	int tpt, chunks, tiles, groups;
+};
+constexpr long long SUMS_ONE_UNIT = 1 << 16;   /* terms */
+constexpr int HALF_WARPS = NT / 64;
+CCF_HD SumsShape sums_shape(int total, int S, int R, int N, int nch, int rows, int sms)
+{
+	SumsShape p;
+	p.chunks = (long long)total * (R + N) <= SUMS_ONE_UNIT ? nch : 1;
+	p.groups = (nch + p.chunks - 1) / p.chunks;
+	p.tpt = TPT;
+	p.tiles = (total + TILE / S - 1) / (TILE / S);
+	if ((long long)p.tiles * p.groups * rows < sms)
+	{
+		p.tpt = 1;
+		p.tiles = (total + NT / S - 1) / (NT / S);
+		if (S <= HALF_WARPS && (long long)p.tiles * p.groups * rows <= sms)
+		{
+			p.tpt = 0;
+			p.tiles = (total + NT / 2 / S - 1) / (NT / 2 / S);
+		}
+	}
+	return p;
+}
+
+} /* namespace ccf */

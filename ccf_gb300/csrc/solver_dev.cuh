@@ -8,17 +8,12 @@ box.
 
 #include "field_df.cuh"
 #include "kernels.h"
+#include "rows_plan.h"
 
 #include <type_traits>
 
 namespace ccf
 {
-
-constexpr int NT = 256;          /* threads per CTA */
-constexpr int MAX_CLUSTER = 16;  /* CTAs per row (above 8: the non-portable cluster sizes) */
-constexpr int TPT = 2;           /* targets per thread */
-constexpr int TILE = NT * TPT;   /* targets per tile */
-constexpr int CHUNK = 1024;      /* sources per shared-memory stage */
 
 CCF_D void cp_async16(void* smem, const void* gmem)
 {
