@@ -140,49 +140,52 @@ Engine::~Engine()
 	}
 }
 
-/* device memory for the partial sums of the rows a launch_rows works on at
-   once: a 40 060-root row takes 41 MB, one of the 2000-star field 1.6 MB */
-constexpr long long PARTIAL_BYTES = 256LL << 20;
+/* bytes of one row's partial sums: ROWS_PART_BYTES, or CCF_GB300_ROW_SUMS_BYTES
+   (the tests set it to reach the whole sums with small fields) */
+static long long row_sums_limit()
+{
+	const char* e = std::getenv("CCF_GB300_ROW_SUMS_BYTES");
+	const long long v = e ? std::atoll(e) : 0;
+	return v > 0 ? std::min(v, ROWS_PART_BYTES) : ROWS_PART_BYTES;
+}
 
 ccf_status Engine::rows_setup(SolveArgs& A, int which, const std::vector<Field*>& fields, bool mixed, const int rows[2],
 	const int cluster[2])
 {
 	SolverPools& P = pools;
 	cudaStream_t s = stream;
+	const long long limit = row_sums_limit();
 	/* sized for both launches at once: a buffer that grew between them would go
 	   back to the cache under the first */
-	long long stride[2] = {0, 0}, slots[2], part_bytes = 0, most_slots = 0;
-	int bytes = 0, maxR = 0;
+	RowsScratch plan[2];
+	long long part_bytes = 0, shares = 0, units = 0;
+	int maxR = 0;
 	for (const Field* f : fields) maxR = std::max(maxR, f->d.num_roots);
 	for (int k = 0; k < 2; k++)
 	{
-		for (const Field* f : fields)
-		{
-			long long n = 0;
-			bytes = rows_partials(f->d.num_roots, f->d.num_stars, cluster[k], mixed, &n);
-			stride[k] = std::max(stride[k], n);
-		}
-		slots[k] = std::max<long long>(1, std::min<long long>(rows[k], PARTIAL_BYTES / (stride[k] * bytes)));
-		part_bytes = std::max(part_bytes, slots[k] * stride[k] * bytes);
-		most_slots = std::max(most_slots, slots[k]);
+		long long part = 0;
+		for (const Field* f : fields) part = std::max(part, row_part_bytes(f->d.num_roots, f->d.num_stars, cluster[k], mixed, limit));
+		plan[k] = rows_scratch(part, maxR, rows[k]);
+		part_bytes = std::max(part_bytes, plan[k].slots * plan[k].stride);
+		shares = std::max(shares, plan[k].slots * plan[k].shares);
+		units = std::max(units, plan[k].slots * plan[k].units);
 	}
 	CCF_TRY(P.row_state.ensure((size_t)rows[0] + rows[1]), "cudaMalloc(rows)");
 	CCF_TRY(P.row_control.ensure(4), "cudaMalloc(rows)");
 	CCF_TRY(P.row_part.ensure((size_t)part_bytes), "cudaMalloc(rows)");
-	/* a unit's share is 64 to 256 roots; the blocks of a row's segments may end short */
-	const long long units = maxR / MIN_BLOCK + 17, shares = maxR + 17 * 256;
-	CCF_TRY(P.row_share.ensure((size_t)(most_slots * shares)), "cudaMalloc(rows)");
-	CCF_TRY(P.row_counts.ensure((size_t)(most_slots * units)), "cudaMalloc(rows)");
+	CCF_TRY(P.row_share.ensure((size_t)shares), "cudaMalloc(rows)");
+	CCF_TRY(P.row_counts.ensure((size_t)units), "cudaMalloc(rows)");
 	A.share = P.row_share.ptr;
 	A.counts = P.row_counts.ptr;
-	A.share_stride = shares;
-	A.counts_stride = units;
+	A.share_stride = plan[which].shares;
+	A.counts_stride = plan[which].units;
 	A.cluster = cluster[which];
 	A.state = P.row_state.ptr + (which ? rows[0] : 0);
 	A.control = P.row_control.ptr + 2 * which;
 	A.part = P.row_part.ptr;
-	A.part_slots = (int)slots[which];
-	A.part_stride = stride[which];
+	A.part_slots = (int)plan[which].slots;
+	A.part_stride = plan[which].stride;
+	A.part_limit = limit;
 	CCF_TRY(cudaMemsetAsync(A.state, 0, (size_t)rows[which] * sizeof(RowState), s), "memset");
 	CCF_TRY(cudaMemsetAsync(A.control, 0, 2 * sizeof(int), s), "memset");
 	return CCF_OK;

@@ -209,10 +209,10 @@ struct RowState
 	int done;                    /* units of the phase that are finished */
 	int phase, it, j;
 	int total, late;             /* roots of the sweep's list: active; made final by its check */
-	int split, tpt, chunks, tiles;   /* the shape of its sums */
+	int split, tpt, chunks, tiles, whole;   /* the shape of its sums */
 	int complete;
 	int blk;                     /* roots per unit of the phases that evaluate roots */
-	int pad[2];
+	int pad;
 };
 
 struct SolveArgs
@@ -234,9 +234,10 @@ struct SolveArgs
 	/* rows.cu */
 	RowState* state;       /* [num_rows], zeroed before the launch */
 	int* control;          /* next row to start, rows complete; zeroed before the launch */
-	void* part;            /* partial sums: part_slots rows of part_stride elements */
+	void* part;            /* partial sums: part_slots rows of part_stride bytes */
 	int part_slots;
 	long long part_stride;
+	long long part_limit;  /* bytes of one row's above which its sums are whole (rows_plan.h) */
 	int* share;            /* the units' shares of the next list, share_stride a slot */
 	int* counts;           /* and their lengths, counts_stride a slot */
 	long long share_stride, counts_stride;
@@ -474,9 +475,7 @@ size_t fold_binom_size(int nf, int nr, int nq);
 int solver_blocks_per_sm(bool mixed);
 cudaError_t launch_solve(cudaStream_t s, const SolveArgs& a, bool mixed, bool initial);
 /* rows.cu: launch_solve with every row spread over the GPU; cluster then only
-   sets the order of summation.  rows_partials: the elements of one row's
-   partial sums, and the bytes of one */
-int rows_partials(int R, int N, int cluster, bool mixed, long long* elements);
+   sets the order of summation (their memory: rows_plan.h) */
 cudaError_t launch_rows(cudaStream_t s, const SolveArgs& a, bool mixed, bool initial, int num_sms, int max_roots, int max_stars);
 cudaError_t launch_track_mark(cudaStream_t s, const TrackArgs& a, int* cls);
 cudaError_t launch_track_item_order(cudaStream_t s, const TrackArgs& a, int* work, int* order);

@@ -42,8 +42,9 @@ are summed by a 256-thread CTA (solve_kernel has a warp sum those beyond
 OFF_CAP of a block, which a block of 64 never has).  (With another
 order of summation a few rows in 1e5 trade roots: the iteration is chaotic
 before it converges.)  The price is the partial sums in memory, 8 or 16 bytes
-per target, chunk and share, so large launches run PARTIAL_BYTES of rows at a
-time; ccf_continue_branch_noalloc, which has no memory for them, keeps
+per target, chunk and share, so large launches run ROWS_PART_BYTES of rows at a
+time, and a row of more than that alone has its units add their chunks up
+(rows_plan.h); ccf_continue_branch_noalloc, which has no memory for them, keeps
 solve_kernel.
 ******************************************************************************/
 #define CCF_EVAL_UNROLL 4
@@ -273,8 +274,10 @@ CCF_D double widen(float x)
 }
 CCF_D double widen(double x) { return x; }
 
-/* one unit of the sums phase: tile against a group of chunks */
-template <bool MIXED, int TP>
+/* one unit of the sums phase: tile against a group of chunks.  WHOLE: against
+   all of them, the chunks of the roots and those of the stars added up in FP64
+   in order, as gather_sums adds the chunks' sums. */
+template <bool MIXED, int TP, bool WHOLE>
 __device__ void sums_unit(const SolveArgs& A, RowShared<MIXED>& Sh, const int* list, typename PartT<MIXED>::T* part_out)
 {
 	using SrcT = typename Src<MIXED>::T;
@@ -319,6 +322,23 @@ __device__ void sums_unit(const SolveArgs& A, RowShared<MIXED>& Sh, const int* l
 		if constexpr (MIXED) zs[t] = g[t] < total ? __ldcg(rsrc + __ldcg(list + g[t])) : make_float4(0, 0, 0, 0);
 		else zs[t] = g[t] < total ? __ldcg(rsrc + __ldcg(list + g[t])) : make_double2(0, 0);
 	}
+	double2 tot[WHOLE ? TP : 1];
+	if constexpr (WHOLE)
+	{
+#pragma unroll
+		for (int t = 0; t < TP; t++) tot[t] = make_double2(0, 0);
+	}
+	auto add_whole = [&](int t, int ch, double x, double y) {
+		if constexpr (WHOLE)
+		{
+			tot[t].x += x;
+			tot[t].y -= y;
+			if (ch != nrc - 1 && ch != nch - 1) return;
+			double2* whole = reinterpret_cast<double2*>(part_out) + (size_t)((ch < nrc ? 0 : S) + part) * total;
+			if (g[t] < total) whole[g[t]] = tot[t];
+			tot[t] = make_double2(0, 0);
+		}
+	};
 	for (int ch = ch0; ch < ch1; ch++)
 	{
 		const int buf = (ch - ch0) & 1;
@@ -352,7 +372,10 @@ __device__ void sums_unit(const SolveArgs& A, RowShared<MIXED>& Sh, const int* l
 			}
 #pragma unroll
 			for (int t = 0; t < TP; t++)
-				if (g[t] < total) out[g[t]] = make_float2(ax[t], ay[t]);
+			{
+				if constexpr (WHOLE) add_whole(t, ch, (double)ax[t], (double)ay[t]);
+				else if (g[t] < total) out[g[t]] = make_float2(ax[t], ay[t]);
+			}
 		}
 		else
 		{
@@ -376,10 +399,21 @@ __device__ void sums_unit(const SolveArgs& A, RowShared<MIXED>& Sh, const int* l
 			}
 #pragma unroll
 			for (int t = 0; t < TP; t++)
-				if (g[t] < total) out[g[t]] = make_double2(ax[t], ay[t]);
+			{
+				if constexpr (WHOLE) add_whole(t, ch, ax[t], ay[t]);
+				else if (g[t] < total) out[g[t]] = make_double2(ax[t], ay[t]);
+			}
 		}
 		__syncthreads();
 	}
+}
+
+/* out of line: only rows beyond ROWS_PART_BYTES take it */
+template <bool MIXED>
+__device__ __noinline__ void sums_unit_whole(const SolveArgs& A, RowShared<MIXED>& Sh, const int* list, typename PartT<MIXED>::T* part_out)
+{
+	if (Sh.shape.tpt <= 1) sums_unit<MIXED, 1, true>(A, Sh, list, part_out);
+	else sums_unit<MIXED, TPT, true>(A, Sh, list, part_out);
 }
 
 /* The sums of position g of the row's list.  Every lane adds up its own root's,
@@ -388,11 +422,24 @@ __device__ void sums_unit(const SolveArgs& A, RowShared<MIXED>& Sh, const int* l
    x, y) of share q.  Either way a share's chunks are added in order, then the
    shares in order. */
 template <bool MIXED>
-CCF_D void gather_sums(const typename PartT<MIXED>::T* part, bool act, int g, int total, int S, int nrc, int nch, double2& totR,
-	double2& totS)
+CCF_D void gather_sums(const typename PartT<MIXED>::T* part, bool act, int g, int total, int S, int nrc, int nch, bool whole,
+	double2& totR, double2& totS)
 {
 	const unsigned full = 0xffffffffu;
 	totR = totS = make_double2(0, 0);
+	if (whole)
+	{
+		/* the chunks are added up already (sums_unit) */
+		if (!act) return;
+		const double2* p = reinterpret_cast<const double2*>(part) + g;
+		for (int q = 0; q < S; q++)
+		{
+			const double2 r = __ldcg(p + (size_t)q * total), s = __ldcg(p + (size_t)(S + q) * total);
+			totR = q == 0 ? r : cadd(totR, r);
+			totS = q == 0 ? s : cadd(totS, s);
+		}
+		return;
+	}
 	unsigned m = __ballot_sync(full, act);
 	/* FP64 additions in a row: 2 per chunk and share; or the longer of the two
 	   chunk ranges, the shares and the loads' latency (~10), per root */
@@ -494,6 +541,7 @@ __global__ void __launch_bounds__(NT, 2) rows_kernel(const SolveArgs A, const in
 			Sh.shape.tpt = load_volatile(&st->tpt);
 			Sh.shape.chunks = load_volatile(&st->chunks);
 			Sh.shape.tiles = load_volatile(&st->tiles);
+			Sh.shape.whole = load_volatile(&st->whole);
 			return true;
 		};
 		const bool kept = Sh.own_next != 0;
@@ -649,13 +697,14 @@ __global__ void __launch_bounds__(NT, 2) rows_kernel(const SolveArgs A, const in
 		int* const share = only ? list : shares + (size_t)Sh.unit * blk;
 		int* const share_end = only ? list + R : share + blk;
 		int* const share_count = only ? nullptr : counts + Sh.unit;
-		typename PartT<MIXED>::T* part = reinterpret_cast<typename PartT<MIXED>::T*>(A.part) +
-			(size_t)(row % A.part_slots) * A.part_stride;
+		typename PartT<MIXED>::T* part = reinterpret_cast<typename PartT<MIXED>::T*>(
+			reinterpret_cast<unsigned char*>(A.part) + (size_t)(row % A.part_slots) * A.part_stride);
 
 		if (Sh.phase == PHASE_SUMS)
 		{
-			if (Sh.shape.tpt <= 1) sums_unit<MIXED, 1>(A, Sh, list, part);
-			else sums_unit<MIXED, TPT>(A, Sh, list, part);
+			if (Sh.shape.whole) sums_unit_whole<MIXED>(A, Sh, list, part);
+			else if (Sh.shape.tpt <= 1) sums_unit<MIXED, 1, false>(A, Sh, list, part);
+			else sums_unit<MIXED, TPT, false>(A, Sh, list, part);
 		}
 		else
 		{
@@ -670,7 +719,7 @@ __global__ void __launch_bounds__(NT, 2) rows_kernel(const SolveArgs A, const in
 				const int a = own ? __ldcg(list + (act ? g : R - 1 - (g - total))) : 0;
 				double2 z = own ? __ldcg(A.master + base + a) : make_double2(0, 0);
 				double2 totR, totS;
-				gather_sums<MIXED>(part, act, g, total, Sh.split, nrc, nch, totR, totS);
+				gather_sums<MIXED>(part, act, g, total, Sh.split, nrc, nch, Sh.shape.whole != 0, totR, totS);
 				if (act)
 				{
 					const double2 f = __ldcg(A.fval + 2 * (base + a)), df = __ldcg(A.fval + 2 * (base + a) + 1);
@@ -851,7 +900,8 @@ __global__ void __launch_bounds__(NT, 2) rows_kernel(const SolveArgs A, const in
 				{
 					phase = PHASE_SUMS;
 					Sh.split = source_split(Sh.total, csize);
-					Sh.shape = sums_shape(Sh.total, Sh.split, R, N, nch, rows_at_work, (int)gridDim.x / 2);
+					Sh.shape = sums_shape(Sh.total, Sh.split, R, N, nch, rows_at_work, (int)gridDim.x / 2,
+						sums_whole(Sh.total, Sh.split, nch, MIXED, A.part_limit));
 					units = Sh.shape.tiles * Sh.shape.groups;
 					const unsigned long long terms = (unsigned long long)Sh.total * (unsigned long long)(R - 1 + N);
 					atomicAdd(&stats[3], terms);
@@ -882,6 +932,7 @@ __global__ void __launch_bounds__(NT, 2) rows_kernel(const SolveArgs A, const in
 					st->tpt = Sh.shape.tpt;
 					st->chunks = Sh.shape.chunks;
 					st->tiles = Sh.shape.tiles;
+					st->whole = Sh.shape.whole;
 					__threadfence();
 					atomicExch(&st->ticket, ticket_open(units) | 1ull);
 				}
@@ -891,16 +942,6 @@ __global__ void __launch_bounds__(NT, 2) rows_kernel(const SolveArgs A, const in
 	}
 }
 
-}
-
-int rows_partials(int R, int N, int cluster, bool mixed, long long* elements)
-{
-	/* S total is at most 10.5 tiles of the cluster with S >= 4, 2 R with S = 2
-	   (source_split's costs), and 8 R */
-	const long long chunks = (R + CHUNK - 1) / CHUNK + (N + CHUNK - 1) / CHUNK;
-	const long long targets = std::min<long long>(8LL * R, std::max<long long>(2LL * R, 21LL * TILE * cluster / 2));
-	*elements = chunks * targets;
-	return mixed ? (int)sizeof(float2) : (int)sizeof(double2);
 }
 
 cudaError_t launch_rows(cudaStream_t s, const SolveArgs& a, bool mixed, bool initial, int num_sms, int max_roots, int max_stars)

@@ -7,6 +7,8 @@ Host and device code, so that the plan can be checked on the host.
 
 #include "common.cuh"
 
+#include <algorithm>
+
 namespace ccf
 {
 
@@ -80,17 +82,21 @@ CCF_HD int source_split(int total, int csize)
    stars in FP64 6.3 ms against 8.6, the full-sum continuation of 400 stars 4.1
    against 4.3); and
    chunks per unit, all of them where the whole sweep is less work than handing
-   units around (~5 us). */
+   units around (~5 us), or where it is whole: the partial sums of its chunks
+   would take more than the row's memory allows (RowsScratch), so a unit adds
+   its chunks up itself, in the same order, and a row's memory stays
+   proportional to its roots. */
 struct SumsShape
 {
-	int tpt, chunks, tiles, groups;
+	int tpt, chunks, tiles, groups, whole;
 };
 constexpr long long SUMS_ONE_UNIT = 1 << 16;   /* terms */
 constexpr int HALF_WARPS = NT / 64;
-CCF_HD SumsShape sums_shape(int total, int S, int R, int N, int nch, int rows, int sms)
+CCF_HD SumsShape sums_shape(int total, int S, int R, int N, int nch, int rows, int sms, bool whole)
 {
 	SumsShape p;
-	p.chunks = (long long)total * (R + N) <= SUMS_ONE_UNIT ? nch : 1;
+	p.whole = whole ? 1 : 0;
+	p.chunks = whole || (long long)total * (R + N) <= SUMS_ONE_UNIT ? nch : 1;
 	p.groups = (nch + p.chunks - 1) / p.chunks;
 	p.tpt = TPT;
 	p.tiles = (total + TILE / S - 1) / (TILE / S);
@@ -104,6 +110,54 @@ CCF_HD SumsShape sums_shape(int total, int S, int R, int N, int nch, int rows, i
 			p.tiles = (total + NT / 2 / S - 1) / (NT / 2 / S);
 		}
 	}
+	return p;
+}
+
+/* whether a sweep's sums are whole: its partial sums, one per target, chunk
+   and source share, take more than limit bytes */
+CCF_HD bool sums_whole(int total, int S, int nch, bool mixed, long long limit)
+{
+	return (long long)S * total * nch * (mixed ? (long long)sizeof(float2) : (long long)sizeof(double2)) > limit;
+}
+
+/* Device memory of a launch's rows at work: of each, its partial sums (stride
+   bytes), the units' shares of the next list and their lengths; slots rows at
+   once, the others wait for one.  One row of a 20 000-star field has 41 MB of
+   partial sums, of the 2000-star one 1.6 MB.  They grow with the square of the
+   stars: a row whose sums would take more than limit bytes (from 52 000 stars
+   on) has whole sums in the sweeps that exceed it, two FP64 sums per target
+   and share (64 bytes a root), and its other sweeps as before.  Whole sweeps
+   have fewer and longer units, which fill the GPU less evenly: the initial
+   solve of 100 000 stars 159 ms, with every chunk's sums kept 149, of 200 000
+   540 and 492; but such a field holds 0.6 and 0.5 GB on the device instead of
+   1.5 and 4.2. */
+constexpr long long ROWS_PART_BYTES = 256LL << 20;
+struct RowsScratch
+{
+	long long stride, slots, shares, units;   /* bytes; rows; ints a slot; ints a slot */
+	CCF_HD long long bytes() const { return slots * (stride + 4 * (shares + units)); }
+};
+/* the partial sums of one row of R roots and N stars, at most, in bytes.  S
+   total is at most 10.5 tiles of the cluster with S >= 4, 2 R with S = 2
+   (source_split's costs), and 8 R */
+inline long long row_part_bytes(long long R, long long N, int cluster, bool mixed, long long limit)
+{
+	const long long chunks = (R + CHUNK - 1) / CHUNK + (N + CHUNK - 1) / CHUNK;
+	const long long targets = std::min<long long>(8 * R, std::max<long long>(2 * R, 21LL * TILE * cluster / 2));
+	const long long full = chunks * targets * (long long)(mixed ? sizeof(float2) : sizeof(double2));
+	const long long b = full <= limit ? full : std::max<long long>(limit, 2 * targets * (long long)sizeof(double2));
+	return (b + 15) / 16 * 16;
+}
+/* part: the largest row_part_bytes of the launch's rows, maxR: its most roots */
+inline RowsScratch rows_scratch(long long part, long long maxR, long long rows)
+{
+	RowsScratch p;
+	p.stride = part;
+	/* a unit's share is 64 to 256 roots; the blocks of a row's segments may end short */
+	p.shares = maxR + 17 * NT;
+	p.units = maxR / MIN_BLOCK + 17;
+	p.slots = 1;
+	p.slots = std::max(1LL, std::min(rows, ROWS_PART_BYTES / p.bytes()));
 	return p;
 }
 

@@ -113,3 +113,21 @@ def test_rows_do_not_depend_on_the_sums_tiles(n, nb, precision):
     b = fs[-1].results()
     assert np.array_equal(r["ccs"][:, 4], b["ccs"][:, 4])
     assert O.match_sets(r["ccs"], b["ccs"], nb)["max_dist"] <= 1e-11
+
+
+@pytest.mark.parametrize("precision", ["mixed", "fp64"])
+@pytest.mark.parametrize("n, rectangular", [(1, 0), (40, 1), (129, 0), (520, 1), (1500, 0)])
+def test_whole_sums_are_the_chunks_sums(monkeypatch, n, rectangular, precision):
+    """A row whose partial sums would exceed its memory has its units add their
+    chunks up, in the order in which the step adds them otherwise: the same
+    bits with every sweep whole (1 byte) and with the first ones whole."""
+    outs = []
+    for limit in (None, "1", "60000"):
+        if limit:
+            monkeypatch.setenv("CCF_GB300_ROW_SUMS_BYTES", limit)
+        c = field(n, rectangular, nb=2, num_phi=8, continuation="aberth", precision=precision)
+        assert c.run(-1), c.last_error()
+        outs.append(c.results())
+    for r in outs[1:]:
+        for k in ("ccs", "caustics", "errs"):
+            assert np.array_equal(outs[0][k], r[k]), k

@@ -34,7 +34,7 @@ def test_a_ticket_holds_any_number_of_units(tmp_path):
         const int R = (int)(2 * n), N = (int)n, nch = (R + CHUNK - 1) / CHUNK + (N + CHUNK - 1) / CHUNK;
         for (int total : {1, R / 1000 + 1, R})
         {
-            const SumsShape p = sums_shape(total, source_split(total, 16), R, N, nch, 1, 152);
+            const SumsShape p = sums_shape(total, source_split(total, 16), R, N, nch, 1, 152, false);
             const int units = p.tiles * p.groups;
             if (units < 1 || p.groups * p.chunks < nch) bad++;
             unsigned long long t = ticket_open(units) | 1ull;
@@ -45,4 +45,36 @@ def test_a_ticket_holds_any_number_of_units(tmp_path):
             if (ticket_units(t) != units || ticket_next(t) != units + 304) bad++;
         }
     }
+""")
+
+
+def test_a_rows_partial_sums_stay_within_their_memory(tmp_path):
+    """Every sweep of a row fits the bytes its plan gives it, whole sums or one
+    per chunk, and from 52 000 stars on those bytes grow with the stars and no
+    longer with their square."""
+    run_program(tmp_path, r"""
+    for (long long n : {1LL, 31LL, 700LL, 5000LL, 20000LL, 52000LL, 60000LL, 100000LL, 605000LL, 2000000LL})
+        for (int cluster : {1, 2, 4, 8, 16})
+            for (bool mixed : {false, true})
+                for (long long limit : {1LL, 100000LL, ROWS_PART_BYTES})
+                {
+                    const int R = (int)(2 * n), N = (int)n, nch = (R + CHUNK - 1) / CHUNK + (N + CHUNK - 1) / CHUNK;
+                    const long long bytes = row_part_bytes(R, N, cluster, mixed, limit);
+                    if (bytes % 16 != 0) bad++;
+                    if (limit == ROWS_PART_BYTES && bytes > std::max(ROWS_PART_BYTES, 64LL * R + 32LL * 21 * TILE * 8)) bad++;
+                    for (int total = 1; total <= R; total += total < 20000 ? 1 : 997)
+                    {
+                        const int S = source_split(total, cluster);
+                        const bool whole = sums_whole(total, S, nch, mixed, limit);
+                        const long long need = (long long)S * total * (whole ? 2 * 16 : nch * (mixed ? 8 : 16));
+                        if (need > bytes) bad++;
+                        const SumsShape p = sums_shape(total, S, R, N, nch, 1, 152, whole);
+                        if (whole && p.groups != 1) bad++;
+                    }
+                    for (long long rows : {1LL, 64LL, 12288LL})
+                    {
+                        const RowsScratch q = rows_scratch(bytes, R, rows);
+                        if (q.slots < 1 || q.slots > rows || (q.slots > 1 && q.bytes() > ROWS_PART_BYTES)) bad++;
+                    }
+                }
 """)
