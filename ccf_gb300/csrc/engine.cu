@@ -191,11 +191,6 @@ ccf_status Engine::rows_setup(SolveArgs& A, int which, const std::vector<Field*>
 	return CCF_OK;
 }
 
-/* room for the roots that leave the box: a few per row do (20 of 160 000 on
-   the 20 000-star field); those beyond it stay in their items */
-constexpr int FAR_EVICT_CAP = 8192;
-constexpr int OUT_LIST_CAP = 1 << 18;   /* 2 MB */
-
 cudaError_t Engine::far_setup(TrackArgs& T, long long roots, long long smooth, int max_stars, long long out_points)
 {
 	cudaError_t e;
@@ -903,9 +898,6 @@ static size_t nb_total(const std::vector<Field*>& fields)
 	for (const Field* f : fields) n += (size_t)f->params.num_branches;
 	return n;
 }
-
-/* largest number of branches per solved centre the engine picks by itself */
-constexpr int MAX_SEG = 16;
 
 int Engine::solved_seg(const Field& f, bool track) const
 {

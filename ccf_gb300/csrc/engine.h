@@ -262,6 +262,12 @@ struct UploadPack
    setup) is built by one CTA (batch.cu) */
 constexpr int BATCH_SETUP_MAX_STARS = 8192;
 
+/* largest number of branches per solved centre the engine picks by itself */
+constexpr int MAX_SEG = 16;
+
+/* bytes of a window of streamed outputs (stream.cu) */
+size_t chunk_bytes();
+
 /* the root's half length (include/ccf.cuh:746) and the leaf limit: the
    reference's 32 unless leaf_max_stars lowers it */
 inline double root_half_length(const Derived& d)

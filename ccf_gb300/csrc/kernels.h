@@ -267,6 +267,11 @@ struct FarState
 	int row, root, head, hn, run, t0, t1, j, tt, it, evs, refine;
 };
 
+/* room for the roots that leave the box: a few per row do (20 of 160 000 on
+   the 20 000-star field); those beyond it stay in their items */
+constexpr int FAR_EVICT_CAP = 8192;
+constexpr int OUT_LIST_CAP = 1 << 18;   /* TrackArgs::out_list, 2 MB */
+
 struct TrackArgs
 {
 	const FieldView* fields;

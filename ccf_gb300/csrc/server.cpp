@@ -11,8 +11,8 @@ admitted requests hold, counted from admission until the caller releases the
 request.
 ******************************************************************************/
 #include "../../include/ccf_gb300.h"
-#include "common.cuh"
-#include "params.h"
+#include "engine.h"
+#include "rows_plan.h"
 
 #include <chrono>
 #include <condition_variable>
@@ -29,34 +29,70 @@ request.
 namespace
 {
 
-/* Upper estimate of the device bytes of one run (engine.cu's buffers). */
+/* Upper estimate of the device bytes of one run (engine.cu's buffers, and
+   stream.cu's). */
 unsigned long long estimate_bytes(const ccf_params& p, const ccf::Derived& d)
 {
-	const unsigned long long N = (unsigned long long)d.num_stars;
-	const unsigned long long R = (unsigned long long)d.num_roots;
-	const unsigned long long nb = (unsigned long long)p.num_branches;
-	const unsigned long long cols = (unsigned long long)(p.num_phi / p.num_branches + 1);
-	const unsigned long long P1 = (unsigned long long)ccf::MAX_ORDER + 1;
+	typedef unsigned long long u64;
+	const u64 N = (u64)d.num_stars;
+	const u64 R = (u64)d.num_roots;
+	const u64 nb = (u64)p.num_branches;
+	const u64 cols = (u64)(p.num_phi / p.num_branches + 1);
+	const u64 P1 = (u64)ccf::MAX_ORDER + 1;
+	const bool mixed = p.precision == CCF_PRECISION_MIXED;
+	const bool track = p.continuation == CCF_CONTINUATION_TRACK;
 	/* stars: generation and tree order, scratch copies, masses, split forms */
-	unsigned long long b = N * (16 + 16 + 16 + 8 + 8 + 16 + 8);
+	u64 b = N * (16 + 16 + 16 + 8 + 8 + 16 + 8);
 	/* tree and FMM: at most ~N leaves; nodes <= 4/3 of the leaves, per node the
 	   structure arrays and the multipole and local coefficients */
-	const unsigned long long nodes = 2 * N + 64;
+	const u64 nodes = 2 * N + 64;
 	b += nodes * (224 + 2 * P1 * 16);
-	/* leaves: near lists (FP64 and double-float), local blocks, FP32 copy */
+	/* leaves: near lists (FP64 and double-float), local blocks, FP32 copy; the
+	   packed near lists and blocks; the blocks with the smooth mass folded in */
 	b += nodes * (32 * 32 + 3 * P1 * 16 + P1 * 8 + 32 * 24 + 2 * P1 * 16 + 64);
+	if (mixed)
+	{
+		b += nodes * ((u64)ccf::NEAR_PAIRS * ccf::NEAR_PAIR_F4 * 16 + 2 * P1 * 16);
+		if (d.rectangular && p.approx) b += nodes * (2 * P1 * 16 + P1 * 8 + 3 * P1 * 16 + 1) + 3 * 256 * 256 * 8;
+	}
 	/* solver rows: centres and (branch, side) rows, 69 bytes per root */
 	b += 3 * nb * R * 69;
-	/* tracker: column tables (2 R slots of 8 bytes per phi step of every row),
-	   solo-root lists (9 bytes per root of a row), row records and statistics */
-	if (p.continuation == CCF_CONTINUATION_TRACK) b += 2 * nb * (cols / 2) * 2 * R * 8 + 2 * nb * R * 9 + 2 * nb * (40 + 40);
-	/* outputs in the file layout (none on the device with host_outputs) */
-	const unsigned long long pts = R * nb * cols;
-	if (!p.host_outputs)
+	/* the rows at work: their states, and one launch's partial sums and shares
+	   (rows_plan.h).  The widest order of summation: a cluster of at least 256
+	   roots a CTA, or the caller's */
 	{
-		b += pts * (16 + 8);
-		if (p.write_caustics) b += pts * 16;
-		if (p.write_mu_length_scales) b += pts * 8;
+		int cluster = 1;
+		while (cluster < ccf::MAX_CLUSTER && R / (2 * (u64)cluster) >= 256) cluster *= 2;
+		const ccf::RowsScratch one = ccf::rows_scratch(
+			ccf::row_part_bytes((long long)R, (long long)N, std::max(cluster, p.init_cluster), mixed, ccf::ROWS_PART_BYTES), (long long)R, 1);
+		const u64 cap = (u64)ccf::ROWS_PART_BYTES, rows = 2 * nb, lists = 4 * (u64)(one.shares + one.units);
+		b += 3 * nb * sizeof(ccf::RowState);
+		b += std::min(rows * (u64)one.stride, std::max(cap, (u64)one.stride));
+		b += std::min(rows * lists, std::max(cap, lists));
+	}
+	/* outputs in the file layout (with host_outputs below) */
+	const u64 pts = R * nb * cols;
+	const u64 point = 16 + 8 + (p.write_caustics ? 16 : 0) + (p.write_mu_length_scales ? 8 : 0);
+	/* tracker: column tables (2 R slots of 8 bytes per phi step of every row),
+	   solo-root lists (9 bytes per root of a row), row records and statistics,
+	   the queue of items, the phases, the roots handed to the far launch and
+	   the points whose FP64 outputs are formed after the launch */
+	if (track)
+	{
+		b += 2 * nb * (cols / 2) * 2 * R * 8 + 2 * nb * R * 9 + 2 * nb * (40 + 40);
+		b += 2 * nb * (R / 32 + 1) * 16 + (u64)p.num_phi * sizeof(ccf::PhaseEntry);
+		b += std::min<u64>(2 * nb * R, ccf::FAR_EVICT_CAP) * sizeof(ccf::FarState);
+		if (!mixed || p.write_mu_length_scales) b += std::min<u64>(pts, ccf::OUT_LIST_CAP) * 8;
+	}
+	/* the polish's list of points */
+	b += std::min<u64>(1ull << 24, std::max<u64>(1ull << 16, pts / 128)) * 8;
+	if (!p.host_outputs) b += pts * point;
+	/* streamed outputs: the centre columns and two windows of branches */
+	if (p.host_outputs == 2)
+	{
+		const u64 seg = !track ? 1 : p.solved_centres > 0 ? nb / (u64)p.solved_centres : std::min<u64>(nb, ccf::MAX_SEG);
+		const u64 window = std::max((u64)ccf::chunk_bytes(), R * (seg + 1) * cols * point);
+		b += R * nb * point + 2 * std::min(window, pts * point);
 	}
 	return b + (64ull << 20);
 }

@@ -41,14 +41,6 @@ namespace
 
 constexpr size_t CHUNK_BYTES = (size_t)2 << 30;
 
-/* the chunk size target: CHUNK_BYTES, or CCF_GB300_CHUNK_BYTES (bytes) */
-size_t chunk_bytes()
-{
-	const char* e = std::getenv("CCF_GB300_CHUNK_BYTES");
-	const long long v = e ? std::atoll(e) : 0;
-	return v > 0 ? (size_t)v : CHUNK_BYTES;
-}
-
 #define CCF_TRY_S(expr, what)                                   \
 	do                                                          \
 	{                                                           \
@@ -87,6 +79,14 @@ std::vector<CopyRun> window_runs(const std::vector<unsigned char>& mask, int w_b
 }
 
 } /* namespace */
+
+/* the chunk size target: CHUNK_BYTES, or CCF_GB300_CHUNK_BYTES (bytes) */
+size_t chunk_bytes()
+{
+	const char* e = std::getenv("CCF_GB300_CHUNK_BYTES");
+	const long long v = e ? std::atoll(e) : 0;
+	return v > 0 ? (size_t)v : CHUNK_BYTES;
+}
 
 ccf_status Engine::solve_chunked(Field& f, int verbose)
 {

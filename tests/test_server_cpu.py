@@ -100,3 +100,23 @@ def _has_gpu() -> bool:
         return torch.cuda.is_available()
     except Exception:
         return False
+
+
+@pytest.mark.parametrize("num_stars, extra, sums", [
+    # the partial sums of the rows at work, at least (rows, chunks of 1024 roots and of stars, 2 R or more targets)
+    (600, dict(precision="fp64", continuation="aberth", num_branches=256, num_phi=512), 512 * 3 * 2 * 1200 * 16),
+    (20000, dict(num_branches=32, num_phi=64), 4 * 60 * 2 * 40000 * 8),
+    (100000, dict(num_branches=1, num_phi=2), 256 << 20),
+    (200000, dict(num_branches=1, num_phi=2, precision="fp64"), 256 << 20),
+])
+def test_estimate_holds_the_rows_sums(num_stars, extra, sums):
+    """The estimate of a field exceeds that of its stars, tree, roots and
+    outputs, which the sums of reciprocals come on top of."""
+    p = {**SMALL, "num_stars": num_stars, **extra}
+    n, R, nb = num_stars, 2 * num_stars, p["num_branches"]
+    P1, nodes, cols = 32, 2 * n + 64, p["num_phi"] // nb + 1
+    rest = n * 88 + nodes * (224 + 2 * P1 * 16 + 32 * 32 + 3 * P1 * 16 + P1 * 8 + 32 * 24 + 2 * P1 * 16 + 64)
+    rest += 3 * nb * R * 69 + R * nb * cols * 40 + (64 << 20)
+    if p.get("continuation") != "aberth":
+        rest += 2 * nb * (cols // 2) * 2 * R * 8 + 2 * nb * R * 9
+    assert _bare(**p).estimate_device_bytes() >= rest + sums

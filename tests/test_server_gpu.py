@@ -5,12 +5,19 @@ solver is deterministic (Jacobi sweeps, fixed cluster shapes), so a field's
 results are the same bits whether it runs alone or while other requests run
 beside it.  The memory budget bounds how many requests are admitted at once.
 """
+import json
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 
 from ccf_gb300 import CCF, Server, run_batch, submit_batch, _lib
 
 pytestmark = pytest.mark.gpu
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 FIELDS = [
     dict(kappa_tot=0.3, kappa_star=0.3, shear=0.1, num_stars=60, num_phi=64, num_branches=2, random_seed=11),
@@ -98,3 +105,41 @@ def test_submitted_batch_equals_run_batch():
         rx, ry = x.results(stars=False), y.results(stars=False)
         assert np.array_equal(rx["ccs"], ry["ccs"])
         assert np.array_equal(rx["caustics"], ry["caustics"])
+
+
+HELD = r"""
+import json, sys
+import torch
+from ccf_gb300 import CCF
+cases = json.loads(sys.argv[1])
+warm = [CCF(kappa_tot=0.3, kappa_star=0.25, shear=0.1, num_stars=300, num_phi=8, num_branches=1, random_seed=1,
+            rectangular=1, **{k: c[k] for k in ("precision", "continuation") if k in c}) for c in cases]
+for w in warm:      # the kernels are loaded, the device's stacks allocated
+    assert w.run(-1), w.last_error()
+fields, out = [], []
+for c in cases:
+    f = CCF(kappa_tot=0.45, kappa_star=0.4, shear=0.2, mass_function="equal", random_seed=5, **c)
+    before = torch.cuda.mem_get_info()[0]
+    assert f.run(-1), f.last_error()
+    out.append([before - torch.cuda.mem_get_info()[0], f.estimate_device_bytes()])
+    fields.append(f)
+print(json.dumps(out))
+"""
+
+
+def test_estimate_is_above_what_a_run_holds():
+    """In a fresh process (no block kept from an earlier field): the device
+    memory that a run takes, against the estimate that admits it."""
+    cases = [
+        dict(num_stars=600, num_phi=512, num_branches=256, precision="fp64", continuation="aberth"),
+        dict(num_stars=2000, num_phi=512, num_branches=32, rectangular=1),
+        dict(num_stars=900, num_phi=256, num_branches=64, rectangular=1, write_mu_length_scales=1),
+        dict(num_stars=20000, num_phi=64, num_branches=8, rectangular=1),
+        dict(num_stars=20000, num_phi=8, num_branches=2, precision="fp64"),
+        dict(num_stars=1000, num_phi=1024, num_branches=16, host_outputs=2),
+        dict(num_stars=120000, num_phi=2, num_branches=1),
+    ]
+    r = subprocess.run([sys.executable, "-c", HELD, json.dumps(cases)], capture_output=True, text=True, cwd=ROOT)
+    assert r.returncode == 0, r.stderr
+    for case, (held, estimate) in zip(cases, json.loads(r.stdout.splitlines()[-1])):
+        assert held <= estimate, (case, held, estimate)
