@@ -34,12 +34,13 @@ over every SM.  No CTA waits for one that is not running: a phase's missing
 units are held by CTAs at work, and a CTA without work may leave (it does
 after POLL_LIMIT polls).
 
-The results are those of solve_kernel to the bit, for any number of CTAs: a
-unit's partial sums run over the same sources in the same order, the chunks'
-FP32 sums are added in FP64 in chunk order, the source shares S of a tile are
-those solve_kernel's cluster of `cluster` CTAs would choose, and off-box points
-are summed by a 256-thread CTA (solve_kernel has a warp sum those beyond
-OFF_CAP of a block, which a block of 64 never has).  (With another
+The results do not depend on the number of CTAs, nor on how the row is cut into
+blocks and units: a unit's partial sums run over the same sources in the same
+order, the chunks' FP32 sums are added in FP64 in chunk order, the source shares
+S of a tile are those that solve_kernel's cluster of `cluster` CTAs would choose,
+and every off-box point is summed by a 256-thread CTA (offbox_sums).  That is
+the order of summation of solve_kernel, but for a block's off-box points beyond
+OFF_CAP, which it leaves to a warp each.  (With another
 order of summation a few rows in 1e5 trade roots: the iteration is chaotic
 before it converges.)  The price is the partial sums in memory, 8 or 16 bytes
 per target, chunk and share, so large launches run ROWS_PART_BYTES of rows at a
@@ -94,7 +95,7 @@ struct RowShared
 	int warp_list[NT / 32], warp_late[NT / 32];
 	int own_next;           /* the next unit was kept by this CTA */
 	int cand, claimed, started, quit;
-	int noff, nan_err, nan_step;
+	int nan_err, nan_step;
 	unsigned long long unconv;
 	double maxerr;
 	double2 offz[OFF_CAP];
@@ -102,6 +103,34 @@ struct RowShared
 	__align__(16) typename Src<MIXED>::T buf[2 * CHUNK];
 };
 static_assert(OFF_CAP * (NT / 32) * 6 * sizeof(double) <= 2 * CHUNK * 16, "off-field scratch");
+
+/* Star sums of the CTA's points off the root box (the threads with off set):
+   OFF_CAP of them at a time, in thread order, each by the whole CTA, so that a
+   point's sum is the same wherever and with whatever other points it is formed.
+   Every thread calls it. */
+template <bool MIXED, bool NEED1, bool S3DF>
+__device__ void offbox_sums(const FieldView& F, RowShared<MIXED>& S, bool off, double2 z, NearSums& sums)
+{
+	if (!__syncthreads_or(off)) return;
+	const unsigned m = __ballot_sync(0xffffffffu, off);
+	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+	if (lane == 0) S.warp_list[warp] = __popc(m);
+	__syncthreads();
+	int q = __popc(m & ((1u << lane) - 1u)), n = 0;
+	for (int w = 0; w < NT / 32; w++)
+	{
+		if (w < warp) q += S.warp_list[w];
+		n += S.warp_list[w];
+	}
+	for (int q0 = 0; q0 < n; q0 += OFF_CAP)
+	{
+		const bool now = off && q >= q0 && q < q0 + OFF_CAP;
+		if (now) S.offz[q - q0] = z;
+		__syncthreads();
+		offfield_sums_cta<MIXED, NEED1, S3DF>(F, S.offz, min(n - q0, OFF_CAP), S.offs, reinterpret_cast<double*>(S.buf));
+		if (now) sums = S.offs[q - q0];
+	}
+}
 
 /* Newton check of a thread's root a at phase (cphi, sphi), at z: a root whose
    Newton step is under the tolerance takes it and is final; the others keep
@@ -115,23 +144,9 @@ __device__ void check_roots(const SolveArgs& A, RowShared<MIXED>& S, int* share,
 	const FieldView& F = S.F;
 	const long long base = S.R.base;
 	const int leaf = act ? find_leaf(F, z) : 0;
-	int slot = -1;
-	if (threadIdx.x == 0) S.noff = 0;
-	__syncthreads();
-	if (act && leaf < 0)
-	{
-		const int q = atomicAdd(&S.noff, 1);
-		if (q < OFF_CAP)
-		{
-			S.offz[q] = z;
-			slot = q;
-		}
-	}
-	__syncthreads();
-	const int K = min(S.noff, OFF_CAP);
-	if (K) offfield_sums_cta<MIXED, false, true>(F, S.offz, K, S.offs, reinterpret_cast<double*>(S.buf));
-	const NearSums off = slot >= 0 ? S.offs[slot] : zero_sums();
-	const FdF e = eval_fdf_warp<MIXED>(F, act, z, leaf, slot >= 0, off, cphi, sphi);
+	NearSums off = zero_sums();
+	offbox_sums<MIXED, false, true>(F, S, act && leaf < 0, z, off);
+	const FdF e = eval_fdf_warp<MIXED>(F, act, z, leaf, leaf < 0, off, cphi, sphi);
 	bool still = act, late = false;
 	if (act)
 	{
@@ -771,31 +786,13 @@ __global__ void __launch_bounds__(NT, 2) rows_kernel(const SolveArgs A, const in
 					int ob[2] = {c, c}, ok[2] = {O.half, 0};
 					const int nslot = initial ? 1 : row_slots(O.nb, O.half, O.seg, c, side, j, ob, ok);
 					const int leaf = own ? find_leaf(F, z) : 0;
-					int slot = -1;
-					if (threadIdx.x == 0) Sh.noff = 0;
-					__syncthreads();
-					if (own && leaf < 0)
-					{
-						const int q = atomicAdd(&Sh.noff, 1);
-						if (q < OFF_CAP)
-						{
-							Sh.offz[q] = z;
-							slot = q;
-						}
-					}
-					__syncthreads();
-					const int K = min(Sh.noff, OFF_CAP);
-					if (K)
-					{
-						double* red = reinterpret_cast<double*>(Sh.buf);
-						if (O.mu) offfield_sums_cta<MIXED, true, true>(F, Sh.offz, K, Sh.offs, red);
-						else offfield_sums_cta<MIXED, true, false>(F, Sh.offz, K, Sh.offs, red);
-					}
+					NearSums off = zero_sums();
+					if (O.mu) offbox_sums<MIXED, true, true>(F, Sh, own && leaf < 0, z, off);
+					else offbox_sums<MIXED, true, false>(F, Sh, own && leaf < 0, z, off);
 					const size_t out = out_slot(O, own ? a : 0, ob[0], ok[0]);
 					const size_t out2 = nslot > 1 ? out_slot(O, own ? a : 0, ob[1], ok[1]) : NO_SLOT;
-					const NearSums off = slot >= 0 ? Sh.offs[slot] : zero_sums();
 					const bool unconv = own && __ldcg(A.fin + base + a) != 1;
-					if (!point_epilogue_warp<MIXED>(F, O, own, z, leaf, slot >= 0, off, out, out2, cphi, sphi, &Sh.maxerr, unconv))
+					if (!point_epilogue_warp<MIXED>(F, O, own, z, leaf, leaf < 0, off, out, out2, cphi, sphi, &Sh.maxerr, unconv))
 						Sh.nan_err = 1;
 					if (unconv) atomicAdd(&Sh.unconv, 1ull);
 					if (own && initial)

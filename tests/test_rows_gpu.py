@@ -1,7 +1,6 @@
-"""The full-sum rows cut into units over the whole GPU (rows.cu) against the
-cluster-per-row kernel that ccf_continue_branch_noalloc keeps: the same order of
-summation, so the same roots to the bit, whatever number of CTAs takes the
-units.  Sizes at the edges of the units: rows of one block and one unit, blocks
+"""The full-sum rows cut into units over the whole GPU (rows.cu): the same bits
+whatever number of CTAs takes the units and however they are cut, and the zeros
+of the cluster-per-row kernel that ccf_continue_branch_noalloc keeps.  Sizes at the edges of the units: rows of one block and one unit, blocks
 and chunks that end short, several tiles, more rows than fit the partial sums'
 slots, steps with no root left after the first check.
 """
@@ -131,3 +130,29 @@ def test_whole_sums_are_the_chunks_sums(monkeypatch, n, rectangular, precision):
     for r in outs[1:]:
         for k in ("ccs", "caustics", "errs"):
             assert np.array_equal(outs[0][k], r[k]), k
+
+
+@pytest.mark.parametrize("precision", ["mixed", "fp64"])
+@pytest.mark.parametrize("n, shear, scale", [(60, 0.02, 1.18), (60, 0.0, 1.2), (200, 0.06, 1.2)])
+def test_more_off_box_roots_than_one_pass_takes(n, shear, scale, precision):
+    """A nearly square rectangle with a long Taylor series has 72 to 93 roots
+    off the root box at the end of its row, more than the 64 of one pass of the
+    CTA's star sums: the same bits alone (blocks of 64 roots) and in a batch of
+    40 (blocks of 256)."""
+    def make():
+        return CCF(kappa_tot=0.45, kappa_star=0.4, shear=shear, mass_function="equal", rectangular=1, num_stars=n,
+                   num_branches=4, num_phi=32, random_seed=3, safety_scale=scale, continuation="aberth", init_cluster=1,
+                   precision=precision)
+    a = make()
+    assert a.run(-1), a.last_error()
+    r = a.results()
+    i = r["info"]
+    z = r["ccs"].reshape(i["num_roots"], 4, -1)[:, 0, 4]
+    off = np.maximum(np.abs(z.real), np.abs(z.imag)) > i["root_half_length"]
+    assert np.count_nonzero(off[-256:]) > 64
+    fs = [make() for _ in range(40)]
+    assert run_batch(fs, -1), fs[0].last_error()
+    for f in (fs[0], fs[-1]):
+        b = f.results()
+        for k in ("ccs", "caustics", "errs"):
+            assert np.array_equal(r[k], b[k]), k
