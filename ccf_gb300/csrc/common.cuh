@@ -61,6 +61,13 @@ CCF_D double2 cdiv(double2 a, double2 b)
 	return make_double2((a.x * b.x + a.y * b.y) * r, (a.y * b.x - a.x * b.y) * r);
 }
 CCF_D double cabs64(double2 a) { return hypot(a.x, a.y); }
+/* |a|, without hypot's scaling where a's square needs none */
+CCF_HD double cabs_plain(double2 a)
+{
+	const double m = fmax(fabs(a.x), fabs(a.y));
+	if (m < 1e150 && m > 1e-150) return sqrt(fma(a.x, a.x, a.y * a.y));
+	return hypot(a.x, a.y);
+}
 
 /* ---------------- FP32 complex ---------------- */
 CCF_HD float2 fx(float r, float i) { return make_float2(r, i); }

@@ -954,16 +954,6 @@ __device__ __noinline__ SmoothSeries smooth_series_warp(const FieldView& F, doub
 	return out;
 }
 
-/* |a| for the error bound, never below it: in FP32 (2^-20 above) where a's
-   square stays in the FP32 range, else in FP64 (an FP64 hypot is a chain of
-   ~30 instructions of 64 cycles) */
-CCF_D double bound_abs(double2 a)
-{
-	const double m = fmax(fabs(a.x), fabs(a.y));
-	if (m < 1e18 && m > 1e-18) return (double)(hypotf((float)a.x, (float)a.y) * (1.f + 0x1p-20f));
-	return hypot(a.x, a.y);
-}
-
 /* The iteration quantities of the tracker (TrackEval) for the warp's lanes
    with off set, which lie outside the root box: direct double-float sums over
    every star (by the warp, one lane at a time; CTA: lane 0's by the CTA),
@@ -999,29 +989,61 @@ __device__ __noinline__ TrackEval track_offfield(const FieldView& F, bool off, d
 	r.af = 0;
 	r.wpart = {{0.f, 0.f}, {0.f, 0.f}};
 	r.wmode = 2;
-	if (!off) return r;
 	/* f as eval_f_df and w as eval_point_df off the root box, with the
 	   smooth-mass d alpha / d zbar series evaluated once */
-	const double2 ds = series ? sm.ds : smooth_dzbar_any(F, z);
-	const double a = 1 - F.kappa_tot - smooth_dz(F, z);
-	const double2 f = make_double2(F.shear + F.theta2 * ns.s2.x - ds.x - a * cphi, F.theta2 * ns.s2.y + ds.y + a * sphi);
-	const double2 df = series ? make_double2(-2 * F.theta2 * ns.s3.x - sm.d2s.x, -2 * F.theta2 * ns.s3.y + sm.d2s.y)
-	                          : eval_df_mixed(F, -1, z, ns.s3);
-	double2 S = make_double2(0, 0);
-	if (disc_exact)
+	double2 v[5];   /* what the error bound takes the moduli of */
+#pragma unroll
+	for (int k = 0; k < 5; k++) v[k] = make_double2(0, 0);
+	if (off)
 	{
-		const double2 iz = cinv(z);
-		S = make_double2(2 * iz.x, 2 * iz.y);
+		const double2 ds = series ? sm.ds : smooth_dzbar_any(F, z);
+		const double a = 1 - F.kappa_tot - smooth_dz(F, z);
+		const double2 f = make_double2(F.shear + F.theta2 * ns.s2.x - ds.x - a * cphi, F.theta2 * ns.s2.y + ds.y + a * sphi);
+		const double2 df = series ? make_double2(-2 * F.theta2 * ns.s3.x - sm.d2s.x, -2 * F.theta2 * ns.s3.y + sm.d2s.y)
+		                          : eval_df_mixed(F, -1, z, ns.s3);
+		double2 S = make_double2(0, 0);
+		if (disc_exact)
+		{
+			const double2 iz = cinv(z);
+			S = make_double2(2 * iz.x, 2 * iz.y);
+		}
+		const double2 st = cdiv(f, cadd(df, cmul(f, S)));
+		r.step = make_float2((float)st.x, (float)st.y);
+		const double as2 = st.x * st.x + st.y * st.y;
+		r.as2 = as2 < 3e38 ? (float)as2 : INFINITY;   /* a step beyond the FP32 range fails */
+		r.fz = make_float2((float)f.x, (float)f.y);
+		const double2 fs = cmul(df, make_double2(r.step.x, r.step.y));
+		v[0] = make_double2(f.x - fs.x, f.y - fs.y);
+		v[1] = ns.s2;
+		v[2] = ds;
+		v[3] = z;
+		v[4] = df;
 	}
-	const double2 st = cdiv(f, cadd(df, cmul(f, S)));
-	r.step = make_float2((float)st.x, (float)st.y);
-	const double as2 = st.x * st.x + st.y * st.y;
-	r.as2 = as2 < 3e38 ? (float)as2 : INFINITY;   /* a step beyond the FP32 range fails */
-	r.fz = make_float2((float)f.x, (float)f.y);
-	const double2 fs = cmul(df, make_double2(r.step.x, r.step.y));
-	r.af = __double2float_ru(bound_abs(make_double2(f.x - fs.x, f.y - fs.y)) +
-		7.2e-15 * (F.theta2 * bound_abs(ns.s2) + bound_abs(ds) + 1 + F.shear) +
-		1.2e-16 * bound_abs(z) * bound_abs(df));
+	/* a square root is a chain of FP64 instructions of 64 cycles each: a lane
+	   alone hands its five to five lanes */
+	double m[5];
+	const unsigned holders = __ballot_sync(full, off);
+	if (__popc(holders) == 1)
+	{
+		const int src = __ffs(holders) - 1;
+		double2 mine = make_double2(0, 0);
+#pragma unroll
+		for (int k = 0; k < 5; k++)
+		{
+			const double2 t = make_double2(__shfl_sync(full, v[k].x, src), __shfl_sync(full, v[k].y, src));
+			if (lane == k) mine = t;
+		}
+		const double t = cabs_plain(mine);
+#pragma unroll
+		for (int k = 0; k < 5; k++) m[k] = __shfl_sync(full, t, k);
+	}
+	else
+	{
+#pragma unroll
+		for (int k = 0; k < 5; k++) m[k] = off ? cabs_plain(v[k]) : 0;
+	}
+	if (!off) return r;
+	r.af = __double2float_ru(m[0] + 7.2e-15 * (F.theta2 * m[1] + m[2] + 1 + F.shear) + 1.2e-16 * m[3] * m[4]);
 	/* the lens map only where the point can be final: a step below the
 	   tolerance, or a stalled root kept as it is */
 	if (r.as2 < wtol2)
