@@ -95,7 +95,7 @@ struct RowShared
 	int warp_list[NT / 32], warp_late[NT / 32];
 	int own_next;           /* the next unit was kept by this CTA */
 	int cand, claimed, started, quit;
-	int nan_err, nan_step;
+	int noff, nan_err, nan_step;
 	unsigned long long unconv;
 	double maxerr;
 	double2 offz[OFF_CAP];
@@ -104,29 +104,31 @@ struct RowShared
 };
 static_assert(OFF_CAP * (NT / 32) * 6 * sizeof(double) <= 2 * CHUNK * 16, "off-field scratch");
 
-/* Star sums of the CTA's points off the root box (the threads with off set):
-   OFF_CAP of them at a time, in thread order, each by the whole CTA, so that a
-   point's sum is the same wherever and with whatever other points it is formed.
-   Every thread calls it. */
+/* Star sums of the CTA's points off the root box (the threads with off set),
+   each by the whole CTA, OFF_CAP of them at a time: which pass takes a point is
+   no matter, its sum is the same wherever and with whatever others it is formed.
+   Every thread calls it, with a barrier of the CTA between two calls. */
 template <bool MIXED, bool NEED1, bool S3DF>
 __device__ void offbox_sums(const FieldView& F, RowShared<MIXED>& S, bool off, double2 z, NearSums& sums)
 {
-	if (!__syncthreads_or(off)) return;
-	const unsigned m = __ballot_sync(0xffffffffu, off);
-	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-	if (lane == 0) S.warp_list[warp] = __popc(m);
+	if (threadIdx.x == 0) S.noff = 0;
 	__syncthreads();
-	int q = __popc(m & ((1u << lane) - 1u)), n = 0;
-	for (int w = 0; w < NT / 32; w++)
+	int q = -1;
+	if (off)
 	{
-		if (w < warp) q += S.warp_list[w];
-		n += S.warp_list[w];
+		q = atomicAdd(&S.noff, 1);
+		if (q < OFF_CAP) S.offz[q] = z;
 	}
+	__syncthreads();
+	const int n = S.noff;
 	for (int q0 = 0; q0 < n; q0 += OFF_CAP)
 	{
-		const bool now = off && q >= q0 && q < q0 + OFF_CAP;
-		if (now) S.offz[q - q0] = z;
-		__syncthreads();
+		const bool now = q >= q0 && q < q0 + OFF_CAP;
+		if (q0 > 0)
+		{
+			if (now) S.offz[q - q0] = z;
+			__syncthreads();
+		}
 		offfield_sums_cta<MIXED, NEED1, S3DF>(F, S.offz, min(n - q0, OFF_CAP), S.offs, reinterpret_cast<double*>(S.buf));
 		if (now) sums = S.offs[q - q0];
 	}
