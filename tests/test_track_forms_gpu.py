@@ -111,3 +111,43 @@ def test_roots_split_over_lanes_find_the_same_zeros(n, rectangular, num_phi, nb)
         d = O.match_sets(a["ccs"], copies[-1].results()["ccs"], nb)
         assert d["non_finite"] == 0 and d["non_bijective_cols"] == 0
         assert d["max_dist"] <= 1e-11
+
+
+@pytest.mark.parametrize("n, rectangular, num_phi, nb", [
+    (4096, 1, 16, 2),     # the smallest field whose off-box roots have a CTA of several warps each
+    (4501, 1, 24, 1),     # an odd number of stars
+    (4501, 0, 16, 1),     # few roots off the box
+])
+def test_fp64_roots_off_the_box_find_the_full_sum_zeros(n, rectangular, num_phi, nb):
+    """The FP64 far launch, whose warps share a root's stars: the zeros of the
+    full-sum continuation, and the oracle's lens map of them (1e-11 as in the
+    tests above)."""
+    field = dict(kappa_tot=0.45, kappa_star=0.4, shear=0.3, mass_function="equal", rectangular=rectangular, num_stars=n,
+                 random_seed=7 + n)
+    cfg = dict(field, num_phi=num_phi, num_branches=nb, precision="fp64")
+    t = run(cfg)
+    a = run(cfg, continuation="aberth")
+    d = O.match_sets(t["ccs"], a["ccs"], nb)
+    assert d["non_finite"] == 0 and d["non_bijective_cols"] == 0
+    assert d["max_dist"] <= 1e-11
+    h = t["info"]["root_half_length"]
+    z, w = t["ccs"].ravel(), t["caustics"].ravel()
+    off = np.flatnonzero(np.maximum(np.abs(z.real), np.abs(z.imag)) > h)
+    assert off.size > 0 or not rectangular
+    off = off[:: max(1, off.size // 200)]
+    want = O.eval_field(z[off], **field)["w"]
+    assert np.all(np.abs(w[off] - want) <= 1e-11 * (1 + np.abs(want) + np.abs(z[off])))
+
+
+@pytest.mark.parametrize("precision, mu", [("mixed", 0), ("mixed", 1), ("fp64", 0)])
+@pytest.mark.parametrize("n, num_phi, nb", [(4096, 32, 4), (9001, 16, 2)])
+def test_streamed_far_launches_give_the_same_bits(monkeypatch, n, num_phi, nb, precision, mu):
+    """One group of centres at a time, each with far launches of several warps
+    of its own, against the whole field at once."""
+    cfg = dict(kappa_tot=0.45, kappa_star=0.4, shear=0.3, mass_function="equal", rectangular=1, num_stars=n,
+               num_phi=num_phi, num_branches=nb, random_seed=7 + n, precision=precision, write_mu_length_scales=mu)
+    a = run(cfg)
+    monkeypatch.setenv("CCF_GB300_CHUNK_BYTES", "1")
+    b = run(cfg, host_outputs=2)
+    for k in ("ccs", "caustics", "errs") + (("mu_length_scales",) if mu else ()):
+        assert np.array_equal(a[k], b[k]), k
