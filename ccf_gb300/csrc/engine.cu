@@ -264,7 +264,6 @@ bool Engine::ensure_device(int dev)
 	cudaDeviceProp prop;
 	cudaGetDeviceProperties(&prop, dev);
 	num_sms = prop.multiProcessorCount;
-	slots_per_sm = std::min(solver_blocks_per_sm(true), solver_blocks_per_sm(false));
 	device = dev;
 	initialized = true;
 	return true;
@@ -1119,14 +1118,15 @@ ccf_status Engine::solve(std::vector<Field*>& fields, int verbose)
 		CCF_TRY(P.item_start.ensure(rc.size()), "cudaMalloc(rows)");
 	}
 
-	/* CTAs per row: fill the resident slots without a second wave */
-	const int slots = num_sms * slots_per_sm;
+	/* CTAs per row whose order of summation is kept: they would fill the GPU
+	   without a second wave */
+	const int slots = num_sms * CLUSTER_CTAS_PER_SM;
 	auto pick_cluster = [&](int rows) {
 		int cl = 1;
 		while (cl < 16 && (long long)rows * cl * 2 <= slots && minR / (cl * 2) >= 256) cl *= 2;
 		return cl;
 	};
-	/* the initial solve's CTAs per row: as given, else as many as fill the GPU once */
+	/* the initial solve's: as given, else by that rule */
 	const int init_cluster = fields[0]->params.init_cluster;
 	SolveArgs A;
 	std::memset(&A, 0, sizeof(A));

@@ -358,7 +358,6 @@ private:
 	std::vector<std::unique_ptr<Engine>> setup_workers;
 	std::vector<cudaEvent_t> setup_events;
 	bool initialized = false;
-	int slots_per_sm = 1;
 };
 
 } /* namespace ccf */

@@ -477,10 +477,10 @@ void launch_fold_smooth(cudaStream_t s, int num_leaves, int P, const double2* le
 size_t fold_binom_size(int nf, int nr, int nq);
 
 /* solver.cu */
-int solver_blocks_per_sm(bool mixed);
-cudaError_t launch_solve(cudaStream_t s, const SolveArgs& a, bool mixed, bool initial);
-/* rows.cu: launch_solve with every row spread over the GPU; cluster then only
-   sets the order of summation (their memory: rows_plan.h) */
+cudaError_t launch_solve(cudaStream_t s, const SolveArgs& a, bool mixed);   /* continuation rows, one cluster each */
+/* rows.cu: the initial solve and the full-sum continuation with every row
+   spread over the GPU; cluster only sets the order of summation (their memory:
+   rows_plan.h) */
 cudaError_t launch_rows(cudaStream_t s, const SolveArgs& a, bool mixed, bool initial, int num_sms, int max_roots, int max_stars);
 cudaError_t launch_track_mark(cudaStream_t s, const TrackArgs& a, int* cls);
 cudaError_t launch_track_item_order(cudaStream_t s, const TrackArgs& a, int* work, int* order);

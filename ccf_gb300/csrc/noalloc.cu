@@ -24,6 +24,7 @@ the columns this call wrote.
 ******************************************************************************/
 #include "../../include/ccf_gb300.h"
 #include "engine.h"
+#include "rows_plan.h"
 
 #include <mutex>
 #include <string>
@@ -194,7 +195,7 @@ extern "C" ccf_status ccf_continue_branch_noalloc(ccf_handle* h, int branch, int
 	A.rows = (const ccf::RowDesc*)(base + o_row);
 	A.num_rows = 1;
 	int cl = 1;
-	while (cl < 8 && R / (cl * 2) >= 256) cl *= 2;
+	while (cl < ccf::MAX_SOLVE_CLUSTER && R / (cl * 2) >= 256) cl *= 2;
 	A.cluster = cl;
 	A.master = (double2*)(base + o_master);
 	A.snap32 = mixed ? (float4*)(base + o_snap) : nullptr;
@@ -204,7 +205,7 @@ extern "C" ccf_status ccf_continue_branch_noalloc(ccf_handle* h, int branch, int
 	A.fval = (double2*)(base + o_fval);
 	A.star_hilo = (const float4* const*)(base + o_hilo);
 	A.error = nullptr;
-	e = ccf::launch_solve(s, A, mixed, false);
+	e = ccf::launch_solve(s, A, mixed);
 	if (e == cudaSuccess)
 	{
 		/* the FP64 polish of ccf_run, over the columns written here */

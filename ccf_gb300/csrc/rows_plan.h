@@ -13,10 +13,14 @@ namespace ccf
 {
 
 constexpr int NT = 256;          /* threads per CTA */
-constexpr int MAX_CLUSTER = 16;  /* CTAs per row (above 8: the non-portable cluster sizes) */
+constexpr int MAX_SOLVE_CLUSTER = 8;   /* CTAs per row of solve_kernel (the portable cluster sizes) */
+constexpr int MAX_CLUSTER = 16;  /* and of the clusters whose order of summation rows_kernel keeps */
 constexpr int TPT = 2;           /* targets per thread */
 constexpr int TILE = NT * TPT;   /* targets per tile */
 constexpr int CHUNK = 1024;      /* sources per shared-memory stage */
+
+constexpr int CLUSTER_CTAS_PER_SM = 2;   /* CTAs of such a cluster that an SM holds (the rule of the order
+                                            of summation, Engine::solve, fills the GPU with them once) */
 
 /* ticket of a row: the units of the open phase and the next unit (0: none) in
    one word, each as wide as the int it is read into (of 22 bits a first sweep

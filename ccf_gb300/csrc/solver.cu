@@ -45,22 +45,20 @@ namespace ccf
 {
 
 template <bool MIXED>
-__global__ void __launch_bounds__(NT, 2) solve_kernel(const SolveArgs A, const int initial)
+__global__ void __launch_bounds__(NT, 2) solve_kernel(const SolveArgs A)
 {
 	using SrcT = typename Src<MIXED>::T;
 	cg::cluster_group cluster = cg::this_cluster();
 	const int csize = (int)cluster.num_blocks();
 	const int crank = (int)cluster.block_rank();
 	const int item = blockIdx.x / csize;
-	/* the same for every CTA of the cluster, so a cluster leaves as a whole */
-	if (item >= (A.num_rows_dev ? min(*A.num_rows_dev, A.num_rows) : A.num_rows)) return;
 
 	__shared__ FieldView sF;
 	__shared__ FieldOut sO;
 	__shared__ RowDesc sR;
 	__shared__ int s_fill;
 	__shared__ int s_cnt;
-	__shared__ int s_pre[MAX_CLUSTER + 1];
+	__shared__ int s_pre[MAX_SOLVE_CLUSTER + 1];
 	__shared__ unsigned long long s_upd, s_terms, s_unconv;
 	__shared__ double s_maxerr;
 	__shared__ int s_nan_err, s_nan_step;   /* set by plain stores: every writer stores 1 */
@@ -93,9 +91,9 @@ __global__ void __launch_bounds__(NT, 2) solve_kernel(const SolveArgs A, const i
 	const int nb = sO.nb;
 	const int o0 = (int)((long long)R * crank / csize);
 	const int o1 = (int)((long long)R * (crank + 1) / csize);
-	const int j0 = initial ? 0 : sO.step_first;
-	const int j1 = initial ? 0 : sR.steps;
-	const int max_it = initial ? sO.max_iters_init : sO.max_iters_step;
+	const int j0 = sO.step_first;
+	const int j1 = sR.steps;
+	const int max_it = sO.max_iters_step;
 	double2* __restrict__ master = A.master + base;
 	unsigned char* __restrict__ fin = A.fin + base;
 	int* __restrict__ list = A.list + base;
@@ -124,9 +122,8 @@ __global__ void __launch_bounds__(NT, 2) solve_kernel(const SolveArgs A, const i
 
 	for (int j = j0; j <= j1; j++)
 	{
-		const double phi = initial ? (PI / nb + c * 2 * PI / nb) : row_phi(c, nb, sO.nphi, side, j);
 		double sphi, cphi;
-		sincos(phi, &sphi, &cphi);
+		sincos(row_phi(c, nb, sO.nphi, side, j), &sphi, &cphi);
 		for (int a = o0 + threadIdx.x; a < o1; a += NT) fin[a] = 0;
 		__syncthreads();
 
@@ -438,7 +435,7 @@ __global__ void __launch_bounds__(NT, 2) solve_kernel(const SolveArgs A, const i
 
 		/* epilogue: outputs of this phi step for the roots this CTA owns */
 		int ob[2] = {c, c}, ok[2] = {sO.half, 0};
-		const int nslot = initial ? 1 : row_slots(nb, sO.half, sO.seg, c, side, j, ob, ok);
+		const int nslot = row_slots(nb, sO.half, sO.seg, c, side, j, ob, ok);
 		for (int a0 = o0; a0 < o1; a0 += NT)
 		{
 			/* uniform trip count: the epilogue is a warp-wide call */
@@ -468,25 +465,7 @@ __global__ void __launch_bounds__(NT, 2) solve_kernel(const SolveArgs A, const i
 			const bool unconv = v && fin[a] != 1;
 			if (!point_epilogue_warp<MIXED>(F, sO, v, z, leaf, slot >= 0, off, out, out2, cphi, sphi, &s_maxerr, unconv))
 				s_nan_err = 1;
-			if (!v) continue;
-			if (unconv) atomicAdd(&s_unconv, 1ull);
-			if (initial)
-			{
-				long long cb = sR.cont_base;
-				sO.cont_master[cb + a] = z;
-				sO.cont_master[cb + R + a] = z;
-				if constexpr (MIXED)
-				{
-					float4 h = split_hilo(z);
-					sO.cont_snap32[cb + a] = h;
-					sO.cont_snap32[cb + R + a] = h;
-				}
-				else
-				{
-					sO.cont_snap64[cb + a] = z;
-					sO.cont_snap64[cb + R + a] = z;
-				}
-			}
+			if (v && unconv) atomicAdd(&s_unconv, 1ull);
 		}
 		cluster.sync();
 	}
@@ -501,13 +480,8 @@ __global__ void __launch_bounds__(NT, 2) solve_kernel(const SolveArgs A, const i
 		if (flags) atomicOr(&st[1], flags);
 		atomicAdd(&st[2], s_upd);
 		atomicAdd(&st[3], s_terms);
-		if (initial)
-		{
-			atomicAdd(&st[7], s_upd);
-			atomicAdd(&st[8], s_terms);
-		}
 		atomicAdd(&st[4], s_unconv);
-		atomicMax(&st[initial ? 5 : 6], (unsigned long long)sweeps_max);
+		atomicMax(&st[6], (unsigned long long)sweeps_max);
 	}
 }
 
@@ -2236,29 +2210,10 @@ cudaError_t launch_collect_rerun(cudaStream_t s, const TrackArgs& a, RowDesc* re
 	return cudaGetLastError();
 }
 
-int solver_blocks_per_sm(bool mixed)
-{
-	int n = 0;
-	if (mixed) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, solve_kernel<true>, NT, 0);
-	else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, solve_kernel<false>, NT, 0);
-	return n < 1 ? 1 : n;
-}
-
-cudaError_t launch_solve(cudaStream_t s, const SolveArgs& a, bool mixed, bool initial)
+cudaError_t launch_solve(cudaStream_t s, const SolveArgs& a, bool mixed)
 {
 	if (a.num_rows == 0) return cudaSuccess;
-	if (a.cluster < 1 || a.cluster > MAX_CLUSTER) return cudaErrorInvalidValue;
-	if (a.cluster > 8)
-	{
-		static bool allowed[2] = {false, false};
-		if (!allowed[mixed ? 1 : 0])
-		{
-			cudaError_t e = mixed ? cudaFuncSetAttribute(solve_kernel<true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1)
-			                      : cudaFuncSetAttribute(solve_kernel<false>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-			if (e != cudaSuccess) return e;
-			allowed[mixed ? 1 : 0] = true;
-		}
-	}
+	if (a.cluster < 1 || a.cluster > MAX_SOLVE_CLUSTER) return cudaErrorInvalidValue;
 	cudaLaunchConfig_t cfg = {};
 	cfg.gridDim = dim3(a.num_rows * a.cluster, 1, 1);
 	cfg.blockDim = dim3(NT, 1, 1);
@@ -2271,8 +2226,8 @@ cudaError_t launch_solve(cudaStream_t s, const SolveArgs& a, bool mixed, bool in
 	attr[0].val.clusterDim.z = 1;
 	cfg.attrs = attr;
 	cfg.numAttrs = 1;
-	if (mixed) return cudaLaunchKernelEx(&cfg, solve_kernel<true>, a, initial ? 1 : 0);
-	return cudaLaunchKernelEx(&cfg, solve_kernel<false>, a, initial ? 1 : 0);
+	if (mixed) return cudaLaunchKernelEx(&cfg, solve_kernel<true>, a);
+	return cudaLaunchKernelEx(&cfg, solve_kernel<false>, a);
 }
 
 /* pointwise evaluation of f, f', the lens map, the 1/mu bound and the

@@ -26,6 +26,7 @@ keep a chunk within CHUNK_BYTES (2 GiB; CCF_GB300_CHUNK_BYTES sets another
 target, at least one centre per group).
 ******************************************************************************/
 #include "engine.h"
+#include "rows_plan.h"
 
 #include <algorithm>
 #include <cstdlib>
@@ -368,7 +369,7 @@ ccf_status Engine::solve_chunked(Field& f, int verbose)
 	A.rows = P.rows_init.ptr;
 	A.num_rows = K;
 	auto pick_cluster = [&](int rows) {
-		const int slots = num_sms * slots_per_sm;
+		const int slots = num_sms * CLUSTER_CTAS_PER_SM;
 		int cl = 1;
 		while (cl < 16 && (long long)rows * cl * 2 <= slots && R / (cl * 2) >= 256) cl *= 2;
 		return cl;
