@@ -219,14 +219,14 @@ class ClockSampler:
 
 # DRAM bytes (read + write) of the continuation launch per continuation point,
 # from the full-size one-pass capture summarised in
-# profiles/track_kernel_n2000_salpeter_phi512.md: 35.5 + 172.2 MB for the
+# profiles/track_kernel_n2000_salpeter_phi512.md: 39.2 + 178.6 MB for the
 # 4056 * 2048 continuation points of the bench field's launch (the 40-byte
 # outputs, part of which L2 still holds when the launch ends; leaf records
 # and stars stay in L2).
-CONT_DRAM_BYTES_PER_POINT = (35.51e6 + 172.24e6) / (4056 * 2048)
+CONT_DRAM_BYTES_PER_POINT = (39.19e6 + 178.59e6) / (4056 * 2048)
 # FP64-pipe activity of the continuation kernel in the --set full capture of
 # the same profile (sm__pipe_fp64_cycles_active over active cycles)
-CONT_FP64_PIPE_ACTIVE = 0.251
+CONT_FP64_PIPE_ACTIVE = 0.301
 
 
 def hbm_peak_gbs() -> float | None:

@@ -5,8 +5,10 @@ ccf_autotune times candidate settings on the handle's own field (whole
 runs, CUDA-event spans, best of two after a warm-up run) by coordinate
 descent from the library's defaults:
 
-  * init_cluster: CTAs per branch-centre row of the initial Aberth solve
-    (1, 2, 4, 8, 16);
+  * init_cluster: the order of summation of the initial Aberth solve (1, 2,
+    4, 8, 16; it moves the solve's time by 2 to 10 %, repeatably: 600 stars
+    1.33 to 1.45 ms, 2000 2.99 to 3.12, 20 000 12.5 to 13.2, 600 in FP64 5.5
+    to 6.3);
   * solved_centres: branch centres solved by the initial Aberth solve, the
     others reached by tracking (the default's count, half and twice it);
   * with fmm = 1 also leaf_max_stars (24, 16, 12) and expansion_order (the

@@ -931,12 +931,12 @@ ccf_status Engine::solve(std::vector<Field*>& fields, int verbose)
 	/* Solved centres: with the full-sum continuation every branch centre, as
 	   the reference.  With the tracker, every seg-th centre, seg the largest
 	   divisor of num_branches up to 16 that still gives the continuation about
-	   two resident waves of tracked roots (2 rows of R roots per centre): the
-	   initial solve costs O(R (R + N)) per sweep and centre, the tracker only
-	   its evaluations, and rows from a centre then cover seg branches.  The cap
-	   bounds the chain of a root that starts off the root box, which one warp
-	   tracks alone with direct star sums (on the 20000-star field 8 of 128
-	   centres take 0.62 s per field, 2 centres 3.2 s, all 128 1.50 s). */
+	   two waves of 16 warps of tracked roots per SM (2 rows of R roots per
+	   centre): the initial solve costs O(R (R + N)) per sweep and centre, the
+	   tracker only its evaluations, and rows from a centre then cover seg
+	   branches.  The cap bounds the chain of one root's phi steps (20000 stars,
+	   128 branches, 10240 phi steps: 8 centres 0.27 s per field, 2 centres 0.31,
+	   32 centres 0.35, all 128 0.81). */
 	std::vector<int> seg(nf);
 	for (int i = 0; i < nf; i++) seg[i] = solved_seg(*fields[i], track);
 	/* row offsets */

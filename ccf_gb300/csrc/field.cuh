@@ -106,7 +106,7 @@ struct FieldView
 	const float2* leaf_loc3f_fold;    /* like leaf_loc3f */
 	const double2* leaf_loc_fold64;   /* like leaf_loc, in FP64 (the FP64 polish) */
 	/* the tracker's leaf records, two values side by side for the packed
-	   evaluator (eval_track_pk) */
+	   evaluator (eval_track_df with PK) */
 	const float4* leaf_near_pk;  /* [(leaf * NEAR_PAIRS + pair) * NEAR_PAIR_F4 + k], see near_pair */
 	const float4* leaf_loc_pk;   /* [(leaf * (P + 1) + i) * 2 + {0 leading, 1 low}]: alpha_i and
 	                                (d/dzbar)_(i+1), the folded blocks where the leaf is folded */

@@ -313,7 +313,8 @@ struct TrackArgs
 	unsigned long long* out_list;
 	int* num_out;               /* their number (zeroed before the tracking launch) */
 	int out_cap;                /* beyond it they are formed with the others */
-	int scales;                 /* a field of the launch writes length scales */
+	int scales;                 /* a field of the launch writes length scales: all its fields take the scalar
+	                               evaluator, the predictor of five points and no far launch of solo roots */
 };
 
 /* stars.cu */

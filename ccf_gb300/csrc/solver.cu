@@ -1,16 +1,19 @@
 /******************************************************************************
-solver.cu -- the Aberth-Ehrlich root solver and the phi continuation.
+solver.cu -- the Aberth-Ehrlich continuation by one cluster per row
+(solve_kernel), the continuation tracker (track_kernel), its outputs and
+checks.
 
-For a branch centre (initial solve) or a (branch, side) continuation row,
-every root z_k of the critical-curve function f(z; phi) is updated by the
+solve_kernel runs the rows of ccf_continue_branch_noalloc; the initial solve
+and the full-sum continuation of a run are rows_kernel's (rows.cu), the same
+sweep cut into units for the whole GPU.  In a (branch, side) row every root z_k of the critical-curve function f(z; phi) is updated by the
 Aberth step of the reference (include/ccf_functions.cuh:193-243):
 
     z_k <- z_k - f / (f' + f (2 sum_i 1/(z_k - z_i) - sum_{j != k} 1/(z_k - z_j)))
 
-and the continuation advances phi step by step away from the branch centre
+as phi advances step by step away from the branch centre
 (include/ccf_functions.cuh:261-394, include/ccf.cuh:979-1033).
 
-GB300 design:
+GB300 design of the sweep:
   * one thread-block cluster owns one row for all of its phi steps, so a
     whole continuation is a single launch; the CTAs of the cluster split the
     row's active roots and meet at cluster barriers between sweeps;
@@ -511,7 +514,7 @@ dependence on the other roots.
     with such a pair, a root lost after the sub-step and evaluation limits,
     or a non-finite 1/mu bound is tracked again from its branch-centre roots
     with sub-steps of 1/TRACK_FINE_SUB of a step, and a row failing that too
-    is run by the full-sum continuation (solve_kernel), so every row written
+    is run by the full-sum continuation (rows_kernel), so every row written
     is either a verified tracked row or the reference's scheme.  Rows whose
     results are kept report their statistics through collect_rerun_kernel;
     re-run rows through the full-sum kernel. */
@@ -1650,7 +1653,7 @@ __global__ void __launch_bounds__(FAR ? 32 * FAR_MAX_WARPS : TNT, FAR || G > 1 ?
 					/* next target: predict, restart the corrector */
 					tt = tn;
 					const int hp = min(hn, smooth && !T.scales ? TRACK_HIST : TRACK_HIST_ROUGH);
-				z = track_predict<NL>(hz, head, hp, tt - t1 == t1 - t0 && run >= hp - 1, t0, t1, tt);
+					z = track_predict<NL>(hz, head, hp, tt - t1 == t1 - t0 && run >= hp - 1, t0, t1, tt);
 					it = 0;
 					prev2 = 0;
 					track_phase(O, c, side, tt, gp, cp, sp, cpd, spd);

@@ -18,8 +18,8 @@ The outputs of a field take 40 bytes per point (16.6 GB for 20000 stars and
     while the next group computes into the other buffer.
 
 The results are the bits of Engine::solve's: the same rows run the same
-kernels; only the rows' launch grouping differs, and a row's results do not
-depend on what else its launch holds.  Device-resident outputs: the centre
+kernels in the same forms (those that depend on a launch's size go by the
+whole run's, TrackArgs::run_items); only the rows' launch grouping differs.  Device-resident outputs: the centre
 buffer and the two chunk buffers (4.4 GB on the field above, each chunk 2.2
 GB).  A group is as many centres (a power of two dividing their number) as
 keep a chunk within CHUNK_BYTES (2 GiB; CCF_GB300_CHUNK_BYTES sets another

@@ -120,8 +120,10 @@ typedef struct ccf_params
 	                                (include/tree_node.cuh:14, :321-345); 4 .. 32 (a smaller
 	                                leaf makes the near sums shorter and the tree deeper; it
 	                                changes the far field as expansion_order does) */
-	int init_cluster;            /* CTAs per branch-centre row of the initial Aberth solve:
-	                                0 (default) = as many as fill the GPU once; 1, 2, 4, 8, 16 */
+	int init_cluster;            /* order of summation of the initial Aberth solve: that of a row shared by
+	                                so many CTAs (its blocks of roots begin, and its sources are split,
+	                                as theirs); 1, 2, 4, 8, 16, 0 (default) = as many as would fill the
+	                                GPU once.  Every row uses the whole GPU whatever the value */
 	int autotune;                /* 1: ccf_run applies the settings ccf_autotune found for fields
 	                                of this shape (init_cluster, solved_centres), tuning on the
 	                                first run of a shape; 2: also expansion_order and
@@ -212,7 +214,7 @@ typedef struct ccf_info
 	long long points_polished;         /* points the polish worked on */
 	long long points_above_target;     /* polished points whose FP64 1/mu error stays above
 	                                      1e-9 although |f| is above the FP64 floor (below) */
-	int init_cluster;                  /* CTAs per row of the initial Aberth solve */
+	int init_cluster;                  /* the initial Aberth solve's order of summation (ccf_params) */
 	int leaf_max_stars;                /* the tree's leaf limit (32: the reference's rule) */
 	long long points_at_fp64_floor;    /* polished points whose 1/mu error stays above 1e-9
 	                                      because |f| is within four times |f'| times half the
@@ -358,7 +360,7 @@ ccf_status ccf_fmm_error(ccf_handle* h, double* max_error);
 ccf_status ccf_autotune(ccf_handle* h, int fmm, int verbose, ccf_params* best, double* best_seconds);
 
 /* Device memory a run with parameters p will hold (stars, tree, FMM and leaf
-   records, solver rows, outputs), an upper estimate used for admission.  No
+   records, solver rows and the partial sums of those at work, outputs), an upper estimate used for admission.  No
    reference counterpart (the reference allocates managed memory as it goes,
    include/ccf.cuh:131-143). */
 ccf_status ccf_estimate_device_bytes(const ccf_params* p, unsigned long long* bytes);
