@@ -151,3 +151,21 @@ def test_streamed_far_launches_give_the_same_bits(monkeypatch, n, num_phi, nb, p
     b = run(cfg, host_outputs=2)
     for k in ("ccs", "caustics", "errs") + (("mu_length_scales",) if mu else ()):
         assert np.array_equal(a[k], b[k]), k
+
+
+@pytest.mark.parametrize("n, rectangular, num_phi, nb", [(137, 0, 24, 2), (150, 1, 24, 2), (4501, 1, 24, 1)])
+def test_a_batch_mate_with_length_scales_leaves_the_zeros(n, rectangular, num_phi, nb):
+    """One field with length scales moves its whole batch to the scalar
+    evaluator and its off-box roots to the items: the same zeros as alone."""
+    cfg = dict(kappa_tot=0.45, kappa_star=0.4, shear=0.3, mass_function="equal", rectangular=rectangular, num_stars=n,
+               num_phi=num_phi, num_branches=nb, random_seed=7 + n)
+    mate = dict(cfg, num_stars=40, write_mu_length_scales=1)
+    alone, mate_alone = run(cfg), run(mate)
+    fs = [CCF(**cfg), CCF(**mate)]
+    assert run_batch(fs, -1), fs[0].last_error()
+    for f, want in zip(fs, (alone, mate_alone)):
+        r = f.results()
+        for k in ("ccs", "caustics"):
+            d = O.match_sets(r[k], want[k], nb)
+            assert d["non_finite"] == 0 and d["non_bijective_cols"] == 0
+        assert O.match_sets(r["ccs"], want["ccs"], nb)["max_dist"] <= 1e-11
